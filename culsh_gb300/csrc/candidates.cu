@@ -467,23 +467,96 @@ __global__ void __launch_bounds__(WT) k_candidates_ws(WsArgs a) {
 constexpr int DT = 256;
 constexpr int DW = DT / 32;
 
+// Shared memory of scan_words: candidate ids of DT words, per-warp lists.
+struct ScanSmem {
+    uint32_t* clist;   // [DT * 32]
+    float* wd;         // [DW][K]
+    uint32_t* wi;      // [DW][K]
+};
+__device__ __forceinline__ ScanSmem scan_smem(void* p, int K) {
+    ScanSmem s;
+    s.clist = static_cast<uint32_t*>(p);
+    s.wd = reinterpret_cast<float*>(s.clist + DT * 32);
+    s.wi = reinterpret_cast<uint32_t*>(s.wd + DW * K);
+    return s;
+}
+constexpr size_t scan_bytes(int K) { return 4 * (size_t)DT * 32 + (size_t)DW * K * (sizeof(float) + sizeof(uint32_t)); }
+
+// Exact top-K of the points whose bits are set in words word(0 .. nwords),
+// DT words at a time, written padded to oid / od by one block; returns the
+// number of set bits (every thread).
+template <class Word>
+__device__ __forceinline__ unsigned long long scan_words(const float* __restrict__ X, int D, int K, uint32_t nwords,
+                                                         Word word, const float* qs, bool vec, const ScanSmem& sc,
+                                                         int32_t* oid, float* od) {
+    __shared__ uint32_t s_ws[DW], s_wn[DW];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    float* wd = sc.wd + warp * K;
+    uint32_t* wi = sc.wi + warp * K;
+    int n = 0;
+    float thr_d = FLT_MAX;
+    uint32_t thr_i = 0;
+    unsigned long long U = 0;
+    for (uint32_t w0 = 0; w0 < nwords; w0 += DT) {
+        const uint32_t w = w0 + tid;
+        const uint32_t bits = w < nwords ? word(w) : 0u;
+        // block exclusive scan of the set-bit counts
+        const uint32_t c = __popc(bits);
+        uint32_t x = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+            if (lane >= o) x += y;
+        }
+        if (lane == 31) s_ws[warp] = x;
+        __syncthreads();
+        uint32_t before = 0, total = 0;
+        for (int i = 0; i < DW; ++i) {
+            const uint32_t v = s_ws[i];
+            before += i < warp ? v : 0u;
+            total += v;
+        }
+        uint32_t k = before + x - c;
+        for (uint32_t m = bits; m; m &= m - 1) sc.clist[k++] = w * 32 + (uint32_t)(__ffs((int)m) - 1);
+        __syncthreads();
+        fp32_dist_pass<DW>(X, D, qs, vec, total, [](uint32_t j) { return j; },
+                           [&](uint32_t ci) { return sc.clist[ci]; }, [](uint32_t, float&) { return false; }, wd, wi,
+                           K, n, thr_d, thr_i);
+        U += total;
+        __syncthreads();
+    }
+    if (lane == 0) s_wn[warp] = n;
+    __syncthreads();
+    if (warp == 0) {
+        for (int ww = 1; ww < DW; ++ww) {
+            const int nw = s_wn[ww];
+            for (int e = 0; e < nw; ++e) {
+                const float d = sc.wd[ww * K + e];
+                const uint32_t id = sc.wi[ww * K + e];
+                if (!lessp(d, id, thr_d, thr_i)) break;
+                warp_insert(wd, wi, n, K, d, id, thr_d, thr_i);
+            }
+        }
+        for (int k = lane; k < K; k += 32) {
+            oid[k] = k < n ? (int32_t)wi[k] : -1;
+            od[k] = k < n ? wd[k] : FLT_MAX;
+        }
+    }
+    return U;
+}
+
 __global__ void __launch_bounds__(DT, 1) k_candidates_dense(WsArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ GatherSmem<DT, GCH> s_gather;
     __shared__ int s_q;
-    __shared__ uint32_t s_ws[DW], s_wn[DW];
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int tid = threadIdx.x;
     const int D = a.D, K = a.K, L = a.L, T = a.T;
     const int Dp = (D + 3) & ~3;
     const uint32_t nwords = (uint32_t)((a.N + 31) >> 5);
     const uint32_t nwp = (nwords + 3) & ~3u;
     float* qs = reinterpret_cast<float*>(smem);
     uint32_t* bits = reinterpret_cast<uint32_t*>(qs + Dp);
-    uint32_t* clist = bits + nwp;                       // DT * 32 candidate ids
-    float* wd_all = reinterpret_cast<float*>(clist + DT * 32);
-    uint32_t* wi_all = reinterpret_cast<uint32_t*>(wd_all + DW * K);
-    float* wd = wd_all + warp * K;
-    uint32_t* wi = wi_all + warp * K;
+    const ScanSmem sc = scan_smem(bits + nwp, K);
     const bool vec = (D & 3) == 0;
     const unsigned int ndense = *a.n_dense;
 
@@ -503,62 +576,33 @@ __global__ void __launch_bounds__(DT, 1) k_candidates_dense(WsArgs a) {
                                    [&](uint32_t id) { atomicOr(&bits[id >> 5], 1u << (id & 31)); });
         __syncthreads();
 
-        int n = 0;
-        float thr_d = FLT_MAX;
-        uint32_t thr_i = 0;
-        unsigned long long U = 0;   // unique candidates (summed by every thread alike)
-        for (uint32_t w0 = 0; w0 < nwords; w0 += DT) {
-            const uint32_t w = w0 + tid;
-            const uint32_t word = w < nwords ? bits[w] : 0u;
-            // block exclusive scan of the set-bit counts
-            const uint32_t c = __popc(word);
-            uint32_t x = c;
-#pragma unroll
-            for (int o = 1; o < 32; o <<= 1) {
-                const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-                if (lane >= o) x += y;
-            }
-            if (lane == 31) s_ws[warp] = x;
-            __syncthreads();
-            uint32_t before = 0, total = 0;
-            for (int i = 0; i < DW; ++i) {
-                const uint32_t v = s_ws[i];
-                before += i < warp ? v : 0u;
-                total += v;
-            }
-            uint32_t k = before + x - c;
-            for (uint32_t m = word; m; m &= m - 1) clist[k++] = w * 32 + (uint32_t)(__ffs((int)m) - 1);
-            __syncthreads();
-            fp32_dist_pass<DW>(a.X, D, qs, vec, total, [](uint32_t j) { return j; },
-                               [&](uint32_t ci) { return clist[ci]; }, [](uint32_t, float&) { return false; }, wd,
-                               wi, K, n, thr_d, thr_i);
-            U += total;
-            __syncthreads();
+        const unsigned long long U = scan_words(a.X, D, K, nwords, [&](uint32_t w) { return bits[w]; }, qs, vec, sc,
+                                                a.out_ids + (int64_t)q * K, a.out_d + (int64_t)q * K);
+        if (tid == 0) {
+            a.cu[q] = U;
+            atomicAdd(a.totals + 0, U);
+            atomicAdd(a.totals + 1, a.cnu[q]);
         }
-        if (lane == 0) s_wn[warp] = n;
         __syncthreads();
-        if (warp == 0) {
-            for (int ww = 1; ww < DW; ++ww) {
-                const int nw = s_wn[ww];
-                for (int e = 0; e < nw; ++e) {
-                    const float d = wd_all[ww * K + e];
-                    const uint32_t id = wi_all[ww * K + e];
-                    if (!lessp(d, id, thr_d, thr_i)) break;
-                    warp_insert(wd, wi, n, K, d, id, thr_d, thr_i);
-                }
-            }
-            int32_t* oid = a.out_ids + (int64_t)q * K;
-            float* od = a.out_d + (int64_t)q * K;
-            for (int k2 = lane; k2 < K; k2 += 32) {
-                oid[k2] = k2 < n ? (int32_t)wi[k2] : -1;
-                od[k2] = k2 < n ? wd[k2] : FLT_MAX;
-            }
-            if (lane == 0) {
-                a.cu[q] = U;
-                atomicAdd(a.totals + 0, U);
-                atomicAdd(a.totals + 1, a.cnu[q]);
-            }
-        }
+    }
+}
+
+// Exact scan of the queries the tensor-core merge could not finish (their
+// survivors outgrew its lists): the candidates come from the query's
+// membership row, distances and top-K as in k_candidates_dense.
+__global__ void __launch_bounds__(DT, 1) k_knn_scan_rows(KnnSearch k) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    const int tid = threadIdx.x, D = k.D, K = k.K;
+    float* qs = reinterpret_cast<float*>(smem);
+    const ScanSmem sc = scan_smem(qs + ((D + 3) & ~3), K);
+    const unsigned int nf = *k.n_fallback;
+    for (unsigned int f = blockIdx.x; f < nf; f += gridDim.x) {
+        const int i = k.fallback[f], q = k.dense_q[i];
+        for (int d = tid; d < D; d += DT) qs[d] = k.queries[(int64_t)q * D + d];
+        __syncthreads();
+        const uint32_t* row = k.bm + (int64_t)i * k.nwp;
+        scan_words(k.X, D, K, (uint32_t)((k.N + 31) >> 5), [&](uint32_t w) { return __ldg(row + w); }, qs,
+                   (D & 3) == 0, sc, k.out_ids + (int64_t)q * K, k.out_d + (int64_t)q * K);
         __syncthreads();
     }
 }
@@ -580,18 +624,34 @@ __global__ void __launch_bounds__(DT, 1) k_candidates_dense(WsArgs a) {
 // per four words. The set is the same either way.
 constexpr int BT = 1024;
 constexpr int BU = 8;
-constexpr uint32_t BSEG = 1024;
-constexpr int BCH = 256;   // (table, probe) slots per compaction chunk
+constexpr int BCH = 512;   // (table, probe) slots per compaction chunk
 constexpr uint32_t BROWS = 64;
 
 struct BitmapSmem {
-    uint64_t base[BCH];     // ids offset of each matched bucket
-    uint32_t size[BCH];
-    uint32_t upre[BCH + 1]; // units before each matched bucket
-    uint32_t n;
+    // id lists of a chunk's matched buckets (whole buckets, or the tails of
+    // bank lists), as one flattened range
+    uint64_t lbase[BCH];    // offset of each list (top bit: in the tails)
+    uint32_t lpre[BCH];     // ids up to and including each list
+    // bank lists: first entry and units up to and including each list
+    uint64_t bbase[BCH];
+    uint32_t bsize[BCH];    // groups of 128 entries
+    uint32_t bpre[BCH];
+    uint32_t wsum[2][BT / 32];
+    uint32_t nl, nb;
     uint32_t nrow;          // matched buckets with a bucket row (may exceed BROWS)
     uint32_t row[BROWS];    // their rows
 };
+
+// First of the n ascending inclusive prefixes that exceeds i.
+__device__ __forceinline__ uint32_t list_of(const uint32_t* pre, uint32_t n, uint32_t i) {
+    uint32_t lo = 0, hi = n - 1;
+    while (lo < hi) {
+        const uint32_t mid = (lo + hi) >> 1;
+        if (pre[mid] > i) hi = mid;
+        else lo = mid + 1;
+    }
+    return lo;
+}
 
 // Row of global bucket gi among the n ascending bucket numbers of big_gi, -1
 // if it has none.
@@ -607,34 +667,131 @@ __device__ __forceinline__ int big_row(const uint64_t* __restrict__ big_gi, int 
     return -1;
 }
 
-__global__ void __launch_bounds__(BT, 1) k_cand_bitmap(WsArgs a, uint32_t* __restrict__ bm, int nwp) {
+// Ids of the ascending list b[0 .. n) below p.
+__device__ __forceinline__ uint32_t ids_below(const uint32_t* __restrict__ b, uint32_t n, uint32_t p) {
+    uint32_t lo = 0;
+    while (n > 0) {
+        const uint32_t half = n >> 1;
+        const bool below = __ldg(b + lo + half) < p;
+        lo = below ? lo + half + 1 : lo;
+        n = below ? n - half - 1 : half;
+    }
+    return lo;
+}
+
+// Sets the bit of a bank-list entry (the low 16 bits of e: word row << 5 | bit)
+// in the column of words at `col`.
+__device__ __forceinline__ void or_entry(uint32_t* col, uint32_t e) {
+    atomicOr(col + (e & 0xFFE0u), __funnelshift_l(0u, 1u, e));   // 1 << (e & 31)
+}
+
+// Sample words of a segment for f = 32 / G: chunk c's i-th point is bit
+// (c % G) f of word c / G + i s32 / G, so G chunks share their reads.
+template <int G>
+__device__ __forceinline__ void sample_words(const uint32_t* bits, uint32_t* srow, int s32) {
+    const int step = s32 / G;   // s32 is a multiple of 4
+    for (int c = threadIdx.x; c < step; c += BT) {
+        uint32_t word[G];
+#pragma unroll
+        for (int j = 0; j < G; ++j) word[j] = 0;
+#pragma unroll 8
+        for (int i = 0; i < 32; ++i) {
+            const uint32_t w = bits[c + i * step];
+#pragma unroll
+            for (int j = 0; j < G; ++j) word[j] |= ((w >> (j * (32 / G))) & 1u) << i;
+        }
+#pragma unroll
+        for (int j = 0; j < G; ++j) srow[c * G + j] = word[j];
+    }
+}
+
+// ORs unit u of the bank lists of g (BU groups of one list) into the bitmap;
+// one warp, every load in flight before the first is ORed in.
+__device__ __forceinline__ void or_bank_unit(const WsArgs& a, const BitmapSmem& g, uint32_t u, uint32_t* bits) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t h = list_of(g.bpre, g.nb, u);
+    const uint32_t first = (u - (h ? g.bpre[h - 1] : 0u)) * BU;
+    const uint32_t cnt = min((uint32_t)BU, g.bsize[h] - first);
+    // lane b's four entries of a group are bits of words with bank b, so a
+    // warp's atomics never share a bank
+    const uint2* src = reinterpret_cast<const uint2*>(a.bank + g.bbase[h]) + (size_t)first * 32 + lane;
+    uint32_t* col = bits + lane;
+    uint2 v[BU];
+#pragma unroll
+    for (int b = 0; b < BU; ++b)
+        if (b < (int)cnt) v[b] = __ldg(src + b * 32);
+#pragma unroll
+    for (int b = 0; b < BU; ++b) {
+        if (b >= (int)cnt) break;   // warp-uniform
+        or_entry(col, v[b].x);
+        or_entry(col, v[b].x >> 16);
+        or_entry(col, v[b].y);
+        or_entry(col, v[b].y >> 16);
+    }
+}
+
+// ORs ids [32 BU u, 32 BU (u + 1)) of the flattened id lists into the bitmap
+// (one warp): short lists share a unit, so that its loads are in flight
+// together whatever the list lengths.
+__device__ __forceinline__ void or_id_unit(const WsArgs& a, const BitmapSmem& g, uint32_t u, uint32_t total,
+                                           uint32_t* bits, uint32_t p0) {
+    const int lane = threadIdx.x & 31;
+    uint32_t h = list_of(g.lpre, g.nl, u * (32 * BU));
+    uint32_t v[BU];
+#pragma unroll
+    for (int b = 0; b < BU; ++b) {
+        const uint32_t i = u * (32 * BU) + b * 32 + lane;
+        if (i < total) {
+            while (g.lpre[h] <= i) ++h;
+            const uint64_t base = g.lbase[h];
+            const uint32_t* src = (base >> 63 ? a.bank_tail : a.ids) + (base & ~(1ull << 63));
+            v[b] = __ldg(src + (i - (h ? g.lpre[h - 1] : 0u)));
+        }
+    }
+#pragma unroll
+    for (int b = 0; b < BU; ++b)
+        if (u * (32 * BU) + b * 32 + lane < total) {
+            const uint32_t w = v[b] - p0;   // p0 is a multiple of 32
+            atomicOr(&bits[w >> 5], __funnelshift_l(0u, 1u, w));
+        }
+}
+
+__global__ void __launch_bounds__(BT, 1) k_cand_bitmap(WsArgs a, KnnSearch k, uint32_t* __restrict__ bm) {
     extern __shared__ __align__(16) uint32_t bits[];
     __shared__ BitmapSmem g;
-    __shared__ int s_q, s_k;
+    __shared__ int s_q;
+    __shared__ unsigned int s_item;
     __shared__ unsigned long long s_cnt[BT / 32];
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
     constexpr int NW = BT / 32;
-    const unsigned int ndense = *a.n_dense;
+    const unsigned int nseg = (unsigned int)k.nseg;
+    const unsigned int nitems = (unsigned int)k.nd * nseg;
     const int T = a.T, LT = a.L * a.T;
-    // Thread 0 claims the next query while the block works on the current
+    // Thread 0 claims the next item while the block works on the current
     // one (the claim's round trip overlaps the work) and publishes it at the
-    // end of the query, before the block's last barrier.
+    // end of the item, before the block's last barrier.
     if (tid == 0) {
-        const unsigned int k = atomicAdd(a.dense_next, 1u);
-        s_k = (int)k;
-        s_q = k < ndense ? a.dense_q[k] : -1;
+        const unsigned int it = atomicAdd(a.dense_next, 1u);
+        s_item = it;
+        s_q = it < nitems ? k.dense_q[it / nseg] : -1;
     }
     __syncthreads();
     for (;;) {
-        const int q = s_q, k = s_k;
+        const int q = s_q;
         if (q < 0) break;
+        const unsigned int kq = s_item / nseg, g0 = s_item % nseg;
+        // the item's points: [p0, p1), word offset w0 of its row
+        const uint32_t p0 = g0 * (uint32_t)k.seg;
+        const uint32_t p1 = g0 + 1 == nseg ? (uint32_t)a.N : p0 + (uint32_t)k.seg;
+        const int w0 = (int)(p0 >> 5);
+        const int nwp = (g0 + 1 == nseg ? k.nwp : (int)(p1 >> 5)) - w0;
         unsigned int knext = 0;
         if (tid == 0) knext = atomicAdd(a.dense_next, 1u);
         for (int i = tid * 4; i < nwp; i += BT * 4) *reinterpret_cast<uint4*>(bits + i) = make_uint4(0u, 0u, 0u, 0u);
         for (int c0 = 0; c0 < LT; c0 += BCH) {
             // matched buckets of this chunk of (table, probe) slots, with sizes
             if (tid == 0) {
-                g.n = 0;
+                g.nl = g.nb = 0;
                 if (c0 == 0) g.nrow = 0;
             }
             __syncthreads();
@@ -644,7 +801,7 @@ __global__ void __launch_bounds__(BT, 1) k_cand_bitmap(WsArgs a, uint32_t* __res
                 const int32_t j = __ldg(a.qbuckets + (int64_t)l * a.Q * T + (int64_t)q * T + t);
                 if (j >= 0) {
                     const uint64_t gi = __ldg(a.boff + l) + (uint32_t)j;
-                    const uint32_t st = __ldg(a.starts + gi), sz = __ldg(a.sizes + gi);
+                    uint32_t st = __ldg(a.starts + gi), sz = __ldg(a.sizes + gi);
                     if (a.nbig > 0 && sz >= a.big_min) {
                         const int r = big_row(a.big_gi, a.nbig, gi);
                         if (r >= 0) {
@@ -655,98 +812,115 @@ __global__ void __launch_bounds__(BT, 1) k_cand_bitmap(WsArgs a, uint32_t* __res
                             }
                         }
                     }
-                    if (sz) {
-                        const uint32_t kk = atomicAdd(&g.n, 1u);
-                        g.base[kk] = (uint64_t)l * (uint64_t)a.N + st;
-                        g.size[kk] = sz;
+                    if (nseg > 1 && sz) {
+                        // the bucket's ids ascend: its part inside the segment
+                        const uint32_t* b = a.ids + (uint64_t)l * (uint64_t)a.N + st;
+                        const uint32_t lo = ids_below(b, sz, p0), hi = ids_below(b, sz, p1);
+                        st += lo;
+                        sz = hi - lo;
+                    }
+                    const uint64_t off = (uint64_t)l * (uint64_t)a.N + st;
+                    uint64_t lb = off;
+                    uint32_t ls = sz;
+                    if (a.bank_meta && sz >= a.bank_min) {
+                        const uint2 mt = __ldg(a.bank_meta + gi);
+                        if (mt.x) {
+                            const uint32_t kk = atomicAdd(&g.nb, 1u);
+                            g.bbase[kk] = (off + 3) & ~3ull;
+                            g.bsize[kk] = mt.x;
+                        }
+                        lb = off | (1ull << 63);
+                        ls = mt.y;
+                    }
+                    if (ls) {
+                        const uint32_t kk = atomicAdd(&g.nl, 1u);
+                        g.lbase[kk] = lb;
+                        g.lpre[kk] = ls;
                     }
                 }
             }
             __syncthreads();
-            const uint32_t n = g.n;
-            if (n == 0) continue;   // uniform
-            if (warp == 0) {
-                // exclusive scan of the units per bucket
-                uint32_t carry = 0;
-                for (uint32_t b0 = 0; b0 < n; b0 += 32) {
-                    const uint32_t kk = b0 + lane;
-                    const uint32_t c = kk < n ? (g.size[kk] + BSEG - 1) / BSEG : 0u;
-                    uint32_t x = c;
+            const uint32_t nl = g.nl, nb = g.nb;
+            if (nl + nb == 0) continue;   // uniform
+            {
+                // inclusive scans: ids per list (threads of the lower half),
+                // units per bank list (upper half)
+                static_assert(2 * BCH <= BT && BCH % 32 == 0, "one list per thread");
+                const int half = tid / BCH, t = tid % BCH;
+                uint32_t c = 0;
+                if (half == 0 && t < (int)nl) c = g.lpre[t];
+                if (half == 1 && t < (int)nb) c = (g.bsize[t] + BU - 1) / BU;
+                uint32_t x = c;
 #pragma unroll
-                    for (int o = 1; o < 32; o <<= 1) {
-                        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
-                        if (lane >= o) x += y;
-                    }
-                    if (kk < n) g.upre[kk] = carry + x - c;
-                    carry += __shfl_sync(0xffffffffu, x, 31);
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+                    if (lane >= o) x += y;
                 }
-                if (lane == 0) g.upre[n] = carry;
+                constexpr int HW = BCH / 32;   // warps per half
+                if (half < 2 && lane == 31) g.wsum[half][warp % HW] = x;
+                __syncthreads();
+                if (half < 2) {
+                    uint32_t before = lane < warp % HW ? g.wsum[half][lane] : 0u;
+                    before = __reduce_add_sync(0xffffffffu, before);
+                    if (half == 0 && t < (int)nl) g.lpre[t] = before + x;
+                    if (half == 1 && t < (int)nb) g.bpre[t] = before + x;
+                }
             }
             __syncthreads();
-            const uint32_t units = g.upre[n];
+            const uint32_t bunits = nb ? g.bpre[nb - 1] : 0u;
+            const uint32_t ids = nl ? g.lpre[nl - 1] : 0u;
+            const uint32_t units = bunits + (ids + 32 * BU - 1) / (32 * BU);
             for (uint32_t u = warp; u < units; u += NW) {
-                // bucket of unit u: the last b with upre[b] <= u
-                uint32_t lo = 0, hi = n - 1;
-                while (lo < hi) {
-                    const uint32_t mid = (lo + hi + 1) >> 1;
-                    if (g.upre[mid] <= u) lo = mid;
-                    else hi = mid - 1;
-                }
-                const uint32_t off = (u - g.upre[lo]) * BSEG;
-                const uint32_t cnt = min(BSEG, g.size[lo] - off);
-                const uint32_t* src = a.ids + g.base[lo] + off;
-                uint32_t j0 = 0;
-                for (; j0 + 32 * BU <= cnt; j0 += 32 * BU) {   // full blocks: BU loads in flight per lane
-                    uint32_t v[BU];
-#pragma unroll
-                    for (int b = 0; b < BU; ++b) v[b] = __ldg(src + j0 + b * 32 + lane);
-#pragma unroll
-                    for (int b = 0; b < BU; ++b) atomicOr(&bits[v[b] >> 5], 1u << (v[b] & 31));
-                }
-                for (; j0 < cnt; j0 += 32) {
-                    const uint32_t j = j0 + lane;
-                    if (j < cnt) {
-                        const uint32_t v = __ldg(src + j);
-                        atomicOr(&bits[v >> 5], 1u << (v & 31));
-                    }
-                }
+                if (u < bunits) or_bank_unit(a, g, u, bits);
+                else or_id_unit(a, g, u - bunits, ids, bits, p0);
             }
             __syncthreads();
         }
-        uint32_t* row = bm + (int64_t)k * nwp;
+        uint32_t* row = bm + (int64_t)kq * k.nwp + w0;
         const uint32_t nrow = min(g.nrow, BROWS);
         unsigned long long cnt = 0;
         for (int i = tid * 4; i < nwp; i += BT * 4) {
             uint4 v = *reinterpret_cast<const uint4*>(bits + i);
 #pragma unroll 4
             for (uint32_t r = 0; r < nrow; ++r) {
-                const uint4 w = __ldg(reinterpret_cast<const uint4*>(a.big_rows + (size_t)g.row[r] * nwp + i));
+                const uint4 w = __ldg(reinterpret_cast<const uint4*>(a.big_rows + (size_t)g.row[r] * k.nwp + w0 + i));
                 v.x |= w.x;
                 v.y |= w.y;
                 v.z |= w.z;
                 v.w |= w.w;
             }
             *reinterpret_cast<uint4*>(row + i) = v;
+            if (nrow > 0 && k.f > 0) *reinterpret_cast<uint4*>(bits + i) = v;   // for the sample words
             cnt += __popc(v.x) + __popc(v.y) + __popc(v.z) + __popc(v.w);
         }
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) cnt += __shfl_xor_sync(0xffffffffu, cnt, o);
         if (lane == 0) s_cnt[warp] = cnt;
         __syncthreads();
+        // the segment's sample chunks: chunk c holds points (i s32 + c) f of it
+        uint32_t* srow = k.bm_sample + (int64_t)kq * k.nws + g0 * k.s32;
+        if (k.f == 16) sample_words<2>(bits, srow, k.s32);
+        else if (k.f == 8) sample_words<4>(bits, srow, k.s32);
+        else
+            for (int c = tid; c < k.s32; c += BT) {
+                uint32_t word = 0, p = (uint32_t)c * k.f;
+#pragma unroll 8
+                for (int i = 0; i < 32; ++i, p += (uint32_t)k.s32 * k.f) word |= ((bits[p >> 5] >> (p & 31)) & 1u) << i;
+                srow[c] = word;
+            }
         if (tid == 0) {
             unsigned long long U = 0;
             for (int w = 0; w < NW; ++w) U += s_cnt[w];
-            a.cu[q] = U;
+            if (nseg == 1) a.cu[q] = U;
+            else atomicAdd(a.cu + q, U);   // zeroed by the planner
             atomicAdd(a.totals + 0, U);
-            atomicAdd(a.totals + 1, a.cnu[q]);
-            s_k = (int)knext;
-            s_q = knext < ndense ? a.dense_q[knext] : -1;
+            if (g0 == 0) atomicAdd(a.totals + 1, a.cnu[q]);
+            s_item = knext;
+            s_q = knext < nitems ? k.dense_q[knext / nseg] : -1;
         }
         __syncthreads();
     }
 }
-
-size_t bitmap_smem_bytes(int64_t N) { return 4 * (size_t)((((N + 31) >> 5) + 3) & ~3ll); }
 
 __global__ void k_big_find(const uint32_t* __restrict__ sizes, uint64_t totB, uint32_t big_min, uint64_t* gi,
                            uint32_t* sz, unsigned int* cnt, unsigned int cap) {
@@ -760,6 +934,58 @@ __global__ void k_big_find(const uint32_t* __restrict__ sizes, uint64_t totB, ui
             }
         }
     }
+}
+
+// Bank lists (one block per bucket of the list gi): a bucket's ids as 16-bit
+// entries (word row << 5 | bit of the id in an N-bit bitmap whose words are 32
+// banks wide), arranged so that a warp of the membership kernel ORs 32
+// entries into 32 different banks: entry slot [group][bank][4] holds four
+// ids of one bank. Every bank gets as many slots as an even split of the
+// bucket would fill; a bank with fewer ids fills the rest with an entry of the
+// word row past the bitmap (never copied out), one with more sends the remaining ids to the bucket's tail (32-bit ids). The order
+// within a bank is arbitrary: the entries are ORed. 32 random banks cost 3.5
+// cycles a warp instruction, distinct ones one, and an entry is half an id:
+// (figures at k_cand_bitmap).
+constexpr int BF = 256;
+__global__ void __launch_bounds__(BF) k_bank_fill(const uint64_t* __restrict__ gi, const unsigned int* __restrict__ n,
+                                                 unsigned int cap, const uint64_t* __restrict__ boff, int L,
+                                                 const uint32_t* __restrict__ starts, const uint32_t* __restrict__ sizes,
+                                                 const uint32_t* __restrict__ ids, int64_t N, uint16_t* bank,
+                                                 uint32_t* tail, uint2* meta) {
+    __shared__ uint32_t cnt[32], ntail;
+    const unsigned int nb = min(*n, cap);
+    const uint16_t dummy = (uint16_t)(((uint32_t)(N + 1023) >> 10) << 5);
+    for (unsigned int r = blockIdx.x; r < nb; r += gridDim.x) {
+        const uint64_t b = gi[r];
+        int l = 0;
+        while (l + 1 < L && boff[l + 1] <= b) ++l;
+        const uint64_t off = (uint64_t)l * N + starts[b], base = (off + 3) & ~3ull;
+        const uint32_t sz = sizes[b];
+        const uint32_t R = ((sz - 3) / 32) & ~3u;   // slots per bank; 32 R entries fit from base on
+        __syncthreads();
+        if (threadIdx.x < 32) cnt[threadIdx.x] = 0;
+        if (threadIdx.x == 32) ntail = 0;
+        __syncthreads();
+        for (uint32_t j = threadIdx.x; j < sz; j += BF) {
+            const uint32_t v = ids[off + j], bk = (v >> 5) & 31u;
+            const uint32_t k = atomicAdd(&cnt[bk], 1u);
+            if (k < R) bank[base + (uint64_t)(k >> 2) * 128 + bk * 4 + (k & 3)] = (uint16_t)(((v >> 10) << 5) | (v & 31u));
+            else tail[off + atomicAdd(&ntail, 1u)] = v;
+        }
+        __syncthreads();
+        for (uint32_t s = threadIdx.x; s < 32 * R; s += BF) {
+            const uint32_t bk = (s >> 2) & 31u, k = ((s >> 7) << 2) | (s & 3u);
+            if (k >= cnt[bk]) bank[base + s] = dummy;
+        }
+        if (threadIdx.x == 0) meta[b] = make_uint2(R / 4, ntail);
+    }
+}
+
+cudaError_t launch_bank_fill(const uint64_t* gi, const unsigned int* n, unsigned int cap, const uint64_t* boff, int L,
+                             const uint32_t* starts, const uint32_t* sizes, const uint32_t* ids, int64_t N,
+                             uint16_t* bank, uint32_t* tail, uint2* meta, cudaStream_t st) {
+    k_bank_fill<<<152 * 8, BF, 0, st>>>(gi, n, cap, boff, L, starts, sizes, ids, N, bank, tail, meta);
+    return cudaGetLastError();
 }
 
 // Row r (blockIdx.y) gets the bits of bucket gi[r]'s ids (table tl[r]).
@@ -793,19 +1019,34 @@ cudaError_t launch_big_fill(const uint64_t* gi, const int32_t* tl, int nbig, con
     return cudaGetLastError();
 }
 
-cudaError_t launch_cand_bitmap(const WsArgs& a, uint32_t* bm, int nwp, int grid, cudaStream_t st) {
+// (less the block's lists and the bank lists' word row)
+size_t bitmap_smem(int max_smem) { return (size_t)max_smem - sizeof(BitmapSmem) - 2048; }
+
+cudaError_t launch_cand_bitmap(const WsArgs& a, const KnnSearch& k, uint32_t* bm, int grid, cudaStream_t st) {
     static std::atomic<size_t> cap{0};
-    const size_t smem = 4 * (size_t)nwp;
+    // the longest segment is the last one
+    size_t smem = 4 * (size_t)(k.nwp - (k.nseg - 1) * (k.seg >> 5));
+    if (a.bank_meta) smem = 4 * ((size_t)((a.N + 1023) >> 10) + 1) * 32;   // and the word row of unused entries
     const cudaError_t e = opt_in_smem(k_cand_bitmap, smem, cap);
     if (e != cudaSuccess) return e;
-    k_cand_bitmap<<<grid, BT, smem, st>>>(a, bm, nwp);
+    k_cand_bitmap<<<grid, BT, smem, st>>>(a, k, bm);
+    return cudaGetLastError();
+}
+
+size_t knn_scan_smem(int D, int K) { return sizeof(float) * (size_t)((D + 3) & ~3) + scan_bytes(K); }
+
+cudaError_t launch_knn_scan_rows(const KnnSearch& k, int grid, cudaStream_t st) {
+    static std::atomic<size_t> cap{0};
+    const size_t smem = knn_scan_smem(k.D, k.K);
+    const cudaError_t e = opt_in_smem(k_knn_scan_rows, smem, cap);
+    if (e != cudaSuccess) return e;
+    k_knn_scan_rows<<<grid, DT, smem, st>>>(k);
     return cudaGetLastError();
 }
 
 size_t dense_smem_bytes(int64_t N, int D, int K) {
     const size_t nwp = (size_t)((((N + 31) >> 5) + 3) & ~3ll);
-    return sizeof(float) * (size_t)((D + 3) & ~3) + 4 * nwp + 4 * (size_t)DT * 32 +
-           (size_t)DW * K * (sizeof(float) + sizeof(uint32_t));
+    return sizeof(float) * (size_t)((D + 3) & ~3) + 4 * nwp + scan_bytes(K);
 }
 
 size_t ws_smem_bytes(int D, int K, int wt, int bf16, int slots) {

@@ -142,9 +142,9 @@ struct culsh_index {
     DevBuf<uint16_t> xb;    // bf16 copy of the device dataset (search precision form), built on first use
     DevBuf<uint8_t> xflag;  // per row: 1 exact in bf16, 2 always re-check in FP32, 0 bound applies
     bool xb_valid = false;
-    // tensor-core k-NN rows of the dataset (bf16 parts, weights, flags), built on first use
-    DevBuf<uint16_t> kx_h, kx_l;
-    DevBuf<float> kw_exact, kw_bound;
+    // tensor-core k-NN rows of the dataset (fp16 operand, norms, state), built on first use
+    DevBuf<uint16_t> kx_h;
+    DevBuf<float> kx_w;
     DevBuf<KnnState> kstate;
     KnnState h_kstate{};
     bool kx_valid = false;
@@ -156,6 +156,12 @@ struct culsh_index {
     DevBuf<unsigned int> big_cnt;
     int nbig = 0;
     uint32_t big_min = UINT32_MAX;
+    // bank lists of the buckets of kBankMin ids or more (same life as the bucket rows)
+    DevBuf<uint64_t> bank_gi;
+    DevBuf<uint16_t> bank;
+    DevBuf<uint32_t> bank_tail;
+    DevBuf<uint2> bank_meta;
+    bool has_bank = false;
     bool big_valid = false;
     int KW = 1;
     std::vector<int32_t> h_cmin, h_cmax;
@@ -254,12 +260,12 @@ struct culsh_search {
     DevBuf<uint8_t> item_p;
     DevBuf<float> part_d;
     DevBuf<uint32_t> part_i;
-    // tensor-core k-NN path: membership rows, query rows, partial lists, fallback list
-    DevBuf<uint32_t> kbm;
-    DevBuf<uint16_t> kq_h, kq_l;
-    DevBuf<float> kq_sq, kq_base, kpart_key;
-    DevBuf<unsigned int> kq_bound;
-    DevBuf<uint32_t> kpart_id;
+    // tensor-core k-NN path: membership rows, query rows, sample, survivor lists, scan list
+    DevBuf<uint32_t> kbm, kbm_sample;
+    DevBuf<uint16_t> kq_h;
+    DevBuf<KnnQuery> kq_info;
+    DevBuf<float> kq_lim, kw_sample, ksmin;
+    DevBuf<uint2> kpart;
     DevBuf<int> kpart_n, kfallback;
     int knn_queries = 0, knn_fallback = 0;   // last search: dense queries on the tensor cores, re-run
     int bucket_rows = 0;                     // last search: bucket rows its membership rows could use
@@ -917,9 +923,9 @@ constexpr int kWsPartitions = 64;              // most partitions of one query
 // to the host after it): [0] unique and [1] non-unique candidate totals,
 // [2] overflow-arena top, [3] deferred queries, [4] work-stealing item
 // counter (low) and overflow flag (high), [5] items, [6] BF16 re-checks,
-// [7] dense queries (low) and their claim counter (high), [8..9] the dense
-// queries' k-NN row state, [10] tensor-core fallback queries, [11] its error
-// flags, [12..13] totals of re-runs that must not count twice.
+// [7] dense queries (low) and their claim counter (high), [8..9] unused,
+// [10] dense queries scanned exactly after the tensor-core merge, [11] the
+// tensor-core kernels' error flags, [12..15] unused.
 constexpr int kStatWords = 16;
 constexpr size_t kWsPartialBytes = size_t(64) << 20;
 
@@ -945,22 +951,21 @@ struct SearchPlan {
     float* vals;
     ProbeArgs pa;
     int probe_generic;
-    int use_ws, ws_grid, use_dense, dense_grid;
-    int use_knn;        // dense queries on the tensor cores (membership rows + masked GEMM)
-    uint32_t* kbm;      // their membership rows
-    KnnSearch kn;
+    int use_ws, ws_grid;
+    int use_dense;      // some query can be dense: the planner lists those, run_dense serves them
+    int use_knn;        // ... on the tensor cores (membership rows + masked GEMM)
     CandArgs ca;
     WsArgs wa;
     unsigned long long* stats;
     unsigned long long* h_stats;
     unsigned long long* cnu;
-    cudaEvent_t ev[5];  // stage boundaries; ev[4]: membership rows done (tensor-core path)
+    cudaEvent_t ev[4];  // stage boundaries
     int stage_events;   // 0: no stage events in the graph (they cost a few microseconds each)
 };
 
 static_assert(sizeof(SearchPlan) <= kPlanBytes, "graph key buffer too small");
 
-// Dataset rows of the tensor-core k-NN path (bf16 parts, weights, flags),
+// Dataset rows of the tensor-core k-NN path (fp16 operand, norms, state),
 // made once per dataset. The stream is drained before they are published:
 // searches on other streams read them as soon as they see them.
 int ensure_knn_rows(culsh_index* ix, cudaStream_t st) {
@@ -968,13 +973,10 @@ int ensure_knn_rows(culsh_index* ix, cudaStream_t st) {
     const int N = ix->N, D = ix->D, Dp = (D + 63) / 64 * 64;
     const int64_t pad = ((int64_t)N + 255) / 256 * 256;
     CU_TRY(ix->kx_h.reserve((size_t)N * Dp));
-    CU_TRY(ix->kx_l.reserve((size_t)N * Dp));
-    CU_TRY(ix->kw_exact.reserve((size_t)pad));
-    CU_TRY(ix->kw_bound.reserve((size_t)pad));
+    CU_TRY(ix->kx_w.reserve((size_t)pad));
     CU_TRY(ix->kstate.reserve(1));
     CU_TRY(cudaMemsetAsync(ix->kstate.p, 0, sizeof(KnnState), st));
-    CU_TRY(launch_knn_rows_dataset(ix->dev_x(), N, D, Dp, ix->kx_h.p, ix->kx_l.p, ix->kw_exact.p, ix->kw_bound.p, pad,
-                                   knn_bound_factor(D), ix->kstate.p, st));
+    CU_TRY(launch_knn_rows_dataset(ix->dev_x(), N, D, Dp, ix->kx_h.p, ix->kx_w.p, pad, ix->kstate.p, st));
     CU_TRY(cudaMemcpyAsync(&ix->h_kstate, ix->kstate.p, sizeof(KnnState), cudaMemcpyDeviceToHost, st));
     CU_TRY(cudaStreamSynchronize(st));
     ix->kx_valid = true;
@@ -983,19 +985,38 @@ int ensure_knn_rows(culsh_index* ix, cudaStream_t st) {
 
 // Bucket rows: every bucket of at least big_min ids gets an N-bit row (nwp
 // words), which the membership kernel ORs into a dense query's row instead of
-// setting the bucket's bits id by id. big_min = max(1024, N/64), where a row
-// (N/8 bytes) is at most twice the bucket's ids (4 bytes each); there are then
-// at most 64 L rows. CULSH_BIG_ROWS_MIN overrides big_min (0: no rows). Rows
+// setting the bucket's bits id by id. big_min = max(1024, N/32): a row is N/8
+// bytes to read; the bucket's bank list is about 2.2 bytes and a thirty-second
+// of a warp's atomic per id, about as much at N/32 ids; there are then at most
+// 32 L rows. CULSH_BIG_ROWS_MIN overrides big_min (0: no rows). Rows
 // beyond kBigRowsBytes keep only the largest buckets. Made once per index; the
 // stream is drained before they are published.
 constexpr size_t kBigRowsBytes = size_t(1) << 30;
 
-int ensure_big_rows(culsh_index* ix, int nwp, cudaStream_t st) {
+int ensure_big_rows(culsh_index* ix, int nwp, int nseg, cudaStream_t st) {
     if (ix->big_valid) return CULSH_OK;
     const int L = ix->L, N = ix->N;
     ix->nbig = 0;
     ix->big_min = UINT32_MAX;
-    long long bmin = std::max(1024ll, (long long)N / 64);
+    ix->has_bank = false;
+    if (nseg == 1 && N <= kBankMaxN && ix->max_bucket >= kBankMin) {
+        // Bank lists for the one-segment membership kernel.
+        const size_t LN = (size_t)L * N, totB = ix->h_boff[L];
+        const unsigned int cap = (unsigned int)std::min<size_t>(LN / kBankMin + 1, totB);
+        CU_TRY(ix->bank_gi.reserve(cap));
+        CU_TRY(ix->big_sz.reserve(cap));
+        CU_TRY(ix->big_cnt.reserve(1));
+        CU_TRY(ix->bank.reserve(LN));
+        CU_TRY(ix->bank_tail.reserve(LN));
+        CU_TRY(ix->bank_meta.reserve(totB));
+        CU_TRY(cudaMemsetAsync(ix->big_cnt.p, 0, sizeof(unsigned int), st));
+        CU_TRY(launch_big_find(ix->sizes.p, totB, kBankMin, ix->bank_gi.p, ix->big_sz.p, ix->big_cnt.p, cap, st));
+        CU_TRY(launch_bank_fill(ix->bank_gi.p, ix->big_cnt.p, cap, ix->boff.p, L, ix->starts.p, ix->sizes.p, ix->ids.p,
+                                N, ix->bank.p, ix->bank_tail.p, ix->bank_meta.p, st));
+        CU_TRY(cudaStreamSynchronize(st));
+        ix->has_bank = true;
+    }
+    long long bmin = std::max(1024ll, (long long)N / 32);
     if (const char* e = getenv("CULSH_BIG_ROWS_MIN")) bmin = atoll(e);
     if (bmin <= 0 || (long long)ix->max_bucket < bmin) {
         ix->big_valid = true;
@@ -1053,77 +1074,131 @@ int ensure_big_rows(culsh_index* ix, int nwp, cudaStream_t st) {
     return CULSH_OK;
 }
 
-// Whether the dataset's values allow the exact form (integers of magnitude
-// <= 256, D max|v|^2 < 2^24 and D (max - min)^2 < 2^24); the queries must
-// qualify too, which the kernels check on the device.
-bool knn_dataset_exact(const culsh_index* ix) {
-    const KnnState& k = ix->h_kstate;
-    if (k.flags & (kKnnNotSmallInt | kKnnNonFinite) || k.mneg == 0 || k.mpos == 0) return false;
-    const long long lo = 257 - k.mneg, hi = k.mpos - 257, mag = std::max(-lo, hi);
-    return (long long)ix->D * mag * mag < (1ll << 24) && (long long)ix->D * (hi - lo) * (hi - lo) < (1ll << 24);
+// Whether the dataset's magnitudes suit the tensor-core path (its squares
+// stay inside the float range).
+bool knn_dataset_fits(const KnnState& k) {
+    float amax;
+    std::memcpy(&amax, &k.amax, 4);
+    return !(k.flags & kKnnNonFinite) && amax <= kKnnMaxValue && (amax == 0.0f || amax >= kKnnMinValue);
 }
 
-// Membership rows above this size send the dense queries to the SIMT kernel.
-constexpr size_t kKnnMaxBitmapBytes = size_t(16) << 30;
+constexpr int kKnnEstimateSmem = 227 * 1024;   // shared memory a block may opt into, for estimates without a device
 
-// Plans the tensor-core path for the dense queries of a search of Q queries
-// (sets *ok); it declines dimensions above 128, K above kMaxKnnK, datasets
-// whose N-bit bitmap does not fit a block's shared memory and membership rows
-// above kKnnMaxBitmapBytes.
-int plan_knn(culsh_search* s, SearchPlan& P, int Q, int32_t* d_ids, float* d_d, cudaStream_t st, bool* ok) {
-    *ok = false;
-    culsh_index* ix = s->ix;
-    KnnSearch& k = P.kn;
+// Most membership-row bytes at a time; further dense queries take turns.
+constexpr size_t kKnnChunkBytes = size_t(2) << 30;
+
+// Shapes of the tensor-core path for nd dense queries at a time (as many as
+// kKnnChunkBytes of membership rows allow); false when it does not serve the
+// index and K.
+bool knn_shapes(const culsh_index* ix, int K, int nd, int sms, int smem_optin, KnnSearch* out) {
+    KnnSearch& k = *out;
+    k = KnnSearch{};
     k.N = ix->N;
     k.D = ix->D;
-    k.K = s->K;
-    k.Qcap = (Q + 2 * kKnnTileQ - 1) / (2 * kKnnTileQ) * (2 * kKnnTileQ);   // whole 256-query tiles
-    k.grid = s->sms;
-    if (!knn_plan(k, s->smem_optin)) return CULSH_OK;
-    if (bitmap_smem_bytes(ix->N) + 8192 > (size_t)s->smem_optin) return CULSH_OK;
-    const size_t bm_words = (size_t)k.Qcap * k.nwp;
-    if (4 * bm_words > kKnnMaxBitmapBytes) return CULSH_OK;
-    TRY(ensure_knn_rows(ix, st));
-    if (ix->h_kstate.flags & kKnnNonFinite) return CULSH_OK;
-    TRY(ensure_big_rows(ix, k.nwp, st));
-    k.exact_possible = knn_dataset_exact(ix) && k.ops_exact > 0;
-    k.C = knn_bound_factor(ix->D);
-    CU_TRY(s->kbm.reserve(bm_words));
-    CU_TRY(s->kq_h.reserve((size_t)k.Qcap * k.Dp));
-    CU_TRY(s->kq_l.reserve((size_t)k.Qcap * k.Dp));
-    CU_TRY(s->kq_sq.reserve(k.Qcap));
-    CU_TRY(s->kq_base.reserve(k.Qcap));
-    CU_TRY(s->kq_bound.reserve(k.Qcap));
-    CU_TRY(s->kpart_key.reserve(knn_part_entries(k)));
-    CU_TRY(s->kpart_id.reserve(knn_part_entries(k)));
-    CU_TRY(s->kpart_n.reserve(knn_part_lists(k)));
-    CU_TRY(s->kfallback.reserve(k.Qcap));
+    k.K = K;
+    const size_t row = 4 * (size_t)(((size_t)ix->N + 31) / 32 + 3);
+    const size_t most = std::max<size_t>(kKnnChunkBytes / row / kKnnTileQ, 1) * kKnnTileQ;
+    k.nd = (int)std::min<size_t>((size_t)nd, most);
+    k.Qcap = (k.nd + kKnnTileQ - 1) / kKnnTileQ * kKnnTileQ;
+    k.grid = sms;
+    return knn_plan(k, smem_optin, bitmap_smem(smem_optin)) && knn_scan_smem(k.D, k.K) + 8192 <= (size_t)smem_optin;
+}
+
+// Serves the nd dense queries the planner listed (s->dense_q) once the rest of
+// the search has run: their number is known here, so that a search without
+// any launches nothing for them and buffers are sized by those it has. The
+// tensor-core path, or the SIMT bitmap kernel where that does not apply;
+// *left is set when neither does (the caller re-runs them per query).
+int run_dense(culsh_search* s, const SearchPlan& P, int nd, cudaStream_t st, bool* left) {
+    culsh_index* ix = s->ix;
+    WsArgs a = P.wa;
+    KnnSearch k;
+    bool knn = P.use_knn && knn_shapes(ix, s->K, nd, s->sms, s->smem_optin, &k);
+    *left = false;
+    if (knn) {
+        std::lock_guard<std::mutex> lk(alloc_capture_mutex());
+        TRY(ensure_knn_rows(ix, st));
+        knn = knn_dataset_fits(ix->h_kstate);
+        if (knn) {
+            TRY(ensure_big_rows(ix, k.nwp, k.nseg, st));
+            CU_TRY(s->kbm.reserve((size_t)k.Qcap * k.nwp));
+            CU_TRY(s->kbm_sample.reserve((size_t)k.Qcap * k.nws));
+            CU_TRY(s->kq_h.reserve((size_t)k.Qcap * k.Dp));
+            CU_TRY(s->kq_info.reserve(k.Qcap));
+            CU_TRY(s->kq_lim.reserve(k.Qcap));
+            CU_TRY(s->kw_sample.reserve((size_t)k.nws * 32));
+            CU_TRY(s->ksmin.reserve((size_t)k.Qcap * k.nws));
+            CU_TRY(s->kpart.reserve(knn_part_entries(k)));
+            CU_TRY(s->kpart_n.reserve(knn_part_lists(k)));
+            CU_TRY(s->kfallback.reserve(k.Qcap));
+        }
+    }
+    if (!knn) {
+        if (dense_smem_bytes(ix->N, ix->D, s->K) + 8192 > (size_t)s->smem_optin) {
+            *left = true;
+            return CULSH_OK;
+        }
+        CU_TRY(launch_candidates_dense(a, s->sms, st));
+        s->launches += 1;
+        if (P.stage_events) CU_TRY(cudaEventRecord(s->ev[3], st));
+        CU_TRY(cudaMemcpyAsync(s->h_stats.p, s->stats.p, 8 * kStatWords, cudaMemcpyDeviceToHost, st));
+        CU_TRY(cudaStreamSynchronize(st));
+        return CULSH_OK;
+    }
+    if (ix->nbig > 0 && !getenv("CULSH_NO_BIG_ROWS")) {
+        a.big_gi = ix->big_gi.p;
+        a.big_rows = ix->big_rows.p;
+        a.nbig = ix->nbig;
+        a.big_min = ix->big_min;
+    }
+    if (ix->has_bank && k.nseg == 1) {
+        a.bank = ix->bank.p;
+        a.bank_tail = ix->bank_tail.p;
+        a.bank_meta = ix->bank_meta.p;
+        a.bank_min = kBankMin;
+    }
+    k.gamma = knn_gamma(ix->D);
     k.xh = ix->kx_h.p;
-    k.xl = ix->kx_l.p;
-    k.w_exact = ix->kw_exact.p;
-    k.w_bound = ix->kw_bound.p;
+    k.w = ix->kx_w.p;
     k.dstate = ix->kstate.p;
     k.X = ix->dev_x();
     k.queries = P.ca.queries;
-    k.dense_q = s->dense_q.p;
-    k.n_dense = P.wa.n_dense;
     k.qh = s->kq_h.p;
-    k.ql = s->kq_l.p;
-    k.qsq = s->kq_sq.p;
-    k.qbase = s->kq_base.p;
-    k.qbound = s->kq_bound.p;
-    k.qstate = reinterpret_cast<KnnState*>(s->stats.p + 8);
+    k.qinfo = s->kq_info.p;
+    k.qlim = s->kq_lim.p;
+    k.w_sample = s->kw_sample.p;
+    k.smin = s->ksmin.p;
     k.bm = s->kbm.p;
-    k.part_key = s->kpart_key.p;
-    k.part_id = s->kpart_id.p;
+    k.bm_sample = s->kbm_sample.p;
+    k.part = s->kpart.p;
     k.part_n = s->kpart_n.p;
-    k.out_ids = d_ids;
-    k.out_d = d_d;
+    k.out_ids = P.ca.out_ids;
+    k.out_d = P.ca.out_d;
     k.fallback = s->kfallback.p;
     k.n_fallback = reinterpret_cast<unsigned int*>(s->stats.p + 10);
     k.err = reinterpret_cast<int*>(s->stats.p + 11);
-    P.kbm = s->kbm.p;
-    *ok = true;
+    const int chunk = k.nd;
+    s->knn_queries = nd;
+    s->bucket_rows = a.nbig;
+    for (int at = 0; at < nd; at += chunk) {
+        k.nd = std::min(chunk, nd - at);   // buffers and lists stay those of a whole chunk
+        k.dense_q = s->dense_q.p + at;
+        if (at > 0) {
+            CU_TRY(cudaMemsetAsync(a.dense_next, 0, sizeof(unsigned int), st));
+            CU_TRY(cudaMemsetAsync(s->stats.p + 10, 0, 8, st));
+        }
+        CU_TRY(launch_cand_bitmap(a, k, s->kbm.p, s->sms, st));
+        if (P.stage_events) CU_TRY(cudaEventRecord(s->ev[5], st));
+        CU_TRY(launch_knn_search(k, st));
+        CU_TRY(launch_knn_scan_rows(k, s->sms, st));
+        s->launches += 2 + knn_launches(k);
+        if (P.stage_events) CU_TRY(cudaEventRecord(s->ev[3], st));
+        CU_TRY(cudaMemcpyAsync(s->h_stats.p, s->stats.p, 8 * kStatWords, cudaMemcpyDeviceToHost, st));
+        CU_TRY(cudaStreamSynchronize(st));
+        if ((s->h_stats.p[11] & 0xffffffffu) != 0)
+            return fail(CULSH_ERR_DEVICE, "tensor-core k-NN: a bounded device wait gave up");
+        s->knn_fallback += (int)(s->h_stats.p[10] & 0xffffffffu);
+    }
     return CULSH_OK;
 }
 
@@ -1314,9 +1389,9 @@ int plan_search(culsh_search* s, const float* dQ, int Q, int32_t* d_ids, float* 
         // take the tensor-core path (membership rows and a masked GEMM over
         // the whole dataset; default threshold max(4096, N/256)) or, where
         // that path does not apply, the SIMT bitmap kernel (max(32768, N/16)).
-        // The tuning or CULSH_DENSE_MIN override the threshold. The dense
-        // kernels are launched only when some query could reach it (L*T*largest
-        // bucket) and the N-bit bitmap fits the shared memory of a block.
+        // The tuning or CULSH_DENSE_MIN override the threshold. The planner
+        // lists them when some query could reach it (L*T*largest bucket) and
+        // the kernels can serve them; run_dense then takes the list.
         a.n_dense = reinterpret_cast<unsigned int*>(s->stats.p + 7);
         a.dense_next = reinterpret_cast<unsigned int*>(s->stats.p + 7) + 1;
         const unsigned long long reach = (unsigned long long)L * T * ix->max_bucket;
@@ -1327,11 +1402,10 @@ int plan_search(culsh_search* s, const float* dQ, int Q, int32_t* d_ids, float* 
             if (const char* e = getenv("CULSH_DENSE_MIN")) d = std::max(1ll, atoll(e));
             return d;
         };
-        bool knn = false;
-        if (tu.dense_tc && !getenv("CULSH_NO_KNN_TC") && reach >= dense_min_for(true)) {
-            CU_TRY(s->dense_q.reserve(Q));
-            TRY(plan_knn(s, P, Q, d_ids, d_d, st, &knn));
-        }
+        KnnSearch shapes;
+        const bool knn = tu.dense_tc && !getenv("CULSH_NO_KNN_TC") && reach >= dense_min_for(true) &&
+                         !(ix->kx_valid && !knn_dataset_fits(ix->h_kstate)) &&
+                         knn_shapes(ix, K, Q, s->sms, s->smem_optin, &shapes);
         const unsigned long long dmin = dense_min_for(knn);
         const bool dense_fits = knn || dense_smem_bytes(ix->N, D, K) + 8192 <= (size_t)s->smem_optin;
         P.use_dense = dense_fits && reach >= dmin;
@@ -1340,17 +1414,9 @@ int plan_search(culsh_search* s, const float* dQ, int Q, int32_t* d_ids, float* 
         if (P.use_dense) {
             CU_TRY(s->dense_q.reserve(Q));
             a.dense_q = s->dense_q.p;
-            P.dense_grid = s->sms;
-            if (P.use_knn) P.kn.dense_q = s->dense_q.p;
         }
         a.nbig = 0;
         a.big_min = UINT32_MAX;
-        if (P.use_knn && ix->nbig > 0 && !getenv("CULSH_NO_BIG_ROWS")) {
-            a.big_gi = ix->big_gi.p;
-            a.big_rows = ix->big_rows.p;
-            a.nbig = ix->nbig;
-            a.big_min = ix->big_min;
-        }
         if (tu.ws_order) {
             CU_TRY(s->qorder.reserve(Q));
             CU_TRY(s->qorder_bins.reserve(kOrderBins + 1));
@@ -1375,7 +1441,6 @@ int plan_search(culsh_search* s, const float* dQ, int Q, int32_t* d_ids, float* 
     P.h_stats = s->h_stats.p;
     P.cnu = s->cnu.p;
     for (int i = 0; i < 4; ++i) P.ev[i] = s->ev[i];
-    P.ev[4] = s->ev[5];
     P.stage_events = s->stage_events ? 1 : 0;
     return CULSH_OK;
 }
@@ -1401,20 +1466,12 @@ int enqueue_search(const SearchPlan& P, cudaStream_t st, bool capturing, int* la
         if (P.wa.order) CU_TRY(launch_order_queries(P.wa, st));
         CU_TRY(launch_plan_items(P.wa, st));
         CU_TRY(launch_candidates_ws(P.wa, P.ws_grid, st));
-        if (P.use_knn) {
-            CU_TRY(launch_cand_bitmap(P.wa, P.kbm, P.kn.nwp, P.dense_grid, st));
-            if (P.stage_events) CU_TRY(cudaEventRecordWithFlags(P.ev[4], st, evf));
-            CU_TRY(launch_knn_search(P.kn, st));
-        } else if (P.use_dense) {
-            CU_TRY(launch_candidates_dense(P.wa, P.dense_grid, st));
-        }
     } else {
         CU_TRY(launch_candidates(P.ca, st));
     }
     if (P.stage_events) CU_TRY(cudaEventRecordWithFlags(P.ev[3], st, evf));
     CU_TRY(cudaMemcpyAsync(P.h_stats, P.stats, 8 * kStatWords, cudaMemcpyDeviceToHost, st));
-    const int dense_launches = P.use_knn ? 1 + knn_launches(P.kn) : (P.use_dense ? 1 : 0);
-    *launches = (P.use_ws ? 3 + dense_launches + (P.wa.order ? 3 : 0) : 2) + probe_launches(P.pa);
+    *launches = (P.use_ws ? 3 + (P.wa.order ? 3 : 0) : 2) + probe_launches(P.pa);
     return CULSH_OK;
 }
 
@@ -1614,29 +1671,22 @@ int finish_search(culsh_search* s, const SearchPlan& P, cudaStream_t st) {
         s->deferred_queries = (int)ndef;
         TRY(rerun_queries(s, ca, std::move(dl), Q, st));
     }
-    s->tot_unique = s->h_stats.p[0];
-    s->tot_nonunique = s->h_stats.p[1];
     s->knn_queries = s->knn_fallback = s->bucket_rows = 0;
-    if (P.use_knn && !s->ws_overflow) {
-        if ((s->h_stats.p[11] & 0xffffffffu) != 0)
-            return fail(CULSH_ERR_DEVICE, "tensor-core k-NN: a bounded device wait gave up");
-        s->knn_queries = (int)(s->h_stats.p[7] & 0xffffffffu);
-        s->bucket_rows = P.wa.nbig;
-        // queries whose bound-form lists could not prove their top-K: the
-        // exact per-query kernel (their counts were taken already)
-        const unsigned int nfb = (unsigned int)(s->h_stats.p[10] & 0xffffffffu);
-        if (nfb) {
-            std::vector<int> fl(nfb);
-            CU_TRY(cudaMemcpyAsync(fl.data(), s->kfallback.p, 4 * (size_t)nfb, cudaMemcpyDeviceToHost, st));
+    const int nd = P.use_dense && !s->ws_overflow ? (int)(s->h_stats.p[7] & 0xffffffffu) : 0;
+    if (nd) {
+        bool left = false;
+        TRY(run_dense(s, P, nd, st, &left));
+        if (left) {   // extreme data in a set too large for the bitmap kernel
+            std::vector<int> dl(nd);
+            CU_TRY(cudaMemcpyAsync(dl.data(), s->dense_q.p, 4 * (size_t)nd, cudaMemcpyDeviceToHost, st));
             CU_TRY(cudaStreamSynchronize(st));
-            CandArgs cb = ca;
-            cb.totals = s->stats.p + 12;
-            TRY(rerun_queries(s, cb, std::move(fl), Q, st));
-            s->knn_fallback = (int)nfb;
+            TRY(rerun_queries(s, ca, std::move(dl), Q, st));
         }
     }
+    s->tot_unique = s->h_stats.p[0];
+    s->tot_nonunique = s->h_stats.p[1];
     s->rechecked = P.use_ws && P.wa.bf16 && !s->ws_overflow ? (long long)s->h_stats.p[6] : 0;
-    s->dense_queries = P.use_ws && P.use_dense && !s->ws_overflow ? (int)(s->h_stats.p[7] & 0xffffffffu) : 0;
+    s->dense_queries = nd;
     return CULSH_OK;
 }
 
@@ -2097,19 +2147,21 @@ long long culsh_search_device_bytes(culsh_search* s) {
     add(s->qorder);
     add(s->qorder_bins);
     add(s->kbm);
+    add(s->kbm_sample);
     add(s->kq_h);
-    add(s->kq_l);
-    add(s->kq_sq);
-    add(s->kq_base);
-    add(s->kq_bound);
-    add(s->kpart_key);
-    add(s->kpart_id);
+    add(s->kq_info);
+    add(s->kq_lim);
+    add(s->kw_sample);
+    add(s->ksmin);
+    add(s->kpart);
     add(s->kpart_n);
     add(s->kfallback);
     return (long long)b;
 }
 
-long long culsh_search_estimate_bytes(const culsh_index* ix, int Q, int K, int T) {
+} // extern "C"
+
+long long culsh::search_estimate(const culsh_index* ix, int Q, int K, int T, bool tensor_cores) {
     if (!ix || Q <= 0 || K <= 0 || T <= 0) return 0;
     const size_t L = ix->L, M = ix->M, q = (size_t)Q, k = (size_t)K;
     size_t b = 4 * L * M * q + 4 * L * q * (size_t)T + 8 * q + 8 * q + 64 + 8 * q + 4 * kArenaInitialWords;
@@ -2119,17 +2171,22 @@ long long culsh_search_estimate_bytes(const culsh_index* ix, int Q, int K, int T
     b += 16 * q + cap * per_item;   // per-query plan arrays, dense-query list, partial lists
     b += 4 * q + 4 * (kOrderBins + 1);   // locality order
     if (M <= 16) b += 12 * L * q * (size_t)T + 48 * L * q;   // split probe lookups
-    if (ix->D <= 128 && K <= kMaxKnnK) {
+    KnnSearch kn;
+    // one tensor-core CTA per SM, at most 160
+    if (tensor_cores && knn_shapes(ix, K, Q, 160, kKnnEstimateSmem, &kn)) {
         // tensor-core path for dense queries: membership rows, query rows,
-        // partial lists (at most 160 CTAs' list sets plus one per query tile)
-        const size_t qc = (q + 2 * kKnnTileQ - 1) / (2 * kKnnTileQ) * (2 * kKnnTileQ);
-        const size_t dp = ((size_t)ix->D + 63) / 64 * 64;
-        const size_t nwp = (((size_t)ix->N + 31) / 32 + 3) / 4 * 4;
-        const size_t lists = (160 + qc / kKnnTileQ) * 2 * kKnnTileQ;
-        const size_t bmb = 4 * qc * nwp;
-        if (bmb <= kKnnMaxBitmapBytes) b += bmb + 4 * qc * dp + 12 * qc + lists * (4 + 8 * (size_t)kMaxKnnK);
+        // sample, survivor lists
+        const size_t qc = kn.Qcap, nws = kn.nws;
+        b += 4 * qc * kn.nwp + 8 * qc * nws + 128 * nws + 2 * qc * kn.Dp + (sizeof(KnnQuery) + 8) * qc +
+             8 * knn_part_entries(kn) + 4 * knn_part_lists(kn);
     }
     return (long long)b;
+}
+
+extern "C" {
+
+long long culsh_search_estimate_bytes(const culsh_index* ix, int Q, int K, int T) {
+    return culsh::search_estimate(ix, Q, K, T, true);
 }
 
 int culsh_search_release(culsh_search* s) {
@@ -2161,13 +2218,13 @@ int culsh_search_release(culsh_search* s) {
     s->qorder.release();
     s->qorder_bins.release();
     s->kbm.release();
+    s->kbm_sample.release();
     s->kq_h.release();
-    s->kq_l.release();
-    s->kq_sq.release();
-    s->kq_base.release();
-    s->kq_bound.release();
-    s->kpart_key.release();
-    s->kpart_id.release();
+    s->kq_info.release();
+    s->kq_lim.release();
+    s->kw_sample.release();
+    s->ksmin.release();
+    s->kpart.release();
     s->kpart_n.release();
     s->kfallback.release();
     s->Q = 0;

@@ -379,7 +379,17 @@ struct WsArgs {
     const uint32_t* big_rows;          // [nbig][nwp]
     int nbig;
     uint32_t big_min;
+    // Bank lists (tensor-core path, one membership segment): the ids of every
+    // bucket of bank_min ids or more again, arranged for the membership kernel
+    // (k_bank_fill). bank_meta[g] of global bucket g: (groups of 128 entries,
+    // tail ids). nullptr: none.
+    const uint16_t* bank;
+    const uint32_t* bank_tail;
+    const uint2* bank_meta;
+    uint32_t bank_min;
 };
+constexpr uint32_t kBankMin = 512;            // smallest bucket that has a bank list
+constexpr int64_t kBankMaxN = (int64_t(1) << 21) - 1024;   // 11 bits of word row (one past the bitmap), 5 of bit
 constexpr int kOrderBins = 4096;
 cudaError_t launch_order_queries(const WsArgs& a, cudaStream_t st);   // 3 kernels + 1 memset
 size_t dense_smem_bytes(int64_t N, int D, int K);
@@ -396,82 +406,108 @@ cudaError_t launch_big_find(const uint32_t* sizes, uint64_t totB, uint32_t big_m
 cudaError_t launch_big_fill(const uint64_t* gi, const int32_t* tl, int nbig, const uint32_t* starts,
                             const uint32_t* sizes, const uint32_t* ids, int64_t N, uint32_t* rows, int nwp,
                             cudaStream_t st);
+// Bank lists of the n buckets gi (any order): see k_bank_fill.
+cudaError_t launch_bank_fill(const uint64_t* gi, const unsigned int* n, unsigned int cap, const uint64_t* boff, int L,
+                             const uint32_t* starts, const uint32_t* sizes, const uint32_t* ids, int64_t N,
+                             uint16_t* bank, uint32_t* tail, uint2* meta, cudaStream_t st);
 cudaError_t launch_candidates_ws(const WsArgs& a, int grid, cudaStream_t st);
 
 // ---------------------------------------------------------------------------
 // Tensor-core k-NN over candidate membership rows (knn_tc.cu): the dense
 // queries' candidate distances and top-K as a masked GEMM.
 
-// Properties of a set of rows (the dataset, or one search's dense queries),
-// accumulated by k_knn_rows. Zero is the empty state.
+// Properties of the dataset's values, accumulated by k_knn_scan and
+// k_knn_rows. Zero is the empty state.
 enum KnnFlags : int {
-    kKnnHasLo = 1,         // some value is not exact in bf16
     kKnnNotSmallInt = 2,   // some value is not an integer of magnitude <= 256
     kKnnNonFinite = 4,
 };
 struct KnnState {
     int flags;
-    int mneg;   // max over the small-integer values v of 257 - v (0: none)
-    int mpos;   // max over them of v + 257
-    int pad;
+    int mneg;        // max over the small-integer values v of 257 - v (0: none)
+    int mpos;        // max over them of v + 257
+    uint32_t amax;   // largest magnitude (float bits)
+    uint32_t rho;    // largest relative fp16 residual of a row (float bits)
 };
-constexpr int kMaxKnnK = 64;    // list length limit of the tensor-core k-NN path
-constexpr int kKnnTileQ = 128;  // queries per tensor-core tile
+// A dense query's key multipliers and error terms (knn_tc.cu).
+enum KnnQueryFlags : int {
+    kKnnExact = 1,   // small integers: keys are exact
+    kKnnUnfit = 2,   // magnitudes outside the tensor-core path: scanned exactly
+};
+struct KnnQuery {
+    float m_lo, m_up;     // of the lower- and upper-bound keys
+    float sq;             // |q|^2
+    float kappa, slack;
+    int flags;
+};
+constexpr int kMaxKnnK = 256;           // neighbours the tensor-core path serves
+constexpr int kMaxKnnD = 2048;          // dimensions
+constexpr int kKnnTileQ = 256;          // queries per tensor-core tile
+constexpr int kKnnMaxSurvivors = 4096;  // candidates of a query the merge takes
+constexpr int kKnnMaxChosen = 1024;     // of those, distances it computes
+// Magnitudes (largest of a row or of the dataset) outside which squares could
+// leave the float range.
+constexpr float kKnnMaxValue = 1e17f, kKnnMinValue = 1e-12f;
 
 // Everything the k-NN kernels of one search read and write.
 struct KnnSearch {
-    int N, D, Dp, K, Qcap;            // Qcap: rows of the query buffers (a multiple of 128)
+    int N, D, Dp, K;
+    int nd, Qcap;                      // dense queries; rows of the query buffers (nd rounded up to kKnnTileQ)
     int grid;                          // persistent CTAs of the tensor-core kernels
-    int exact_possible;                // dataset qualifies for the exact form (launch its kernel)
-    int kl_exact, kl_bound;            // list length per query (exact: K; bound: K + margin)
-    int ops_exact, ops_bound;          // point-tile ring stages per form
-    size_t smem_exact, smem_bound;     // dynamic shared memory per form
+    int ops;                           // operand ring stages
+    size_t smem;                       // dynamic shared memory of the tensor-core kernels
     int nwp;                           // membership words per query row (a multiple of 4)
-    float C;                           // bound-form factor (|d~ - d| <= C S)
+    // sample pass: every f-th point (0: none) of nseg segments of seg points,
+    // in s32 chunks of 32 each; chunk c of segment g holds the points
+    // g seg + (i s32 + c) f, i < 32
+    int f, nseg, seg, s32;
+    int nws;                           // sample membership words per query row
+    float gamma;
     // dataset side (per index)
-    const void* xh;                    // [N][Dp] bf16
-    const void* xl;                    // [N][Dp] bf16
-    const float* w_exact;              // [ntp256 * 256]: |x|^2, FLT_MAX past N
-    const float* w_bound;              // [ntp256 * 256]: |x|^2 - C |x|^2_up, FLT_MAX past N
+    const void* xh;                    // [N][Dp] fp16, scaled
+    const float* w;                    // [N padded to 256]: |x|^2, FLT_MAX past N
     const KnnState* dstate;
-    const float* X;                    // [N][D] f32 (the bound form's exact recomputation)
+    const float* X;                    // [N][D] f32 (exact distances)
     // query side (per search)
     const float* queries;              // [Q][D] f32
     const int* dense_q;                // dense list (query ids)
-    const unsigned int* n_dense;
-    void* qh;                          // [Qcap][Dp] bf16, dense-list order
-    void* ql;
-    float* qsq;                        // [Qcap]
-    float* qbase;                      // [Qcap]
-    KnnState* qstate;                  // cleared before the search
-    unsigned int* qbound;              // [Qcap] exact form: per-query shared key bound
+    void* qh;                          // [Qcap][Dp] fp16, dense-list order
+    KnnQuery* qinfo;                   // [Qcap]
+    float* qlim;                       // [Qcap]
+    float* w_sample;                   // [nws * 32]
+    float* smin;                       // [Qcap][nws] chunk minima
     const uint32_t* bm;                // [Qcap][nwp] membership rows (k_cand_bitmap)
-    float* part_key;                   // partial lists, see k_knn_tc
-    uint32_t* part_id;
+    uint32_t* bm_sample;               // [Qcap][nws] their sample points
+    uint2* part;                       // survivor lists, list_cap entries each
     int* part_n;
+    int list_cap;
     int32_t* out_ids;
     float* out_d;
-    int* fallback;                     // [Qcap] queries the bound form could not prove
+    int* fallback;                     // [Qcap] dense positions to scan exactly
     unsigned int* n_fallback;
     int* err;
 };
 // Buffer sizes of one search (elements).
-size_t knn_part_entries(const KnnSearch& k);   // part_key / part_id entries
+size_t knn_part_entries(const KnnSearch& k);   // part entries
 size_t knn_part_lists(const KnnSearch& k);     // part_n entries
-// Plans the shared memory and stages of both forms for D, K on this device;
-// false when the tensor-core path cannot serve them (D > 128, K too large).
-bool knn_plan(KnnSearch& k, int max_smem);
-// The bound-form factor C for dimension D (see knn_tc.cu).
-float knn_bound_factor(int D);
-// Dataset rows: bf16 parts, weights, flags (once per index).
-cudaError_t launch_knn_rows_dataset(const float* X, int64_t N, int D, int Dp, void* xh, void* xl, float* w_exact,
-                                    float* w_bound, int64_t pad, float C, KnnState* st, cudaStream_t s);
-// Query rows, tensor-core kernels and merge of one search (3 or 4 launches).
+// Plans shared memory, sample and list sizes for N, D, K, Qcap and grid; false
+// when the tensor-core path does not serve them. bitmap_smem: shared memory
+// the membership kernel may use for its bitmap.
+bool knn_plan(KnnSearch& k, int max_smem, size_t bitmap_smem);
+// Relative error terms beside the operand residuals (see knn_tc.cu).
+float knn_gamma(int D);
+// Dataset rows: fp16 operand, norms, state (once per index).
+cudaError_t launch_knn_rows_dataset(const float* X, int64_t N, int D, int Dp, void* xh, float* w, int64_t pad,
+                                    KnnState* st, cudaStream_t s);
+// Query rows, tensor-core passes and merge of one search.
 cudaError_t launch_knn_search(const KnnSearch& k, cudaStream_t s);
 int knn_launches(const KnnSearch& k);
-// Membership rows of the dense queries (candidates.cu).
-size_t bitmap_smem_bytes(int64_t N);
-cudaError_t launch_cand_bitmap(const WsArgs& a, uint32_t* bm, int nwp, int grid, cudaStream_t st);
+// Membership rows of the dense queries, and the exact scan of the queries the
+// merge could not finish (candidates.cu).
+size_t bitmap_smem(int max_smem);   // bytes of bits a membership block can hold
+cudaError_t launch_cand_bitmap(const WsArgs& a, const KnnSearch& k, uint32_t* bm, int grid, cudaStream_t st);
+cudaError_t launch_knn_scan_rows(const KnnSearch& k, int grid, cudaStream_t st);
+size_t knn_scan_smem(int D, int K);
 
 // Opts `func` into `dyn` bytes of dynamic shared memory when static plus
 // dynamic shared memory could pass the 48 KB default (the kernels here keep
@@ -491,6 +527,8 @@ cudaError_t opt_in_smem(F* func, size_t dyn, std::atomic<size_t>& cap) {
 // Process-wide lock held while a search plans (and grows) its buffers and
 // captures its graph: no thread frees device memory while another captures.
 std::mutex& alloc_capture_mutex();
+// culsh_search_estimate_bytes, with or without the tensor-core path's buffers.
+long long search_estimate(const culsh_index* ix, int Q, int K, int T, bool tensor_cores);
 // Sets the calling thread's culsh_last_error() message; returns code.
 int set_last_error(int code, const char* msg);
 

@@ -8,51 +8,61 @@
 // path: the same ids and bit-identical squared distances.
 //
 // Formulation. A query's candidates are marked in an N-bit membership row
-// (k_cand_bitmap, candidates.cu). A tile of 128 queries is multiplied with
-// every 256- (or 128-) point tile of the dataset by tcgen05.mma
-// (q . x in FP32 accumulators in TMEM, bf16 operands staged by TMA), and the
-// epilogue turns each accumulator into a ranking key
-//     t = w_x - 2 q.x,     w_x = |x|^2 (exact form) or |x|^2 - C S_x (bound form)
-// so that d = t + |q|^2 (exact form) or t + |q|^2 - C S_q <= d (bound form).
-// Each query keeps the Kl smallest keys among its candidates (membership
-// bit set) in shared memory; a chunk of 32 columns is only examined when its
-// smallest key beats the query's current Kl-th key.
+// (k_cand_bitmap, candidates.cu). Tiles of 256 queries are multiplied with
+// tiles of 128 points by tcgen05.mma: fp16 operands (each query row and the
+// dataset scaled by a power of two), FP32 accumulators in TMEM, operands
+// staged by TMA. The epilogue turns each accumulator into a key
+//     t = |x|^2 + m q.x       (m = -2 / scales, per query)
+// and three steps use the keys:
+//  1. Sample pass: over every f-th point (f <= 16), the smallest key among
+//     the candidates of each 32-point chunk. The K-th smallest of a query's
+//     chunk minima belongs to K different candidates, so the upper end of its
+//     error interval bounds the K-th distance from above (k_knn_limit).
+//  2. Full pass: every candidate whose certified lower bound does not exceed
+//     that limit is appended to the list of its (CTA, column slice, query)
+//     in global memory. About f K candidates of a query survive, so the
+//     epilogue is one comparison of a 32-column minimum almost everywhere.
+//  3. Merge: the survivors of a query are cut at the K-th smallest key, the
+//     exact FP32 lane-order distances of those K and of whatever their largest
+//     distance does not exclude are computed, and (distance, id) sorted.
+// A query whose survivors outgrow their lists is scanned exactly from its
+// membership row (k_knn_scan_rows, candidates.cu).
 //
-//  * Exact form: every coordinate of the dataset and the queries is an
-//    integer with |v| <= 256 (exact in bf16), and D max|v|^2 < 2^24 and
-//    D (max v - min v)^2 < 2^24. Every product, partial sum and norm is then an
-//    integer below 2^24, so the tensor-core sum is exact in any order, t is
-//    exact, and d = t + |q|^2 is the exact squared distance, which is also
-//    what the reference's FP32 lane order computes (all of its partial sums
-//    are exact too). One bf16 product per element.
-//  * Bound form (any finite data): q = qh + ql, x = xh + xl split into bf16
-//    parts; the tensor cores sum qh.xh + qh.xl + ql.xh. With S = |q|^2 + |x|^2
-//    (upper bounds), |d~ - d| <= C S covers the split residue, the
-//    accumulation, the norms and the FP32 lane order of the exact distance,
-//    so key + base is a lower bound of the exact distance. The merge kernel
-//    recomputes the exact FP32 lane-order distance of the listed candidates
-//    in ascending bound order and stops once the bound passes the K-th exact
-//    distance. A query whose full list's largest bound does not exceed its
-//    K-th exact distance (the list was too short to prove the result) is
-//    re-run by the exact per-query kernel.
+// Error interval. With |q - qh| <= r_q, |x - xh| <= rho |x| + a for every row
+// (measured when the rows are converted), g the accumulation, norm and
+// lane-order terms (knn_gamma) and 2 |q| |x| <= |q|^2 + |x|^2 = S, the exact
+// FP32 distance d differs from |x|^2 - 2 qh.xh + |q|^2 by at most kappa S + e,
+// kappa = 1.01 (r_q / |q| + rho) + g and e = 2.02 |q| a. Since the bound is
+// linear in |x|^2 it is folded into m:
+//     d >= (1 - kappa) (|x|^2 + m_lo q.x + |q|^2) - e,  m_lo = -2 / (1 - kappa)
+//     d <= (1 + kappa) (|x|^2 + m_up q.x + |q|^2) + e,  m_up = -2 / (1 + kappa)
+// One fp16 product per element bounds d to about 2^-11 S; a split into two
+// bf16 parts and three products (2^-13 S), with sorted lists kept in the
+// epilogue, was the earlier form: 8.8 ms against 2.6 + 0.2 ms (both passes) at
+// 9,973 queries, 1M x 100.
+// Queries and datasets of small integers (|v| <= 256, D max|v|^2 < 2^24 and
+// D (max v - min v)^2 < 2^24) have kappa = e = 0: every product, partial sum
+// and norm is an integer below 2^24, the key plus |q|^2 is the exact distance
+// and no row is read again.
 //
 // Work split: the (query tile, point tile) pairs are cut into gridDim.x
 // contiguous ranges, one per persistent CTA, so that every CTA does the same
 // number of tensor-core tiles. A CTA's range covers part of one or a few
-// query tiles; for each it leaves one partial list per query (list set
-// blockIdx.x + query tile, unique because the ranges are ordered), which the
-// merge kernel combines.
+// query tiles; for each it leaves one list per query and column slice (list
+// set blockIdx.x + query tile, unique because the ranges are ordered), which
+// the merge kernel combines.
 //
-// Roles: warp 0 issues TMA loads (the query tile's operand once per query
-// tile, point tiles into a ring, membership words and per-point weights into
-// a second ring); warp 1 owns TMEM and issues tcgen05.mma (M = 128, N = the
-// point tile, K = 16 per instruction) into two accumulators, so that the
-// epilogue of one tile overlaps the products of the next; the other warps read
-// TMEM with tcgen05.ld and keep the per-query lists. Every mbarrier wait is
-// bounded: on timeout the kernel raises kErrSpin, drains its copies and
-// products, frees TMEM and returns; the host then reports the error.
+// Roles: warp 0 issues TMA loads (point tiles into a ring of 64-column slabs,
+// membership words and point norms into a second ring; the query tile once
+// per query tile for D <= 128, otherwise slab by slab beside the points);
+// warp 1 owns TMEM and issues tcgen05.mma (M = 128 twice, N = 128, K = 16
+// per instruction) into two accumulator sets, so that the epilogue of one tile
+// overlaps the products of the next; the other sixteen warps read TMEM with
+// tcgen05.ld. Every mbarrier wait is bounded: on timeout the kernel raises
+// kErrSpin, drains its copies and products, frees TMEM and returns; the host
+// then reports the error.
 #include <cuda.h>
-#include <cuda_bf16.h>
+#include <cuda_fp16.h>
 
 #include <algorithm>
 #include <atomic>
@@ -69,11 +79,23 @@ namespace culsh {
 namespace {
 
 constexpr int KM = 128;                 // rows of one MMA (TMEM lanes)
-// Tile shapes: MQ queries (MQ / 128 MMAs of M = 128) x BN points per tile,
-// NEPI epilogue warps, NCH = 32 NEPI / MQ column slices of 64 per query.
-constexpr int kBnExact = 128, kMqExact = 256, kNepiExact = 16;   // exact form: two MMAs share a point tile
-constexpr int kBnBound = 128, kMqBound = 128, kNepiBound = 8;    // bound form: three products per element
-constexpr int kNchExact = 32 * kNepiExact / kMqExact, kNchBound = 32 * kNepiBound / kMqBound;
+constexpr int MQ = kKnnTileQ;           // queries per tile: two MMAs share a point tile
+constexpr int BN = 128;                 // points per tile
+constexpr int MH = MQ / KM;
+constexpr int MW = MH;                  // MMA warps, one per half of the query tile
+constexpr int NEPI = 16;                // epilogue warps
+constexpr int kKnnThreads = 32 * (1 + MW + NEPI);
+constexpr int NT = 32 * NEPI;           // one (query, accumulator set) each
+constexpr int NCH = NT / MQ;            // warp groups: one per accumulator set, alternating tiles
+constexpr int BW = BN / 32;             // membership words per query row and point tile
+constexpr uint32_t kXSlab = (uint32_t)BN * 128;   // bytes of 64 columns of a point tile
+constexpr uint32_t kQSlab = (uint32_t)MQ * 128;   // ... of a query tile
+constexpr uint32_t kBmBytes = (uint32_t)MQ * BW * 4, kWBytes = (uint32_t)BN * 4;
+constexpr uint32_t kEpStride = kBmBytes + kWBytes;
+constexpr int kEpStages = 4;            // membership / norm ring stages
+constexpr int kMaxOpStages = 6;         // operand ring stages
+constexpr int kResidentD = 128;         // query tile kept in shared memory up to this dimension
+static_assert(NCH * MQ == NT && NCH == 2, "one warp group, and one list per query, per accumulator set");
 // Bounded waits: each poll suspends the thread in hardware for up to
 // kKnnSuspendNs (it resumes as soon as the phase completes, and takes no issue
 // slots meanwhile), at most kKnnPoll polls (a few seconds) in all.
@@ -101,9 +123,19 @@ __device__ __forceinline__ bool bar_try_wait(uint64_t* bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
+__device__ __forceinline__ bool bar_test(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(ok)
+        : "r"(smem_addr(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
 // Bounded wait for the phase of the given parity; on timeout raises the
 // block's abort flag and kErrSpin.
 __device__ __forceinline__ bool bar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* err) {
+    if (bar_test(bar, parity)) return true;
     for (uint32_t i = 0; i < kKnnPoll; ++i) {
         if (bar_try_wait(bar, parity)) return true;
         if (*abort_flag) return false;
@@ -126,6 +158,13 @@ __device__ __forceinline__ void tma_2d(void* dst, const CUtensorMap* map, uint64
         "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_addr(bar)), "r"(x), "r"(y)
         : "memory");
 }
+__device__ __forceinline__ void tma_4d(void* dst, const CUtensorMap* map, uint64_t* bar, int x, int y, int z, int w) {
+    asm volatile(
+        "cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], "
+        "[%2];" ::"r"(smem_addr(dst)),
+        "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_addr(bar)), "r"(x), "r"(y), "r"(z), "r"(w)
+        : "memory");
+}
 __device__ __forceinline__ void bulk_copy(void* dst, const void* src, uint32_t bytes, uint64_t* bar) {
     asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
                      smem_addr(dst)),
@@ -138,7 +177,7 @@ __device__ __forceinline__ uint64_t desc_sw128(uint32_t saddr) {
     return (uint64_t)((saddr >> 4) & 0x3FFFu) | ((uint64_t)1 << 16) | ((uint64_t)(1024 >> 4) << 32) |
            ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
-__device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+__device__ __forceinline__ void mma_f16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                          uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(
@@ -150,38 +189,40 @@ __device__ __forceinline__ void mma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_addr(bar))
                  : "memory");
 }
+// One lane of the (converged) warp, the same on every call.
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(p));
+    return p != 0;
+}
 __device__ __forceinline__ void fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
-// The 32 accumulator columns [taddr, taddr + 32) of this thread's TMEM lane,
-// loaded and waited for in one statement, so that no use of r can be
-// scheduled before the wait.
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, "
-        "%15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];\n\t"
-        "tcgen05.wait::ld.sync.aligned;"
-        : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]),
-          "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]),
-          "=r"(r[17]), "=r"(r[18]), "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-          "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]), "=r"(r[31])
-        : "r"(taddr)
-        : "memory");
+// Starts loading the 16 accumulator columns [taddr, taddr + 16) of this
+// thread's TMEM lane; r holds them after tmem_wait16.
+__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
+                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+                 : "r"(taddr)
+                 : "memory");
+}
+// Waits for this thread's TMEM loads; the values pass through the statement,
+// so that no use of them can be scheduled before it.
+__device__ __forceinline__ void tmem_wait16(uint32_t (&r)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;" : "+r"(r[0]), "+r"(r[1]), "+r"(r[2]), "+r"(r[3]), "+r"(r[4]), "+r"(r[5]), "+r"(r[6]), "+r"(r[7]), "+r"(r[8]), "+r"(r[9]), "+r"(r[10]), "+r"(r[11]), "+r"(r[12]), "+r"(r[13]), "+r"(r[14]), "+r"(r[15])::"memory");
 }
 
-// Element k (0..31) of 32 register values, by a tree of selects on k's bits
+// Element k (0..15) of 16 register values, by a tree of selects on k's bits
 // (no local memory).
-__device__ __forceinline__ float select32(const uint32_t* v, int k) {
-    float a[16];
+__device__ __forceinline__ float select16(const uint32_t (&v)[16], int k) {
+    float a[8];
 #pragma unroll
-    for (int i = 0; i < 16; ++i) a[i] = __uint_as_float((k & 1) ? v[2 * i + 1] : v[2 * i]);
+    for (int i = 0; i < 8; ++i) a[i] = __uint_as_float((k & 1) ? v[2 * i + 1] : v[2 * i]);
 #pragma unroll
-    for (int i = 0; i < 8; ++i) a[i] = (k & 2) ? a[2 * i + 1] : a[2 * i];
+    for (int i = 0; i < 4; ++i) a[i] = (k & 2) ? a[2 * i + 1] : a[2 * i];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) a[i] = (k & 4) ? a[2 * i + 1] : a[2 * i];
-#pragma unroll
-    for (int i = 0; i < 2; ++i) a[i] = (k & 8) ? a[2 * i + 1] : a[2 * i];
-    return (k & 16) ? a[1] : a[0];
+    for (int i = 0; i < 2; ++i) a[i] = (k & 4) ? a[2 * i + 1] : a[2 * i];
+    return (k & 8) ? a[1] : a[0];
 }
 
 // Three-input minimum (sm_100 and later).
@@ -191,44 +232,28 @@ __device__ __forceinline__ float fmin3(float a, float b, float c) {
     return d;
 }
 
-// Order-preserving encoding of a float key as an unsigned word (unsigned
-// comparison of encodings = float comparison of keys), so that a shared bound
-// can be lowered with atomicMin.
-__host__ __device__ __forceinline__ uint32_t key_enc(float f) {
-    uint32_t u;
-    memcpy(&u, &f, 4);
+// Order-preserving encoding of a float key as an unsigned word.
+__device__ __forceinline__ uint32_t key_enc(float f) {
+    const uint32_t u = __float_as_uint(f);
     return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
 }
 __device__ __forceinline__ float key_dec(uint32_t e) {
     return __uint_as_float((e & 0x80000000u) ? (e & 0x7FFFFFFFu) : ~e);
 }
-constexpr uint32_t kNoBound = 0xFF800000u;   // key_enc(+infinity)
-
-// Exact form of the search (see the file comment), from the flags and value
-// ranges of the dataset and of the dense queries.
-__device__ __forceinline__ bool exact_form(const KnnState* ds, const KnnState* qs, int D) {
-    if ((ds->flags | qs->flags) & (kKnnNotSmallInt | kKnnNonFinite)) return false;
-    const int mneg = max(ds->mneg, qs->mneg), mpos = max(ds->mpos, qs->mpos);
-    if (mneg == 0 || mpos == 0) return false;
-    const long long lo = 257 - mneg, hi = mpos - 257;
-    const long long mag = max(-lo, hi);
-    return (long long)D * mag * mag < (1ll << 24) && (long long)D * (hi - lo) * (hi - lo) < (1ll << 24);
-}
 
 struct KnnArgs {
-    int N, D, Dp;
-    int exact_launched;               // the exact form's kernel is part of this search
-    long long ntp_exact, ntp_bound;   // point tiles of 256 / 128
-    int kl_exact, kl_bound;
-    int op_stages, ep_stages;
-    const unsigned int* n_dense;
-    const KnnState* dstate;
-    const KnnState* qstate;
-    unsigned int* qbound;             // [dense position] shared key bound of the exact form (key_enc)
-    const float* w_exact;
-    const float* w_bound;
-    float* part_key;
-    uint32_t* part_id;
+    int Dp;
+    long long ntp;                    // point tiles of this pass
+    int op_stages;
+    int s32;                          // sample pass: chunks per segment
+    unsigned int nd;                  // dense queries
+    const KnnQuery* qinfo;            // [dense position]
+    const float* qlim;                // [dense position] key limit of the full pass
+    const float* w;                   // |x|^2 of the pass's points, FLT_MAX past the last
+    float* smin;                      // sample pass: [Qcap][nws] smallest member key of each chunk
+    int nws;
+    uint2* part;                      // full pass: lists of (key, id), list_cap each
+    int list_cap;
     int* part_n;
     int* err;
 };
@@ -239,77 +264,62 @@ __device__ __forceinline__ int owner_cta(long long p, long long U, int G) {
     return (int)(((p + 1) * G - 1) / U);
 }
 
-// MQ queries per tile (MQ / 128 MMAs of M = 128 share each point tile of BN
-// points), NEPI epilogue warps: each lane keeps one query's list over one of
-// the NCH column slices of the tile (32 * NEPI == MQ * NCH).
-template <int BN, int MQ, int NEPI, bool kExact>
-__global__ void __launch_bounds__(64 + 32 * NEPI, 1)
-    k_knn_tc(const __grid_constant__ CUtensorMap tm_qh, const __grid_constant__ CUtensorMap tm_ql,
-             const __grid_constant__ CUtensorMap tm_xh, const __grid_constant__ CUtensorMap tm_xl,
+// kSample: the sample pass (chunk minima), else the full pass (lists).
+// kStream: D > kResidentD, query slabs travel with the point slabs.
+template <bool kSample, bool kStream>
+__global__ void __launch_bounds__(kKnnThreads, 1)
+    k_knn_tc(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_x,
              const __grid_constant__ CUtensorMap tm_bm, KnnArgs a) {
-    constexpr int NT = 32 * NEPI;          // list-keeping threads: one (query, column slice) each
-    constexpr int MH = MQ / KM;            // M = 128 halves of the query tile
-    constexpr int NCH = NT / MQ;           // column slices of a tile
-    constexpr int CW = BN / NCH;           // columns per slice
-    constexpr int BW = BN / 32;            // membership words per query row and point tile
     constexpr uint32_t kTmemCols = 2 * MH * BN;
-    static_assert(NCH * MQ == NT && CW == 64, "64-column slices, one list per (query, slice)");
-    // the other form's kernel runs (the exact one only where it was launched)
-    if ((a.exact_launched && exact_form(a.dstate, a.qstate, a.D)) != kExact) return;
-    const unsigned int nd = *a.n_dense;
+    const unsigned int nd = a.nd;
     const long long nqt = ((long long)nd + MQ - 1) / MQ;
-    const long long ntp = kExact ? a.ntp_exact : a.ntp_bound;
+    const long long ntp = a.ntp;
     const long long U = nqt * ntp;
     const int G = (int)min((long long)gridDim.x, U);
     if ((int)blockIdx.x >= G) return;
     const long long p0 = (long long)blockIdx.x * U / G, p1 = (long long)(blockIdx.x + 1) * U / G;
-    const int Dp = a.Dp, atoms = Dp / 64, ksteps = Dp / 16;
-    const int Kl = kExact ? a.kl_exact : a.kl_bound;
-    const int ops = a.op_stages, eps = a.ep_stages;
-    const int need_xl = kExact ? 0 : ((a.dstate->flags & kKnnHasLo) != 0);
-    const int need_ql = kExact ? 0 : ((a.qstate->flags & kKnnHasLo) != 0);
+    const int atoms = a.Dp / 64;
+    const int apst = kStream ? 1 : atoms;   // 64-column slabs per operand stage
+    const int nst = kStream ? atoms : 1;    // operand stages per tile
+    const int ops = a.op_stages;
 
     extern __shared__ __align__(1024) unsigned char smraw[];
     unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smraw) + 1023) & ~uintptr_t(1023));
-    const uint32_t qbytes = (uint32_t)MQ * Dp * 2, xbytes = (uint32_t)BN * Dp * 2;
-    unsigned char* sQh = base;
-    unsigned char* sQl = sQh + qbytes;                                  // bound form only
-    unsigned char* sX = sQh + (kExact ? 1u : 2u) * qbytes;             // op ring: [xh][xl] per stage
-    const uint32_t op_stride = (kExact ? 1u : 2u) * xbytes;
-    unsigned char* sE = sX + (size_t)ops * op_stride;                  // ep ring: [membership][weights] per stage
-    const uint32_t bm_bytes = (uint32_t)MQ * BW * 4, w_bytes = (uint32_t)BN * 4;
-    const uint32_t ep_stride = bm_bytes + w_bytes;
-    float* lkey = reinterpret_cast<float*>(sE + (size_t)eps * ep_stride);   // [Kl][NT]
-    uint32_t* lid = reinterpret_cast<uint32_t*>(lkey + (size_t)Kl * NT);
-    uint64_t* bars = reinterpret_cast<uint64_t*>(lid + (size_t)Kl * NT);
+    unsigned char* sQ = base;                                                  // resident query tile
+    unsigned char* sOp = sQ + (kStream ? 0u : (uint32_t)atoms * kQSlab);       // ring: [points][queries if streamed]
+    const uint32_t xbytes = (uint32_t)apst * kXSlab;
+    const uint32_t op_stride = xbytes + (kStream ? kQSlab : 0u);
+    unsigned char* sE = sOp + (size_t)ops * op_stride;                         // ring: [membership][norms]
+    uint64_t* bars = reinterpret_cast<uint64_t*>(sE + (size_t)kEpStages * kEpStride);
     uint64_t* a_full = bars;
     uint64_t* a_empty = bars + 1;
-    uint64_t* tfull = bars + 2;     // [2]
-    uint64_t* tempty = bars + 4;    // [2]
-    uint64_t* done_bar = bars + 6;
-    uint64_t* full_op = bars + 7;             // [ops]
-    uint64_t* empty_op = full_op + ops;       // [ops]
-    uint64_t* full_ep = empty_op + ops;       // [eps]
-    uint64_t* empty_ep = full_ep + eps;       // [eps]
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(empty_ep + eps);
+    uint64_t* tfull = bars + 2;                      // [accumulator set][half]
+    uint64_t* tempty = tfull + 2 * MH;               // [accumulator set][half]
+    uint64_t* done_bar = tempty + 2 * MH;
+    uint64_t* full_op = done_bar + 1;                // [ops]
+    uint64_t* empty_op = full_op + ops;              // [ops]
+    uint64_t* full_ep = empty_op + ops;              // [kEpStages]
+    uint64_t* empty_ep = full_ep + kEpStages;        // [kEpStages]
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(empty_ep + kEpStages);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // known to be warp-uniform
     if (tid == 0) {
         bar_init(a_full, 1);
-        bar_init(a_empty, 1);
-        for (int s = 0; s < 2; ++s) {
+        bar_init(a_empty, MW);
+        for (int s = 0; s < 2 * MH; ++s) {
             bar_init(tfull + s, 1);
-            bar_init(tempty + s, NEPI);
+            bar_init(tempty + s, KM / 32);
         }
-        bar_init(done_bar, 1);
+        bar_init(done_bar, MW);
         for (int s = 0; s < ops; ++s) {
             bar_init(full_op + s, 1);
-            bar_init(empty_op + s, 1);
+            bar_init(empty_op + s, MW);
         }
-        for (int s = 0; s < eps; ++s) {
+        for (int s = 0; s < kEpStages; ++s) {
             bar_init(full_ep + s, 1);
-            bar_init(empty_ep + s, NEPI);
+            bar_init(empty_ep + s, NEPI / NCH);
         }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -329,40 +339,60 @@ __global__ void __launch_bounds__(64 + 32 * NEPI, 1)
         // ---- TMA producer ----
         long long cur_qt = -1;
         int j = -1;
-        long long i = 0;
-        // (query tile, point tile) of pair p and both rings' stage and round
-        // parity, advanced incrementally (no 64-bit division per tile)
+        // (query tile, point tile) and both rings' stage and round parity,
+        // advanced incrementally (no 64-bit division per tile)
         long long qt = p0 / ntp, pt = p0 - qt * ntp;
         int s = 0, e = 0;
         uint32_t spar = 0, epar = 0;
         long long issued_op = 0, issued_ep = 0;   // copies issued into each ring
-        for (long long p = p0; p < p1 && !*abort_flag; ++p, ++i) {
-            if (qt != cur_qt) {
+        bool ok = true;
+        for (long long p = p0; p < p1 && ok && !*abort_flag; ++p) {
+            if (!kStream && qt != cur_qt) {
                 ++j;
                 cur_qt = qt;
                 if (j >= 1 && !bar_wait(a_empty, (uint32_t)((j - 1) & 1), abort_flag, a.err)) break;
-                bar_expect_tx(a_full, qbytes * (need_ql ? 2u : 1u));
-                for (int k = 0; k < atoms; ++k) {
-                    tma_2d(sQh + (size_t)k * MQ * 128, &tm_qh, a_full, k * 64, (int)(qt * MQ));
-                    if (need_ql) tma_2d(sQl + (size_t)k * MQ * 128, &tm_ql, a_full, k * 64, (int)(qt * MQ));
+                bar_expect_tx(a_full, (uint32_t)atoms * kQSlab);
+                for (int k = 0; k < atoms; ++k)
+                    tma_2d(sQ + (size_t)k * kQSlab, &tm_q, a_full, k * 64, (int)(qt * MQ));
+            }
+            for (int sl = 0; sl < nst; ++sl) {
+                if (issued_op >= ops && !bar_wait(empty_op + s, spar ^ 1u, abort_flag, a.err)) {
+                    ok = false;
+                    break;
+                }
+                unsigned char* xs = sOp + (size_t)s * op_stride;
+                bar_expect_tx(full_op + s, op_stride);
+                for (int k = 0; k < apst; ++k) {
+                    const int col = (sl * apst + k) * 64;
+                    if constexpr (kSample) {
+                        // a tile is four chunks of 32 sample points
+#pragma unroll
+                        for (int i = 0; i < BN / 32; ++i) {
+                            const int c = (int)(pt * (BN / 32)) + i;
+                            const int seg = c / a.s32;
+                            tma_4d(xs + (size_t)k * kXSlab + i * 32 * 128, &tm_x, full_op + s, col, c - seg * a.s32, 0,
+                                   seg);
+                        }
+                    } else {
+                        tma_2d(xs + (size_t)k * kXSlab, &tm_x, full_op + s, col, (int)(pt * BN));
+                    }
+                }
+                if constexpr (kStream) tma_2d(xs + xbytes, &tm_q, full_op + s, sl * 64, (int)(qt * MQ));
+                ++issued_op;
+                if (++s == ops) { s = 0; spar ^= 1u; }
+                if (sl == 0) {
+                    if (issued_ep >= kEpStages && !bar_wait(empty_ep + e, epar ^ 1u, abort_flag, a.err)) {
+                        ok = false;
+                        break;
+                    }
+                    unsigned char* es = sE + (size_t)e * kEpStride;
+                    bar_expect_tx(full_ep + e, kEpStride);
+                    tma_2d(es, &tm_bm, full_ep + e, (int)(pt * BW), (int)(qt * MQ));
+                    bulk_copy(es + kBmBytes, a.w + pt * BN, kWBytes, full_ep + e);
+                    ++issued_ep;
+                    if (++e == kEpStages) { e = 0; epar ^= 1u; }
                 }
             }
-            if (i >= ops && !bar_wait(empty_op + s, spar ^ 1u, abort_flag, a.err)) break;
-            unsigned char* xs = sX + (size_t)s * op_stride;
-            bar_expect_tx(full_op + s, xbytes * (need_xl ? 2u : 1u));
-            for (int k = 0; k < atoms; ++k) {
-                tma_2d(xs + (size_t)k * BN * 128, &tm_xh, full_op + s, k * 64, (int)(pt * BN));
-                if (need_xl) tma_2d(xs + xbytes + (size_t)k * BN * 128, &tm_xl, full_op + s, k * 64, (int)(pt * BN));
-            }
-            ++issued_op;
-            if (i >= eps && !bar_wait(empty_ep + e, epar ^ 1u, abort_flag, a.err)) break;
-            unsigned char* es = sE + (size_t)e * ep_stride;
-            bar_expect_tx(full_ep + e, ep_stride);
-            tma_2d(es, &tm_bm, full_ep + e, (int)(pt * BW), (int)(qt * MQ));
-            bulk_copy(es + bm_bytes, (kExact ? a.w_exact : a.w_bound) + pt * BN, w_bytes, full_ep + e);
-            ++issued_ep;
-            if (++s == ops) { s = 0; spar ^= 1u; }
-            if (++e == eps) { e = 0; epar ^= 1u; }
             if (++pt == ntp) { pt = 0; ++qt; }
         }
         // Drain: every copy issued into a ring stage completes before exit.
@@ -370,377 +400,665 @@ __global__ void __launch_bounds__(64 + 32 * NEPI, 1)
             const long long last = st + ((issued_op - 1 - st) / ops) * ops;
             bar_drain(full_op + st, (uint32_t)((last / ops) & 1), a.err);
         }
-        for (int et = 0; et < eps && et < issued_ep; ++et) {
-            const long long last = et + ((issued_ep - 1 - et) / eps) * eps;
-            bar_drain(full_ep + et, (uint32_t)((last / eps) & 1), a.err);
+        for (int et = 0; et < kEpStages && et < issued_ep; ++et) {
+            const long long last = et + ((issued_ep - 1 - et) / kEpStages) * kEpStages;
+            bar_drain(full_ep + et, (uint32_t)((last / kEpStages) & 1), a.err);
         }
         if (j >= 0) bar_drain(a_full, (uint32_t)(j & 1), a.err);
-    } else if (warp == 1 && lane == 0) {
-        // ---- MMA issuer ----
-        // kind::f16: FP32 accumulator, bf16 A and B, both K-major, N = BN, M = 128.
-        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(BN >> 3) << 17) |
-                               ((uint32_t)(KM >> 4) << 24);
-        const uint64_t qhdesc = desc_sw128(smem_addr(sQh)), qldesc = desc_sw128(smem_addr(sQl));
-        const uint64_t xdesc = desc_sw128(smem_addr(sX));
+    } else if (warp >= 1 && warp <= MW) {
+        // ---- MMA issuers ----
+        // One warp per half of the query tile: while one waits for a barrier
+        // (a few hundred cycles even for a completed phase) the other's
+        // products keep the tensor pipe busy. The whole warp walks the loop, so
+        // that descriptors and counters are warp-uniform values; one elected
+        // lane issues (a loop run by one lane alone moved every descriptor
+        // through vector registers and issued one product in 178 cycles; the
+        // pipe takes 64).
+        // kind::f16: FP32 accumulator, fp16 A and B, both K-major, N = BN, M = 128.
+        const int hq = warp - 1;
+        const uint32_t idesc = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(KM >> 4) << 24);
+        const uint64_t qdesc = desc_sw128(smem_addr(kStream ? sOp + xbytes : sQ) + (uint32_t)(hq * KM * 128));
+        const uint64_t xdesc = desc_sw128(smem_addr(sOp));
+        const bool leader = elect_one();
         long long cur_qt = -1;
         int j = -1;
         long long i = 0;
         long long qt = p0 / ntp, pt = p0 - qt * ntp;
         int s = 0;
         uint32_t spar = 0;
-        for (long long p = p0; p < p1; ++p, ++i) {
-            if (qt != cur_qt) {
-                if (j >= 0) mma_commit(a_empty);
+        bool ok = true;
+        for (long long p = p0; p < p1 && ok; ++p, ++i) {
+            if (!kStream && qt != cur_qt) {
+                if (j >= 0 && leader) mma_commit(a_empty);
                 ++j;
                 cur_qt = qt;
-                if (!bar_wait(a_full, (uint32_t)(j & 1), abort_flag, a.err)) break;
+                ok = __all_sync(0xffffffffu, bar_wait(a_full, (uint32_t)(j & 1), abort_flag, a.err));
+                if (!ok) break;
             }
+            const bool work = qt * MQ + hq * KM < (long long)nd;   // a half without queries is left out
             if (++pt == ntp) { pt = 0; ++qt; }
             const int acc = (int)(i & 1);
-            if (i >= 2 && !bar_wait(tempty + acc, (uint32_t)(((i >> 1) - 1) & 1), abort_flag, a.err)) break;
-            if (!bar_wait(full_op + s, spar, abort_flag, a.err)) break;
-            fence_after();
-            // descriptors advance by adding the byte offset / 16 to their
-            // start-address field (shared addresses stay below 2^18: no carry)
-            const uint64_t dxh = xdesc + (uint64_t)(s * (op_stride >> 4)), dxl = dxh + (xbytes >> 4);
-            for (int hq = 0; hq < MH; ++hq) {
-                const uint32_t d = tmem + (uint32_t)((acc * MH + hq) * BN);
-#pragma unroll 4
-                for (int ks = 0; ks < ksteps; ++ks) {
-                    const uint64_t ao = (uint64_t)(((ks >> 2) * MQ * 128 + hq * KM * 128 + (ks & 3) * 32) >> 4);
-                    const uint64_t bo = (uint64_t)(((ks >> 2) * BN * 128 + (ks & 3) * 32) >> 4);
-                    mma_bf16(d, qhdesc + ao, dxh + bo, idesc, ks > 0 ? 1u : 0u);
-                    if (!kExact) {
-                        if (need_xl) mma_bf16(d, qhdesc + ao, dxl + bo, idesc, 1u);
-                        if (need_ql) mma_bf16(d, qldesc + ao, dxh + bo, idesc, 1u);
-                    }
+            const int ab = acc * MH + hq;
+            ok = i < 2 || __all_sync(0xffffffffu, bar_wait(tempty + ab, (uint32_t)(((i >> 1) - 1) & 1), abort_flag, a.err));
+            if (!ok) break;
+            const uint32_t d = tmem + (uint32_t)(ab * BN);
+            for (int sl = 0; sl < nst; ++sl) {
+                ok = __all_sync(0xffffffffu, bar_wait(full_op + s, spar, abort_flag, a.err));
+                if (!ok) break;
+                fence_after();
+                // descriptors advance by adding the byte offset / 16 to their
+                // start-address field (shared addresses stay below 2^18: no carry)
+                const uint64_t so = (uint64_t)(s * (op_stride >> 4));
+                const uint64_t dx = xdesc + so, dq = kStream ? qdesc + so : qdesc;
+                if (leader) {
+                    if (work)
+                        for (int at = 0; at < apst; ++at) {
+                            const uint64_t da = dq + (uint64_t)((at * kQSlab) >> 4);
+                            const uint64_t db = dx + (uint64_t)((at * kXSlab) >> 4);
+#pragma unroll
+                            for (int ks = 0; ks < 4; ++ks)
+                                mma_f16(d, da + (uint64_t)(ks * 2), db + (uint64_t)(ks * 2), idesc,
+                                        (ks | at | sl) > 0 ? 1u : 0u);
+                        }
+                    mma_commit(empty_op + s);
+                    if (sl + 1 == nst) mma_commit(tfull + ab);
                 }
+                __syncwarp();
+                if (++s == ops) { s = 0; spar ^= 1u; }
             }
-            mma_commit(empty_op + s);
-            mma_commit(tfull + acc);
-            if (++s == ops) { s = 0; spar ^= 1u; }
         }
         // every product has landed before TMEM is released
-        mma_commit(done_bar);
-        bar_drain(done_bar, 0, a.err);
-    } else if (warp >= 2) {
-        // ---- epilogue: ranking keys, per-query lists ----
-        const int ew = warp - 2;
+        if (leader) mma_commit(done_bar);
+        __syncwarp();
+    } else if (warp > MW) {
+        // ---- epilogue ----
+        // Eight warps per accumulator set, so that a warp visits every second
+        // tile: the fixed cost of a visit (barrier waits, loads of the query's
+        // membership) is paid once per 128 columns instead of once per 64, and
+        // two tiles' epilogues overlap.
+        const int ew = warp - 1 - MW;
         const int quad = warp & 3;                    // TMEM lanes this warp may read
         const int hq = (ew >> 2) % MH;                // query half (its own accumulator)
-        const int ch = (ew >> 2) / MH;                // column slice
+        const int acc = (ew >> 2) / MH;               // accumulator set, of tiles acc, acc + 2, ...
+        const int ab = acc * MH + hq;
         const int row = hq * KM + quad * 32 + lane;   // query of the tile
-        const int lt = ew * 32 + lane;
-        float* mk = lkey + lt;
-        uint32_t* mi = lid + lt;
-        int n = 0;
-        float thr = INFINITY;
+        int n = 0;                                    // survivors in this lane's list
+        uint2* list = nullptr;
+        float m = 0.0f, lim = 0.0f;
         long long cur_qt = -1;
-        long long i = 0;
-        // Exact form: the lists of one query (column slices, CTAs) share a
-        // bound in global memory, the smallest K-th key of any full list (an
-        // upper bound of the query's K-th key: that list holds K candidates at
-        // or below it). A candidate above it cannot be in the top-K; one equal
-        // to it still enters (it may win the tie on its id).
-        auto flush = [&](long long qt) {
-            const long long lst = ((long long)blockIdx.x + qt) * NCH + ch;
-            const long long lb = lst * (long long)Kl;
-            for (int k = 0; k < n; ++k) {
-                a.part_key[(lb + k) * MQ + row] = mk[k * NT];
-                a.part_id[(lb + k) * MQ + row] = mi[k * NT];
-            }
-            a.part_n[lst * MQ + row] = n;
+        auto close_list = [&](long long q) {
+            a.part_n[(((long long)blockIdx.x + q) * NCH + acc) * MQ + row] = n;
         };
         long long qt = p0 / ntp, pt = p0 - qt * ntp;
-        int e = 0;
-        uint32_t epar = 0;
-        for (long long p = p0; p < p1; ++p, ++i) {
-            if (qt != cur_qt) {
-                if (cur_qt >= 0) flush(cur_qt);
-                cur_qt = qt;
-                n = 0;
-                thr = INFINITY;
-            }
-            const int acc = (int)(i & 1);
+        // A query tile can be crossed between this group's visits: its list is
+        // opened (and closed, if empty) all the same.
+        auto open_list = [&]() {
+            if (!kSample && cur_qt >= 0) close_list(cur_qt);
+            cur_qt = qt;
+            n = 0;
             const int gq = (int)qt * MQ + row;   // dense position of this lane's query
-            // the shared bound is read before the waits (its latency overlaps
-            // them): it only decreases, so an earlier value is still a bound
-            const uint32_t ext_enc = kExact ? __ldcg(a.qbound + gq) : 0u;
-            // every lane waits (and so sees the copied data); the warp leaves
-            // together if any lane gave up, since tcgen05.ld is warp-wide
-            const bool ok = bar_wait(tfull + acc, (uint32_t)((i >> 1) & 1), abort_flag, a.err) &&
-                            bar_wait(full_ep + e, epar, abort_flag, a.err);
-            if (!__all_sync(0xffffffffu, ok)) break;
-            fence_after();
-            const unsigned char* es = sE + (size_t)e * ep_stride;
-            const float ext = kExact ? key_dec(ext_enc) : INFINITY;
-            // a key enters iff key < thr and key <= ext, i.e. key < lim
-            const float ext_up = nextafterf(ext, INFINITY);
-            float lim = fminf(thr, ext_up);
-            const uint2 mw = *reinterpret_cast<const uint2*>(es + (size_t)row * BW * 4 + ch * 8);   // 2 words: 64 columns
-            const float* wv = reinterpret_cast<const float*>(es + bm_bytes) + ch * CW;
-            const uint32_t id0 = (uint32_t)(pt * BN + ch * CW);
-            const uint32_t tbase =
-                tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)((acc * MH + hq) * BN + ch * CW);
+            const bool live = (unsigned int)gq < nd;
+            m = live ? (kSample ? a.qinfo[gq].m_up : a.qinfo[gq].m_lo) : 0.0f;
+            if constexpr (!kSample) {
+                lim = live ? a.qlim[gq] : -INFINITY;   // no key is below -infinity
+                list = a.part + ((((long long)blockIdx.x + qt) * NCH + acc) * MQ + row) * a.list_cap;
+            }
+        };
+        int e = 0;
+        uint32_t epar = 0, tpar = 0;
+        bool mine = acc == 0;
+        for (long long p = p0; p < p1; ++p, mine = !mine) {
+            if (qt != cur_qt) open_list();
+            if (mine) {
+                // every lane waits (and so sees the copied data); the warp leaves
+                // together if any lane gave up, since tcgen05.ld is warp-wide
+                const bool ok = bar_wait(full_ep + e, epar, abort_flag, a.err) &&
+                                bar_wait(tfull + ab, tpar, abort_flag, a.err);
+                if (!__all_sync(0xffffffffu, ok)) break;
+                tpar ^= 1u;
+                fence_after();
+                const bool work = qt * MQ + hq * KM < (long long)nd;   // warp-uniform
+                if (work) {
+                    const unsigned char* es = sE + (size_t)e * kEpStride;
+                    const uint4 mw = *reinterpret_cast<const uint4*>(es + (size_t)row * BW * 4);
+                    const float* wv = reinterpret_cast<const float*>(es + kBmBytes);
+                    const uint32_t tbase = tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(ab * BN);
+                    // 16 columns at a time in two register sets: the next ones
+                    // are loaded while these are examined. The accumulator goes
+                    // back to the MMA warp as soon as the last ones are in
+                    // registers.
+                    uint32_t rc[2][16];
+                    float mprev = INFINITY;   // sample pass: minimum of a chunk's first half
+                    __syncwarp();   // tcgen05.ld is warp-collective
+                    tmem_ld16(tbase, rc[0]);
 #pragma unroll
-            for (int c = 0; c < 2; ++c) {
-                // The slice's two 32-column halves are loaded and ranked in
-                // turn, so that only 32 keys are live at a time; the
-                // accumulator goes back to the MMA warp as soon as the second
-                // half is in registers (the next products into it overlap the
-                // rest of this tile's key work).
-                uint32_t rc[32];
-                if (c == 1) __syncwarp();   // tcgen05.ld is warp-collective: reconverge after the inserts
-                tmem_ld32(tbase + (uint32_t)(c * 32), rc);
-                if (c == 1) {
-                    fence_before();
-                    __syncwarp();
-                    if (lane == 0) bar_arrive(tempty + acc);
-                }
-                // keys t = w - 2 q.x (packed FMA, in place)
-#pragma unroll
-                for (int j = 0; j < 32; j += 4) {
-                    const float4 w4 = *reinterpret_cast<const float4*>(wv + c * 32 + j);
-                    const float2 a2 = __ffma2_rn(make_float2(-2.0f, -2.0f),
-                                                 make_float2(__uint_as_float(rc[j]), __uint_as_float(rc[j + 1])),
-                                                 make_float2(w4.x, w4.y));
-                    const float2 b2 = __ffma2_rn(make_float2(-2.0f, -2.0f),
-                                                 make_float2(__uint_as_float(rc[j + 2]), __uint_as_float(rc[j + 3])),
-                                                 make_float2(w4.z, w4.w));
-                    rc[j] = __float_as_uint(a2.x);
-                    rc[j + 1] = __float_as_uint(a2.y);
-                    rc[j + 2] = __float_as_uint(b2.x);
-                    rc[j + 3] = __float_as_uint(b2.y);
-                }
-                const uint32_t mbits = c == 0 ? mw.x : mw.y;
-                float mm[11];
-#pragma unroll
-                for (int k = 0; k < 10; ++k)
-                    mm[k] = fmin3(__uint_as_float(rc[3 * k]), __uint_as_float(rc[3 * k + 1]), __uint_as_float(rc[3 * k + 2]));
-                mm[10] = fminf(__uint_as_float(rc[30]), __uint_as_float(rc[31]));
-                const float m = fmin3(fmin3(mm[0], mm[1], mm[2]), fmin3(mm[3], mm[4], mm[5]),
-                                      fmin3(fmin3(mm[6], mm[7], mm[8]), mm[9], mm[10]));
-                if (m < lim && mbits) {
-                    // this lane's candidate columns whose key beats its list;
-                    // lanes insert in parallel, each into its own sorted list
-                    uint32_t pm = 0;
-#pragma unroll
-                    for (int k = 0; k < 32; ++k) pm |= (__uint_as_float(rc[k]) < lim ? 1u : 0u) << k;
-                    pm &= mbits;
-                    for (; pm; pm &= pm - 1) {
-                        const int k = __ffs((int)pm) - 1;
-                        const float key = select32(rc, k);
-                        if (!(key < lim)) continue;
-                        // ids arrive in ascending order, so a key equal to a
-                        // listed one goes after it
-                        int pos = n < Kl ? n : Kl - 1;
-                        while (pos > 0 && mk[(pos - 1) * NT] > key) {
-                            mk[pos * NT] = mk[(pos - 1) * NT];
-                            mi[pos * NT] = mi[(pos - 1) * NT];
-                            --pos;
+                    for (int c = 0; c < BN / 16; ++c) {
+                        uint32_t(&v)[16] = rc[c & 1];
+                        tmem_wait16(v);
+                        if (c + 1 < BN / 16) {
+                            __syncwarp();
+                            tmem_ld16(tbase + (uint32_t)((c + 1) * 16), rc[(c + 1) & 1]);
+                        } else {
+                            fence_before();
+                            __syncwarp();
+                            if (lane == 0) bar_arrive(tempty + ab);
                         }
-                        mk[pos * NT] = key;
-                        mi[pos * NT] = id0 + (uint32_t)(c * 32 + k);
-                        if (n < Kl) ++n;
-                        if (n == Kl) {
-                            thr = mk[(Kl - 1) * NT];
-                            lim = fminf(thr, ext_up);
+                        // keys t = |x|^2 + m acc (packed FMA, in place)
+#pragma unroll
+                        for (int k = 0; k < 16; k += 4) {
+                            const float4 w4 = *reinterpret_cast<const float4*>(wv + c * 16 + k);
+                            const float2 a2 = __ffma2_rn(make_float2(m, m),
+                                                         make_float2(__uint_as_float(v[k]), __uint_as_float(v[k + 1])),
+                                                         make_float2(w4.x, w4.y));
+                            const float2 b2 = __ffma2_rn(make_float2(m, m),
+                                                         make_float2(__uint_as_float(v[k + 2]), __uint_as_float(v[k + 3])),
+                                                         make_float2(w4.z, w4.w));
+                            v[k] = __float_as_uint(a2.x);
+                            v[k + 1] = __float_as_uint(a2.y);
+                            v[k + 2] = __float_as_uint(b2.x);
+                            v[k + 3] = __float_as_uint(b2.y);
+                        }
+                        const uint32_t word = c < 2 ? mw.x : c < 4 ? mw.y : c < 6 ? mw.z : mw.w;
+                        const uint32_t mbits = (c & 1) ? word >> 16 : word & 0xFFFFu;
+                        if constexpr (kSample) {
+#pragma unroll
+                            for (int k = 0; k < 16; ++k) v[k] = ((mbits >> k) & 1u) ? v[k] : 0x7f800000u;
+                        }
+                        float mm[5];
+#pragma unroll
+                        for (int k = 0; k < 5; ++k)
+                            mm[k] = fmin3(__uint_as_float(v[3 * k]), __uint_as_float(v[3 * k + 1]),
+                                          __uint_as_float(v[3 * k + 2]));
+                        const float mn = fmin3(fmin3(mm[0], mm[1], mm[2]), fminf(mm[3], mm[4]), __uint_as_float(v[15]));
+                        if constexpr (kSample) {
+                            if (c & 1)
+                                a.smin[(qt * MQ + row) * a.nws + pt * (BN / 32) + (c >> 1)] = fminf(mn, mprev);
+                            else
+                                mprev = mn;
+                        } else if (mn < lim && mbits) {
+                            const uint32_t id0 = (uint32_t)(pt * BN + c * 16);
+                            uint32_t pm = 0;
+#pragma unroll
+                            for (int k = 0; k < 16; ++k) pm |= (__uint_as_float(v[k]) < lim ? 1u : 0u) << k;
+                            for (pm &= mbits; pm; pm &= pm - 1) {
+                                const int k = __ffs((int)pm) - 1;
+                                if (n < a.list_cap)
+                                    list[n] = make_uint2(__float_as_uint(select16(v, k)), id0 + (uint32_t)k);
+                                ++n;   // a count above list_cap marks the list as overflowed
+                            }
                         }
                     }
+                } else {
+                    fence_before();
+                    __syncwarp();
+                    if (lane == 0) bar_arrive(tempty + ab);
                 }
+                __syncwarp();
+                if (lane == 0) bar_arrive(empty_ep + e);
             }
-            if (kExact && n == Kl && thr < ext) atomicMin(a.qbound + gq, key_enc(thr));
-            __syncwarp();
-            if (lane == 0) bar_arrive(empty_ep + e);
-            if (++e == eps) { e = 0; epar ^= 1u; }
+            if (++e == kEpStages) { e = 0; epar ^= 1u; }
             if (++pt == ntp) { pt = 0; ++qt; }
         }
-        if (cur_qt >= 0 && !*abort_flag) flush(cur_qt);
+        if (!kSample && cur_qt >= 0 && !*abort_flag) close_list(cur_qt);
     }
+    if (warp == 1) bar_drain(done_bar, 0, a.err);   // both MMA warps' products
     __syncthreads();
     fence_after();
     if (warp == 1)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
 }
 
-
-// bf16 parts, squared norm and bound weight of rows (the dataset once per
-// index, the dense queries once per search), and the rows' flags. Row r is
-// src[list ? list[r] : r]; there are *count rows (or n). Rows from there up to
-// the padded count (a multiple of pad_to, or pad) are zero rows with weight
-// FLT_MAX. sq[r] = |x|^2 (RN FP32 chain, exact for small integers);
-// wb[r] = |x|^2 - C |x|^2_up rounded down (the bound form's weight, and for a
-// query its base). One warp per row.
-__global__ void k_knn_rows(const float* __restrict__ src, int D, int Dp, const int* __restrict__ list,
-                           const unsigned int* __restrict__ count, int64_t n, int64_t pad, int pad_to,
-                           __nv_bfloat16* __restrict__ xh, __nv_bfloat16* __restrict__ xl, float* __restrict__ sq,
-                           float* __restrict__ wb, float C, KnnState* __restrict__ st,
-                           unsigned int* __restrict__ bound) {
-    const int lane = threadIdx.x & 31;
-    const int64_t nrows = count ? (int64_t)*count : n;
-    const int64_t npad = count ? ((nrows + pad_to - 1) / pad_to) * pad_to : pad;
-    const int64_t w0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+// Largest magnitude, value range and finiteness of the dataset.
+__global__ void k_knn_scan(const float* __restrict__ X, int64_t n, KnnState* __restrict__ st) {
     int flags = 0, mneg = 0, mpos = 0;
-    for (int64_t r = w0; r < npad; r += nw) {
-        if (bound && lane == 0) bound[r] = kNoBound;
-        if (r >= nrows) {
-            if (r < n || count) {   // operand rows exist only up to the buffer's rows
-                for (int d = lane; d < Dp; d += 32) {
-                    xh[r * Dp + d] = __float2bfloat16_rn(0.0f);
-                    xl[r * Dp + d] = __float2bfloat16_rn(0.0f);
-                }
-            }
-            if (lane == 0) {
-                sq[r] = FLT_MAX;
-                wb[r] = FLT_MAX;
-            }
-            continue;
-        }
-        const float* row = src + (list ? (int64_t)list[r] : r) * D;
-        float s = 0.0f, su = 0.0f;
-        for (int d = lane; d < Dp; d += 32) {
-            const float x = d < D ? __ldg(row + d) : 0.0f;
-            const __nv_bfloat16 h = __float2bfloat16_rn(x);
-            const __nv_bfloat16 l = __float2bfloat16_rn(__fsub_rn(x, __bfloat162float(h)));
-            xh[r * Dp + d] = h;
-            xl[r * Dp + d] = l;
-            if (__bfloat16_as_ushort(l) & 0x7FFF) flags |= kKnnHasLo;
-            if (!(fabsf(x) <= FLT_MAX)) flags |= kKnnNonFinite;
-            if (x == rintf(x) && fabsf(x) <= 256.0f) {
-                const int v = (int)x;
-                mneg = max(mneg, 257 - v);
-                mpos = max(mpos, v + 257);
-            } else {
-                flags |= kKnnNotSmallInt;
-            }
-            s = __fmaf_rn(x, x, s);
-            su = __fmaf_ru(x, x, su);
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            s = __fadd_rn(s, __shfl_xor_sync(0xffffffffu, s, o));
-            su = __fadd_ru(su, __shfl_xor_sync(0xffffffffu, su, o));
-        }
-        if (lane == 0) {
-            sq[r] = s;
-            wb[r] = __fsub_rd(s, __fmul_ru(C, su));
+    float amax = 0.0f;
+    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+        const float x = __ldg(X + i);
+        if (!(fabsf(x) <= FLT_MAX)) flags |= kKnnNonFinite;
+        else amax = fmaxf(amax, fabsf(x));
+        if (x == rintf(x) && fabsf(x) <= 256.0f) {
+            mneg = max(mneg, 257 - (int)x);
+            mpos = max(mpos, 257 + (int)x);
+        } else {
+            flags |= kKnnNotSmallInt;
         }
     }
-    const unsigned full = 0xffffffffu;
-    flags = __reduce_or_sync(full, flags);
-    mneg = __reduce_max_sync(full, mneg);
-    mpos = __reduce_max_sync(full, mpos);
-    if (lane == 0) {
+    flags = __reduce_or_sync(0xffffffffu, flags);
+    mneg = __reduce_max_sync(0xffffffffu, mneg);
+    mpos = __reduce_max_sync(0xffffffffu, mpos);
+    const uint32_t am = __reduce_max_sync(0xffffffffu, __float_as_uint(amax));   // non-negative floats order as words
+    if ((threadIdx.x & 31) == 0) {
         if (flags) atomicOr(&st->flags, flags);
         if (mneg) atomicMax(&st->mneg, mneg);
         if (mpos) atomicMax(&st->mpos, mpos);
+        if (am) atomicMax(&st->amax, am);
     }
 }
 
-// Exact FP32 squared distance in the reference's lane order
-// (cuLSH_Kernels.cu:323-346): partial j chains columns j, j+8, ... with FMA,
-// then (p0+p4, p1+p5, p2+p6, p3+p7) -> (t0+t2) + (t1+t3). One thread.
-__device__ __forceinline__ float lane_order_distance(const float* __restrict__ q, const float* __restrict__ x, int D) {
-    float p[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) p[j] = 0.0f;
-    int c = 0;
-    for (; c + 8 <= D; c += 8) {
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-            const float df = __fsub_rn(__ldg(q + c + j), __ldg(x + c + j));
-            p[j] = __fmaf_rn(df, df, p[j]);
-        }
-    }
-#pragma unroll
-    for (int j = 0; j < 8; ++j)
-        if (c + j < D) {
-            const float df = __fsub_rn(__ldg(q + c + j), __ldg(x + c + j));
-            p[j] = __fmaf_rn(df, df, p[j]);
-        }
-    const float t0 = __fadd_rn(p[0], p[4]), t1 = __fadd_rn(p[1], p[5]);
-    const float t2 = __fadd_rn(p[2], p[6]), t3 = __fadd_rn(p[3], p[7]);
-    return __fadd_rn(__fadd_rn(t0, t2), __fadd_rn(t1, t3));
+// Power-of-two scale that takes magnitudes up to amax below 2^15 (1 for zero).
+__device__ __forceinline__ float knn_scale(float amax) {
+    if (!(amax > 0.0f)) return 1.0f;
+    return scalbnf(1.0f, 14 - ilogbf(amax));
 }
 
-constexpr int MERGE_WARPS = 4;
-constexpr int kEpStages = 4;   // membership / weight ring stages
+// Shared row conversion of a warp: fp16(row * scale) into xh, the squared
+// norm (RN) and the squared residual norm in scaled units (rounded up).
+__device__ __forceinline__ void knn_row(const float* __restrict__ row, int D, int Dp, float scale, __half* xh, float& s,
+                                        float& rr) {
+    const int lane = threadIdx.x & 31;
+    s = rr = 0.0f;
+    for (int d = lane; d < Dp; d += 32) {
+        const float x = d < D ? __ldg(row + d) : 0.0f;
+        const float xs = x * scale;   // exact: a power of two, no overflow
+        const __half h = __float2half_rn(xs);
+        const float r = __fsub_rn(xs, __half2float(h));
+        xh[d] = h;
+        s = __fmaf_rn(x, x, s);
+        rr = __fmaf_ru(r, r, rr);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        s = __fadd_rn(s, __shfl_xor_sync(0xffffffffu, s, o));
+        rr = __fadd_ru(rr, __shfl_xor_sync(0xffffffffu, rr, o));
+    }
+}
 
-// Merges the partial lists of each dense query into its top-K (one warp per
-// query). Lists are walked in ascending key order and left as soon as the
-// lower bound key + base passes the K-th distance found so far. Exact form:
-// key + |q|^2 is the distance. Bound form: the exact FP32 lane-order distance
-// of each entry not yet excluded is recomputed; a query with a full list whose
-// last bound does not exceed its K-th distance is handed to the fallback list.
-__global__ void __launch_bounds__(32 * MERGE_WARPS) k_knn_merge(KnnSearch k) {
-    __shared__ float s_d[MERGE_WARPS][kMaxKnnK];
-    __shared__ uint32_t s_i[MERGE_WARPS][kMaxKnnK];
+// Residual that any row of D elements in scaled units may have beside the
+// relative 2^-11 of its normal fp16 values (subnormals: half of 2^-24 each).
+__device__ __forceinline__ float knn_abs_residual(int D) { return 1.01f * 2.98023224e-8f * sqrtf((float)D); }
+
+// Dataset rows (once per index): fp16 operand, |x|^2 (FLT_MAX from row N up to
+// the padded count) and the largest relative residual. One warp per row.
+__global__ void k_knn_rows(const float* __restrict__ X, int64_t N, int D, int Dp, int64_t pad, __half* __restrict__ xh,
+                           float* __restrict__ w, KnnState* __restrict__ st) {
+    const int lane = threadIdx.x & 31;
+    const int64_t w0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
+    const float scale = knn_scale(__uint_as_float(*(volatile uint32_t*)&st->amax));
+    const float ar = knn_abs_residual(D);
+    float rho = 0.0f;
+    for (int64_t r = w0; r < pad; r += nw) {
+        if (r >= N) {
+            if (lane == 0) w[r] = FLT_MAX;
+            continue;
+        }
+        float s, rr;
+        knn_row(X + r * D, D, Dp, scale, xh + r * Dp, s, rr);
+        // |x| scaled, rounded down; a zero row has no residual
+        const float nx = sqrtf(s) * scale * 0.9999f, res = sqrtf(rr) * 1.0001f;
+        if (res > ar && nx > 0.0f) rho = fmaxf(rho, (res - ar) / nx * 1.0001f);
+        if (lane == 0) w[r] = s;
+    }
+    const uint32_t rm = __float_as_uint(rho);
+    if (lane == 0 && rm) atomicMax(&st->rho, rm);
+}
+
+// Query rows of one search, in dense-list order (zero rows up to the next
+// tile): fp16 operand, |q|^2, key multipliers and error terms. The norms of
+// the sample points are gathered beside them. One warp per row.
+__global__ void k_knn_qrows(KnnSearch k) {
+    const int lane = threadIdx.x & 31;
+    const int64_t g0 = (int64_t)blockIdx.x * blockDim.x + threadIdx.x, gn = (int64_t)gridDim.x * blockDim.x;
+    if (k.f > 0) {
+        const int64_t S = (int64_t)k.nseg * k.s32 * 32;
+        for (int64_t j = g0; j < S; j += gn) {
+            const int c = (int)(j >> 5), i = (int)(j & 31), seg = c / k.s32;
+            k.w_sample[j] = k.w[(int64_t)seg * k.seg + ((int64_t)i * k.s32 + (c - seg * k.s32)) * k.f];
+        }
+    }
+    const unsigned int nd = (unsigned int)k.nd;
+    const int64_t npad = ((int64_t)nd + MQ - 1) / MQ * MQ;
+    const KnnState ds = *k.dstate;
+    const float sx = knn_scale(__uint_as_float(ds.amax));
+    for (int64_t r = g0 >> 5; r < npad; r += gn >> 5) {
+        __half* qh = static_cast<__half*>(k.qh) + r * k.Dp;
+        if (r >= nd) {
+            for (int d = lane; d < k.Dp; d += 32) qh[d] = __float2half_rn(0.0f);
+            continue;
+        }
+        const float* row = k.queries + (int64_t)k.dense_q[r] * k.D;
+        int bad = 0, mneg = 0, mpos = 0;
+        float amax = 0.0f;
+        for (int d = lane; d < k.D; d += 32) {
+            const float x = __ldg(row + d);
+            // beyond these magnitudes squares could leave the float range
+            if (!(fabsf(x) <= kKnnMaxValue)) bad |= 2;
+            else amax = fmaxf(amax, fabsf(x));
+            if (x == rintf(x) && fabsf(x) <= 256.0f) {
+                mneg = max(mneg, 257 - (int)x);
+                mpos = max(mpos, 257 + (int)x);
+            } else {
+                bad |= 1;
+            }
+        }
+        bad = __reduce_or_sync(0xffffffffu, bad);
+        mneg = max(__reduce_max_sync(0xffffffffu, mneg), ds.mneg);
+        mpos = max(__reduce_max_sync(0xffffffffu, mpos), ds.mpos);
+        amax = __uint_as_float(__reduce_max_sync(0xffffffffu, __float_as_uint(amax)));
+        const bool unfit = (bad & 2) || (amax > 0.0f && amax < kKnnMinValue);
+        const float sq = unfit ? 0.0f : knn_scale(amax);
+        float s, rr;
+        knn_row(row, k.D, k.Dp, sq, qh, s, rr);
+        if (lane) continue;
+        KnnQuery qi;
+        qi.sq = s;
+        if (unfit) {   // scanned exactly (k_knn_scan_rows); no survivors here
+            qi = KnnQuery{0.0f, 0.0f, 0.0f, 0.0f, 0.0f, kKnnUnfit};
+            k.fallback[atomicAdd(k.n_fallback, 1u)] = (int)r;
+        } else {
+            const long long lo = 257 - mneg, hi = mpos - 257, mag = max(-lo, hi);
+            const bool exact = !(ds.flags & kKnnNotSmallInt) && !bad && mneg > 0 && mpos > 0 &&
+                               k.D * mag * mag < (1ll << 24) && k.D * (hi - lo) * (hi - lo) < (1ll << 24);
+            const float m0 = -2.0f / (sq * sx);   // scales are powers of two
+            if (exact) {
+                qi.m_lo = qi.m_up = m0;
+                qi.kappa = qi.slack = 0.0f;
+                qi.flags = kKnnExact;
+            } else {
+                const float nq = sqrtf(s);
+                const float rq = s > 0.0f ? sqrtf(rr) * 1.0001f / (sq * nq * 0.9999f) : 0.0f;
+                qi.kappa = 1.01f * (rq + __uint_as_float(ds.rho)) + k.gamma;
+                qi.slack = 2.02f * nq * (knn_abs_residual(k.D) / sx) + 1e-37f;
+                qi.m_lo = m0 / (1.0f - qi.kappa);
+                qi.m_up = m0 / (1.0f + qi.kappa);
+                qi.flags = 0;
+            }
+        }
+        k.qinfo[r] = qi;
+        if (k.f == 0) k.qlim[r] = unfit ? -INFINITY : INFINITY;   // no sample pass
+    }
+}
+
+// One warp: the bin of a 256-bin histogram that holds the want-th entry (in
+// bin order, want >= 1) and the entry's rank within it. False when the bins
+// hold fewer than want entries.
+__device__ __forceinline__ bool select_bin(const uint32_t* hist, uint32_t want, uint32_t& bin, uint32_t& rest) {
+    const int lane = threadIdx.x & 31;
+    uint32_t mine = 0;
+#pragma unroll
+    for (int b = 0; b < 8; ++b) mine += hist[lane * 8 + b];
+    uint32_t x = mine;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    const uint32_t hit = __ballot_sync(0xffffffffu, x >= want);
+    if (hit == 0) return false;
+    const int src = __ffs((int)hit) - 1;
+    uint32_t r = want - (x - mine), b = (uint32_t)lane * 8;
+    if (lane == src)
+        while (hist[b] < r) r -= hist[b++];
+    bin = __shfl_sync(0xffffffffu, b, src);
+    rest = __shfl_sync(0xffffffffu, r, src);
+    return true;
+}
+
+constexpr int LW = 8;   // queries (warps) per block of k_knn_limit
+
+// Key limit of each dense query's full pass from its chunk minima (one warp
+// per query): the K-th smallest, then every key whose lower bound can reach its
+// upper bound. The minima are read once, folded into 32 R groups held in
+// registers (any K groups hold K different candidates; with at least 16 K
+// groups two of the K nearest rarely share one), and the K-th smallest group
+// is selected by radix passes over a 256-bin histogram, from the highest bit
+// in which the groups differ (bits above it would send every lane to one bin).
+// 10,000 queries of 1,953 chunks: 345 us with four passes over global memory
+// from the top bit, 108 us from the first differing bit.
+template <int R>
+__global__ void __launch_bounds__(32 * LW) k_knn_limit(KnnSearch k) {
+    __shared__ uint32_t hist[LW][256];
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const unsigned int nd = *k.n_dense;
-    const bool exact = k.exact_possible && exact_form(k.dstate, k.qstate, k.D);
-    const int K = k.K;
-    const int Kl = exact ? k.kl_exact : k.kl_bound;
-    const int MQ = exact ? kMqExact : kMqBound;
-    const int NCH = exact ? kNchExact : kNchBound;
-    const int BN = exact ? kBnExact : kBnBound;
-    const long long ntp = (k.N + BN - 1) / BN;
-    const long long nqt = ((long long)nd + MQ - 1) / MQ;
-    const long long U = nqt * ntp;
+    const unsigned int i = blockIdx.x * LW + w;
+    if (i >= (unsigned int)k.nd) return;   // warps work alone
+    const int nc = k.nws;
+    const float* src = k.smin + (int64_t)i * nc;
+    float v[R];
+#pragma unroll
+    for (int j = 0; j < R; ++j) v[j] = INFINITY;
+    for (int c0 = 0; c0 < nc; c0 += 32 * R) {
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+            const int c = c0 + j * 32 + lane;
+            if (c < nc) v[j] = fminf(v[j], __ldg(src + c));
+        }
+    }
+    uint32_t e[R], lo = 0xFFFFFFFFu, hi = 0, cnt = 0;   // encoded keys; range and count of the groups with a candidate
+#pragma unroll
+    for (int j = 0; j < R; ++j) {
+        e[j] = v[j] < FLT_MAX ? key_enc(v[j]) : 0xFFFFFFFFu;
+        if (e[j] != 0xFFFFFFFFu) {
+            lo = min(lo, e[j]);
+            hi = max(hi, e[j]);
+            ++cnt;
+        }
+    }
+    lo = __reduce_min_sync(0xffffffffu, lo);
+    hi = __reduce_max_sync(0xffffffffu, hi);
+    cnt = __reduce_add_sync(0xffffffffu, cnt);
+    const KnnQuery q = k.qinfo[i];
+    if (cnt < (uint32_t)k.K || (q.flags & kKnnUnfit)) {   // uniform: no limit, or no survivors
+        if (lane == 0) k.qlim[i] = (q.flags & kKnnUnfit) ? -INFINITY : INFINITY;
+        return;
+    }
+    uint32_t prefix = 0, want = (uint32_t)k.K;   // want-th smallest of e - lo with this prefix
+    for (int top = 32 - __clz((int)(hi - lo)); top > 0;) {
+        const int sh = max(top - 8, 0);
+        for (int b = lane; b < 256; b += 32) hist[w][b] = 0;
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < R; ++j) {
+            const uint32_t d = e[j] - lo;
+            if (e[j] != 0xFFFFFFFFu && (top >= 32 ? 0u : d >> top) == prefix)
+                atomicAdd(&hist[w][(d >> sh) & ((1u << (top - sh)) - 1u)], 1u);
+        }
+        __syncwarp();
+        uint32_t bin = 0, rest = 0;
+        select_bin(hist[w], want, bin, rest);
+        prefix = (prefix << (top - sh)) | bin;
+        want = rest;
+        top = sh;
+        __syncwarp();
+    }
+    if (lane) return;
+    const float key = key_dec(lo + prefix);
+    const double u = (1.0 + (double)q.kappa) * ((double)key + q.sq) + q.slack;
+    const double l = (u + q.slack) / (1.0 - (double)q.kappa) - q.sq;
+    k.qlim[i] = (float)(l + 1e-6 * (fabs(u) + q.sq));   // keys below it survive
+}
+
+constexpr int MT = 128;   // threads of k_knn_merge
+
+// Top-K of each dense query from its survivors (one block per query): step 3
+// of the file comment. Survivors are (encoded key, id) words in shared memory;
+// the chosen ones become (distance bits, id) words and are sorted.
+__global__ void __launch_bounds__(MT) k_knn_merge(KnnSearch k) {
+    extern __shared__ __align__(16) unsigned char msm[];
+    unsigned long long* ent = reinterpret_cast<unsigned long long*>(msm);   // [kKnnMaxSurvivors]
+    unsigned long long* sel = ent + kKnnMaxSurvivors;                       // [kKnnMaxChosen]
+    float* qs = reinterpret_cast<float*>(sel + kKnnMaxChosen);              // [D]
+    __shared__ uint32_t hist[256];
+    __shared__ uint32_t s_cnt, s_bad, s_bin, s_rest, s_dmax, s_m, s_lo, s_hi;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const unsigned int nd = (unsigned int)k.nd;
+    const int K = k.K, D = k.D;
+    const long long ntp = ((long long)k.N + BN - 1) / BN;
+    const long long U = (((long long)nd + MQ - 1) / MQ) * ntp;
     const int G = (int)min((long long)k.grid, U);
-    float* wd = s_d[w];
-    uint32_t* wi = s_i[w];
-    for (long long i = (long long)blockIdx.x * MERGE_WARPS + w; i < nd; i += (long long)gridDim.x * MERGE_WARPS) {
+    const bool vec = (D & 3) == 0;
+    for (unsigned int i = blockIdx.x; i < nd; i += gridDim.x) {
+        const KnnQuery qi = k.qinfo[i];
+        if (qi.flags & kKnnUnfit) continue;   // uniform
         const int q = k.dense_q[i];
         const long long qt = i / MQ;
         const int r = (int)(i - qt * MQ);
         const int c0 = owner_cta(qt * ntp, U, G), c1 = owner_cta(qt * ntp + ntp - 1, U, G);
-        const float base = exact ? k.qsq[i] : k.qbase[i];
-        const float* qrow = k.queries + (int64_t)q * k.D;
-        int n = 0;
-        float thr_d = FLT_MAX;
-        uint32_t thr_i = 0;
-        float minlast = INFINITY;   // smallest last bound over the full lists
-        for (int c = c0; c <= c1; ++c) {
-            for (int h = 0; h < NCH; ++h) {   // the column slices
-                const long long lst = ((long long)c + qt) * NCH + h;
-                const int cnt = k.part_n[lst * MQ + r];
-                const long long lb = lst * (long long)Kl;
-                if (!exact && cnt == Kl)
-                    minlast = fminf(minlast, __fadd_rd(k.part_key[(lb + Kl - 1) * MQ + r], base));
-                for (int e0 = 0; e0 < cnt; e0 += 32) {
-                    const int e = e0 + lane;
-                    const bool valid = e < cnt;
-                    const float key = valid ? k.part_key[(lb + e) * MQ + r] : INFINITY;
-                    const uint32_t id = valid ? k.part_id[(lb + e) * MQ + r] : 0u;
-                    const float low = exact ? __fadd_rn(key, base) : __fadd_rd(key, base);
-                    // entries are in ascending key order: lane 0 holds the chunk's smallest
-                    if (__shfl_sync(0xffffffffu, low, 0) > thr_d) break;
-                    float d = INFINITY;
-                    if (valid && low <= thr_d) d = exact ? low : lane_order_distance(qrow, k.X + (int64_t)id * k.D, k.D);
-                    uint32_t want = __ballot_sync(0xffffffffu, valid && lessp(d, id, thr_d, thr_i));
-                    while (want) {
-                        const int src = __ffs(want) - 1;
-                        want &= want - 1;
-                        const float cd = __shfl_sync(0xffffffffu, d, src);
-                        const uint32_t cid = __shfl_sync(0xffffffffu, id, src);
-                        if (lessp(cd, cid, thr_d, thr_i)) warp_insert(wd, wi, n, K, cd, cid, thr_d, thr_i);
-                    }
-                }
+        const int nl = (c1 - c0 + 1) * NCH;
+        __syncthreads();
+        if (tid == 0) {
+            s_cnt = s_bad = s_dmax = s_m = s_hi = 0;
+            s_lo = 0xFFFFFFFFu;
+        }
+        __syncthreads();
+        // gather the lists: 16 lanes per list
+        for (int l = tid >> 4; l < nl; l += MT / 16) {
+            const long long lst = (((long long)(c0 + l / NCH) + qt) * NCH + l % NCH) * MQ + r;
+            const int cnt = k.part_n[lst], have = min(cnt, k.list_cap);
+            const uint2* src = k.part + lst * k.list_cap;
+            uint32_t at = 0;
+            if ((tid & 15) == 0) {
+                at = atomicAdd(&s_cnt, (uint32_t)have);
+                if (cnt > k.list_cap) s_bad = 1;
+            }
+            at = __shfl_sync(0xffffu << (lane & 16), at, lane & 16);
+            for (int e = tid & 15; e < have; e += 16) {
+                const uint2 v = src[e];
+                if (at + e < (uint32_t)kKnnMaxSurvivors)
+                    ent[at + e] = ((unsigned long long)key_enc(__uint_as_float(v.x)) << 32) | v.y;
             }
         }
-        if (!exact && minlast <= thr_d) {
-            // a list may have dropped an entry that belongs to the top-K
-            if (lane == 0) k.fallback[atomicAdd(k.n_fallback, 1u)] = q;
+        for (int d = tid; d < D; d += MT) qs[d] = k.queries[(int64_t)q * D + d];
+        __syncthreads();
+        const uint32_t n = s_cnt;
+        if (s_bad) {   // uniform
+            if (tid == 0) k.fallback[atomicAdd(k.n_fallback, 1u)] = (int)i;
             continue;
         }
+        // every survivor, from shared memory or (more than it holds) the lists
+        auto each = [&](auto f) {
+            if (n <= (uint32_t)kKnnMaxSurvivors) {
+                for (uint32_t e = tid; e < n; e += MT) f(ent[e]);
+                return;
+            }
+            for (int l = tid >> 4; l < nl; l += MT / 16) {
+                const long long lst = (((long long)(c0 + l / NCH) + qt) * NCH + l % NCH) * MQ + r;
+                const int have = k.part_n[lst];
+                const uint2* src = k.part + lst * k.list_cap;
+                for (int e = tid & 15; e < have; e += 16) {
+                    const uint2 v = src[e];
+                    f(((unsigned long long)key_enc(__uint_as_float(v.x)) << 32) | v.y);
+                }
+            }
+        };
+        // K-th smallest encoded key (no limit when there are no more than K)
+        uint32_t thr = 0xFFFFFFFFu;
+        if (n > (uint32_t)K) {
+            // digits from the highest bit in which the keys differ
+            uint32_t lo = 0xFFFFFFFFu, hi = 0;
+            each([&](unsigned long long v) {
+                lo = min(lo, (uint32_t)(v >> 32));
+                hi = max(hi, (uint32_t)(v >> 32));
+            });
+            __syncwarp();
+            atomicMin(&s_lo, __reduce_min_sync(0xffffffffu, lo));
+            atomicMax(&s_hi, __reduce_max_sync(0xffffffffu, hi));
+            __syncthreads();
+            lo = s_lo;
+            uint32_t prefix = 0, want = (uint32_t)K;
+            for (int top = 32 - __clz((int)(s_hi - lo)); top > 0;) {
+                const int sh = max(top - 8, 0);
+                for (int b = tid; b < 256; b += MT) hist[b] = 0;
+                __syncthreads();
+                each([&](unsigned long long w) {
+                    const uint32_t v = (uint32_t)(w >> 32) - lo;
+                    if ((top >= 32 ? 0u : v >> top) == prefix) atomicAdd(&hist[(v >> sh) & ((1u << (top - sh)) - 1u)], 1u);
+                });
+                __syncthreads();
+                if (warp == 0) {
+                    uint32_t bin = 0, rest = 0;
+                    select_bin(hist, want, bin, rest);
+                    if (lane == 0) {
+                        s_bin = bin;
+                        s_rest = rest;
+                    }
+                }
+                __syncthreads();
+                prefix = (prefix << (top - sh)) | s_bin;
+                want = s_rest;
+                top = sh;
+            }
+            thr = lo + prefix;
+        }
+        auto choose = [&](unsigned long long v) {
+            const uint32_t at = atomicAdd(&s_m, 1u);
+            if (at < (uint32_t)kKnnMaxChosen) sel[at] = v;
+        };
+        each([&](unsigned long long v) {
+            if ((uint32_t)(v >> 32) <= thr) choose(v);
+        });
+        __syncthreads();
+        uint32_t m = min(s_m, (uint32_t)kKnnMaxChosen);
+        if (qi.flags & kKnnExact) {
+            for (uint32_t e = tid; e < m; e += MT) {
+                const float d = __fadd_rn(key_dec((uint32_t)(sel[e] >> 32)), qi.sq);
+                sel[e] = ((unsigned long long)__float_as_uint(d) << 32) | (uint32_t)sel[e];
+            }
+        } else {
+            // exact FP32 lane-order distances of sel[from, to): two lanes per
+            // row (eight where D % 4 != 0)
+            auto distances = [&](uint32_t from, uint32_t to) {
+                const int per = vec ? 16 : 4, sub = vec ? lane >> 1 : lane >> 3;
+                for (uint32_t b = from + warp * per; b < to; b += (MT / 32) * per) {
+                    const uint32_t e = b + sub;
+                    const bool on = e < to;
+                    const uint32_t id = on ? (uint32_t)sel[e] : 0u;
+                    const float d = row_distance(k.X + (int64_t)id * D, D, qs, vec, on);
+                    __syncwarp();
+                    if (on && (lane & (vec ? 1 : 7)) == 0) {
+                        const uint32_t bits = d <= FLT_MAX ? __float_as_uint(d) : 0x7f800000u;   // NaN, inf: never listed
+                        sel[e] = ((unsigned long long)bits << 32) | id;
+                        atomicMax(&s_dmax, bits);
+                    }
+                }
+            };
+            distances(0, m);
+            __syncthreads();
+            if (n > (uint32_t)K) {
+                // those K distances bound the K-th: the entries whose lower
+                // bound they do not exclude
+                const float top = __uint_as_float(s_dmax);
+                each([&](unsigned long long v) {
+                    const uint32_t ek = (uint32_t)(v >> 32);
+                    if (ek <= thr) return;
+                    const float low = __fsub_rd(__fmul_rd(1.0f - qi.kappa, __fadd_rd(key_dec(ek), qi.sq)), qi.slack);
+                    if (low <= top) choose(v);
+                });
+                __syncthreads();
+                const uint32_t m2 = min(s_m, (uint32_t)kKnnMaxChosen);
+                distances(m, m2);
+                m = m2;
+            }
+        }
+        __syncthreads();
+        if (s_m > (uint32_t)kKnnMaxChosen) {   // uniform
+            if (tid == 0) k.fallback[atomicAdd(k.n_fallback, 1u)] = (int)i;
+            continue;
+        }
+        // ascending (distance, id): bitonic over the next power of two
+        uint32_t P = 32;
+        while (P < m) P <<= 1;
+        for (uint32_t e = m + tid; e < P; e += MT) sel[e] = ~0ull;
+        __syncthreads();
+        for (uint32_t a = 2; a <= P; a <<= 1)
+            for (uint32_t b = a >> 1; b > 0; b >>= 1) {
+                for (uint32_t t = tid; t < P / 2; t += MT) {
+                    const uint32_t x = 2 * t - (t & (b - 1)), y = x + b;
+                    const unsigned long long u = sel[x], v = sel[y];
+                    if ((u > v) == ((x & a) == 0)) {
+                        sel[x] = v;
+                        sel[y] = u;
+                    }
+                }
+                __syncthreads();
+            }
         int32_t* oid = k.out_ids + (int64_t)q * K;
         float* od = k.out_d + (int64_t)q * K;
-        for (int j = lane; j < K; j += 32) {
-            oid[j] = j < n ? (int32_t)wi[j] : -1;
-            od[j] = j < n ? wd[j] : FLT_MAX;
+        for (int j = tid; j < K; j += MT) {
+            const unsigned long long v = (uint32_t)j < m ? sel[j] : ~0ull;
+            const bool have = (uint32_t)(v >> 32) < 0x7F7FFFFFu;   // finite, below FLT_MAX
+            oid[j] = have ? (int32_t)(uint32_t)v : -1;
+            od[j] = have ? __uint_as_float((uint32_t)(v >> 32)) : FLT_MAX;
         }
-        __syncwarp();
     }
 }
 
@@ -766,164 +1084,183 @@ EncodeTiledFn knn_encode_fn() {
     return f;
 }
 
-// 2-D map over a row-major [rows][cols] array with a (box_cols x box_rows) box.
-bool knn_map(CUtensorMap* m, const void* ptr, CUtensorMapDataType dt, int esize, uint64_t cols, uint64_t rows,
-             uint32_t box_cols, uint32_t box_rows, bool swizzle) {
+
+// Map over an array of `rank` dimensions (strides in bytes, from the second).
+bool knn_map(CUtensorMap* m, const void* ptr, CUtensorMapDataType dt, int rank, const cuuint64_t* dims,
+             const cuuint64_t* strides, const cuuint32_t* box, bool swizzle) {
     EncodeTiledFn fn = knn_encode_fn();
     if (!fn) return false;
-    const cuuint64_t dims[2] = {cols, rows};
-    const cuuint64_t strides[1] = {cols * (uint64_t)esize};
-    const cuuint32_t box[2] = {box_cols, box_rows};
-    const cuuint32_t es[2] = {1, 1};
-    return fn(m, dt, 2, const_cast<void*>(ptr), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+    const cuuint32_t es[4] = {1, 1, 1, 1};
+    return fn(m, dt, (cuuint32_t)rank, const_cast<void*>(ptr), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
               swizzle ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
-
-size_t knn_smem(bool exact, int Dp, int Kl, int ops, int eps) {
-    const int MQ = exact ? kMqExact : kMqBound, BN = exact ? kBnExact : kBnBound;
-    const int nepi = exact ? kNepiExact : kNepiBound;
-    const size_t q = (size_t)MQ * Dp * 2 * (exact ? 1 : 2);
-    const size_t op = (size_t)BN * Dp * 2 * (exact ? 1 : 2);
-    const size_t ep = (size_t)MQ * (BN / 32) * 4 + (size_t)BN * 4;
-    const size_t lists = (size_t)32 * nepi * Kl * 8;   // one list per (query, column slice)
-    const size_t bars = 8 * (7 + 2 * ops + 2 * eps) + 16;
-    return 1024 + q + ops * op + eps * ep + lists + bars;
+bool knn_map_rows(CUtensorMap* m, const void* ptr, uint64_t cols, uint64_t rows, uint32_t box_rows) {
+    const cuuint64_t dims[2] = {cols, rows}, strides[1] = {2 * cols};
+    const cuuint32_t box[2] = {64, box_rows};
+    return knn_map(m, ptr, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, dims, strides, box, true);
+}
+bool knn_map_bits(CUtensorMap* m, const void* ptr, uint64_t words, uint64_t rows) {
+    const cuuint64_t dims[2] = {words, rows}, strides[1] = {4 * words};
+    const cuuint32_t box[2] = {BW, MQ};
+    return knn_map(m, ptr, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, dims, strides, box, false);
 }
 
-template <int BN, int MQ, int NEPI, bool kExact>
-cudaError_t launch_knn_form(const KnnSearch& k, const CUtensorMap& mxh, const CUtensorMap& mxl, cudaStream_t s) {
+size_t knn_smem(int Dp, int ops) {
+    const size_t atoms = Dp / 64;
+    const bool stream = Dp > kResidentD;
+    const size_t op = stream ? kXSlab + kQSlab : atoms * kXSlab;
+    return 1024 + (stream ? 0 : atoms * kQSlab) + ops * op + (size_t)kEpStages * kEpStride +
+           8 * (3 + 4 * MH + 2 * ops + 2 * kEpStages) + 16;
+}
+
+template <bool kSample, bool kStream>
+cudaError_t launch_knn_pass(const KnnSearch& k, cudaStream_t s) {
     static std::atomic<size_t> cap{0};
-    const size_t smem = kExact ? k.smem_exact : k.smem_bound;
-    if (smem > cap.load()) {
-        const cudaError_t e = cudaFuncSetAttribute(k_knn_tc<BN, MQ, NEPI, kExact>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (k.smem > cap.load()) {
+        const cudaError_t e = cudaFuncSetAttribute(k_knn_tc<kSample, kStream>,
+                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem);
         if (e != cudaSuccess) return e;
-        cap = smem;
+        cap = k.smem;
     }
-    CUtensorMap mbm, mqh, mql;
-    if (!knn_map(&mbm, k.bm, CU_TENSOR_MAP_DATA_TYPE_UINT32, 4, (uint64_t)k.nwp, (uint64_t)k.Qcap, BN / 32, MQ,
-                 false) ||
-        !knn_map(&mqh, k.qh, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)k.Dp, (uint64_t)k.Qcap, 64, MQ, true) ||
-        !knn_map(&mql, k.ql, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)k.Dp, (uint64_t)k.Qcap, 64, MQ, true))
-        return cudaErrorNotSupported;
+    CUtensorMap mq, mx, mb;
+    if (!knn_map_rows(&mq, k.qh, k.Dp, k.Qcap, MQ)) return cudaErrorNotSupported;
     KnnArgs a;
-    a.N = k.N;
-    a.D = k.D;
     a.Dp = k.Dp;
-    a.exact_launched = k.exact_possible;
-    a.ntp_exact = (k.N + kBnExact - 1) / kBnExact;
-    a.ntp_bound = (k.N + kBnBound - 1) / kBnBound;
-    a.kl_exact = k.kl_exact;
-    a.kl_bound = k.kl_bound;
-    a.op_stages = kExact ? k.ops_exact : k.ops_bound;
-    a.ep_stages = kEpStages;
-    a.n_dense = k.n_dense;
-    a.dstate = k.dstate;
-    a.qstate = k.qstate;
-    a.qbound = k.qbound;
-    a.w_exact = k.w_exact;
-    a.w_bound = k.w_bound;
-    a.part_key = k.part_key;
-    a.part_id = k.part_id;
+    a.op_stages = k.ops;
+    a.s32 = k.s32;
+    a.nd = (unsigned int)k.nd;
+    a.qinfo = k.qinfo;
+    a.qlim = k.qlim;
+    a.smin = k.smin;
+    a.nws = k.nws;
+    a.part = k.part;
+    a.list_cap = k.list_cap;
     a.part_n = k.part_n;
     a.err = k.err;
-    k_knn_tc<BN, MQ, NEPI, kExact><<<k.grid, 64 + 32 * NEPI, smem, s>>>(mqh, mql, mxh, mxl, mbm, a);
+    if (kSample) {
+        // sample point (segment g, chunk c, i) is row g seg + (i s32 + c) f
+        const uint64_t row = 2 * (uint64_t)k.Dp;
+        const cuuint64_t dims[4] = {(cuuint64_t)k.Dp, (cuuint64_t)k.s32, 32, (cuuint64_t)k.nseg};
+        const cuuint64_t strides[3] = {(cuuint64_t)k.f * row, (cuuint64_t)k.s32 * k.f * row, (cuuint64_t)k.seg * row};
+        const cuuint32_t box[4] = {64, 1, 32, 1};
+        if (!knn_map(&mx, k.xh, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4, dims, strides, box, true) ||
+            !knn_map_bits(&mb, k.bm_sample, k.nws, k.Qcap))
+            return cudaErrorNotSupported;
+        a.ntp = (long long)k.nseg * k.s32 / (BN / 32);
+        a.w = k.w_sample;
+    } else {
+        if (!knn_map_rows(&mx, k.xh, k.Dp, k.N, BN) || !knn_map_bits(&mb, k.bm, k.nwp, k.Qcap))
+            return cudaErrorNotSupported;
+        a.ntp = ((long long)k.N + BN - 1) / BN;
+        a.w = k.w;
+    }
+    k_knn_tc<kSample, kStream><<<k.grid, kKnnThreads, k.smem, s>>>(mq, mx, mb, a);
     return cudaGetLastError();
 }
 
+size_t merge_smem(int D) { return 8 * (size_t)(kKnnMaxSurvivors + kKnnMaxChosen) + 4 * (size_t)D; }
+
 }  // namespace
 
-float knn_bound_factor(int D) {
-    // split residue (three products) and accumulation of 3D products, as in
-    // the projection's bound; the exact distance's own FP32 lane order
-    // (gamma_n, n = ceil(D/8) + 6, twice: d~ <= 2 S); norms and key
-    // arithmetic ((D + 16) u); all with a 10 % margin.
-    const double u = std::ldexp(1.0, -24), u23 = std::ldexp(1.0, -23), u16 = std::ldexp(1.0, -16);
-    const double kappa = 1.25 * (3.02 * u16 + (3.0 * D + 16) * u23);
-    const double nn = (double)((D + 7) / 8 + 6);
-    const double gamma = nn * u / (1.0 - nn * u);
-    return std::nextafter((float)(1.1 * (kappa + 2.0 * gamma + (D + 16) * u)), INFINITY);
+float knn_gamma(int D) {
+    // accumulation of D products (one 2^-23 step per summed product), norms
+    // and key arithmetic ((D + 16) + 8 roundings), the exact distance's own
+    // FP32 lane order (gamma_n, n = ceil(D/8) + 6, twice: d <= 2 S); all with
+    // margins.
+    const double u = std::ldexp(1.0, -24), nn = (double)((D + 7) / 8 + 6);
+    const double gn = nn * u / (1.0 - nn * u);
+    return std::nextafter((float)(1.1 * (1.25 * (D + 16) * 2.0 * u + 2.0 * gn + (D + 24) * u)), INFINITY);
 }
 
-bool knn_plan(KnnSearch& k, int max_smem) {
-    if (k.D < 1 || k.D > 128 || k.K < 1 || k.K > kMaxKnnK || k.N < 1) return false;
+bool knn_plan(KnnSearch& k, int max_smem, size_t bitmap_smem) {
+    if (k.D < 1 || k.D > kMaxKnnD || k.K < 1 || k.K > kMaxKnnK || k.N < 1) return false;
+    // A sample of N / f points bounds the K-th distance when it has at least
+    // 3 K chunks of 32; below 128 K points even the whole dataset is too coarse
+    // a sample, and without a limit every candidate survives: allowed only
+    // where all of them fit the merge.
+    if (k.N < 128ll * k.K && k.N > kKnnMaxSurvivors) return false;
     k.Dp = (k.D + 63) / 64 * 64;
-    k.kl_exact = k.K;
-    // bound form: K plus a margin of entries that the error bound may reorder;
-    // CULSH_KNN_LIST_MARGIN sets the margin (the tests use 0 to reach the
-    // exact fallback)
-    int margin = std::max(8, k.K / 2);
-    if (const char* e = getenv("CULSH_KNN_LIST_MARGIN")) margin = std::max(0, atoi(e));
-    k.kl_bound = std::min(kMaxKnnK, k.K + margin);
-    k.ops_exact = k.ops_bound = 0;
-    // the deepest point-tile ring (1 to 4 stages) that fits
-    for (int ops = 4; ops >= 1 && !k.ops_exact; --ops) {
-        const size_t sm = knn_smem(true, k.Dp, k.kl_exact, ops, kEpStages);
-        if (sm <= (size_t)max_smem) {
-            k.ops_exact = ops;
-            k.smem_exact = sm;
+    k.ops = 0;
+    for (int ops = kMaxOpStages; ops >= 2 && !k.ops; --ops)
+        if (knn_smem(k.Dp, ops) <= (size_t)max_smem) {
+            k.ops = ops;
+            k.smem = knn_smem(k.Dp, ops);
         }
-    }
-    for (int ops = 4; ops >= 1 && !k.ops_bound; --ops) {
-        const size_t sm = knn_smem(false, k.Dp, k.kl_bound, ops, kEpStages);
-        if (sm <= (size_t)max_smem) {
-            k.ops_bound = ops;
-            k.smem_bound = sm;
-        }
-    }
-    // the bound form serves every search; the exact form only when it fits too
-    if (!k.ops_bound) return false;
-    if (!k.ops_exact) k.exact_possible = 0;
+    if (!k.ops) return false;
     k.nwp = (int)((((int64_t)k.N + 31) / 32 + 3) / 4 * 4);
+    k.f = 0;
+    if (k.N >= 128ll * k.K) {
+        // survivors are about f K: 1,024 of them at most, and a sixteenth of
+        // the points (6 % more tensor work) is enough for any K up to 64
+        k.f = 16;
+        while (k.f > 1 && (k.f * k.K > 1024 || k.N / (32ll * k.f) < 3ll * k.K)) k.f >>= 1;
+    }
+    // segments of the membership kernel: as few as fit a block's bitmap (the
+    // last one also takes what rounding leaves over)
+    const int step = 128 * std::max(k.f, 1);
+    const int64_t bits = (int64_t)bitmap_smem * 8 - 128;
+    if (bits < 4 * step) return false;
+    for (k.nseg = 1;; ++k.nseg) {
+        k.seg = (int)((int64_t)k.N / k.nseg / step * step);
+        if ((int64_t)k.N - (int64_t)(k.nseg - 1) * k.seg <= bits) break;
+    }
+    if (k.seg == 0) {   // fewer points than a sample step: one segment, no sample
+        k.seg = k.N;
+        k.f = 0;
+    }
+    k.s32 = k.f ? k.seg / (32 * k.f) : 0;
+    k.nws = k.nseg * k.s32;
+    // List capacity: within 512 MB of lists, at least 64 entries, never more
+    // than a CTA's range can hold. CULSH_KNN_LIST_MARGIN sets it to K plus a
+    // margin (the tests use 0 to reach the exact scan).
+    const int64_t ntp = ((int64_t)k.N + BN - 1) / BN, nqt = k.Qcap / MQ;
+    const int64_t sets = std::min<int64_t>(k.grid, nqt * ntp) + nqt;
+    int64_t lc = std::min<int64_t>(1024, (int64_t(512) << 20) / (8 * sets * NT));
+    lc = std::min<int64_t>(std::max<int64_t>(lc, 64), BN * (nqt * ntp / k.grid / NCH + 2));
+    if (const char* e = getenv("CULSH_KNN_LIST_MARGIN")) lc = k.K + std::max(0, atoi(e));
+    k.list_cap = (int)lc;
     return true;
 }
 
 size_t knn_part_lists(const KnnSearch& k) {
-    // list sets blockIdx.x + query tile < grid + Qcap / MQ, with MQ rows and
-    // NCH column slices each
-    const size_t e = (size_t)(k.grid + k.Qcap / kMqExact) * kMqExact * kNchExact;
-    const size_t b = (size_t)(k.grid + k.Qcap / kMqBound) * kMqBound * kNchBound;
-    return std::max(e, b);
+    const int64_t ntp = ((int64_t)k.N + BN - 1) / BN, nqt = k.Qcap / MQ;
+    return (size_t)(std::min<int64_t>(k.grid, nqt * ntp) + nqt) * NT;
 }
-size_t knn_part_entries(const KnnSearch& k) {
-    return knn_part_lists(k) * (size_t)std::max(k.kl_exact, k.kl_bound);
-}
+size_t knn_part_entries(const KnnSearch& k) { return knn_part_lists(k) * (size_t)k.list_cap; }
 
-cudaError_t launch_knn_rows_dataset(const float* X, int64_t N, int D, int Dp, void* xh, void* xl, float* w_exact,
-                                    float* w_bound, int64_t pad, float C, KnnState* st, cudaStream_t s) {
+cudaError_t launch_knn_rows_dataset(const float* X, int64_t N, int D, int Dp, void* xh, float* w, int64_t pad,
+                                    KnnState* st, cudaStream_t s) {
+    const int64_t n = N * D;
+    k_knn_scan<<<(unsigned)std::min<int64_t>((n + 1023) / 1024, 152 * 16), 256, 0, s>>>(X, n, st);
     const int blocks = (int)std::min<int64_t>((pad * 32 + 255) / 256, 152 * 16);
-    k_knn_rows<<<blocks, 256, 0, s>>>(X, D, Dp, nullptr, nullptr, N, pad, 1, static_cast<__nv_bfloat16*>(xh),
-                                      static_cast<__nv_bfloat16*>(xl), w_exact, w_bound, C, st, nullptr);
+    k_knn_rows<<<blocks, 256, 0, s>>>(X, N, D, Dp, pad, static_cast<__half*>(xh), w, st);
     return cudaGetLastError();
 }
 
-int knn_launches(const KnnSearch& k) { return 3 + (k.exact_possible ? 1 : 0); }
+int knn_launches(const KnnSearch& k) { return k.f > 0 ? 5 : 3; }
 
 cudaError_t launch_knn_search(const KnnSearch& k, cudaStream_t s) {
-    // query rows in dense-list order, zero rows up to the next tile
     const int qblocks = (int)std::min<int64_t>(((int64_t)k.Qcap * 32 + 255) / 256, 152 * 8);
-    k_knn_rows<<<qblocks, 256, 0, s>>>(k.queries, k.D, k.Dp, k.dense_q, k.n_dense, 0, 0, std::max(kMqExact, kMqBound),
-                                       static_cast<__nv_bfloat16*>(k.qh), static_cast<__nv_bfloat16*>(k.ql), k.qsq,
-                                       k.qbase, k.C, k.qstate, k.qbound);
+    k_knn_qrows<<<qblocks, 256, 0, s>>>(k);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    if (k.exact_possible) {
-        CUtensorMap mxh;
-        if (!knn_map(&mxh, k.xh, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)k.Dp, (uint64_t)k.N, 64, kBnExact,
-                     true))
-            return cudaErrorNotSupported;
-        e = launch_knn_form<kBnExact, kMqExact, kNepiExact, true>(k, mxh, mxh, s);
+    const bool stream = k.Dp > kResidentD;
+    if (k.f > 0) {
+        e = stream ? launch_knn_pass<true, true>(k, s) : launch_knn_pass<true, false>(k, s);
         if (e != cudaSuccess) return e;
+        const unsigned lb = (unsigned)((k.Qcap + LW - 1) / LW);
+        if (k.K <= 64) k_knn_limit<32><<<lb, 32 * LW, 0, s>>>(k);
+        else if (k.K <= 128) k_knn_limit<64><<<lb, 32 * LW, 0, s>>>(k);
+        else k_knn_limit<128><<<lb, 32 * LW, 0, s>>>(k);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
-    CUtensorMap mxh, mxl;
-    if (!knn_map(&mxh, k.xh, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)k.Dp, (uint64_t)k.N, 64, kBnBound, true) ||
-        !knn_map(&mxl, k.xl, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, (uint64_t)k.Dp, (uint64_t)k.N, 64, kBnBound, true))
-        return cudaErrorNotSupported;
-    e = launch_knn_form<kBnBound, kMqBound, kNepiBound, false>(k, mxh, mxl, s);
+    e = stream ? launch_knn_pass<false, true>(k, s) : launch_knn_pass<false, false>(k, s);
     if (e != cudaSuccess) return e;
-    const int mblocks = (int)std::min<int64_t>(((int64_t)k.Qcap + MERGE_WARPS - 1) / MERGE_WARPS, 152 * 16);
-    k_knn_merge<<<mblocks, 32 * MERGE_WARPS, 0, s>>>(k);
+    static std::atomic<size_t> cap{0};
+    const size_t smem = merge_smem(k.D);
+    if ((e = opt_in_smem(k_knn_merge, smem, cap)) != cudaSuccess) return e;
+    k_knn_merge<<<(unsigned)std::min<int64_t>(k.Qcap, 152 * 16), MT, smem, s>>>(k);
     return cudaGetLastError();
 }
 

@@ -52,6 +52,7 @@ struct Slot {
     culsh_search* s = nullptr;
     cudaStream_t st = nullptr;
     int K = 0, T = 0;                      // the search object's current reset
+    bool tc = true;                        // the batch's dense queries may take the tensor-core path
     float* d_q = nullptr;
     int* d_ids = nullptr;
     float* d_d = nullptr;
@@ -176,6 +177,13 @@ int run_batch(culsh_server* v, Slot* sl, const std::vector<ReqPtr>& batch) {
         sl->K = K;
         sl->T = T;
     }
+    culsh_tuning tune;
+    rc = culsh_search_get_tuning(sl->s, &tune);
+    if (rc == CULSH_OK && tune.dense_tc != (sl->tc ? 1 : 0)) {
+        tune.dense_tc = sl->tc ? 1 : 0;
+        rc = culsh_search_set_tuning(sl->s, &tune);
+    }
+    if (rc != CULSH_OK) return rc;
     rc = culsh_search_run_device(sl->s, sl->d_q, (int)Q, sl->d_ids, sl->d_d, sl->st);
     if (rc != CULSH_OK) return rc;
     if (cudaMemcpyAsync(sl->h_ids, sl->d_ids, Q * K * 4, cudaMemcpyDeviceToHost, sl->st) != cudaSuccess ||
@@ -271,10 +279,14 @@ void scheduler_loop(culsh_server* v) {
                 break;
             }
         if (!sl) sl = idle();
+        // A request that fits the budget only without the tensor-core path's
+        // buffers runs without that path.
+        bool tc = true;
         auto need_of = [&](size_t q) {
-            return culsh_search_estimate_bytes(v->ix, (int)q, r0->K, r0->T) +
+            return culsh::search_estimate(v->ix, (int)q, r0->K, r0->T, tc) +
                    slot_buffer_bytes(q, q, (size_t)r0->K, v->D);
         };
+        tc = need_of((size_t)r0->Q) <= v->budget;
         long long need = need_of(Qb);
         auto fits = [&]() { return total_reserved(v) - sl->reserved + std::max(need, sl->reserved) <= v->budget; };
         if (!fits()) {
@@ -323,6 +335,7 @@ void scheduler_loop(culsh_server* v) {
             if (it != v->pending.end()) v->pending.erase(it);
         }
         sl->batch = batch;
+        sl->tc = tc;
         sl->busy = true;
         sl->reserved = std::max(sl->reserved, need);
         ++v->in_flight;

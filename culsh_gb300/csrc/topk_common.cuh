@@ -73,6 +73,46 @@ __device__ __forceinline__ void set_insert(uint32_t* hset, uint32_t mask, uint32
     }
 }
 
+// Exact FP32 squared distance of row x to the query qs (shared memory) in the
+// reference lane order (cuLSH_Kernels.cu:301-348), by the two lanes (vec:
+// D % 4 == 0, four of the eight lane partials each from 16-byte loads) or
+// eight lanes that share the row; lanes without a row pass on = false. Every
+// lane of the warp calls it and every lane of a group gets the distance.
+__device__ __forceinline__ float row_distance(const float* __restrict__ x, int D, const float* qs, bool vec, bool on) {
+    const int lane = threadIdx.x & 31;
+    if (vec) {
+        float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+        if (on) {
+#pragma unroll 8
+            for (int c = 4 * (lane & 1); c < D; c += 8) {
+                const float4 v = __ldg(reinterpret_cast<const float4*>(x + c));
+                const float4 qv = *reinterpret_cast<const float4*>(qs + c);
+                const float d0 = __fsub_rn(qv.x, v.x), d1 = __fsub_rn(qv.y, v.y);
+                const float d2 = __fsub_rn(qv.z, v.z), d3 = __fsub_rn(qv.w, v.w);
+                s0 = __fmaf_rn(d0, d0, s0);
+                s1 = __fmaf_rn(d1, d1, s1);
+                s2 = __fmaf_rn(d2, d2, s2);
+                s3 = __fmaf_rn(d3, d3, s3);
+            }
+        }
+        const float o0 = __shfl_xor_sync(0xffffffffu, s0, 1), o1 = __shfl_xor_sync(0xffffffffu, s1, 1);
+        const float o2 = __shfl_xor_sync(0xffffffffu, s2, 1), o3 = __shfl_xor_sync(0xffffffffu, s3, 1);
+        const float t0 = __fadd_rn(s0, o0), t1 = __fadd_rn(s1, o1), t2 = __fadd_rn(s2, o2), t3 = __fadd_rn(s3, o3);
+        return __fadd_rn(__fadd_rn(t0, t2), __fadd_rn(t1, t3));
+    }
+    float s = 0.f;
+    if (on) {
+#pragma unroll 4
+        for (int c = lane & 7; c < D; c += 8) {
+            const float df = __fsub_rn(qs[c], __ldg(x + c));
+            s = __fmaf_rn(df, df, s);
+        }
+    }
+    const float t = __fadd_rn(s, __shfl_xor_sync(0xffffffffu, s, 4));
+    const float u = __fadd_rn(t, __shfl_xor_sync(0xffffffffu, t, 2));
+    return __fadd_rn(u, __shfl_xor_sync(0xffffffffu, u, 1));
+}
+
 // Exact FP32 squared distances, in the reference lane order
 // (cuLSH_Kernels.cu:301-348), of list entries [0, cnt) into this warp's sorted
 // top-K list (wd, wi, n, thr_d, thr_i). Entry j is candidate ci = idx_of(j)

@@ -317,3 +317,84 @@ def test_bucket_rows_graph_replay(culsh, all_dense, monkeypatch):
         modes.append(st.profile()["graph_mode"])
         assert st.profile()["bucket_rows"] > 0
     assert modes[0] == 1 and modes[-1] == 2
+
+
+def _mixture(N, D, Q, seed, scale=8.0, clusters=40):
+    rng = np.random.default_rng(seed)
+    centers = rng.normal(0, scale, (clusters, D)).astype(np.float32)
+    X = centers[rng.integers(0, clusters, N)] + rng.normal(0, 1, (N, D)).astype(np.float32)
+    Qm = centers[rng.integers(0, clusters, Q)] + rng.normal(0, 1, (Q, D)).astype(np.float32)
+    return X.astype(np.float32), Qm.astype(np.float32), rng
+
+
+# (points, dimensions, queries, neighbours): the largest dimension with the
+# query tile resident in shared memory and the first streamed one, D % 4 != 0,
+# one- and many-slab operands, the largest dimension and the first declined;
+# every sample step (16 to 1 points, none), the largest K and the first
+# declined; a query tile's half filled exactly and crossed.
+@pytest.mark.parametrize("N,D,Q,K", [
+    (20_011, 128, 128, 10), (20_011, 129, 129, 10), (9_001, 130, 257, 10), (6_007, 960, 40, 10),
+    (3_001, 2048, 20, 5), (3_001, 2049, 20, 5), (33_000, 17, 90, 100), (66_000, 20, 40, 256),
+    (66_000, 20, 40, 257), (12_800, 24, 60, 100), (4_096, 24, 60, 100), (2_560, 64, 33, 20),
+    (100_003, 33, 300, 1)])
+def test_sample_list_and_operand_shapes(culsh, all_dense, N, D, Q, K):
+    """The sample, list and operand forms of the tensor-core k-NN at the edges
+    of their rules, on real-valued data (certified bounds, exact distances)."""
+    X, Qm, rng = _mixture(N, D, Q, 31 + D + K)
+    L, M, T, W = 4, 3, 4, 3.0 * np.sqrt(2.0 * D)
+    A = rng.normal(0, 1, (L, M, D)).astype(np.float32)
+    b = (rng.random((L, M)) * W).astype(np.float32)
+    want = _oracle_case(X, Qm, A, b, W, K, T)
+    ht = culsh.HashTables()
+    ht.reset(N, D, L, M, W, A=A, b=b)
+    ht.index(X)
+    st = _search(culsh, ht, Qm, X, K, T, dense_tc=1)
+    _check_against(st, want, Q, X)
+    pr = st.profile()
+    served = D <= 2048 and K <= 256
+    assert pr["knn_queries"] == (int((want["nonunique"] > 0).sum()) if served else 0)
+    assert pr["knn_fallback"] == 0
+
+
+def test_points_beyond_one_bitmap(culsh):
+    """More points than one block's bitmap holds: membership rows made in
+    segments, buckets cut at the segments' ends, sample chunks per segment."""
+    N, D, Q, K, T = 3_700_001, 4, 60, 20, 3
+    X, Qm, rng = _mixture(N, D, Q, 5, scale=30.0, clusters=25)
+    L, M, W = 2, 2, 20.0
+    A = rng.normal(0, 1, (L, M, D)).astype(np.float32)
+    b = (rng.random((L, M)) * W).astype(np.float32)
+    want = _oracle_case(X, Qm, A, b, W, K, T)
+    ht = culsh.HashTables()
+    ht.reset(N, D, L, M, W, A=A, b=b)
+    ht.index(X)
+    st = _search(culsh, ht, Qm, X, K, T, dense_tc=1)
+    _check_against(st, want, Q, X)
+    assert st.profile()["knn_queries"] > Q // 2
+
+
+@pytest.mark.parametrize("scale", [1e-9, 1.0, 1e11, 1e14])
+def test_magnitudes_and_outlier_rows(culsh, all_dense, scale):
+    """Magnitudes far from one (operands are scaled by powers of two), a few
+    rows a thousand times larger or smaller than the rest, zero rows, and
+    queries that are zero, tiny, or beyond the path's range (scanned exactly).
+    A dataset with a magnitude above 1e17 is left to the SIMT kernel."""
+    X, Qm, rng = _mixture(8_000, 32, 64, 9)
+    X[::997] *= 1000.0
+    X[1::997] *= 1e-3
+    X[2::997] = 0.0
+    Qm[0] = 0.0
+    Qm[1] *= 1e-6
+    X, Qm = (X * np.float32(scale)).astype(np.float32), (Qm * np.float32(scale)).astype(np.float32)
+    Qm[2] = np.float32(3e17)
+    L, M, T, K, W = 4, 3, 6, 12, 25.0 * scale
+    A = rng.normal(0, 1, (L, M, 32)).astype(np.float32)
+    b = (rng.random((L, M)) * W).astype(np.float32)
+    want = _oracle_case(X, Qm, A, b, W, K, T)
+    ht = culsh.HashTables()
+    ht.reset(X.shape[0], 32, L, M, W, A=A, b=b)
+    ht.index(X)
+    st = _search(culsh, ht, Qm, X, K, T, dense_tc=1)
+    _check_against(st, want, Qm.shape[0], X)
+    served = np.abs(X).max() <= 1e17
+    assert st.profile()["knn_queries"] == (int((want["nonunique"] > 0).sum()) if served else 0)

@@ -618,7 +618,7 @@ int sort_keys(culsh_index* ix, int N, int passes, cudaStream_t st, const uint32_
     sb.h_hist_words = ix->h_sort_hist.n;
     const int top_passes = passes - 4 * (KW - 1);
     ix->sort_form = 0;
-    if (KW >= 2 && top_passes >= 1 && !getenv("CULSH_SORT_ALL_WORDS")) {
+    if (KW >= 2 && KW <= 4 && top_passes >= 1 && !getenv("CULSH_SORT_ALL_WORDS")) {
         SortBuffers sa = sb;
         sa.keys[0] = ix->ws_keys[0].p + (KW - 1) * LN;   // read first, then a ping-pong slot
         sa.keys[1] = ix->ws_keys[1].p + (KW - 1) * LN;

@@ -72,6 +72,8 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* ws, ui
     return r;
 }
 
+// WIDE: keys of more than 128 bits (KW > 4), assembled word by word.
+template <bool WIDE>
 __global__ void k_pack_keys(const int32_t* __restrict__ codes, int64_t N, int L, int M, int KW,
                             const int32_t* __restrict__ cmin, const uint8_t* __restrict__ fbits,
                             const uint16_t* __restrict__ foff, uint32_t* __restrict__ keys,
@@ -81,6 +83,17 @@ __global__ void k_pack_keys(const int32_t* __restrict__ codes, int64_t N, int L,
          idx += (int64_t)gridDim.x * blockDim.x) {
         const int l = (int)(idx / N);
         const int64_t n = idx - (int64_t)l * N;
+        if constexpr (WIDE) {
+            uint32_t key[kMaxKW] = {};
+            for (int m = 0; m < M; ++m) {
+                const int c = l * M + m;
+                const int bits = __ldg(fbits + c);
+                if (bits) key_put(key, __ldg(foff + c), bits, (uint32_t)(codes[(int64_t)c * N + n] - __ldg(cmin + c)));
+            }
+            for (int w = 0; w < KW; ++w) keys[w * LN + idx] = key[w];
+            vals[idx] = (uint32_t)n;
+            continue;
+        }
         // fields are contiguous, column M - 1 at bit 0 and column 0 on top:
         // shift each column in after the previous one (registers only)
         unsigned __int128 kk = 0;
@@ -91,7 +104,7 @@ __global__ void k_pack_keys(const int32_t* __restrict__ codes, int64_t N, int L,
             kk = (kk << bits) | (uint32_t)(codes[(int64_t)c * N + n] - __ldg(cmin + c));
         }
 #pragma unroll
-        for (int w = 0; w < kMaxKW; ++w)
+        for (int w = 0; w < 4; ++w)
             if (w < KW) keys[w * LN + idx] = (uint32_t)(kk >> (32 * w));
         vals[idx] = (uint32_t)n;
     }
@@ -594,6 +607,7 @@ __global__ void k_bucket_sizes(const uint64_t* __restrict__ boff, const uint32_t
     }
 }
 
+template <bool WIDE>   // KW > 4
 __global__ void k_hash_build(const uint64_t* __restrict__ boff, const uint32_t* __restrict__ ukeys, int M, int KW,
                              const uint16_t* __restrict__ foff, const uint8_t* __restrict__ fbits,
                              const unsigned long long* __restrict__ rmul, const uint64_t* __restrict__ hoff,
@@ -605,17 +619,24 @@ __global__ void k_hash_build(const uint64_t* __restrict__ boff, const uint32_t* 
     const int64_t B = (int64_t)(boff[l + 1] - boff[l]);
     if (j >= B) return;
     const uint32_t* key = ukeys + (boff[l] + j) * KW;
-    unsigned __int128 kk = 0;
-    for (int w = KW - 1; w >= 0; --w) kk = (kk << 32) | key[w];
     const uint32_t gmask = hmask[l];
     uint64_t hs = 0;   // additive lookup hash over the key's fields
-    // fields are contiguous from bit 0 (column M - 1) upwards
-    for (int m = M - 1; m >= 0; --m) {
-        const int c = l * M + m;
-        const int bits = __ldg(fbits + c);
-        const uint32_t f = bits ? (uint32_t)kk & (bits == 32 ? 0xFFFFFFFFu : ((1u << bits) - 1u)) : 0u;
-        kk >>= bits;
-        hs += (uint64_t)f * __ldg(rmul + c);
+    if constexpr (WIDE) {
+        for (int m = 0; m < M; ++m) {
+            const int c = l * M + m;
+            hs += (uint64_t)key_get(key, __ldg(foff + c), __ldg(fbits + c)) * __ldg(rmul + c);
+        }
+    } else {
+        unsigned __int128 kk = 0;
+        for (int w = KW - 1; w >= 0; --w) kk = (kk << 32) | key[w];
+        // fields are contiguous from bit 0 (column M - 1) upwards
+        for (int m = M - 1; m >= 0; --m) {
+            const int c = l * M + m;
+            const int bits = __ldg(fbits + c);
+            const uint32_t f = bits ? (uint32_t)kk & (bits == 32 ? 0xFFFFFFFFu : ((1u << bits) - 1u)) : 0u;
+            kk >>= bits;
+            hs += (uint64_t)f * __ldg(rmul + c);
+        }
     }
     const uint64_t hh = hash_finish(hs);
     const uint32_t h = (uint32_t)hh;
@@ -762,7 +783,8 @@ cudaError_t launch_pack_keys(const int32_t* codes, int64_t N, int L, int M, int 
                              cudaStream_t st) {
     const int64_t LN = (int64_t)L * N;
     const int grid = (int)std::min<int64_t>((LN + NT - 1) / NT, 152 * 32);
-    k_pack_keys<<<grid, NT, 0, st>>>(codes, N, L, M, KW, cmin, fbits, foff, keys, vals);
+    if (KW > 4) k_pack_keys<true><<<grid, NT, 0, st>>>(codes, N, L, M, KW, cmin, fbits, foff, keys, vals);
+    else k_pack_keys<false><<<grid, NT, 0, st>>>(codes, N, L, M, KW, cmin, fbits, foff, keys, vals);
     return cudaGetLastError();
 }
 
@@ -888,8 +910,13 @@ cudaError_t launch_hash_build(const uint64_t* boff, const uint32_t* ukeys, int L
                               uint32_t* filt, const uint64_t* fl_off, const uint32_t* fl_mask, int* err,
                               cudaStream_t st) {
     if (maxB <= 0) return cudaSuccess;
-    k_hash_build<<<dim3(blocks_for(maxB), L), NT, 0, st>>>(boff, ukeys, M, KW, foff, fbits, rmul, hoff, hmask,
-                                                          hslots, filt, fl_off, fl_mask, err);
+    const dim3 grid(blocks_for(maxB), L);
+    if (KW > 4)
+        k_hash_build<true><<<grid, NT, 0, st>>>(boff, ukeys, M, KW, foff, fbits, rmul, hoff, hmask, hslots, filt, fl_off,
+                                               fl_mask, err);
+    else
+        k_hash_build<false><<<grid, NT, 0, st>>>(boff, ukeys, M, KW, foff, fbits, rmul, hoff, hmask, hslots, filt, fl_off,
+                                                fl_mask, err);
     return cudaGetLastError();
 }
 

@@ -77,3 +77,26 @@ def test_all_words_form_agrees(culsh, monkeypatch):
     monkeypatch.setenv("CULSH_SORT_ALL_WORDS", "1")
     p = check(culsh, X, A, b, W)
     assert p["sort_form"] == 0
+
+
+@pytest.mark.parametrize("M,W", [(10, 0.02), (11, 0.02), (16, 0.02), (20, 0.02)])
+def test_keys_wider_than_128_bits(culsh, M, W):
+    """Bucket keys of 4 to 8 words: buckets, codes and a search whose queries
+    are indexed points, against the oracle."""
+    rng = np.random.default_rng(M)
+    N, D, L, T, K = 5000, 32, 3, 4, 5
+    X = rng.normal(0, 1, (N, D)).astype(np.float32)
+    X[N // 2:] = X[:N // 2] + rng.normal(0, 1e-5, (N // 2, D)).astype(np.float32)
+    A = rng.normal(0, 1, (L, M, D)).astype(np.float32)
+    b = (rng.random((L, M)) * W).astype(np.float32)
+    p = check(culsh, X, A, b, W)
+    assert p["key_words"] >= (5 if M > 11 else 4)
+    ht = culsh.HashTables()
+    ht.reset(N, D, L, M, W, A=A, b=b)
+    ht.index(X)
+    st = culsh.SearchTables()
+    st.reset(ht, K, T)
+    st.search(X[:200], dataset=X)
+    want = oracle.search(oracle.build_index(X, A, b, W), X, X[:200], K, T)
+    np.testing.assert_array_equal(st.getKnnIds(), want["knn_ids"])
+    np.testing.assert_array_equal(st.getKnnDistances(), want["knn_dists"])

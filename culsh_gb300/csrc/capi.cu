@@ -201,7 +201,7 @@ struct culsh_index {
     int sort_passes = 0;
     cudaEvent_t bev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};   // build stage boundaries
     bool built_once = false;
-    DevBuf<uint32_t> ws_keys[2], ws_vals, ws_hist, ws_base, ws_status, ws_tcnt, ws_toff, ws_nb;
+    DevBuf<uint32_t> ws_keys[2], ws_low, ws_vals, ws_hist, ws_base, ws_status, ws_tcnt, ws_toff, ws_nb;
     PinBuf<uint32_t> h_sort_hist;
     DevBuf<unsigned long long> ws_run_pos;
     DevBuf<uint32_t> ws_run_len;
@@ -365,12 +365,21 @@ int read_err_flag(culsh_index* ix, cudaStream_t st, const char* what) {
     return CULSH_OK;
 }
 
+// Whether keys of KW words and `bits` bits are sorted top word first: two to
+// four words, and more below the top word than one digit pass over the whole
+// key (at most 8 bits: five passes of 12 bytes a point against four of 8 and
+// the runs' ordering, with nothing to fall back from).
+bool sort_top_word(int KW, int bits) {
+    return KW >= 2 && KW <= 4 && bits > 40 && !getenv("CULSH_SORT_ALL_WORDS");
+}
+
 // Bit widths and offsets of each column's field: column 0 most significant.
 int compute_layout(culsh_index* ix, int* passes) {
     const int L = ix->L, M = ix->M;
     ix->h_fbits.assign((size_t)L * M, 0);
     ix->h_foff.assign((size_t)L * M, 0);
     int smax = 0;
+    std::vector<int> total(L, 0);
     for (int l = 0; l < L; ++l) {
         int off = 0;
         for (int m = M - 1; m >= 0; --m) {
@@ -383,6 +392,7 @@ int compute_layout(culsh_index* ix, int* passes) {
             ix->h_foff[c] = (uint16_t)off;
             off += bits;
         }
+        total[l] = off;
         smax = std::max(smax, off);
     }
     if (smax > 32 * kMaxKW)
@@ -390,6 +400,19 @@ int compute_layout(culsh_index* ix, int* passes) {
                     32 * kMaxKW);
     ix->KW = std::max(1, (smax + 31) / 32);
     *passes = (smax + 7) / 8;
+    if (sort_top_word(ix->KW, smax)) {
+        // top-word-first form: every table's fields end at the top of its key,
+        // so that the top word holds 32 leading bits. (Fields from bit 0 up had
+        // left it what was over, 8 to 16 bits at 40 and 112 key bits: its runs
+        // were long and the sort fell back to passes over every word.)
+        for (int l = 0; l < L; ++l)
+            for (int m = 0; m < M; ++m) {
+                // a column of one code has no field: keep its (unused) offset inside the key
+                const int off = ix->h_foff[l * M + m] + 32 * ix->KW - total[l];
+                ix->h_foff[l * M + m] = (uint16_t)std::min(off, 32 * ix->KW - 1);
+            }
+        *passes = 4 * ix->KW;
+    }
     return CULSH_OK;
 }
 
@@ -594,17 +617,32 @@ int project_tensor_cores(culsh_index* ix, const float* dX, cudaStream_t st, bool
     return CULSH_OK;
 }
 
-// Orders every table's points by packed key (ties by id), the order of the
-// reference's LSD row sort (cuLSH_Indexing.cu:71-93). Multi-word keys first
-// take the digit passes over the top word alone (moving 8 bytes per point a
-// pass instead of 4 (KW + 1)), gather the lower words into sorted order, and
-// order each run of equal top words by (lower words, id); a run longer than
+// Packs every point's key and orders every table's points by it (ties by id),
+// the order of the reference's LSD row sort (cuLSH_Indexing.cu:71-93). Keys of
+// two to four words (sort_top_word) take the digit passes over the top word
+// alone (moving 8 bytes per point a pass instead of 4 (KW + 1)) and then order
+// each run of equal top words by (lower words, id); a run longer than
 // run_max_len() or more runs than the lists hold sends the build through the
-// passes over every word instead. On return *skeys holds the sorted keys
-// ([KW][L*N]) and ix->ids the sorted ids.
-int sort_keys(culsh_index* ix, int N, int passes, cudaStream_t st, const uint32_t** skeys) {
+// passes over every word instead. On return *sk describes the sorted keys and
+// ix->ids holds the sorted ids.
+int sort_keys(culsh_index* ix, int N, int passes, cudaStream_t st, SortedKeys* sk) {
     const int L = ix->L, KW = ix->KW;
     const size_t LN = (size_t)L * N;
+    const bool top_first = passes == 4 * KW && sort_top_word(KW, 32 * KW);
+    const int lw = low_row_words(KW);
+    CU_TRY(ix->ws_vals.reserve(LN));
+    CU_TRY(ix->ids.reserve(LN));
+    CU_TRY(ix->ws_keys[0].reserve(top_first ? LN : LN * KW));
+    CU_TRY(ix->ws_keys[1].reserve(top_first ? LN : LN * KW));
+    if (top_first) CU_TRY(ix->ws_low.reserve(LN * lw));
+    CU_TRY(launch_pack_keys(ix->ws_codes.p, N, L, ix->M, KW, ix->cmin.p, ix->fbits.p, ix->foff.p, ix->ws_keys[0].p,
+                            ix->ids.p, top_first ? ix->ws_low.p : nullptr, lw, st));
+    const int hp = std::max(passes, 1);
+    CU_TRY(ix->ws_hist.reserve((size_t)L * hp * 256));
+    CU_TRY(ix->ws_base.reserve((size_t)L * hp * 256));
+    CU_TRY(ix->ws_status.reserve(sort_status_words(N, L)));
+    CU_TRY(ix->h_sort_hist.reserve((size_t)L * hp * 256));
+    CU_TRY(cudaEventRecord(ix->bev[2], st));
     SortBuffers sb;
     sb.keys[0] = ix->ws_keys[0].p;
     sb.keys[1] = ix->ws_keys[1].p;
@@ -616,21 +654,14 @@ int sort_keys(culsh_index* ix, int N, int passes, cudaStream_t st, const uint32_
     sb.err = ix->err.p;
     sb.h_hist = ix->h_sort_hist.p;
     sb.h_hist_words = ix->h_sort_hist.n;
-    const int top_passes = passes - 4 * (KW - 1);
     ix->sort_form = 0;
-    if (KW >= 2 && KW <= 4 && top_passes >= 1 && !getenv("CULSH_SORT_ALL_WORDS")) {
-        SortBuffers sa = sb;
-        sa.keys[0] = ix->ws_keys[0].p + (KW - 1) * LN;   // read first, then a ping-pong slot
-        sa.keys[1] = ix->ws_keys[1].p + (KW - 1) * LN;
-        bool alt = false;
-        CU_TRY(run_segmented_sort(sa, N, L, 1, top_passes, &alt, st));
-        const uint32_t* top = alt ? sa.keys[1] : sa.keys[0];
+    bool alt = false;
+    if (top_first) {
+        CU_TRY(run_segmented_sort(sb, N, L, 1, 4, &alt, st));
+        const uint32_t* top = sb.keys[alt ? 1 : 0];
         if (alt) ix->ids.swap(ix->ws_vals);
-        // ws_keys[0]'s lower words are still in point order; its top slot may
-        // hold sorted top words (read before being overwritten: other buffer)
-        CU_TRY(launch_gather_lower(ix->ws_keys[0].p, ix->ids.p, top, N, L, KW, ix->ws_keys[1].p, st));
-        const unsigned int tcap = (unsigned int)std::min<size_t>(LN / 2 + 1, (size_t)1 << 23);
-        const unsigned int scap = (unsigned int)std::min<size_t>(LN / 9 + 1, (size_t)1 << 21);
+        const unsigned int tcap = (unsigned int)std::min<size_t>(LN / 3 + 1, (size_t)1 << 25);
+        const unsigned int scap = (unsigned int)std::min<size_t>(LN / 9 + 1, (size_t)1 << 23);
         const unsigned int lcap = (unsigned int)std::min<size_t>(LN / 33 + 1, (size_t)1 << 18);
         const size_t rcap = (size_t)tcap + scap + lcap;
         CU_TRY(ix->ws_run_pos.reserve(rcap));
@@ -648,28 +679,30 @@ int sort_keys(culsh_index* ix, int N, int passes, cudaStream_t st, const uint32_
         rl.llen = ix->ws_run_len.p + tcap + scap;
         rl.lcap = lcap;
         rl.cnt = ix->ws_run_cnt.p;
-        const uint32_t* stop = ix->ws_keys[1].p + (KW - 1) * LN;
-        CU_TRY(launch_run_find(stop, N, L, rl, st));
+        CU_TRY(launch_run_find(top, N, L, KW, ix->ws_low.p, ix->ids.p, rl, st));
         CU_TRY(cudaMemcpyAsync(ix->h_run_cnt.p, rl.cnt, 4 * sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
         CU_TRY(cudaStreamSynchronize(st));
         const unsigned int* hc = ix->h_run_cnt.p;
         if (hc[3] == 0) {
-            CU_TRY(launch_run_sorts(rl, hc, N, L, KW, ix->ws_keys[1].p, ix->ids.p, st));
+            CU_TRY(launch_run_sorts(rl, hc, N, L, KW, ix->ws_low.p, ix->ids.p, st));
             ix->sort_form = 1;
-            *skeys = ix->ws_keys[1].p;
+            *sk = SortedKeys{top, ix->ws_low.p, ix->ids.p, lw};
             return CULSH_OK;
         }
         // a run too long to order in shared memory: repack, sort every word
-        CU_TRY(launch_pack_keys(ix->ws_codes.p, N, L, ix->M, KW, ix->cmin.p, ix->fbits.p, ix->foff.p,
-                                ix->ws_keys[0].p, ix->ids.p, st));
+        ix->sort_form = 2;
+        CU_TRY(ix->ws_keys[0].reserve(LN * KW));
+        CU_TRY(ix->ws_keys[1].reserve(LN * KW));
+        CU_TRY(launch_pack_keys(ix->ws_codes.p, N, L, ix->M, KW, ix->cmin.p, ix->fbits.p, ix->foff.p, ix->ws_keys[0].p,
+                                ix->ids.p, nullptr, 0, st));
+        sb.keys[0] = ix->ws_keys[0].p;
+        sb.keys[1] = ix->ws_keys[1].p;
         sb.vals[0] = ix->ids.p;
         sb.vals[1] = ix->ws_vals.p;
-        ix->sort_form = 2;
     }
-    bool alt = false;
     CU_TRY(run_segmented_sort(sb, N, L, KW, passes, &alt, st));
-    *skeys = ix->ws_keys[alt ? 1 : 0].p;
     if (alt) ix->ids.swap(ix->ws_vals);
+    *sk = SortedKeys{sb.keys[alt ? 1 : 0], nullptr, ix->ids.p, 0};
     return CULSH_OK;
 }
 
@@ -712,21 +745,8 @@ int build_device(culsh_index* ix, const float* dX, cudaStream_t st, FILE* dbg) {
                 "%d key words, %d sort passes\n",
                 N, L, M, ix->tc_recomputed >= 0 ? "tensor cores" : "FP32 SIMT", ix->tc_recomputed, ix->KW, passes);
 
-    // Pack keys and sort all tables at once.
-    const size_t LN = (size_t)L * N;
-    CU_TRY(ix->ws_keys[0].reserve(LN * ix->KW));
-    CU_TRY(ix->ws_keys[1].reserve(LN * ix->KW));
-    CU_TRY(ix->ws_vals.reserve(LN));
-    CU_TRY(ix->ids.reserve(LN));
-    CU_TRY(launch_pack_keys(ix->ws_codes.p, N, L, M, ix->KW, ix->cmin.p, ix->fbits.p, ix->foff.p, ix->ws_keys[0].p,
-                            ix->ids.p, st));
-    const int hp = std::max(passes, 1);
-    CU_TRY(ix->ws_hist.reserve((size_t)L * hp * 256));
-    CU_TRY(ix->ws_base.reserve((size_t)L * hp * 256));
-    CU_TRY(ix->ws_status.reserve(sort_status_words(N, L)));
-    CU_TRY(ix->h_sort_hist.reserve((size_t)L * hp * 256));
-    CU_TRY(cudaEventRecord(ix->bev[2], st));
-    const uint32_t* skeys = nullptr;
+    // Pack keys and sort all tables at once (records bev[2] between the two).
+    SortedKeys skeys{};
     TRY(sort_keys(ix, N, passes, st, &skeys));
     CU_TRY(cudaEventRecord(ix->bev[3], st));
 

@@ -204,10 +204,12 @@ cudaError_t launch_tc_recompute(const float* X, int64_t N, int D, int LM, const 
                                 const unsigned long long* list, unsigned long long cap, const unsigned int* cnt,
                                 int regions, int32_t* codes, int32_t* cmin, int32_t* cmax, int* err, cudaStream_t st);
 
-// Key packing from int codes [LM][N] into SoA keys [KW][L*N] and identity values.
+// Key packing from int codes [LM][N] into SoA keys [KW][L*N] and identity values;
+// with low (KW 2 to 4): the top word into keys [L*N], the lower words into rows
+// of lw words (low_row_words).
 cudaError_t launch_pack_keys(const int32_t* codes, int64_t N, int L, int M, int KW, const int32_t* cmin,
                              const uint8_t* fbits, const uint16_t* foff, uint32_t* keys, uint32_t* vals,
-                             cudaStream_t st);
+                             uint32_t* low, int lw, cudaStream_t st);
 
 // Onesweep segmented LSD radix sort of L segments of N (key, value) pairs.
 // Sorts bits [0, 8*passes) of the KW-word keys. Buffers are ping-ponged; on
@@ -227,10 +229,10 @@ cudaError_t run_segmented_sort(SortBuffers& sb, int64_t N, int L, int KW, int pa
                                cudaStream_t st);
 
 // Top-word-first ordering (sort.cu): after the digit passes over the top key
-// word, gather the lower words into sorted order, find the runs of equal top
-// words and order each run by (lower words, id).
+// word, find the runs of equal top words and order each run by (lower words,
+// id).
 struct RunLists {
-    unsigned long long* tpos;   // runs of 2..8: first sorted position (table * N + i)
+    unsigned long long* tpos;   // runs of 3..8: first sorted position (table * N + i)
     uint32_t* tlen;
     unsigned int tcap;
     unsigned long long* spos;   // runs of 9..32
@@ -241,18 +243,27 @@ struct RunLists {
     unsigned int lcap;
     unsigned int* cnt;          // [4]: tiny, small and large runs; overflow flags (1 run too long, 2 list full)
 };
-cudaError_t launch_gather_lower(const uint32_t* keys0, const uint32_t* ids, const uint32_t* top, int64_t N, int L,
-                                int KW, uint32_t* skeys, cudaStream_t st);
-cudaError_t launch_run_find(const uint32_t* top, int64_t N, int L, const RunLists& rl, cudaStream_t st);
-cudaError_t launch_run_sorts(const RunLists& rl, const unsigned int* counts, int64_t N, int L, int KW, uint32_t* skeys,
+cudaError_t launch_run_find(const uint32_t* top, int64_t N, int L, int KW, const uint32_t* low, uint32_t* ids,
+                            const RunLists& rl, cudaStream_t st);
+cudaError_t launch_run_sorts(const RunLists& rl, const unsigned int* counts, int64_t N, int L, int KW, const uint32_t* low,
                              uint32_t* ids, cudaStream_t st);
 int run_max_len();
 
+// Sorted keys of all tables: KW arrays of L*N words, or (low != nullptr) the
+// sorted top words and the lower words by point, in rows of lw words.
+struct SortedKeys {
+    const uint32_t* keys;
+    const uint32_t* low;
+    const uint32_t* ids;   // [L*N] sorted ids
+    int lw;
+};
+constexpr int low_row_words(int KW) { return KW == 2 ? 1 : KW == 3 ? 2 : 4; }
+
 // Run-length bucketing of sorted keys. Two phases: count (per table bucket
 // totals, written to nb[L]) and write (starts, ukeys).
-cudaError_t launch_rl_count(const uint32_t* keys, int64_t N, int L, int KW, uint32_t* tile_cnt, uint32_t* tile_off,
+cudaError_t launch_rl_count(const SortedKeys& keys, int64_t N, int L, int KW, uint32_t* tile_cnt, uint32_t* tile_off,
                             uint32_t* nb, cudaStream_t st);
-cudaError_t launch_rl_write(const uint32_t* keys, int64_t N, int L, int KW, const uint32_t* tile_off,
+cudaError_t launch_rl_write(const SortedKeys& keys, int64_t N, int L, int KW, const uint32_t* tile_off,
                             const uint64_t* boff, uint32_t* starts, uint32_t* ukeys, cudaStream_t st);
 cudaError_t launch_bucket_sizes(const uint64_t* boff, const uint32_t* starts, int64_t N, int L, int64_t maxB,
                                 uint32_t* sizes, uint32_t* max_size, cudaStream_t st);

@@ -77,7 +77,7 @@ template <bool WIDE>
 __global__ void k_pack_keys(const int32_t* __restrict__ codes, int64_t N, int L, int M, int KW,
                             const int32_t* __restrict__ cmin, const uint8_t* __restrict__ fbits,
                             const uint16_t* __restrict__ foff, uint32_t* __restrict__ keys,
-                            uint32_t* __restrict__ vals) {
+                            uint32_t* __restrict__ vals, uint32_t* __restrict__ low, int lw) {
     const int64_t LN = (int64_t)L * N;
     for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < LN;
          idx += (int64_t)gridDim.x * blockDim.x) {
@@ -102,6 +102,15 @@ __global__ void k_pack_keys(const int32_t* __restrict__ codes, int64_t N, int L,
             const int bits = __ldg(fbits + c);
             if (!bits) continue;
             kk = (kk << bits) | (uint32_t)(codes[(int64_t)c * N + n] - __ldg(cmin + c));
+        }
+        kk <<= __ldg(foff + (int64_t)l * M + M - 1);   // the last column's offset (compute_layout)
+        if (low) {   // top-word-first form: the top word in keys, the lower ones as a row
+            keys[idx] = (uint32_t)(kk >> (32 * (KW - 1)));
+            if (lw == 1) low[idx] = (uint32_t)kk;
+            else if (lw == 2) reinterpret_cast<uint2*>(low)[idx] = make_uint2((uint32_t)kk, (uint32_t)(kk >> 32));
+            else reinterpret_cast<uint4*>(low)[idx] = make_uint4((uint32_t)kk, (uint32_t)(kk >> 32), (uint32_t)(kk >> 64), 0u);
+            vals[idx] = (uint32_t)n;
+            continue;
         }
 #pragma unroll
         for (int w = 0; w < 4; ++w)
@@ -278,81 +287,29 @@ __global__ void __launch_bounds__(NT, 3) k_sort_pass(const uint32_t* __restrict_
 }
 
 // ---- Top-word-first ordering ----
-// The digit passes can run over the key's top word alone (its leading
-// columns), moving that word and the ids. The lower words of every sorted
-// position are then gathered from the packed keys in point order, and each run
-// of equal top words is ordered by (lower words, id): the LSD passes leave a
-// run's ids ascending, so this is the order the full sort produces.
+// The digit passes can run over the key's top word alone (its leading 32
+// bits), moving that word and the ids. The lower words stay in point order, as
+// rows of lw words (1, 2 or 4), and are read through the ids where they are
+// needed: each run of equal top words is ordered by (lower words, id) (the
+// LSD passes leave a run's ids ascending, so this is the order the full sort
+// produces), the run-length passes compare them inside such runs, and a
+// bucket's key takes one row. Rows gathered into sorted order first, word by
+// word, had cost 9.3 ms at 200M keys of four words.
 
-// skeys[w][i] = keys0[w][table + ids[i]] for the lower words w < KW - 1; the
-// sorted top words are copied into skeys' top slot unless they are there.
-__global__ void k_gather_lower(const uint32_t* __restrict__ keys0, const uint32_t* __restrict__ ids,
-                               const uint32_t* top, int64_t N, int L, int KW, uint32_t* skeys) {
-    const int64_t LN = (int64_t)L * N, seg = (int64_t)blockIdx.y * N;
-    uint32_t* stop = skeys + (int64_t)(KW - 1) * LN;
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < N; i += (int64_t)gridDim.x * blockDim.x) {
-        const int64_t idx = seg + i;
-        const uint32_t id = ids[idx];
-        for (int w = 0; w < KW - 1; ++w) skeys[w * LN + idx] = __ldg(keys0 + w * LN + seg + id);
-        if (top != stop) stop[idx] = top[idx];
-    }
-}
-
-// Runs of two or more equal top words, found from their first element, go to
-// three lists by length: 2..8 (tiny), 9..32 (small), 33..kRunMax (large); a
-// longer run or a full list sets cnt[3] (the caller then sorts all words
-// instead). Block (x, table y); each thread examines RUN_ITEMS consecutive
-// positions. List slots are claimed per block (shared counters, then one
-// global atomic per block and class): with tens of thousands of runs per
-// table, one global atomic per run or per warp serialises on the counters.
-constexpr int RUN_ITEMS = 8;
-__global__ void __launch_bounds__(NT) k_run_find(const uint32_t* __restrict__ top, int64_t N, RunLists rl) {
-    __shared__ unsigned int sc[3], sbase[3];
-    if (threadIdx.x < 3) sc[threadIdx.x] = 0;
-    __syncthreads();
-    const uint32_t* t = top + (int64_t)blockIdx.y * N;
-    const int64_t i0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * RUN_ITEMS;
-    uint32_t len[RUN_ITEMS];
-    unsigned int mine[3] = {0u, 0u, 0u};
-#pragma unroll
-    for (int k = 0; k < RUN_ITEMS; ++k) {
-        const int64_t i = i0 + k;
-        len[k] = 0;
-        if (i + 1 < N) {
-            const uint32_t v = t[i];
-            if (t[i + 1] == v && !(i > 0 && t[i - 1] == v)) {
-                int64_t j = i + 2;
-                while (j < N && j - i <= kRunMax && t[j] == v) ++j;
-                if (j - i > kRunMax) atomicOr(rl.cnt + 3, 1u);
-                else len[k] = (uint32_t)(j - i);
-            }
-        }
-        const uint32_t n = len[k];
-        mine[0] += (n >= 2 && n <= 8) ? 1u : 0u;
-        mine[1] += (n > 8 && n <= 32) ? 1u : 0u;
-        mine[2] += n > 32 ? 1u : 0u;
-    }
-    unsigned int off[3];
-#pragma unroll
-    for (int c = 0; c < 3; ++c) off[c] = mine[c] ? atomicAdd(&sc[c], mine[c]) : 0u;
-    __syncthreads();
-    if (threadIdx.x < 3) sbase[threadIdx.x] = sc[threadIdx.x] ? atomicAdd(rl.cnt + threadIdx.x, sc[threadIdx.x]) : 0u;
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < RUN_ITEMS; ++k) {
-        const uint32_t n = len[k];
-        if (n < 2) continue;
-        const int c = n <= 8 ? 0 : (n <= 32 ? 1 : 2);
-        const unsigned int slot = sbase[c] + off[c]++;
-        const unsigned int cap = c == 0 ? rl.tcap : (c == 1 ? rl.scap : rl.lcap);
-        unsigned long long* pos = c == 0 ? rl.tpos : (c == 1 ? rl.spos : rl.lpos);
-        uint32_t* lens = c == 0 ? rl.tlen : (c == 1 ? rl.slen : rl.llen);
-        if (slot < cap) {
-            pos[slot] = (unsigned long long)((int64_t)blockIdx.y * N + i0 + k);
-            lens[slot] = n;
-        } else {
-            atomicOr(rl.cnt + 3, 2u);
-        }
+// Lower words of point `id` of the table that starts at seg.
+template <int KWL>
+__device__ __forceinline__ void low_row(const uint32_t* __restrict__ low, int64_t seg, uint32_t id, uint32_t* e) {
+    if constexpr (KWL == 1) {
+        e[0] = __ldg(low + seg + id);
+    } else if constexpr (KWL == 2) {
+        const uint2 v = __ldg(reinterpret_cast<const uint2*>(low) + seg + id);
+        e[0] = v.x;
+        e[1] = v.y;
+    } else {
+        const uint4 v = __ldg(reinterpret_cast<const uint4*>(low) + seg + id);
+        e[0] = v.x;
+        e[1] = v.y;
+        e[2] = v.z;
     }
 }
 
@@ -365,25 +322,120 @@ __device__ __forceinline__ bool run_less(const uint32_t (&a)[KWL + 1], const uin
     return a[KWL] < b[KWL];
 }
 
-// One thread per run of 2 to 8: an odd-even transposition sort over eight
+// Runs of two or more equal top words, found from their first element. Runs of
+// two, by far the most where points fall nearly alone (of 200M positions of the
+// 10M-point build more than the lists hold), are ordered here; longer ones go
+// to three lists: 3..8 (tiny), 9..32 (small), 33..kRunMax (large); a longer
+// run or a full list sets cnt[3] (the caller then sorts all words instead).
+// Block (x, table y) examines RUN_TILE positions from shared memory, one
+// position in RUN_ITEMS rows per thread (consecutive threads, consecutive
+// positions). List slots are claimed per block (shared counters, then one
+// global atomic per block and class): with tens of thousands of runs per
+// table, one global atomic per run or per warp serialises on the counters.
+constexpr int RUN_ITEMS = 8;
+constexpr int RUN_TILE = NT * RUN_ITEMS;
+template <int KWL>
+__global__ void __launch_bounds__(NT) k_run_find(const uint32_t* __restrict__ top, int64_t N,
+                                                const uint32_t* __restrict__ low, uint32_t* __restrict__ ids,
+                                                RunLists rl) {
+    __shared__ unsigned int sc[3], sbase[3];
+    __shared__ uint32_t w[RUN_TILE + 10];   // positions i0 - 1 .. i0 + RUN_TILE + 8
+    const int64_t seg = (int64_t)blockIdx.y * N;
+    const uint32_t* t = top + seg;
+    const int64_t i0 = (int64_t)blockIdx.x * RUN_TILE;
+    if (threadIdx.x < 3) sc[threadIdx.x] = 0;
+    for (int j = threadIdx.x; j < RUN_TILE + 10; j += NT) {
+        const int64_t i = i0 + j - 1;
+        // past either end of the table: a value that differs from its neighbour
+        if (i >= 0 && i < N) w[j] = t[i];
+        else w[j] = ~t[i < 0 ? 0 : N - 1];
+    }
+    __syncthreads();
+    uint32_t len[RUN_ITEMS];
+    unsigned int mine[3] = {0u, 0u, 0u};
+#pragma unroll
+    for (int k = 0; k < RUN_ITEMS; ++k) {
+        const int j = k * NT + threadIdx.x + 1;
+        const int64_t i = i0 + j - 1;
+        const uint32_t v = w[j];
+        uint32_t n = 1;
+        if (i + 1 < N && w[j + 1] == v && w[j - 1] != v) {
+            n = 2;
+            while (n < 9 && i + n < N && w[j + n] == v) ++n;
+            if (n == 9) {   // the words ascend: halve the rest
+                if (i + kRunMax < N && t[i + kRunMax] == v) {
+                    atomicOr(rl.cnt + 3, 1u);
+                    n = 1;
+                } else {
+                    int64_t lo = i + 9, hi = min(N, i + kRunMax);   // hi: differs, or the end
+                    while (lo < hi) {
+                        const int64_t mid = (lo + hi) >> 1;
+                        if (t[mid] == v) lo = mid + 1;
+                        else hi = mid;
+                    }
+                    n = (uint32_t)(lo - i);
+                }
+            } else if (n == 2) {
+                uint32_t a[KWL + 1], b[KWL + 1];
+                a[KWL] = ids[seg + i];
+                b[KWL] = ids[seg + i + 1];
+                low_row<KWL>(low, seg, a[KWL], a);
+                low_row<KWL>(low, seg, b[KWL], b);
+                if (run_less<KWL>(b, a)) {
+                    ids[seg + i] = b[KWL];
+                    ids[seg + i + 1] = a[KWL];
+                }
+            }
+        }
+        len[k] = n;
+        mine[0] += (n > 2 && n <= 8) ? 1u : 0u;
+        mine[1] += (n > 8 && n <= 32) ? 1u : 0u;
+        mine[2] += n > 32 ? 1u : 0u;
+    }
+    unsigned int off[3];
+#pragma unroll
+    for (int c = 0; c < 3; ++c) off[c] = mine[c] ? atomicAdd(&sc[c], mine[c]) : 0u;
+    __syncthreads();
+    if (threadIdx.x < 3) sbase[threadIdx.x] = sc[threadIdx.x] ? atomicAdd(rl.cnt + threadIdx.x, sc[threadIdx.x]) : 0u;
+    __syncthreads();
+#pragma unroll
+    for (int k = 0; k < RUN_ITEMS; ++k) {
+        const uint32_t n = len[k];
+        if (n <= 2) continue;
+        const int c = n <= 8 ? 0 : (n <= 32 ? 1 : 2);
+        const unsigned int slot = sbase[c] + off[c]++;
+        const unsigned int cap = c == 0 ? rl.tcap : (c == 1 ? rl.scap : rl.lcap);
+        unsigned long long* pos = c == 0 ? rl.tpos : (c == 1 ? rl.spos : rl.lpos);
+        uint32_t* lens = c == 0 ? rl.tlen : (c == 1 ? rl.slen : rl.llen);
+        if (slot < cap) {
+            pos[slot] = (unsigned long long)(seg + i0 + k * NT + threadIdx.x);
+            lens[slot] = n;
+        } else {
+            atomicOr(rl.cnt + 3, 2u);
+        }
+    }
+}
+
+// One thread per run of 3 to 8: an odd-even transposition sort over eight
 // register slots (missing slots hold all-ones, above every element).
 template <int KWL>
 __global__ void k_run_sort_tiny(const unsigned long long* __restrict__ tpos, const uint32_t* __restrict__ tlen,
-                                const unsigned int* __restrict__ cnt, unsigned int tcap, int64_t LN,
-                                uint32_t* __restrict__ skeys, uint32_t* __restrict__ ids) {
+                                const unsigned int* __restrict__ cnt, unsigned int tcap, int64_t N,
+                                const uint32_t* __restrict__ low,
+                                uint32_t* __restrict__ ids) {
     const unsigned int nrun = min(cnt[0], tcap);
     for (unsigned int r = blockIdx.x * blockDim.x + threadIdx.x; r < nrun; r += gridDim.x * blockDim.x) {
         const int64_t pos = (int64_t)tpos[r];
         const int len = (int)tlen[r];
+        const int64_t seg = pos / N * N;
         uint32_t e[8][KWL + 1];
 #pragma unroll
         for (int t = 0; t < 8; ++t) {
 #pragma unroll
             for (int k = 0; k <= KWL; ++k) e[t][k] = 0xFFFFFFFFu;
             if (t < len) {
-#pragma unroll
-                for (int k = 0; k < KWL; ++k) e[t][k] = skeys[k * LN + pos + t];
                 e[t][KWL] = ids[pos + t];
+                low_row<KWL>(low, seg, e[t][KWL], e[t]);
             }
         }
 #pragma unroll
@@ -402,11 +454,7 @@ __global__ void k_run_sort_tiny(const unsigned long long* __restrict__ tpos, con
         }
 #pragma unroll
         for (int t = 0; t < 8; ++t) {
-            if (t < len) {
-#pragma unroll
-                for (int k = 0; k < KWL; ++k) skeys[k * LN + pos + t] = e[t][k];
-                ids[pos + t] = e[t][KWL];
-            }
+            if (t < len) ids[pos + t] = e[t][KWL];
         }
     }
 }
@@ -415,21 +463,22 @@ __global__ void k_run_sort_tiny(const unsigned long long* __restrict__ tpos, con
 // lanes hold all-ones, above every element: ids are below 2^32 - 1).
 template <int KWL>
 __global__ void k_run_sort_small(const unsigned long long* __restrict__ spos, const uint32_t* __restrict__ slen,
-                                 const unsigned int* __restrict__ cnt, unsigned int scap, int64_t LN,
-                                 uint32_t* __restrict__ skeys, uint32_t* __restrict__ ids) {
+                                 const unsigned int* __restrict__ cnt, unsigned int scap, int64_t N,
+                                 const uint32_t* __restrict__ low,
+                                uint32_t* __restrict__ ids) {
     const int lane = threadIdx.x & 31;
     const unsigned int nrun = min(cnt[1], scap);
     for (unsigned int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < nrun;
          r += (gridDim.x * blockDim.x) >> 5) {
         const int64_t pos = (int64_t)spos[r];
         const int len = (int)slen[r];
+        const int64_t seg = pos / N * N;
         uint32_t e[KWL + 1];
 #pragma unroll
         for (int k = 0; k <= KWL; ++k) e[k] = 0xFFFFFFFFu;
         if (lane < len) {
-#pragma unroll
-            for (int k = 0; k < KWL; ++k) e[k] = skeys[k * LN + pos + lane];
             e[KWL] = ids[pos + lane];
+            low_row<KWL>(low, seg, e[KWL], e);
         }
 #pragma unroll
         for (int k = 2; k <= 32; k <<= 1) {
@@ -446,11 +495,7 @@ __global__ void k_run_sort_small(const unsigned long long* __restrict__ spos, co
                 }
             }
         }
-        if (lane < len) {
-#pragma unroll
-            for (int k = 0; k < KWL; ++k) skeys[k * LN + pos + lane] = e[k];
-            ids[pos + lane] = e[KWL];
-        }
+        if (lane < len) ids[pos + lane] = e[KWL];
     }
 }
 
@@ -459,19 +504,26 @@ template <int KWL>
 __global__ void __launch_bounds__(NT) k_run_sort_large(const unsigned long long* __restrict__ lpos,
                                                       const uint32_t* __restrict__ llen,
                                                       const unsigned int* __restrict__ cnt, unsigned int lcap,
-                                                      int64_t LN, uint32_t* __restrict__ skeys,
+                                                      int64_t N, const uint32_t* __restrict__ low,
                                                       uint32_t* __restrict__ ids) {
     __shared__ uint32_t sv[KWL + 1][kRunMax];
     const unsigned int nrun = min(cnt[2], lcap);
     for (unsigned int r = blockIdx.x; r < nrun; r += gridDim.x) {
         const int64_t pos = (int64_t)lpos[r];
         const int len = (int)llen[r];
+        const int64_t seg = pos / N * N;
         int n2 = 64;
         while (n2 < len) n2 <<= 1;
         for (int t = threadIdx.x; t < n2; t += NT) {
+            uint32_t e[KWL + 1];
 #pragma unroll
-            for (int k = 0; k < KWL; ++k) sv[k][t] = t < len ? skeys[k * LN + pos + t] : 0xFFFFFFFFu;
-            sv[KWL][t] = t < len ? ids[pos + t] : 0xFFFFFFFFu;
+            for (int k = 0; k <= KWL; ++k) e[k] = 0xFFFFFFFFu;
+            if (t < len) {
+                e[KWL] = ids[pos + t];
+                low_row<KWL>(low, seg, e[KWL], e);
+            }
+#pragma unroll
+            for (int k = 0; k <= KWL; ++k) sv[k][t] = e[k];
         }
         __syncthreads();
         for (int k = 2; k <= n2; k <<= 1) {
@@ -498,29 +550,38 @@ __global__ void __launch_bounds__(NT) k_run_sort_large(const unsigned long long*
                 __syncthreads();
             }
         }
-        for (int t = threadIdx.x; t < len; t += NT) {
-#pragma unroll
-            for (int k = 0; k < KWL; ++k) skeys[k * LN + pos + t] = sv[k][t];
-            ids[pos + t] = sv[KWL][t];
-        }
+        for (int t = threadIdx.x; t < len; t += NT) ids[pos + t] = sv[KWL][t];
         __syncthreads();
     }
 }
 
-__device__ __forceinline__ bool key_differs(const uint32_t* keys, int64_t LN, int64_t a, int64_t b, int KW) {
+// Whether sorted positions a and a - 1 of the table at seg hold different keys.
+// LOW: top-word-first form, keys = the sorted top words, low = lower words by
+// point; otherwise keys = KW arrays of LN words.
+template <bool LOW>
+__device__ __forceinline__ bool key_differs(const SortedKeys& s, int64_t LN, int64_t seg, int64_t a, int KW) {
+    if constexpr (LOW) {
+        if (s.keys[a] != s.keys[a - 1]) return true;
+        const uint32_t* x = s.low + (seg + s.ids[a]) * s.lw;
+        const uint32_t* y = s.low + (seg + s.ids[a - 1]) * s.lw;
+        for (int w = 0; w < KW - 1; ++w)
+            if (__ldg(x + w) != __ldg(y + w)) return true;
+        return false;
+    }
     for (int w = 0; w < KW; ++w)
-        if (keys[w * LN + a] != keys[w * LN + b]) return true;
+        if (s.keys[w * LN + a] != s.keys[w * LN + a - 1]) return true;
     return false;
 }
 
-__global__ void k_rl_count(const uint32_t* __restrict__ keys, int64_t N, int L, int KW, uint32_t* __restrict__ tile_cnt) {
+template <bool LOW>
+__global__ void k_rl_count(SortedKeys s, int64_t N, int L, int KW, uint32_t* __restrict__ tile_cnt) {
     __shared__ uint32_t ws[SP_WARPS];
     const int l = blockIdx.y, tile = blockIdx.x, tiles = gridDim.x;
     const int64_t LN = (int64_t)L * N, seg = (int64_t)l * N;
     uint32_t c = 0;
     for (int e = threadIdx.x; e < SP_TILE; e += NT) {
         const int64_t i = (int64_t)tile * SP_TILE + e;
-        if (i < N) c += (i == 0 || key_differs(keys, LN, seg + i, seg + i - 1, KW)) ? 1u : 0u;
+        if (i < N) c += (i == 0 || key_differs<LOW>(s, LN, seg, seg + i, KW)) ? 1u : 0u;
     }
     uint32_t tot;
     block_excl_scan(c, ws, &tot);
@@ -547,8 +608,8 @@ __global__ void k_rl_scan(const uint32_t* __restrict__ tile_cnt, int tiles, uint
 // takes positions [512 w, 512 w + 512) as 16 rows of 32 lanes (coalesced key
 // loads), ranks its flagged positions with ballots, and the block scans the
 // warp totals; flagged positions are written in order.
-__global__ void k_rl_write(const uint32_t* __restrict__ keys, int64_t N, int L, int KW,
-                           const uint32_t* __restrict__ tile_off, const uint64_t* __restrict__ boff,
+template <bool LOW>
+__global__ void k_rl_write(SortedKeys s, int64_t N, int L, int KW, const uint32_t* __restrict__ tile_off, const uint64_t* __restrict__ boff,
                            uint32_t* __restrict__ starts, uint32_t* __restrict__ ukeys) {
     __shared__ uint32_t ws[SP_WARPS];
     const int l = blockIdx.y, tile = blockIdx.x, tiles = gridDim.x;
@@ -560,7 +621,7 @@ __global__ void k_rl_write(const uint32_t* __restrict__ keys, int64_t N, int L, 
 #pragma unroll
     for (int k = 0; k < SP_ITEMS; ++k) {
         const int64_t i = w0 + k * 32 + lane;
-        const bool f = i < N && (i == 0 || key_differs(keys, LN, seg + i, seg + i - 1, KW));
+        const bool f = i < N && (i == 0 || key_differs<LOW>(s, LN, seg, seg + i, KW));
         ball[k] = __ballot_sync(0xffffffffu, f);
         c += __popc(ball[k]);
     }
@@ -576,7 +637,13 @@ __global__ void k_rl_write(const uint32_t* __restrict__ keys, int64_t N, int L, 
             const int64_t i = w0 + k * 32 + lane;
             const uint64_t g = bo + r + __popc(ball[k] & below);
             starts[g] = (uint32_t)i;
-            for (int w = 0; w < KW; ++w) ukeys[g * KW + w] = keys[w * LN + seg + i];
+            if constexpr (LOW) {
+                const uint32_t* x = s.low + (seg + s.ids[seg + i]) * s.lw;
+                for (int w = 0; w < KW - 1; ++w) ukeys[g * KW + w] = __ldg(x + w);
+                ukeys[g * KW + KW - 1] = s.keys[seg + i];
+            } else {
+                for (int w = 0; w < KW; ++w) ukeys[g * KW + w] = s.keys[w * LN + seg + i];
+            }
         }
         r += __popc(ball[k]);
     }
@@ -629,7 +696,8 @@ __global__ void k_hash_build(const uint64_t* __restrict__ boff, const uint32_t* 
     } else {
         unsigned __int128 kk = 0;
         for (int w = KW - 1; w >= 0; --w) kk = (kk << 32) | key[w];
-        // fields are contiguous from bit 0 (column M - 1) upwards
+        // fields are contiguous from column M - 1's offset upwards
+        kk >>= __ldg(foff + (int64_t)l * M + M - 1);
         for (int m = M - 1; m >= 0; --m) {
             const int c = l * M + m;
             const int bits = __ldg(fbits + c);
@@ -780,11 +848,11 @@ inline int blocks_for(int64_t n) { return (int)((n + NT - 1) / NT); }
 
 cudaError_t launch_pack_keys(const int32_t* codes, int64_t N, int L, int M, int KW, const int32_t* cmin,
                              const uint8_t* fbits, const uint16_t* foff, uint32_t* keys, uint32_t* vals,
-                             cudaStream_t st) {
+                             uint32_t* low, int lw, cudaStream_t st) {
     const int64_t LN = (int64_t)L * N;
     const int grid = (int)std::min<int64_t>((LN + NT - 1) / NT, 152 * 32);
-    if (KW > 4) k_pack_keys<true><<<grid, NT, 0, st>>>(codes, N, L, M, KW, cmin, fbits, foff, keys, vals);
-    else k_pack_keys<false><<<grid, NT, 0, st>>>(codes, N, L, M, KW, cmin, fbits, foff, keys, vals);
+    if (KW > 4) k_pack_keys<true><<<grid, NT, 0, st>>>(codes, N, L, M, KW, cmin, fbits, foff, keys, vals, nullptr, 0);
+    else k_pack_keys<false><<<grid, NT, 0, st>>>(codes, N, L, M, KW, cmin, fbits, foff, keys, vals, low, lw);
     return cudaGetLastError();
 }
 
@@ -840,60 +908,59 @@ cudaError_t run_segmented_sort(SortBuffers& sb, int64_t N, int L, int KW, int pa
     return e;
 }
 
-cudaError_t launch_gather_lower(const uint32_t* keys0, const uint32_t* ids, const uint32_t* top, int64_t N, int L,
-                                int KW, uint32_t* skeys, cudaStream_t st) {
-    const dim3 grid((unsigned)std::min<int64_t>((N + NT - 1) / NT, 152 * 4), (unsigned)L);
-    k_gather_lower<<<grid, NT, 0, st>>>(keys0, ids, top, N, L, KW, skeys);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_run_find(const uint32_t* top, int64_t N, int L, const RunLists& rl, cudaStream_t st) {
-    const int64_t LN = (int64_t)L * N;
+cudaError_t launch_run_find(const uint32_t* top, int64_t N, int L, int KW, const uint32_t* low, uint32_t* ids,
+                            const RunLists& rl, cudaStream_t st) {
     cudaError_t e = cudaMemsetAsync(rl.cnt, 0, 4 * sizeof(unsigned int), st);
     if (e != cudaSuccess) return e;
-    (void)LN;
-    const dim3 grid((unsigned)((N + (int64_t)NT * RUN_ITEMS - 1) / ((int64_t)NT * RUN_ITEMS)), (unsigned)L);
-    k_run_find<<<grid, NT, 0, st>>>(top, N, rl);
+    const dim3 grid((unsigned)((N + RUN_TILE - 1) / RUN_TILE), (unsigned)L);
+    switch (KW - 1) {
+    case 1: k_run_find<1><<<grid, NT, 0, st>>>(top, N, low, ids, rl); break;
+    case 2: k_run_find<2><<<grid, NT, 0, st>>>(top, N, low, ids, rl); break;
+    case 3: k_run_find<3><<<grid, NT, 0, st>>>(top, N, low, ids, rl); break;
+    default: return cudaErrorInvalidValue;
+    }
     return cudaGetLastError();
 }
 
 int run_max_len() { return kRunMax; }
 
 template <int KWL>
-void launch_run_sorts_w(const RunLists& rl, unsigned int ntiny, unsigned int nsmall, unsigned int nlarge, int64_t LN,
-                        uint32_t* skeys, uint32_t* ids, cudaStream_t st) {
+void launch_run_sorts_w(const RunLists& rl, unsigned int ntiny, unsigned int nsmall, unsigned int nlarge, int64_t N,
+                        const uint32_t* low, uint32_t* ids, cudaStream_t st) {
     const unsigned gt = (unsigned)std::min<unsigned long long>(((unsigned long long)ntiny + NT - 1) / NT, 152 * 16);
     const unsigned gs = (unsigned)std::min<unsigned long long>(((unsigned long long)nsmall * 32 + NT - 1) / NT, 152 * 32);
     const unsigned gl = (unsigned)std::min<unsigned int>(nlarge, 152 * 4);
-    if (gt) k_run_sort_tiny<KWL><<<gt, NT, 0, st>>>(rl.tpos, rl.tlen, rl.cnt, rl.tcap, LN, skeys, ids);
-    if (gs) k_run_sort_small<KWL><<<gs, NT, 0, st>>>(rl.spos, rl.slen, rl.cnt, rl.scap, LN, skeys, ids);
-    if (gl) k_run_sort_large<KWL><<<gl, NT, 0, st>>>(rl.lpos, rl.llen, rl.cnt, rl.lcap, LN, skeys, ids);
+    if (gt) k_run_sort_tiny<KWL><<<gt, NT, 0, st>>>(rl.tpos, rl.tlen, rl.cnt, rl.tcap, N, low, ids);
+    if (gs) k_run_sort_small<KWL><<<gs, NT, 0, st>>>(rl.spos, rl.slen, rl.cnt, rl.scap, N, low, ids);
+    if (gl) k_run_sort_large<KWL><<<gl, NT, 0, st>>>(rl.lpos, rl.llen, rl.cnt, rl.lcap, N, low, ids);
 }
 
-cudaError_t launch_run_sorts(const RunLists& rl, const unsigned int* counts, int64_t N, int L, int KW, uint32_t* skeys,
+cudaError_t launch_run_sorts(const RunLists& rl, const unsigned int* counts, int64_t N, int L, int KW, const uint32_t* low,
                              uint32_t* ids, cudaStream_t st) {
-    const int64_t LN = (int64_t)L * N;
+    (void)L;
     switch (KW - 1) {
-    case 1: launch_run_sorts_w<1>(rl, counts[0], counts[1], counts[2], LN, skeys, ids, st); break;
-    case 2: launch_run_sorts_w<2>(rl, counts[0], counts[1], counts[2], LN, skeys, ids, st); break;
-    case 3: launch_run_sorts_w<3>(rl, counts[0], counts[1], counts[2], LN, skeys, ids, st); break;
+    case 1: launch_run_sorts_w<1>(rl, counts[0], counts[1], counts[2], N, low, ids, st); break;
+    case 2: launch_run_sorts_w<2>(rl, counts[0], counts[1], counts[2], N, low, ids, st); break;
+    case 3: launch_run_sorts_w<3>(rl, counts[0], counts[1], counts[2], N, low, ids, st); break;
     default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();
 }
 
-cudaError_t launch_rl_count(const uint32_t* keys, int64_t N, int L, int KW, uint32_t* tile_cnt, uint32_t* tile_off,
+cudaError_t launch_rl_count(const SortedKeys& keys, int64_t N, int L, int KW, uint32_t* tile_cnt, uint32_t* tile_off,
                             uint32_t* nb, cudaStream_t st) {
     const int tiles = (int)((N + SP_TILE - 1) / SP_TILE);
-    k_rl_count<<<dim3(tiles, L), NT, 0, st>>>(keys, N, L, KW, tile_cnt);
+    if (keys.low) k_rl_count<true><<<dim3(tiles, L), NT, 0, st>>>(keys, N, L, KW, tile_cnt);
+    else k_rl_count<false><<<dim3(tiles, L), NT, 0, st>>>(keys, N, L, KW, tile_cnt);
     k_rl_scan<<<L, NT, 0, st>>>(tile_cnt, tiles, tile_off, nb);
     return cudaGetLastError();
 }
 
-cudaError_t launch_rl_write(const uint32_t* keys, int64_t N, int L, int KW, const uint32_t* tile_off,
+cudaError_t launch_rl_write(const SortedKeys& keys, int64_t N, int L, int KW, const uint32_t* tile_off,
                             const uint64_t* boff, uint32_t* starts, uint32_t* ukeys, cudaStream_t st) {
     const int tiles = (int)((N + SP_TILE - 1) / SP_TILE);
-    k_rl_write<<<dim3(tiles, L), NT, 0, st>>>(keys, N, L, KW, tile_off, boff, starts, ukeys);
+    if (keys.low) k_rl_write<true><<<dim3(tiles, L), NT, 0, st>>>(keys, N, L, KW, tile_off, boff, starts, ukeys);
+    else k_rl_write<false><<<dim3(tiles, L), NT, 0, st>>>(keys, N, L, KW, tile_off, boff, starts, ukeys);
     return cudaGetLastError();
 }
 

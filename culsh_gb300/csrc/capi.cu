@@ -189,7 +189,8 @@ struct culsh_index {
     DevBuf<int32_t> ws_codes, ws_pmin, ws_pmax;
     DevBuf<uint16_t> ws_ah, ws_al, ws_xh, ws_xl;   // bf16 splits for the tensor-core projection
     DevBuf<float> ws_anorm, ws_xnorm;
-    DevBuf<int> ws_tcflags;
+    DevBuf<ProjectState> ws_pstate;
+    PinBuf<float> h_norms;
     double tc_predicted_open = 0.0;   // predicted share of codes the tensor-core bound leaves open
     DevBuf<uint32_t> maxb;
     PinBuf<uint32_t> h_maxb;
@@ -484,19 +485,6 @@ int build_hash(culsh_index* ix, cudaStream_t st) {
     return CULSH_OK;
 }
 
-inline uint16_t bf16_bits_rn(float f) {
-    uint32_t u;
-    std::memcpy(&u, &f, 4);
-    const uint32_t bias = 0x7FFFu + ((u >> 16) & 1u);
-    return (uint16_t)((u + bias) >> 16);
-}
-inline float bf16_to_float(uint16_t h) {
-    const uint32_t u = (uint32_t)h << 16;
-    float f;
-    std::memcpy(&f, &u, 4);
-    return f;
-}
-
 // Index projection on the tensor cores when the shape allows it. On success
 // ws_codes holds every code and cmin/cmax their ranges, exactly as the SIMT
 // kernel would produce; *done stays false when the caller must run the SIMT
@@ -522,61 +510,71 @@ int project_tensor_cores(culsh_index* ix, const float* dX, cudaStream_t st, bool
     struct {
         int Dp, LMp, grid;
     } p = {stream ? sp.Dp : rp.Dp, stream ? sp.LMp : rp.LMp, stream ? sp.grid : rp.grid};
-    // Host split of the projection matrix and upper bounds of its column norms.
-    std::vector<uint16_t> ah((size_t)p.LMp * p.Dp, 0), al((size_t)p.LMp * p.Dp, 0);
-    std::vector<float> an(LM);
-    for (int c = 0; c < LM; ++c) {
-        double ss = 0.0;
-        for (int d = 0; d < D; ++d) {
-            const float v = ix->A[(size_t)c * D + d];
-            const uint16_t h = bf16_bits_rn(v);
-            ah[(size_t)c * p.Dp + d] = h;
-            al[(size_t)c * p.Dp + d] = bf16_bits_rn(v - bf16_to_float(h));
-            ss += (double)v * v;
-        }
-        an[c] = std::nextafter((float)(std::sqrt(ss) * (1.0 + 1e-6)), INFINITY);
-    }
-    CU_TRY(ix->ws_ah.reserve(ah.size()));
-    CU_TRY(ix->ws_al.reserve(al.size()));
+    // Norms of A's columns and of a sample of X, and the operands' scales.
+    const int ns = (int)std::min<int64_t>(N, 4096);
     CU_TRY(ix->ws_anorm.reserve(LM));
-    CU_TRY(cudaMemcpyAsync(ix->ws_ah.p, ah.data(), 2 * ah.size(), cudaMemcpyHostToDevice, st));
-    CU_TRY(cudaMemcpyAsync(ix->ws_al.p, al.data(), 2 * al.size(), cudaMemcpyHostToDevice, st));
-    CU_TRY(cudaMemcpyAsync(ix->ws_anorm.p, an.data(), 4 * LM, cudaMemcpyHostToDevice, st));
-    const size_t nx = (size_t)N * p.Dp;
-    CU_TRY(ix->ws_xh.reserve(nx));
-    CU_TRY(ix->ws_xl.reserve(nx));
-    CU_TRY(ix->ws_xnorm.reserve(N));
-    CU_TRY(ix->ws_tcflags.reserve(4));
-    CU_TRY(cudaMemsetAsync(ix->ws_tcflags.p, 0, 16, st));
-    CU_TRY(launch_split_rows(dX, N, D, p.Dp, ix->ws_xh.p, ix->ws_xl.p, ix->ws_xnorm.p, ix->ws_tcflags.p, st));
-    int flags = 0;
-    CU_TRY(cudaMemcpyAsync(&flags, ix->ws_tcflags.p, 4, cudaMemcpyDeviceToHost, st));
+    CU_TRY(ix->ws_xnorm.reserve(std::max(N, ns)));
+    CU_TRY(ix->ws_pstate.reserve(1));
+    CU_TRY(ix->h_norms.reserve(LM + ns));
+    CU_TRY(launch_project_sample(dX, N, D, ns, ix->dA.p, LM, ix->ws_xnorm.p, ix->ws_anorm.p, ix->ws_pstate.p, st));
+    CU_TRY(cudaMemcpyAsync(ix->h_norms.p, ix->ws_anorm.p, 4 * (size_t)LM, cudaMemcpyDeviceToHost, st));
+    CU_TRY(cudaMemcpyAsync(ix->h_norms.p + LM, ix->ws_xnorm.p, 4 * (size_t)ns, cudaMemcpyDeviceToHost, st));
+    ProjectState ps{};
+    CU_TRY(cudaMemcpyAsync(&ps, ix->ws_pstate.p, sizeof(ps), cudaMemcpyDeviceToHost, st));
     CU_TRY(cudaStreamSynchronize(st));
-    if (flags & 2) return CULSH_OK;   // non-finite data: the SIMT kernel reports it
-    const int need_lo = flags & 1;
     // Bound on |tensor-core sum - canonical FP32 chain| per unit of sum|x||a|
-    // (bounded by |x|_2 |a|_2): split residue, one rounding per summed
-    // product, the canonical chain's rounding; 1.25 margin.
-    const double u24 = std::ldexp(1.0, -24), u23 = std::ldexp(1.0, -23), u16 = std::ldexp(1.0, -16);
-    const double split = need_lo ? 3.02 * u16 : 1.01 * u16;
-    const double accum = ((need_lo ? 3.0 : 2.0) * D + 16) * u23;
-    const float kappa = (float)(1.25 * ((D + 2) * u24 + split + accum));
+    // (bounded by |x|_2 |a|_2): fp16 split residue, one rounding per summed
+    // large product and, at 2^-10 of it, per small one (all products alike in
+    // the streaming form, whose K slices alternate), the canonical chain's
+    // rounding; 1.25 margin.
+    const double u24 = std::ldexp(1.0, -24), u23 = std::ldexp(1.0, -23), u22 = std::ldexp(1.0, -22);
+    auto kappa_for = [&](int need_lo) {
+        const double split = (need_lo ? 3.1 : 1.05) * u22;
+        const double accum = stream ? ((need_lo ? 3.0 : 2.0) * D + 16) * u23
+                                    : (D + 16) * u23 + ((need_lo ? 2.0 : 1.0) * D + 16) * u23 * std::ldexp(1.0, -10);
+        return (float)(1.25 * ((D + 2) * u24 + split + accum));
+    };
+    bool lo = (ps.flags & 8) != 0;
+    float kappa = kappa_for(lo);
     {
         // Predicted share of codes the bound leaves open: a code is open when
         // an integer lies within E / W of its value, E = kappa |x| |a|. Above
         // 6 % the FP32 recomputation costs more than the SIMT projection
-        // itself (e.g. D = 960, W = 0.25: 14 %), so the SIMT kernel runs.
-        const int ns = (int)std::min<int64_t>(N, 4096);
-        std::vector<float> xs(ns);
-        CU_TRY(cudaMemcpyAsync(xs.data(), ix->ws_xnorm.p, 4 * (size_t)ns, cudaMemcpyDeviceToHost, st));
-        CU_TRY(cudaStreamSynchronize(st));
-        std::vector<float> as(an.begin(), an.end());
-        std::nth_element(xs.begin(), xs.begin() + ns / 2, xs.end());
-        std::nth_element(as.begin(), as.begin() + LM / 2, as.end());
+        // itself, so the SIMT kernel runs. Taken before anything of X's size is
+        // converted.
+        float *as = ix->h_norms.p, *xs = ix->h_norms.p + LM;
+        std::nth_element(xs, xs + ns / 2, xs + ns);
+        std::nth_element(as, as + LM / 2, as + LM);
         const double open = 2.0 * (double)kappa * xs[ns / 2] * as[LM / 2] / (double)ix->W;
         ix->tc_predicted_open = open;
-        if (open > 0.06 && !getenv("CULSH_PROJECT_TC")) return CULSH_OK;
+        if (!(open <= 0.06) && !getenv("CULSH_PROJECT_TC")) return CULSH_OK;
     }
+    CU_TRY(ix->ws_ah.reserve((size_t)p.LMp * p.Dp));
+    CU_TRY(ix->ws_al.reserve((size_t)p.LMp * p.Dp));
+    CU_TRY(launch_split_a(ix->dA.p, LM, p.LMp, D, p.Dp, kappa, ix->ws_ah.p, ix->ws_al.p, ix->ws_anorm.p, ix->ws_pstate.p,
+                          st));
+    const size_t nx = (size_t)N * p.Dp;
+    CU_TRY(ix->ws_xh.reserve(nx));
+    // The low parts are made when the sample has one; data that are inexact
+    // elsewhere only, or whose magnitudes the sample's scale takes out of the
+    // fp16 range, are converted again.
+    for (int attempt = 0;; ++attempt) {
+        if (lo) CU_TRY(ix->ws_xl.reserve(nx));
+        CU_TRY(launch_split_rows(dX, N, D, p.Dp, kappa, ix->ws_xh.p, lo ? ix->ws_xl.p : nullptr, ix->ws_xnorm.p,
+                                 ix->ws_pstate.p, attempt > 0, st));
+        CU_TRY(cudaMemcpyAsync(&ps, ix->ws_pstate.p, sizeof(ps), cudaMemcpyDeviceToHost, st));
+        CU_TRY(cudaStreamSynchronize(st));
+        if (ps.flags & 2) return CULSH_OK;   // non-finite data: the SIMT kernel reports it
+        if (attempt == 2 && (ps.flags & 4)) return CULSH_OK;
+        if (!(ps.flags & 4) && (lo || !(ps.flags & 1))) break;
+        lo = lo || (ps.flags & 1);
+        kappa = kappa_for(lo);
+        CU_TRY(cudaMemsetAsync(&ix->ws_pstate.p->flags, 0, sizeof(int), st));
+    }
+    // the accumulators' scale and its reciprocal stay well inside the float range
+    if (!(ps.sx * ps.sa > 1e-25f && ps.sx * ps.sa < 1e25f && ix->W > 1e-10f && ix->W < 1e10f)) return CULSH_OK;
+    const int need_lo = lo ? 1 : 0;
+    ix->tc_need_lo = need_lo;
     // One recomputation region per CTA, sized for 1/6 of its codes.
     const unsigned long long cap = ((unsigned long long)N * LM / 6) / p.grid + 4096;
     CU_TRY(ix->ws_relist.reserve(cap * p.grid));
@@ -585,13 +583,13 @@ int project_tensor_cores(culsh_index* ix, const float* dX, cudaStream_t st, bool
     CU_TRY(ix->ws_pmax.reserve((size_t)p.grid * LM));
     if (stream)
         CU_TRY(launch_project_tc_stream(sp, need_lo, N, D, LM, ix->ws_xh.p, ix->ws_xl.p, ix->ws_ah.p, ix->ws_al.p,
-                                        ix->db.p, ix->ws_anorm.p, ix->ws_xnorm.p, ix->W, kappa, ix->ws_codes.p,
-                                        ix->ws_pmin.p, ix->ws_pmax.p, ix->ws_relist.p, cap, ix->ws_relist_cnt.p,
-                                        ix->err.p, st));
+                                        ix->db.p, ix->ws_anorm.p, ix->ws_xnorm.p, ix->ws_pstate.p, ix->W, kappa,
+                                        ix->ws_codes.p, ix->ws_pmin.p, ix->ws_pmax.p, ix->ws_relist.p, cap,
+                                        ix->ws_relist_cnt.p, ix->err.p, st));
     else
         CU_TRY(launch_project_tc(rp, need_lo, N, D, LM, ix->ws_xh.p, ix->ws_xl.p, ix->ws_ah.p, ix->ws_al.p, ix->db.p,
-                                 ix->ws_anorm.p, ix->ws_xnorm.p, ix->W, kappa, ix->ws_codes.p, ix->ws_pmin.p,
-                                 ix->ws_pmax.p, ix->ws_relist.p, cap, ix->ws_relist_cnt.p, ix->err.p, st));
+                                 ix->ws_anorm.p, ix->ws_xnorm.p, ix->ws_pstate.p, ix->W, kappa, ix->ws_codes.p,
+                                 ix->ws_pmin.p, ix->ws_pmax.p, ix->ws_relist.p, cap, ix->ws_relist_cnt.p, ix->err.p, st));
     CU_TRY(launch_minmax_reduce(ix->ws_pmin.p, ix->ws_pmax.p, p.grid, LM, ix->cmin.p, ix->cmax.p, st));
     std::vector<unsigned int> cnt(p.grid);
     int err = 0;
@@ -612,7 +610,6 @@ int project_tensor_cores(culsh_index* ix, const float* dX, cudaStream_t st, bool
         CU_TRY(launch_tc_recompute(dX, N, D, LM, ix->dA.p, ix->db.p, ix->W, ix->ws_relist.p, cap, ix->ws_relist_cnt.p,
                                    p.grid, ix->ws_codes.p, ix->cmin.p, ix->cmax.p, ix->err.p, st));
     ix->tc_recomputed = (long long)nre;
-    ix->tc_need_lo = need_lo;
     *done = true;
     return CULSH_OK;
 }

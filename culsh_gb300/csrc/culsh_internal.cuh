@@ -167,14 +167,20 @@ cudaError_t launch_copy_f32(const float* src, float* dst, int64_t n, cudaStream_
 cudaError_t launch_minmax_reduce(const int32_t* pmin, const int32_t* pmax, int nparts, int LM, int32_t* cmin,
                                  int32_t* cmax, cudaStream_t st);
 
-// Tensor-core (tcgen05) projection for index builds: plan, bf16 split of X,
+// Tensor-core (tcgen05) projection for index builds: plan, fp16 split of X,
 // the GEMM with the proven-code epilogue, and the canonical recomputation of
 // the codes its error bound could not prove.
+// Scales and properties of a projection's operands (device).
+struct ProjectState {
+    uint32_t amax_x, amax_a;   // largest magnitudes (float bits): X's sample, A
+    float sx, sa;              // power-of-two scales
+    int flags;                 // see k_split_rows
+};
 struct TcPlan {
     bool ok;
-    int Dp, LMp, ntiles, grid, tmem_cols;
+    int Dp, blk, LMp, ntiles, grid;   // columns of one launch, of all launches
     uint32_t b_bytes, x_bytes;
-    int stages[2];        // X-tile ring depth without / with the low bf16 part
+    int stages[2];        // X-tile ring depth without / with the low fp16 part
     size_t smem[2];
 };
 TcPlan tc_plan(int64_t N, int D, int LM, int num_sms, int max_smem);
@@ -189,15 +195,21 @@ struct TcStreamPlan {
 TcStreamPlan tc_plan_stream(int64_t N, int D, int LM, int num_sms, int max_smem);
 cudaError_t launch_project_tc_stream(const TcStreamPlan& p, int need_lo, int64_t N, int D, int LM, const void* xh,
                                      const void* xl, const void* ah, const void* al, const float* b,
-                                     const float* anorm, const float* xnorm, float W, float kappa, int32_t* codes,
-                                     int32_t* pmin, int32_t* pmax, unsigned long long* relist,
+                                     const float* anorm, const float* xnorm, const ProjectState* ps, float W, float kappa,
+                                     int32_t* codes, int32_t* pmin, int32_t* pmax, unsigned long long* relist,
                                      unsigned long long relist_cap, unsigned int* relist_cnt, int* err,
                                      cudaStream_t st);
-cudaError_t launch_split_rows(const float* X, int64_t N, int D, int Dp, void* xh, void* xl, float* xnorm, int* flags,
-                              cudaStream_t st);
+// Norms of A's columns and of ns rows of X, and both scales; fp16 parts of A and
+// of X (xl null: the high part only; rescale: from X's own maximum).
+cudaError_t launch_project_sample(const float* X, int64_t N, int D, int ns, const float* A, int LM, float* xs,
+                                  float* anorm, ProjectState* ps, cudaStream_t st);
+cudaError_t launch_split_a(const float* A, int LM, int LMp, int D, int Dp, float kappa, void* ah, void* al, float* anorm,
+                           const ProjectState* ps, cudaStream_t st);
+cudaError_t launch_split_rows(const float* X, int64_t N, int D, int Dp, float kappa, void* xh, void* xl, float* xnorm,
+                              ProjectState* ps, bool rescale, cudaStream_t st);
 cudaError_t launch_project_tc(const TcPlan& p, int need_lo, int64_t N, int D, int LM, const void* xh, const void* xl,
                               const void* ah, const void* al, const float* b, const float* anorm, const float* xnorm,
-                              float W, float kappa, int32_t* codes, int32_t* pmin, int32_t* pmax,
+                              const ProjectState* ps, float W, float kappa, int32_t* codes, int32_t* pmin, int32_t* pmax,
                               unsigned long long* relist, unsigned long long relist_cap, unsigned int* relist_cnt,
                               int* err, cudaStream_t st);
 cudaError_t launch_tc_recompute(const float* X, int64_t N, int D, int LM, const float* A, const float* b, float W,

@@ -5,25 +5,29 @@
 // GEMM over all L*M columns whose epilogue produces the exact canonical FP32
 // bucket codes.
 //
-// Exactness. X = Xh + Xl and A = Ah + Al are split into bf16 parts (Xl is
-// skipped when the data are exactly representable in bf16). The tensor cores
-// compute y = Xh*Ah' + Xh*Al' (+ Xl*Ah') with FP32 accumulation in TMEM.
-// For each element the distance between y and the canonical sequential FMA
-// chain is bounded by E = kappa * |x|_2 * |a|_2 (Cauchy-Schwarz on sum|x||a|),
-// where kappa covers the split residue (2^-16 per omitted cross term), a
-// rounding at every accumulation of the tensor-core sum (one 2^-23 step per
-// product) and the canonical chain's own rounding ((D + 2) * 2^-24), with a
-// 1.25 margin. A cheap window test on (y - b) * (1/W) proves most codes
-// without the two IEEE divides. Because fl(fl(t - b) / W)
-// is non-decreasing in t, floor(v(y - E)) == floor(v(y + E)) proves the code;
-// every other element is appended to a list and recomputed in the canonical
-// order by k_tc_recompute. Codes are therefore bit-identical to the SIMT
-// kernel and the oracle.
+// Exactness. X and A are scaled by powers of two (the largest magnitude of a
+// sample of X, of all of A, goes to 2^10) and split into fp16 parts, X = Xh + Xl
+// and A = Ah + Al (Xl is skipped when every element is exact in fp16). The
+// tensor cores compute y = Xh*Al' (+ Xl*Ah') + Xh*Ah' with FP32 accumulation
+// in TMEM, the small products first. For each element the distance between y
+// and the canonical sequential FMA chain is bounded by
+// E = kappa * |x|_2 * |a|_2 (Cauchy-Schwarz on sum|x||a|), where kappa covers
+// the split residue (2^-22 per part: fp16 pairs keep 22 bits, bf16 pairs had
+// kept 16), a rounding at every accumulation of the large products (one 2^-23
+// step per product; the small ones accumulate at 2^-11 of that) and the
+// canonical chain's own rounding ((D + 2) * 2^-24), with a 1.25 margin. A window
+// test on (y - b) * (1/W) without a division proves a code: when no integer
+// lies within E / W and the test's own rounding of it, every value the
+// canonical chain can take has the same floor. Every other element is
+// appended to a list and recomputed in the canonical order by k_tc_recompute.
+// Codes are therefore bit-identical to the SIMT kernel and the oracle. With
+// bf16 parts in any order 3.8 % of the codes of 1M x 128 integer features at
+// W = 16 were open (0.69 ms of recomputation); now 1.7 %.
 //
 // Structure: persistent CTAs of 18 warps. Warp 0 issues TMA loads (the
 // projection matrix once, then 128-point X tiles into a 1- or 2-stage ring);
 // warp 1 owns TMEM and issues tcgen05.mma (M=128, N=L*M padded to 16, K=16
-// per instruction, bf16 inputs, FP32 accumulators, two accumulators so that
+// per instruction, fp16 inputs, FP32 accumulators, two accumulators so that
 // the epilogue of one tile overlaps the MMAs of the next); warps 2-17 read
 // TMEM with tcgen05.ld (four warps per lane quadrant, each taking a quarter
 // of the columns) and run the epilogue. Codes the bound leaves open are appended
@@ -31,7 +35,7 @@
 // on timeout the kernel raises kErrSpin and the host falls back to the SIMT
 // kernel.
 #include <cuda.h>
-#include <cuda_bf16.h>
+#include <cuda_fp16.h>
 
 #include <algorithm>
 #include <cfloat>
@@ -54,21 +58,21 @@ struct TcArgs {
     const float* b;        // [LM]
     const float* anorm;    // [LM] upper bounds of |a_c|_2
     const float* xnorm;    // [N]  upper bounds of |x_n|_2
+    const ProjectState* ps;   // scales of X and A
     int32_t* codes;        // [LM][N]
     int32_t* pmin;         // [gridDim.x][LM]
     int32_t* pmax;
     unsigned long long* relist;   // (n << 16) | c of codes to recompute, one region per CTA
     unsigned long long relist_cap;        // entries per CTA region
     unsigned int* relist_cnt;             // [gridDim.x] entries used per region (may exceed the cap)
-    float inv_w;                          // 1/W rounded to nearest
     int* err;
-    uint32_t b_bytes, x_bytes;    // one bf16 operand region of A (LMp x Dp) / of an X tile (128 x Dp)
+    uint32_t b_bytes, x_bytes;    // one fp16 operand region of A (LMp x Dp) / of an X tile (128 x Dp)
     // Streaming form (A too large to keep in shared memory): this launch
     // covers columns [col0, col0 + LM) of LMtot; each ring stage holds one
     // 64-wide K slice of Xh (Xl) and of Ah, Al.
     int col0, LMtot;
     uint32_t stage_bytes;         // streaming: bytes of one ring stage
-    uint32_t a_chunk;             // streaming: bytes of one A slice (LMp x 64 bf16)
+    uint32_t a_chunk;             // streaming: bytes of one A slice (LMp x 64 fp16)
     int list_continue;            // streaming: recompute lists continue from relist_cnt
 };
 
@@ -92,11 +96,27 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
         : "memory");
     return ok != 0;
 }
+__device__ __forceinline__ bool mbar_test_wait(uint64_t* bar, uint32_t parity) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tmbarrier.test_wait.parity.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}\n"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return ok != 0;
+}
+// One lane of the (converged) warp, the same on every call.
+__device__ __forceinline__ bool elect_lane() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}\n" : "=r"(p));
+    return p != 0;
+}
 // Bounded wait for the completion of the phase with the given parity. The
 // single-thread producer and MMA roles back off between polls so that their
 // spinning does not take issue slots from the epilogue warps.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* err,
                                           bool backoff = false) {
+    if (mbar_test_wait(bar, parity)) return true;   // cheaper than a suspending wait when the phase is over
     for (uint32_t i = 0; i < kPollLimit; ++i) {
         if (mbar_try_wait(bar, parity)) return true;
         if (*abort_flag) return false;
@@ -122,7 +142,7 @@ __device__ __forceinline__ uint64_t sw128_desc(uint32_t saddr) {
            ((uint64_t)1 << 46) | ((uint64_t)2 << 61);
 }
 
-__device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
+__device__ __forceinline__ void umma_f16(uint32_t d_tmem, uint64_t adesc, uint64_t bdesc, uint32_t idesc,
                                           uint32_t accumulate) {
     asm volatile(
         "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\ttcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}\n" ::"r"(
@@ -173,13 +193,15 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(bfull + 1);
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr + 1);
     unsigned int* list_top = reinterpret_cast<unsigned int*>(tmem_ptr + 2);
-    int32_t* cmin = reinterpret_cast<int32_t*>(tmem_ptr + 4);
+    int32_t* cmin = reinterpret_cast<int32_t*>(tail + 96);   // 16-byte aligned, past the barriers
     int32_t* cmax = cmin + a.LMp;
-    float* s_an = reinterpret_cast<float*>(cmax + a.LMp);     // |a_c|_2 bounds
-    float* s_b = s_an + a.LMp;                                 // b_c
-    uint32_t* s_unsure = reinterpret_cast<uint32_t*>(s_b + a.LMp);   // [8 words][TC_EPI_WARPS * 32] per-thread masks
+    float* s_an = reinterpret_cast<float*>(cmax + a.LMp);     // |a_c|_2 bounds / W
+    float* s_bw = s_an + a.LMp;                                // -b_c / W
+    float* s_win = s_bw + a.LMp;                               // the window test's own rounding beside |v|
+    uint32_t* s_unsure = reinterpret_cast<uint32_t*>(s_win + a.LMp);   // [8 words][TC_EPI_WARPS * 32] per-thread masks
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);   // known to be warp-uniform
     if (tid == 0) {
         for (int s = 0; s < 2; ++s) {
             mbar_init(full + s, 1);
@@ -195,8 +217,10 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     for (int c = tid; c < a.LMp; c += TC_THREADS) {
         cmin[c] = INT_MAX;
         cmax[c] = INT_MIN;
-        s_an[c] = c < a.LM ? __ldg(a.anorm + a.col0 + c) : 0.0f;
-        s_b[c] = c < a.LM ? __ldg(a.b + a.col0 + c) : 0.0f;
+        const float inv_w = 1.0f / a.W, bc = c < a.LM ? __ldg(a.b + a.col0 + c) : 0.0f;
+        s_an[c] = c < a.LM ? __fmul_ru(__ldg(a.anorm + a.col0 + c), inv_w * 1.0001f) : 0.0f;
+        s_bw[c] = -bc * inv_w;
+        s_win[c] = fabsf(bc * inv_w) * 4.8e-7f + 1.5e-7f;
     }
     if (warp == 1) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_ptr)),
@@ -229,43 +253,50 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                 tma_load_2d(sa + a.a_chunk, &tm_al, full + s, k * 64, a.col0);
             }
         }
-    } else if (kStream && warp == 1 && lane == 0) {
-        // ---- MMA issuer, streaming ----
-        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(a.LMp >> 3) << 17) |
-                               ((uint32_t)(TC_M >> 4) << 24);
+    } else if (kStream && warp == 1) {
+        // ---- MMA issuer, streaming (the whole warp walks, one lane issues) ----
+        // kind::f16 instruction descriptor: FP32 accumulator, fp16 A and B,
+        // both K-major, N = LMp, M = 128.
+        const uint32_t idesc = (1u << 4) | ((uint32_t)(a.LMp >> 3) << 17) | ((uint32_t)(TC_M >> 4) << 24);
         const uint32_t xb = 16384u;
+        const bool leader = elect_lane();
         int i = 0, t = 0;
         bool ok = true;
         for (int tile = blockIdx.x; tile < a.ntiles && ok; tile += gridDim.x, ++t) {
             const int acc = t & 1;
-            if (t >= 2 && !mbar_wait(tempty + acc, (uint32_t)(((t >> 1) - 1) & 1), abort_flag, a.err, true)) break;
+            ok = t < 2 || __all_sync(0xffffffffu, mbar_wait(tempty + acc, (uint32_t)(((t >> 1) - 1) & 1), abort_flag, a.err, true));
+            if (!ok) break;
             const uint32_t d = tmem + (uint32_t)(acc * a.LMp);
             for (int k = 0; k < katoms; ++k, ++i) {
                 const int s = i % a.stages;
-                if (!mbar_wait(full + s, (uint32_t)((i / a.stages) & 1), abort_flag, a.err, true)) {
-                    ok = false;
-                    break;
-                }
+                ok = __all_sync(0xffffffffu, mbar_wait(full + s, (uint32_t)((i / a.stages) & 1), abort_flag, a.err, true));
+                if (!ok) break;
                 tc_fence_after();
-                const uint32_t xh = smem_u32(sX + (size_t)s * stage_bytes);
-                const uint32_t ah = xh + xb * (a.need_lo ? 2u : 1u), al = ah + a.a_chunk;
-                for (int ks = 0; ks < 4; ++ks) {
-                    const uint32_t o = (uint32_t)(ks * 32);
-                    umma_bf16(d, sw128_desc(xh + o), sw128_desc(ah + o), idesc, (k > 0 || ks > 0) ? 1u : 0u);
-                    umma_bf16(d, sw128_desc(xh + o), sw128_desc(al + o), idesc, 1u);
-                    if (a.need_lo) umma_bf16(d, sw128_desc(xh + xb + o), sw128_desc(ah + o), idesc, 1u);
+                const uint32_t xs = smem_u32(sX + (size_t)s * stage_bytes);
+                const uint32_t as = xs + xb * (a.need_lo ? 2u : 1u);
+                const uint64_t xh = sw128_desc(xs), xl = sw128_desc(xs + xb), ah = sw128_desc(as),
+                               al = sw128_desc(as + a.a_chunk);
+                if (leader) {
+#pragma unroll
+                    for (int ks = 0; ks < 4; ++ks)
+                        umma_f16(d, xh + ks * 2, al + ks * 2, idesc, (k > 0 || ks > 0) ? 1u : 0u);
+                    if (a.need_lo)
+#pragma unroll
+                        for (int ks = 0; ks < 4; ++ks) umma_f16(d, xl + ks * 2, ah + ks * 2, idesc, 1u);
+#pragma unroll
+                    for (int ks = 0; ks < 4; ++ks) umma_f16(d, xh + ks * 2, ah + ks * 2, idesc, 1u);
+                    umma_commit(empty + s);
+                    if (k + 1 == katoms) umma_commit(tfull + acc);
                 }
-                umma_commit(empty + s);
+                __syncwarp();
             }
-            if (!ok) break;
-            umma_commit(tfull + acc);
         }
     } else if (!kStream && warp == 0 && lane == 0) {
         // ---- TMA producer ----
         mbar_expect_tx(bfull, 2 * a.b_bytes);
         for (int k = 0; k < katoms; ++k) {
-            tma_load_2d(sAh + (size_t)k * a.LMp * 128, &tm_ah, bfull, k * 64, 0);
-            tma_load_2d(sAl + (size_t)k * a.LMp * 128, &tm_al, bfull, k * 64, 0);
+            tma_load_2d(sAh + (size_t)k * a.LMp * 128, &tm_ah, bfull, k * 64, a.col0);
+            tma_load_2d(sAl + (size_t)k * a.LMp * 128, &tm_al, bfull, k * 64, a.col0);
         }
         int i = 0;
         for (int tile = blockIdx.x; tile < a.ntiles && !*abort_flag; tile += gridDim.x, ++i) {
@@ -279,32 +310,39 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                 if (a.need_lo) tma_load_2d(xh + a.x_bytes + (size_t)k * TC_M * 128, &tm_xl, full + s, k * 64, tile * TC_M);
             }
         }
-    } else if (!kStream && warp == 1 && lane == 0) {
-        // ---- MMA issuer ----
-        // kind::f16 instruction descriptor: FP32 accumulator, bf16 A and B,
-        // both K-major, N = LMp, M = 128.
-        const uint32_t idesc = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(a.LMp >> 3) << 17) |
-                               ((uint32_t)(TC_M >> 4) << 24);
-        if (mbar_wait(bfull, 0, abort_flag, a.err, true)) {
-            int i = 0;
-            for (int tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x, ++i) {
-                const int s = i % a.stages, acc = i & 1;
-                if (i >= 2 && !mbar_wait(tempty + acc, (uint32_t)(((i >> 1) - 1) & 1), abort_flag, a.err, true)) break;
-                if (!mbar_wait(full + s, (uint32_t)((i / a.stages) & 1), abort_flag, a.err, true)) break;
-                tc_fence_after();
-                const uint32_t d = tmem + (uint32_t)(acc * a.LMp);
-                const uint32_t xh = smem_u32(sX + (size_t)s * stage_bytes);
-                const uint32_t ah = smem_u32(sAh), al = smem_u32(sAl);
-                for (int ks = 0; ks < ksteps; ++ks) {
-                    const uint32_t xo = (uint32_t)((ks >> 2) * TC_M * 128 + (ks & 3) * 32);
-                    const uint32_t bo = (uint32_t)((ks >> 2) * a.LMp * 128 + (ks & 3) * 32);
-                    umma_bf16(d, sw128_desc(xh + xo), sw128_desc(ah + bo), idesc, ks > 0 ? 1u : 0u);
-                    umma_bf16(d, sw128_desc(xh + xo), sw128_desc(al + bo), idesc, 1u);
-                    if (a.need_lo) umma_bf16(d, sw128_desc(xh + a.x_bytes + xo), sw128_desc(ah + bo), idesc, 1u);
-                }
+    } else if (!kStream && warp == 1) {
+        // ---- MMA issuer (the whole warp walks, one lane issues) ----
+        const uint32_t idesc = (1u << 4) | ((uint32_t)(a.LMp >> 3) << 17) | ((uint32_t)(TC_M >> 4) << 24);
+        const bool leader = elect_lane();
+        const uint64_t ah = sw128_desc(smem_u32(sAh)), al = sw128_desc(smem_u32(sAl));
+        const uint64_t x0 = sw128_desc(smem_u32(sX));
+        bool ok = __all_sync(0xffffffffu, mbar_wait(bfull, 0, abort_flag, a.err, true));
+        int i = 0;
+        for (int tile = blockIdx.x; tile < a.ntiles && ok; tile += gridDim.x, ++i) {
+            const int s = i % a.stages, acc = i & 1;
+            ok = (i < 2 || __all_sync(0xffffffffu, mbar_wait(tempty + acc, (uint32_t)(((i >> 1) - 1) & 1), abort_flag, a.err, true))) &&
+                 __all_sync(0xffffffffu, mbar_wait(full + s, (uint32_t)((i / a.stages) & 1), abort_flag, a.err, true));
+            if (!ok) break;
+            tc_fence_after();
+            const uint32_t d = tmem + (uint32_t)(acc * a.LMp);
+            const uint64_t xh = x0 + (uint64_t)(s * (stage_bytes >> 4)), xl = xh + (a.x_bytes >> 4);
+            if (leader) {
+                // the small products first: their sums round at 2^-11 of the total
+                auto product = [&](uint64_t x, uint64_t c, bool first) {
+                    for (int ka = 0; ka < katoms; ++ka) {
+                        const uint64_t xo = x + (uint64_t)((ka * TC_M * 128) >> 4), co = c + (uint64_t)((ka * a.LMp * 128) >> 4);
+#pragma unroll
+                        for (int ks = 0; ks < 4; ++ks)
+                            umma_f16(d, xo + ks * 2, co + ks * 2, idesc, (first && (ka | ks) == 0) ? 0u : 1u);
+                    }
+                };
+                product(xh, al, true);
+                if (a.need_lo) product(xl, ah, false);
+                product(xh, ah, false);
                 umma_commit(empty + s);
                 umma_commit(tfull + acc);
             }
+            __syncwarp();
         }
     } else if (warp >= 2) {
         // ---- epilogue: TMEM -> proven codes, list of codes to recompute ----
@@ -317,9 +355,12 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         uint32_t* my_mask = s_unsure + ew * 32 + lane;   // word w at my_mask[w * TC_EPI_WARPS * 32]
         unsigned long long* region = a.relist + (unsigned long long)blockIdx.x * a.relist_cap;
         int i = 0;
+        // v = (y - b) / W up to rounding: acc * k1 - b / W, k1 = 1 / (scales W)
+        const float k1 = __fdiv_rn(1.0f, a.W) / (a.ps->sx * a.ps->sa);   // the scales are powers of two
         for (int tile = blockIdx.x; tile < a.ntiles; tile += gridDim.x, ++i) {
             const int acc = i & 1;
-            if (!mbar_wait(tfull + acc, (uint32_t)((i >> 1) & 1), abort_flag, a.err)) break;
+            const bool ok = mbar_wait(tfull + acc, (uint32_t)((i >> 1) & 1), abort_flag, a.err);
+            if (!__all_sync(0xffffffffu, ok)) break;
             tc_fence_after();
             const int64_t n = (int64_t)tile * TC_M + row;
             const bool valid = n < a.N;
@@ -328,44 +369,64 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
             for (int ch = ch0; ch < ch1; ++ch) {
                 const int c0 = ch * 16;
                 uint32_t r[16];
+                __syncwarp();
                 tmem_ld16(tmem + ((uint32_t)(quad * 32) << 16) + (uint32_t)(acc * a.LMp + c0), r);
                 int32_t* out = a.codes + (int64_t)(a.col0 + c0) * a.N + n;
-                uint32_t unsure = 0;
-                int32_t mylo = INT_MAX, myhi = INT_MIN;
+                const int live = a.LM - c0;                // columns of this chunk that exist
+                const uint32_t cols = live >= 16 ? 0xFFFFu : (1u << live) - 1u;
+                uint32_t unsure = 0, wide = 0;
 #pragma unroll
-                for (int j = 0; j < 16; ++j) {
-                    const int c = c0 + j;
-                    const float y = __uint_as_float(r[j]);
-                    const float E = __fmul_ru(kx, s_an[c]);
-                    const float bc = s_b[c];
-                    // Cheap rigorous test first: v_approx is within |v| * 2^-21 +
-                    // 2^-40 of the canonical v of any t in [y - E, y + E] widened
-                    // by E/W; no integer in that window proves the code.
-                    const float va = (y - bc) * a.inv_w;
-                    const float fa = floorf(va);
-                    const float win = __fmul_ru(E, a.inv_w) * 1.0001f + fabsf(va) * 4.8e-7f + 1e-12f;
-                    bool sure = va - fa > win && (fa + 1.0f) - va > win && fabsf(va) < 2.0e9f;
-                    float fl = fa;
-                    if (!sure) {
-                        fl = floorf(__fdiv_rn(__fsub_rn(__fsub_rd(y, E), bc), a.W));
-                        const float fh = floorf(__fdiv_rn(__fsub_rn(__fadd_ru(y, E), bc), a.W));
-                        sure = fl == fh && fl >= -2147483648.0f && fl < 2147483648.0f;
-                    }
-                    const bool live = valid && c < a.LM;
-                    const int32_t code = sure ? (int32_t)fl : 0;
-                    if (live) out[(int64_t)j * a.N] = code;
-                    if (live && !sure) unsure |= 1u << j;
-                    const bool use = live && sure;
-                    const int32_t lo = __reduce_min_sync(0xffffffffu, use ? code : INT_MAX);
-                    const int32_t hi = __reduce_max_sync(0xffffffffu, use ? code : INT_MIN);
-                    if (lane == j) {
-                        mylo = lo;
-                        myhi = hi;
+                for (int j4 = 0; j4 < 16; j4 += 4) {
+                    const float4 an = *reinterpret_cast<const float4*>(s_an + c0 + j4);
+                    const float4 bw = *reinterpret_cast<const float4*>(s_bw + c0 + j4);
+                    const float4 wn = *reinterpret_cast<const float4*>(s_win + c0 + j4);
+                    const int4 mn = *reinterpret_cast<const int4*>(cmin + c0 + j4);
+                    const int4 mx = *reinterpret_cast<const int4*>(cmax + c0 + j4);
+                    auto one = [&](int j, float ac, float bc, float wc, int lo, int hi) {
+                        // The window test: va is within win of every canonical
+                        // v of a sum in [y - E, y + E]; no integer in that
+                        // window proves the code. (From |va| = 2^21 on win
+                        // exceeds a half: codes near the int32 range stay open.)
+                        const float va = __fmaf_rn(__uint_as_float(r[j]), k1, bc);
+                        const float fa = floorf(va);
+                        const float fr = va - fa;
+                        const float win = __fmaf_ru(kx, ac, __fmaf_ru(fabsf(va), 4.8e-7f, wc));
+                        const bool sure = fminf(fr, 1.0f - fr) > win;
+                        const int32_t code = __float2int_rz(fa);
+                        r[j] = (uint32_t)code;
+                        unsure |= sure ? 0u : 1u << j;
+                        wide |= code < lo || code > hi ? 1u << j : 0u;
+                    };
+                    one(j4, an.x, bw.x, wn.x, mn.x, mx.x);
+                    one(j4 + 1, an.y, bw.y, wn.y, mn.y, mx.y);
+                    one(j4 + 2, an.z, bw.z, wn.z, mn.z, mx.z);
+                    one(j4 + 3, an.w, bw.w, wn.w, mn.w, mx.w);
+                }
+                unsure = valid ? unsure & cols : 0u;
+                wide = valid ? wide & cols & ~unsure : 0u;
+                if (valid) {   // open codes are written over by the recomputation
+#pragma unroll
+                    for (int j = 0; j < 16; ++j) {
+                        if (j < live) *out = (int32_t)r[j];
+                        out += a.N;
                     }
                 }
-                if (lane < 16 && mylo <= myhi) {
-                    atomicMin(cmin + c0 + lane, mylo);
-                    atomicMax(cmax + c0 + lane, myhi);
+                // Column ranges: only columns with a code outside the range seen
+                // so far reduce theirs (a warp reduction per column and value
+                // for every chunk had taken most of the kernel: 0.61 ms at
+                // 1M x 192 columns, now 0.32 ms).
+                for (uint32_t m = __reduce_or_sync(0xffffffffu, wide); m; m &= m - 1) {
+                    const int j = __ffs((int)m) - 1;
+                    int32_t code = 0;
+#pragma unroll
+                    for (int k = 0; k < 16; ++k) code = k == j ? (int32_t)r[k] : code;
+                    const bool use = (wide >> j) & 1u;
+                    const int32_t lo = __reduce_min_sync(0xffffffffu, use ? code : INT_MAX);
+                    const int32_t hi = __reduce_max_sync(0xffffffffu, use ? code : INT_MIN);
+                    if (lane == 0) {
+                        atomicMin(cmin + c0 + j, lo);
+                        atomicMax(cmax + c0 + j, hi);
+                    }
                 }
                 // bit (ch - ch0) * 16 + j of this thread's mask words
                 const int w = (ch - ch0) >> 1;
@@ -414,116 +475,216 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     }
 }
 
-// Splits X into bf16 parts and bounds the row norms from above (warp per row).
-__global__ void k_split_rows(const float* __restrict__ X, int64_t N, int D, int Dp, __nv_bfloat16* __restrict__ xh,
-                             __nv_bfloat16* __restrict__ xl, float* __restrict__ xnorm, int* __restrict__ flags) {
+// Power-of-two scale that takes magnitudes up to amax below 2^11 (1 for zero).
+__device__ __forceinline__ float project_scale(uint32_t amax_bits) {
+    const float amax = __uint_as_float(amax_bits);
+    return amax > 0.0f ? scalbnf(1.0f, 10 - ilogbf(amax)) : 1.0f;
+}
+
+// A row (or column of A) of a warp: fp16 parts of row * scale into h and l
+// (either may be null) and its squared norm, rounded up. Lanes hold four
+// consecutive elements where vec (16-byte aligned rows), one otherwise.
+__device__ __forceinline__ void split_row(const float* __restrict__ row, int D, int Dp, float scale, bool vec, __half* h,
+                                          __half* l, float& ss, bool& inexact, float& amax, bool& bad) {
+    const int lane = threadIdx.x & 31;
+    ss = 0.0f;
+    auto part = [&](float x, __half& hi, __half& lo) {
+        const float xs = x * scale;   // exact but for subnormal results
+        hi = __float2half_rn(xs);
+        lo = __float2half_rn(__fsub_rn(xs, __half2float(hi)));
+        inexact |= (__half_as_ushort(lo) & 0x7FFF) != 0;
+        if (fabsf(x) <= FLT_MAX) amax = fmaxf(amax, fabsf(x));
+        else bad = true;
+        ss = __fmaf_ru(x, x, ss);
+    };
+    if (vec) {
+        for (int d = 4 * lane; d < Dp; d += 128) {
+            const float4 x = d < D ? __ldg(reinterpret_cast<const float4*>(row + d)) : make_float4(0.f, 0.f, 0.f, 0.f);
+            __align__(8) __half hh[4], ll[4];
+            part(x.x, hh[0], ll[0]);
+            part(x.y, hh[1], ll[1]);
+            part(x.z, hh[2], ll[2]);
+            part(x.w, hh[3], ll[3]);
+            if (h) *reinterpret_cast<uint2*>(h + d) = *reinterpret_cast<const uint2*>(hh);
+            if (l) *reinterpret_cast<uint2*>(l + d) = *reinterpret_cast<const uint2*>(ll);
+        }
+    } else {
+        for (int d = lane; d < Dp; d += 32) {
+            __half hh, ll;
+            part(d < D ? __ldg(row + d) : 0.0f, hh, ll);
+            if (h) h[d] = hh;
+            if (l) l[d] = ll;
+        }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) ss = __fadd_ru(ss, __shfl_xor_sync(0xffffffffu, ss, o));
+}
+
+__device__ __forceinline__ float norm_up(float ss) { return __fmul_ru(__fsqrt_ru(ss), 1.00001f); }
+
+// Norms of A's columns and of ns rows spread over X, the largest magnitudes of
+// both (one warp per row); flag 8: some of those rows are not exact in fp16.
+__global__ void k_project_sample(const float* __restrict__ X, int64_t N, int D, int ns, const float* __restrict__ A,
+                                 int LM, float* __restrict__ xs, float* __restrict__ anorm, ProjectState* st) {
+    const int lane = threadIdx.x & 31;
+    const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    if (w >= ns + LM) return;
+    const bool is_a = w >= ns;
+    const float* row = is_a ? A + (int64_t)(w - ns) * D : X + (int64_t)w * (N / ns) * D;
+    float ss, amax = 0.0f;
+    bool inexact = false, bad = false;
+    split_row(row, D, D, 1.0f, false, nullptr, nullptr, ss, inexact, amax, bad);
+    const uint32_t am = __reduce_max_sync(0xffffffffu, __float_as_uint(amax));
+    inexact = __any_sync(0xffffffffu, inexact);
+    if (lane == 0) {
+        if (!is_a && inexact) atomicOr(&st->flags, 8);
+        (is_a ? anorm[w - ns] : xs[w]) = norm_up(ss);
+        atomicMax(is_a ? &st->amax_a : &st->amax_x, am);
+    }
+}
+
+// Scales from the largest magnitudes; forced_x: X's own maximum after a
+// conversion whose sample-based scale overflowed.
+__global__ void k_project_scales(ProjectState* st) {
+    st->sx = project_scale(st->amax_x);
+    st->sa = project_scale(st->amax_a);
+}
+
+// fp16 parts of A (LMp rows, zero past LM; the bounds of its norms get the
+// absolute residue of subnormal parts).
+__global__ void k_split_a(const float* __restrict__ A, int LM, int LMp, int D, int Dp, float kappa, __half* ah,
+                          __half* al, float* anorm, const ProjectState* st) {
+    const int lane = threadIdx.x & 31;
+    const int c = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
+    if (c >= LMp) return;
+    float ss, amax = 0.0f;
+    bool inexact = false, bad = false;
+    // rows past LM: zero dimensions to read
+    split_row(A + (int64_t)min(c, LM - 1) * D, c < LM ? D : 0, Dp, st->sa, false, ah + (int64_t)c * Dp,
+              al + (int64_t)c * Dp, ss, inexact, amax, bad);
+    if (lane == 0 && c < LM) anorm[c] += 1.01f * 2.98023224e-8f * sqrtf((float)D) / (st->sa * kappa);
+}
+
+// fp16 parts of X and upper bounds of its row norms (warp per row); xl is null
+// where the sample was exact in fp16. flags: 1 some element has a low part, 2
+// a value is not finite, 4 a scaled value leaves the fp16 range (amax_x then
+// holds the largest magnitude).
+__global__ void k_split_rows(const float* __restrict__ X, int64_t N, int D, int Dp, float kappa, __half* __restrict__ xh,
+                             __half* __restrict__ xl, float* __restrict__ xnorm, ProjectState* st) {
     const int lane = threadIdx.x & 31;
     const int64_t w0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    int any_lo = 0, bad = 0;
+    const float sx = st->sx, res = 1.01f * 2.98023224e-8f * sqrtf((float)D) / (sx * kappa);
+    const bool vec = (D & 3) == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
+    float amax = 0.0f;
+    bool inexact = false, bad = false;
     for (int64_t n = w0; n < N; n += nw) {
-        const float* row = X + n * D;
-        float ss = 0.0f;
-        for (int d = lane; d < Dp; d += 32) {
-            const float x = d < D ? __ldg(row + d) : 0.0f;
-            const __nv_bfloat16 h = __float2bfloat16_rn(x);
-            const __nv_bfloat16 l = __float2bfloat16_rn(__fsub_rn(x, __bfloat162float(h)));
-            xh[n * Dp + d] = h;
-            xl[n * Dp + d] = l;
-            any_lo |= __bfloat16_as_ushort(l) & 0x7FFF;
-            bad |= !(fabsf(x) <= FLT_MAX);
-            ss = __fmaf_ru(x, x, ss);
-        }
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) ss = __fadd_ru(ss, __shfl_xor_sync(0xffffffffu, ss, o));
-        if (lane == 0) xnorm[n] = __fmul_ru(__fsqrt_ru(ss), 1.0009765625f);
+        float ss;
+        split_row(X + n * D, D, Dp, sx, vec, xh + n * Dp, xl ? xl + n * Dp : nullptr, ss, inexact, amax, bad);
+        if (lane == 0) xnorm[n] = __fadd_ru(norm_up(ss), res);
     }
-    if (__any_sync(0xffffffffu, any_lo != 0) && lane == 0) atomicOr(flags, 1);
-    if (__any_sync(0xffffffffu, bad != 0) && lane == 0) atomicOr(flags, 2);
+    const uint32_t am = __reduce_max_sync(0xffffffffu, __float_as_uint(amax));
+    const int f = (__any_sync(0xffffffffu, inexact) ? 1 : 0) | (__any_sync(0xffffffffu, bad) ? 2 : 0) |
+                  (__uint_as_float(am) * sx > 65000.0f ? 4 : 0);
+    if (lane == 0) {
+        if (f & ~st->flags) atomicOr(&st->flags, f);
+        if (f & 4) atomicMax(&st->amax_x, am);
+    }
 }
 
 // Canonical-order recomputation of the codes the tensor-core bound could not
 // prove (one thread per list entry; entries of CTA region r are
-// list[r * cap .. r * cap + cnt[r])).
-__global__ void k_tc_recompute(const float* __restrict__ X, int64_t N, int D, const float* __restrict__ A,
-                               const float* __restrict__ b, float W, const unsigned long long* __restrict__ list,
-                               unsigned long long cap, const unsigned int* __restrict__ cnt, int regions, int LM,
-                               int stage_a, int32_t* __restrict__ codes, int32_t* __restrict__ cmin,
-                               int32_t* __restrict__ cmax, int* __restrict__ err) {
-    // A staged in shared memory with padded rows, so that the lanes of a warp
-    // (different columns, same d) hit different banks: D + 4 floats when
-    // D % 4 == 0 (16-byte reads; column c starts at bank 4c mod 32), else D + 1.
-    extern __shared__ __align__(16) float sA[];
-    __shared__ int32_t smin[1024], smax[1024];   // per-column ranges of this block (LM <= 1024 here)
+// list[r * cap .. r * cap + cnt[r])). A warp's 32 rows of X are fetched together,
+// RD dimensions at a time: four (RD = 16) consecutive lanes read one row's 16-byte
+// pieces, so that a load covers eight rows' 64 bytes instead of one 16-byte
+// piece of 32 rows (which had bound the kernel on L1 lookups: 0.52 ms for 2.9M
+// codes of 128 dimensions, now 0.34 ms); each lane then takes its own row
+// from shared memory. A is staged there too where it fits (stage_a), with rows
+// padded to D + 4 floats so that different columns at the same d spread over
+// the banks.
+constexpr int RT = 1024;       // threads
+constexpr int RD = 16;         // dimensions per step
+constexpr int RP = RD + 4;     // padded row
+__global__ void __launch_bounds__(RT, 1) k_tc_recompute(const float* __restrict__ X, int64_t N, int D,
+                               const float* __restrict__ A, const float* __restrict__ b, float W,
+                               const unsigned long long* __restrict__ list, unsigned long long cap,
+                               const unsigned int* __restrict__ cnt, int regions, int LM, int stage_a, int stage_x,
+                               int32_t* __restrict__ codes, int32_t* __restrict__ cmin, int32_t* __restrict__ cmax,
+                               int* __restrict__ err) {
+    extern __shared__ __align__(16) float sX[];   // [warps][32][RP], then A
+    __shared__ int32_t smin[1024], smax[1024];    // per-column ranges of this block (LM <= 1024 here)
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    float* wx = sX + (size_t)warp * 32 * RP;
+    float* sA = sX + (stage_x ? (size_t)(RT / 32) * 32 * RP : 0);
     const int Dq = (D & 3) == 0 ? D + 4 : D + 1;
     const bool block_range = LM <= 1024;
     if (block_range)
-        for (int c = threadIdx.x; c < LM; c += blockDim.x) {
+        for (int c = tid; c < LM; c += RT) {
             smin[c] = INT_MAX;
             smax[c] = INT_MIN;
         }
     if (stage_a)
-        for (int i = threadIdx.x; i < LM * D; i += blockDim.x) sA[(i / D) * Dq + (i % D)] = __ldg(A + i);
+        for (int i = tid; i < LM * D; i += RT) sA[(i / D) * Dq + (i % D)] = __ldg(A + i);
     __syncthreads();
-    // Blocks walk the regions (region r is list[r * cap .. r * cap + cnt[r])).
-    for (int r = blockIdx.x % regions, part = blockIdx.x / regions, parts = (gridDim.x + regions - 1) / regions;
-         r < regions; r += gridDim.x) {
-      const unsigned int nr = min((unsigned long long)__ldg(cnt + r), cap);
-      for (unsigned int k = part * blockDim.x + threadIdx.x; k < nr; k += parts * blockDim.x) {
-        const unsigned long long e = list[(unsigned long long)r * cap + k];
-        const int64_t n = (int64_t)(e >> 16);
-        const int c = (int)(e & 0xFFFF);
-        const float* x = X + n * D;
-        float acc = 0.0f;
-        if (stage_a && (D & 3) == 0) {
-            const float* av = sA + (int64_t)c * Dq;
-            for (int d = 0; d < D; d += 4) {
-                const float4 x4 = __ldg(reinterpret_cast<const float4*>(x + d));
-                const float4 a4 = *reinterpret_cast<const float4*>(av + d);
-                acc = __fmaf_rn(x4.x, a4.x, acc);
-                acc = __fmaf_rn(x4.y, a4.y, acc);
-                acc = __fmaf_rn(x4.z, a4.z, acc);
-                acc = __fmaf_rn(x4.w, a4.w, acc);
+    for (int r = blockIdx.x; r < regions; r += gridDim.x) {
+        const unsigned int nr = min((unsigned long long)__ldg(cnt + r), cap);
+        for (unsigned int k0 = warp * 32; k0 < nr; k0 += RT) {
+            const bool on = k0 + lane < nr;
+            const unsigned long long e = on ? list[(unsigned long long)r * cap + k0 + lane] : 0ull;
+            const int64_t n = (int64_t)(e >> 16);
+            const int c = (int)(e & 0xFFFF);
+            const float* av = stage_a ? sA + (int64_t)c * Dq : A + (int64_t)c * D;
+            float acc = 0.0f;
+            if (stage_x) {
+                for (int d0 = 0; d0 < D; d0 += RD) {
+                    const int dl = d0 + 4 * (lane & 3);
+                    float4 v[4];
+#pragma unroll
+                    for (int i = 0; i < 4; ++i) {
+                        const int64_t rn = __shfl_sync(0xffffffffu, n, i * 8 + (lane >> 2));
+                        v[i] = dl < D ? __ldg(reinterpret_cast<const float4*>(X + rn * D + dl)) : make_float4(0.f, 0.f, 0.f, 0.f);
+                    }
+                    __syncwarp();
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
+                        *reinterpret_cast<float4*>(wx + (i * 8 + (lane >> 2)) * RP + 4 * (lane & 3)) = v[i];
+                    __syncwarp();
+                    const int dn = min(RD, D - d0);
+#pragma unroll
+                    for (int d = 0; d < RD; d += 4) {
+                        if (d >= dn) break;   // uniform; D % 4 == 0 here
+                        const float4 x4 = *reinterpret_cast<const float4*>(wx + lane * RP + d);
+                        const float4 a4 = *reinterpret_cast<const float4*>(av + d0 + d);
+                        acc = __fmaf_rn(x4.x, a4.x, acc);
+                        acc = __fmaf_rn(x4.y, a4.y, acc);
+                        acc = __fmaf_rn(x4.z, a4.z, acc);
+                        acc = __fmaf_rn(x4.w, a4.w, acc);
+                    }
+                }
+            } else if (on) {
+                const float* x = X + n * D;
+                for (int d = 0; d < D; ++d) acc = __fmaf_rn(__ldg(x + d), av[d], acc);
             }
-        } else if (stage_a) {
-            const float* av = sA + (int64_t)c * Dq;
-            for (int d = 0; d < D; ++d) acc = __fmaf_rn(__ldg(x + d), av[d], acc);
-        } else if ((D & 3) == 0) {
-            // A too large for shared memory (high D): 16-byte loads of the
-            // row and of the column's A row from L2, same FMA order
-            const float* av = A + (int64_t)c * D;
-#pragma unroll 4
-            for (int d = 0; d < D; d += 4) {
-                const float4 x4 = __ldg(reinterpret_cast<const float4*>(x + d));
-                const float4 a4 = __ldg(reinterpret_cast<const float4*>(av + d));
-                acc = __fmaf_rn(x4.x, a4.x, acc);
-                acc = __fmaf_rn(x4.y, a4.y, acc);
-                acc = __fmaf_rn(x4.z, a4.z, acc);
-                acc = __fmaf_rn(x4.w, a4.w, acc);
+            if (!on) continue;
+            const float v = __fdiv_rn(__fsub_rn(acc, __ldg(b + c)), W);
+            const float f = floorf(v);
+            int32_t code = 0;
+            if (!(fabsf(f) <= FLT_MAX)) atomicOr(err, kErrNonFinite);
+            else if (!(f >= -2147483648.0f && f < 2147483648.0f)) atomicOr(err, kErrCodeRange);
+            else code = (int32_t)f;
+            codes[(int64_t)c * N + n] = code;
+            if (block_range) {
+                if (code < smin[c]) atomicMin(smin + c, code);
+                if (code > smax[c]) atomicMax(smax + c, code);
+            } else {
+                atomicMin(cmin + c, code);
+                atomicMax(cmax + c, code);
             }
-        } else {
-            const float* av = A + (int64_t)c * D;
-            for (int d = 0; d < D; ++d) acc = __fmaf_rn(__ldg(x + d), __ldg(av + d), acc);
         }
-        const float v = __fdiv_rn(__fsub_rn(acc, __ldg(b + c)), W);
-        const float f = floorf(v);
-        int32_t code = 0;
-        if (!(fabsf(f) <= FLT_MAX)) atomicOr(err, kErrNonFinite);
-        else if (!(f >= -2147483648.0f && f < 2147483648.0f)) atomicOr(err, kErrCodeRange);
-        else code = (int32_t)f;
-        codes[(int64_t)c * N + n] = code;
-        if (block_range) {
-            atomicMin(smin + c, code);
-            atomicMax(smax + c, code);
-        } else {
-            atomicMin(cmin + c, code);
-            atomicMax(cmax + c, code);
-        }
-      }
     }
     if (block_range) {
         __syncthreads();
-        for (int c = threadIdx.x; c < LM; c += blockDim.x) {
+        for (int c = tid; c < LM; c += RT) {
             if (smin[c] <= smax[c]) {
                 atomicMin(cmin + c, smin[c]);
                 atomicMax(cmax + c, smax[c]);
@@ -558,7 +719,7 @@ bool make_map(CUtensorMap* m, const void* ptr, uint64_t cols, uint64_t rows, uin
     const cuuint64_t strides[1] = {cols * 2};
     const cuuint32_t box[2] = {64, box_rows};
     const cuuint32_t es[2] = {1, 1};
-    return fn(m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, es,
+    return fn(m, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, es,
               CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
               CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
@@ -568,81 +729,107 @@ bool make_map(CUtensorMap* m, const void* ptr, uint64_t cols, uint64_t rows, uin
 TcPlan tc_plan(int64_t N, int D, int LM, int num_sms, int max_smem) {
     TcPlan p{};
     p.Dp = (D + 63) / 64 * 64;
-    p.LMp = (LM + 15) / 16 * 16;
-    p.ok = N >= 1024 && p.Dp <= 256 && p.LMp >= 16 && p.LMp <= 256 && LM <= 65535 && N < (1ll << 47);
+    p.ok = N >= 1024 && p.Dp <= 256 && LM <= 65535 && N < (1ll << 47);
     if (!p.ok) return p;
-    p.b_bytes = (uint32_t)p.LMp * p.Dp * 2;
-    p.x_bytes = (uint32_t)TC_M * p.Dp * 2;
-    // operands, barriers, per-column ranges / norms / offsets, per-thread masks
-    const size_t fixed = 1024 + 2 * (size_t)p.b_bytes + 128 + 16 * (size_t)p.LMp + 8 * 4 * TC_EPI_WARPS * 32;
-    int tc = 32;
-    while (tc < 2 * p.LMp) tc <<= 1;
-    p.tmem_cols = tc;
     p.ntiles = (int)((N + TC_M - 1) / TC_M);
     p.grid = std::min(p.ntiles, num_sms);
-    for (int need_lo = 0; need_lo < 2; ++need_lo) {
-        const size_t st = (size_t)p.x_bytes * (need_lo ? 2 : 1);
-        int stages = 2;
-        while (stages > 0 && fixed + stages * st > (size_t)max_smem) --stages;
-        p.stages[need_lo] = stages;
-        p.smem[need_lo] = fixed + stages * st;
+    p.ok = false;
+    // as few column blocks as fit shared memory with one or two X stages (two
+    // unless that takes more blocks: every block reads X again)
+    for (int blocks = (LM + 255) / 256; blocks <= (LM + 15) / 16 && !p.ok; ++blocks) {
+        p.blk = ((LM + blocks - 1) / blocks + 15) / 16 * 16;
+        p.LMp = (LM + p.blk - 1) / p.blk * p.blk;
+        p.b_bytes = (uint32_t)p.blk * p.Dp * 2;
+        p.x_bytes = (uint32_t)TC_M * p.Dp * 2;
+        // operands, barriers, per-column constants, per-thread masks
+        const size_t fixed = 1024 + 2 * (size_t)p.b_bytes + 128 + 20 * (size_t)p.blk + 8 * 4 * TC_EPI_WARPS * 32;
+        for (int need_lo = 0; need_lo < 2; ++need_lo) {
+            const size_t st = (size_t)p.x_bytes * (need_lo ? 2 : 1);
+            int stages = 2;
+            while (stages > 0 && fixed + stages * st > (size_t)max_smem) --stages;
+            p.stages[need_lo] = stages;
+            p.smem[need_lo] = fixed + stages * st;
+        }
+        p.ok = p.stages[1] >= 1;
     }
-    p.ok = p.stages[1] >= 1;
     return p;
 }
 
-cudaError_t launch_split_rows(const float* X, int64_t N, int D, int Dp, void* xh, void* xl, float* xnorm, int* flags,
-                              cudaStream_t st) {
+cudaError_t launch_project_sample(const float* X, int64_t N, int D, int ns, const float* A, int LM, float* xs,
+                                  float* anorm, ProjectState* ps, cudaStream_t st) {
+    cudaError_t e = cudaMemsetAsync(ps, 0, sizeof(ProjectState), st);
+    if (e != cudaSuccess) return e;
+    k_project_sample<<<(unsigned)((ns + LM + 7) / 8), 256, 0, st>>>(X, N, D, ns, A, LM, xs, anorm, ps);
+    k_project_scales<<<1, 1, 0, st>>>(ps);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_split_a(const float* A, int LM, int LMp, int D, int Dp, float kappa, void* ah, void* al, float* anorm,
+                           const ProjectState* ps, cudaStream_t st) {
+    k_split_a<<<(unsigned)((LMp + 7) / 8), 256, 0, st>>>(A, LM, LMp, D, Dp, kappa, static_cast<__half*>(ah),
+                                                        static_cast<__half*>(al), anorm, ps);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_split_rows(const float* X, int64_t N, int D, int Dp, float kappa, void* xh, void* xl, float* xnorm,
+                              ProjectState* ps, bool rescale, cudaStream_t st) {
+    if (rescale) k_project_scales<<<1, 1, 0, st>>>(ps);
     const int blocks = (int)std::min<int64_t>((N * 32 + 255) / 256, 152 * 16);
-    k_split_rows<<<blocks, 256, 0, st>>>(X, N, D, Dp, static_cast<__nv_bfloat16*>(xh),
-                                        static_cast<__nv_bfloat16*>(xl), xnorm, flags);
+    k_split_rows<<<blocks, 256, 0, st>>>(X, N, D, Dp, kappa, static_cast<__half*>(xh), static_cast<__half*>(xl), xnorm,
+                                        ps);
     return cudaGetLastError();
 }
 
 cudaError_t launch_project_tc(const TcPlan& p, int need_lo, int64_t N, int D, int LM, const void* xh, const void* xl,
                               const void* ah, const void* al, const float* b, const float* anorm, const float* xnorm,
-                              float W, float kappa, int32_t* codes, int32_t* pmin, int32_t* pmax,
+                              const ProjectState* ps, float W, float kappa, int32_t* codes, int32_t* pmin, int32_t* pmax,
                               unsigned long long* relist, unsigned long long relist_cap, unsigned int* relist_cnt,
                               int* err, cudaStream_t st) {
     CUtensorMap mxh, mxl, mah, mal;
-    if (!make_map(&mxh, xh, p.Dp, N, TC_M) || !make_map(&mxl, xl, p.Dp, N, TC_M) ||
-        !make_map(&mah, ah, p.Dp, p.LMp, p.LMp) || !make_map(&mal, al, p.Dp, p.LMp, p.LMp))
+    if (!make_map(&mxh, xh, p.Dp, N, TC_M) || !make_map(&mxl, need_lo ? xl : xh, p.Dp, N, TC_M) ||
+        !make_map(&mah, ah, p.Dp, p.LMp, p.blk) || !make_map(&mal, al, p.Dp, p.LMp, p.blk))
         return cudaErrorNotSupported;
-    TcArgs a;
-    a.N = N;
-    a.D = D;
-    a.Dp = p.Dp;
-    a.LM = LM;
-    a.LMp = p.LMp;
-    a.ntiles = p.ntiles;
-    a.need_lo = need_lo;
-    a.stages = p.stages[need_lo];
-    a.tmem_cols = p.tmem_cols;
-    a.W = W;
-    a.kappa = kappa;
-    a.b = b;
-    a.anorm = anorm;
-    a.xnorm = xnorm;
-    a.codes = codes;
-    a.pmin = pmin;
-    a.pmax = pmax;
-    a.relist = relist;
-    a.relist_cap = relist_cap;
-    a.relist_cnt = relist_cnt;
-    a.inv_w = 1.0f / W;
-    a.err = err;
-    a.b_bytes = p.b_bytes;
-    a.x_bytes = p.x_bytes;
-    a.col0 = 0;
-    a.LMtot = LM;
-    a.stage_bytes = 0;
-    a.a_chunk = 0;
-    a.list_continue = 0;
     const int smem = (int)p.smem[need_lo];
     cudaError_t e = cudaFuncSetAttribute(k_project_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
-    k_project_tc<false><<<p.grid, TC_THREADS, smem, st>>>(mxh, mxl, mah, mal, a);
-    return cudaGetLastError();
+    e = cudaMemsetAsync(relist_cnt, 0, sizeof(unsigned int) * (size_t)p.grid, st);
+    if (e != cudaSuccess) return e;
+    for (int col0 = 0; col0 < LM; col0 += p.blk) {
+        TcArgs a;
+        a.N = N;
+        a.D = D;
+        a.Dp = p.Dp;
+        a.LM = std::min(p.blk, LM - col0);
+        a.LMp = p.blk;
+        a.ntiles = p.ntiles;
+        a.need_lo = need_lo;
+        a.stages = p.stages[need_lo];
+        a.tmem_cols = 32;
+        while (a.tmem_cols < 2 * p.blk) a.tmem_cols <<= 1;
+        a.W = W;
+        a.kappa = kappa;
+        a.b = b;
+        a.anorm = anorm;
+        a.xnorm = xnorm;
+        a.ps = ps;
+        a.codes = codes;
+        a.pmin = pmin;
+        a.pmax = pmax;
+        a.relist = relist;
+        a.relist_cap = relist_cap;
+        a.relist_cnt = relist_cnt;
+        a.err = err;
+        a.b_bytes = p.b_bytes;
+        a.x_bytes = p.x_bytes;
+        a.col0 = col0;
+        a.LMtot = LM;
+        a.stage_bytes = 0;
+        a.a_chunk = 0;
+        a.list_continue = 1;
+        k_project_tc<false><<<p.grid, TC_THREADS, smem, st>>>(mxh, mxl, mah, mal, a);
+        if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    }
+    return cudaSuccess;
 }
 
 TcStreamPlan tc_plan_stream(int64_t N, int D, int LM, int num_sms, int max_smem) {
@@ -658,14 +845,14 @@ TcStreamPlan tc_plan_stream(int64_t N, int D, int LM, int num_sms, int max_smem)
         // widest column block whose two-stage (or one-stage) ring fits
         for (int blk = 256; blk >= 16; blk -= 16) {
             const size_t stage = 16384u * (need_lo ? 2u : 1u) + 2u * (size_t)blk * 128u;
-            const size_t tail = 128 + 16 * (size_t)blk + 8 * 4 * TC_EPI_WARPS * 32;
+            const size_t tail = 128 + 20 * (size_t)blk + 8 * 4 * TC_EPI_WARPS * 32;
             int stages = 2;
             while (stages > 0 && 1024 + stages * stage + tail > (size_t)max_smem) --stages;
             if (stages == 0) continue;
             p.blk[need_lo] = std::min(blk, p.LMp);
             p.stages[need_lo] = stages;
             p.smem[need_lo] = 1024 + stages * (16384u * (need_lo ? 2u : 1u) + 2u * (size_t)p.blk[need_lo] * 128u) +
-                              128 + 16 * (size_t)p.blk[need_lo] + 8 * 4 * TC_EPI_WARPS * 32;
+                              128 + 20 * (size_t)p.blk[need_lo] + 8 * 4 * TC_EPI_WARPS * 32;
             break;
         }
     }
@@ -675,13 +862,13 @@ TcStreamPlan tc_plan_stream(int64_t N, int D, int LM, int num_sms, int max_smem)
 
 cudaError_t launch_project_tc_stream(const TcStreamPlan& p, int need_lo, int64_t N, int D, int LM, const void* xh,
                                      const void* xl, const void* ah, const void* al, const float* b,
-                                     const float* anorm, const float* xnorm, float W, float kappa, int32_t* codes,
-                                     int32_t* pmin, int32_t* pmax, unsigned long long* relist,
+                                     const float* anorm, const float* xnorm, const ProjectState* ps, float W, float kappa,
+                                     int32_t* codes, int32_t* pmin, int32_t* pmax, unsigned long long* relist,
                                      unsigned long long relist_cap, unsigned int* relist_cnt, int* err,
                                      cudaStream_t st) {
     const int blk = p.blk[need_lo];
     CUtensorMap mxh, mxl;
-    if (!make_map(&mxh, xh, p.Dp, N, TC_M) || !make_map(&mxl, xl, p.Dp, N, TC_M)) return cudaErrorNotSupported;
+    if (!make_map(&mxh, xh, p.Dp, N, TC_M) || !make_map(&mxl, need_lo ? xl : xh, p.Dp, N, TC_M)) return cudaErrorNotSupported;
     const int smem = (int)p.smem[need_lo];
     cudaError_t e = cudaFuncSetAttribute(k_project_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return e;
@@ -717,7 +904,7 @@ cudaError_t launch_project_tc_stream(const TcStreamPlan& p, int need_lo, int64_t
         a.relist = relist;
         a.relist_cap = relist_cap;
         a.relist_cnt = relist_cnt;
-        a.inv_w = 1.0f / W;
+        a.ps = ps;
         a.err = err;
         a.b_bytes = 0;
         a.x_bytes = 16384u;
@@ -736,18 +923,17 @@ cudaError_t launch_project_tc_stream(const TcStreamPlan& p, int need_lo, int64_t
 cudaError_t launch_tc_recompute(const float* X, int64_t N, int D, int LM, const float* A, const float* b, float W,
                                 const unsigned long long* list, unsigned long long cap, const unsigned int* cnt,
                                 int regions, int32_t* codes, int32_t* cmin, int32_t* cmax, int* err, cudaStream_t st) {
-    const size_t smem = sizeof(float) * (size_t)LM * ((D & 3) == 0 ? D + 4 : D + 1);
-    const int stage_a = smem <= 200 * 1024;
-    if (stage_a) {
-        cudaError_t e = cudaFuncSetAttribute(k_tc_recompute, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        if (e != cudaSuccess) return e;
-    }
-    // Grid: a multiple of the region count, so that every block has a region.
-    // 512 threads: with A staged (up to ~100 KB at L*M = 192, D = 128) two
-    // blocks fit an SM, 32 warps to cover the latency of the X row loads.
-    const int grid = regions * (stage_a ? 2 : 8);
-    k_tc_recompute<<<grid, 512, stage_a ? smem : 0, st>>>(
-        X, N, D, A, b, W, list, cap, cnt, regions, LM, stage_a, codes, cmin, cmax, err);
+    // rows of X through shared memory where 16-byte loads apply; A beside them
+    // where both fit
+    const int stage_x = (D & 3) == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
+    const size_t xs = stage_x ? sizeof(float) * (size_t)RT * RP : 0;
+    const size_t as = sizeof(float) * (size_t)LM * ((D & 3) == 0 ? D + 4 : D + 1);
+    const int stage_a = xs + as <= 215 * 1024;
+    const size_t smem = xs + (stage_a ? as : 0);
+    cudaError_t e = cudaFuncSetAttribute(k_tc_recompute, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+    k_tc_recompute<<<regions, RT, smem, st>>>(X, N, D, A, b, W, list, cap, cnt, regions, LM, stage_a, stage_x, codes, cmin,
+                                             cmax, err);
     return cudaGetLastError();
 }
 

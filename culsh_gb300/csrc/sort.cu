@@ -72,50 +72,90 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* ws, ui
     return r;
 }
 
+// Keys of one table's points (blockIdx.y), PK_ITEMS per thread. Fields are
+// contiguous from column M - 1's offset upwards; a column's bit width and
+// offset are the same for every thread, so the words are filled from a 64-bit
+// window with uniform control flow (a 128-bit shift per column had cost 44
+// instructions per code: 0.38 ms for 1M x 192 codes, now 0.23 ms).
 // WIDE: keys of more than 128 bits (KW > 4), assembled word by word.
+constexpr int PK_ITEMS = 4;
 template <bool WIDE>
-__global__ void k_pack_keys(const int32_t* __restrict__ codes, int64_t N, int L, int M, int KW,
+__global__ void __launch_bounds__(NT) k_pack_keys(const int32_t* __restrict__ codes, int64_t N, int L, int M, int KW,
                             const int32_t* __restrict__ cmin, const uint8_t* __restrict__ fbits,
                             const uint16_t* __restrict__ foff, uint32_t* __restrict__ keys,
                             uint32_t* __restrict__ vals, uint32_t* __restrict__ low, int lw) {
     const int64_t LN = (int64_t)L * N;
-    for (int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; idx < LN;
-         idx += (int64_t)gridDim.x * blockDim.x) {
-        const int l = (int)(idx / N);
-        const int64_t n = idx - (int64_t)l * N;
-        if constexpr (WIDE) {
+    const int l = blockIdx.y;
+    const int64_t n0 = (int64_t)blockIdx.x * (NT * PK_ITEMS) + threadIdx.x;
+    const int32_t* cl = codes + (int64_t)l * M * N;
+    if constexpr (WIDE) {
+        for (int i = 0; i < PK_ITEMS; ++i) {
+            const int64_t n = n0 + i * NT;
+            if (n >= N) break;
             uint32_t key[kMaxKW] = {};
             for (int m = 0; m < M; ++m) {
                 const int c = l * M + m;
                 const int bits = __ldg(fbits + c);
-                if (bits) key_put(key, __ldg(foff + c), bits, (uint32_t)(codes[(int64_t)c * N + n] - __ldg(cmin + c)));
+                if (bits) key_put(key, __ldg(foff + c), bits, (uint32_t)(cl[(int64_t)m * N + n] - __ldg(cmin + c)));
             }
-            for (int w = 0; w < KW; ++w) keys[w * LN + idx] = key[w];
-            vals[idx] = (uint32_t)n;
-            continue;
+            for (int w = 0; w < KW; ++w) keys[w * LN + (int64_t)l * N + n] = key[w];
+            vals[(int64_t)l * N + n] = (uint32_t)n;
         }
-        // fields are contiguous, column M - 1 at bit 0 and column 0 on top:
-        // shift each column in after the previous one (registers only)
-        unsigned __int128 kk = 0;
-        for (int m = 0; m < M; ++m) {
+    } else {
+        uint32_t k[4][PK_ITEMS];
+        uint64_t acc[PK_ITEMS];
+#pragma unroll
+        for (int i = 0; i < PK_ITEMS; ++i) {
+            acc[i] = 0;
+#pragma unroll
+            for (int w = 0; w < 4; ++w) k[w][i] = 0;
+        }
+        int pos = __ldg(foff + l * M + M - 1), w = 0;   // next bit within the window, word at its bottom
+        auto emit = [&]() {   // the window's low word is complete
+#pragma unroll
+            for (int i = 0; i < PK_ITEMS; ++i) {
+                const uint32_t v = (uint32_t)acc[i];
+                if (w == 0) k[0][i] = v;
+                else if (w == 1) k[1][i] = v;
+                else if (w == 2) k[2][i] = v;
+                else k[3][i] = v;
+                acc[i] >>= 32;
+            }
+            ++w;
+            pos -= 32;
+        };
+        while (pos >= 32) emit();
+        for (int m = M - 1; m >= 0; --m) {
             const int c = l * M + m;
             const int bits = __ldg(fbits + c);
-            if (!bits) continue;
-            kk = (kk << bits) | (uint32_t)(codes[(int64_t)c * N + n] - __ldg(cmin + c));
-        }
-        kk <<= __ldg(foff + (int64_t)l * M + M - 1);   // the last column's offset (compute_layout)
-        if (low) {   // top-word-first form: the top word in keys, the lower ones as a row
-            keys[idx] = (uint32_t)(kk >> (32 * (KW - 1)));
-            if (lw == 1) low[idx] = (uint32_t)kk;
-            else if (lw == 2) reinterpret_cast<uint2*>(low)[idx] = make_uint2((uint32_t)kk, (uint32_t)(kk >> 32));
-            else reinterpret_cast<uint4*>(low)[idx] = make_uint4((uint32_t)kk, (uint32_t)(kk >> 32), (uint32_t)(kk >> 64), 0u);
-            vals[idx] = (uint32_t)n;
-            continue;
-        }
+            if (bits == 0) continue;
+            const int32_t lo = __ldg(cmin + c);
 #pragma unroll
-        for (int w = 0; w < 4; ++w)
-            if (w < KW) keys[w * LN + idx] = (uint32_t)(kk >> (32 * w));
-        vals[idx] = (uint32_t)n;
+            for (int i = 0; i < PK_ITEMS; ++i) {
+                const int64_t n = n0 + i * NT;
+                const uint32_t f = n < N ? (uint32_t)(__ldcs(cl + (int64_t)m * N + n) - lo) : 0u;
+                acc[i] |= (uint64_t)f << pos;
+            }
+            pos += bits;
+            if (pos >= 32) emit();
+        }
+        if (pos > 0) emit();
+#pragma unroll
+        for (int i = 0; i < PK_ITEMS; ++i) {
+            const int64_t n = n0 + i * NT, idx = (int64_t)l * N + n;
+            if (n >= N) break;
+            if (low) {   // top-word-first form: the top word in keys, the lower ones as a row
+                keys[idx] = lw == 1 ? k[1][i] : lw == 2 ? k[2][i] : k[3][i];
+                if (lw == 1) low[idx] = k[0][i];
+                else if (lw == 2) reinterpret_cast<uint2*>(low)[idx] = make_uint2(k[0][i], k[1][i]);
+                else reinterpret_cast<uint4*>(low)[idx] = make_uint4(k[0][i], k[1][i], k[2][i], 0u);
+            } else {
+#pragma unroll
+                for (int v = 0; v < 4; ++v)
+                    if (v < KW) keys[v * LN + idx] = k[v][i];
+            }
+            vals[idx] = (uint32_t)n;
+        }
     }
 }
 
@@ -849,8 +889,7 @@ inline int blocks_for(int64_t n) { return (int)((n + NT - 1) / NT); }
 cudaError_t launch_pack_keys(const int32_t* codes, int64_t N, int L, int M, int KW, const int32_t* cmin,
                              const uint8_t* fbits, const uint16_t* foff, uint32_t* keys, uint32_t* vals,
                              uint32_t* low, int lw, cudaStream_t st) {
-    const int64_t LN = (int64_t)L * N;
-    const int grid = (int)std::min<int64_t>((LN + NT - 1) / NT, 152 * 32);
+    const dim3 grid((unsigned)((N + NT * PK_ITEMS - 1) / (NT * PK_ITEMS)), (unsigned)L);
     if (KW > 4) k_pack_keys<true><<<grid, NT, 0, st>>>(codes, N, L, M, KW, cmin, fbits, foff, keys, vals, nullptr, 0);
     else k_pack_keys<false><<<grid, NT, 0, st>>>(codes, N, L, M, KW, cmin, fbits, foff, keys, vals, low, lw);
     return cudaGetLastError();

@@ -47,15 +47,29 @@ __global__ void __launch_bounds__(PT_PLAN) k_plan_items(WsArgs a) {
     const int q0 = blockIdx.x * PT_PLAN;
     const int q = q0 + tid < a.Q ? (a.order ? (int)a.order[q0 + tid] : q0 + tid) : a.Q;
     uint32_t P = 0;
-    bool dense = false;
+    bool dense = false, small = false;
     if (q < a.Q) {
         const unsigned long long C = a.cnu[q];
         // near-exhaustive candidate sets go to the bitmap kernel instead
         dense = C >= a.dense_min;
-        P = (C == 0 || dense) ? 0u : (uint32_t)min((unsigned long long)a.pmax, (C + a.chunk - 1) / a.chunk);
+        // (FP32 form, enough queries to fill the device: one item while its set
+        // holds every candidate, since each item scans the query's whole list)
+        P = (C == 0 || dense) ? 0u
+            : C <= a.whole        ? 1u
+                                  : (uint32_t)min((unsigned long long)a.pmax, (C + a.chunk - 1) / a.chunk);
         if (dense) a.dense_q[atomicAdd(a.n_dense, 1u)] = q;
+        // a handful of candidates: one warp each (k_candidates_small)
+        small = !dense && C > 0 && C <= a.small_max;
+        if (small) P = 0;
     }
-    s_empty[tid] = q < a.Q && P == 0 && !dense;
+    const uint32_t sm = __ballot_sync(0xffffffffu, small);
+    if (sm) {
+        uint32_t at = 0;
+        if (lane == 0) at = atomicAdd(a.n_small, (uint32_t)__popc(sm));
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(sm & ((1u << lane) - 1u));
+        if (small) a.small_q[at] = q;
+    }
+    s_empty[tid] = q < a.Q && P == 0 && !dense && !small;
     uint32_t x = P;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
@@ -163,6 +177,442 @@ __global__ void k_order_scatter(WsArgs a) {
     if (q < a.Q) a.order[atomicAdd(a.order_bins + order_bin(a, q), 1u)] = (uint32_t)q;
 }
 
+// ---- FP32 form ----
+// Top-K of an item by selection instead of insertion: the item's distances
+// take the place of its hash set as (distance bits, id) words, one histogram
+// pass over the distances' range (two or three where many share a bin) finds a
+// threshold that K of them and few more do not exceed, and those few are
+// sorted. Kept sorted lists (one per warp, merged by one warp) cost a warp-wide
+// insertion of some 150 cycles per entry, and with K = 100 nearly every
+// candidate of an item was inserted (a serving burst over 10M points, K 10 and
+// 100: 8.5 ms of this kernel, now 4.6).
+
+struct SelectSmem {
+    uint32_t hist[256];
+    uint32_t lo, hi, valid;   // range and count of the finite distances
+    uint32_t m, bin, rest;
+};
+constexpr uint32_t kNoDist = 0xFFFFFFFFu;   // distance bits of an entry that is never listed
+
+// Chooses from ent[0 .. n) at least the min(K, valid) smallest (distance, id)
+// entries, sorts them and leaves their positions in idx; returns
+// min(K, valid). All WT threads; sm.lo, hi and valid are set and visible.
+template <int WT>
+__device__ __forceinline__ uint32_t block_top(const unsigned long long* ent, uint32_t n, uint32_t K, uint32_t* idx,
+                                              SelectSmem& sm) {
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t lo = sm.lo, valid = sm.valid;
+    uint32_t edge = 0, sh = 32;   // chosen: (bits - lo) >> sh <= edge
+    if (valid > K && valid > 32) {
+        uint32_t prefix = 0, want = K;
+        for (int top = 32 - __clz((int)(sm.hi - lo)); top > 0;) {
+            const int s = max(top - 8, 0);
+            for (int b = tid; b < 256; b += WT) sm.hist[b] = 0;
+            __syncthreads();
+            for (uint32_t e = tid; e < n; e += WT) {
+                const uint32_t v = (uint32_t)(ent[e] >> 32) - lo;
+                if ((uint32_t)(ent[e] >> 32) != kNoDist && (top >= 32 ? 0u : v >> top) == prefix)
+                    atomicAdd(&sm.hist[(v >> s) & ((1u << (top - s)) - 1u)], 1u);
+            }
+            __syncthreads();
+            if (warp == 0) {
+                uint32_t mine = 0;
+#pragma unroll
+                for (int b = 0; b < 8; ++b) mine += sm.hist[lane * 8 + b];
+                uint32_t x = mine;
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+                    if (lane >= o) x += y;
+                }
+                if (lane == __ffs((int)__ballot_sync(0xffffffffu, x >= want)) - 1) {
+                    uint32_t r = want - (x - mine), b = (uint32_t)lane * 8;
+                    while (sm.hist[b] < r) r -= sm.hist[b++];
+                    sm.bin = b;
+                    sm.rest = r;
+                }
+            }
+            __syncthreads();
+            prefix = (prefix << (top - s)) | sm.bin;
+            want = sm.rest;
+            top = s;
+            edge = prefix;
+            sh = (uint32_t)s;
+            // entries up to this bin: K - want below it and the bin itself
+            const bool few = K - want + sm.hist[sm.bin] <= max(K + K / 2, 32u);
+            __syncthreads();
+            if (few) break;   // uniform
+        }
+    }
+    if (tid == 0) sm.m = 0;
+    __syncthreads();
+    for (uint32_t b = warp * 32; b < n; b += WT) {
+        const uint32_t e = b + lane;
+        const uint32_t bits = e < n ? (uint32_t)(ent[e] >> 32) : kNoDist;
+        const bool take = bits != kNoDist && (sh >= 32 || ((bits - lo) >> sh) <= edge);
+        const uint32_t bal = __ballot_sync(0xffffffffu, take);
+        uint32_t at = 0;
+        if (lane == 0 && bal) at = atomicAdd(&sm.m, (uint32_t)__popc(bal));
+        at = __shfl_sync(0xffffffffu, at, 0) + __popc(bal & ((1u << lane) - 1u));
+        if (take) idx[at] = e;
+    }
+    __syncthreads();
+    const uint32_t m = sm.m;
+    auto key = [&](uint32_t i) { return i == 0xFFFFFFFFu ? ~0ull : ent[i]; };
+    if (m <= 32) {
+        if (warp == 0) {
+            uint32_t i = lane < (int)m ? idx[lane] : 0xFFFFFFFFu;
+            unsigned long long v = key(i);
+#pragma unroll
+            for (int a = 2; a <= 32; a <<= 1) {
+#pragma unroll
+                for (int b = a >> 1; b > 0; b >>= 1) {
+                    const unsigned long long ov = __shfl_xor_sync(0xffffffffu, v, b);
+                    const uint32_t oi = __shfl_xor_sync(0xffffffffu, i, b);
+                    const bool keep_min = ((lane & b) == 0) == ((lane & a) == 0);
+                    if (ov != v && (ov < v) == keep_min) {
+                        v = ov;
+                        i = oi;
+                    }
+                }
+            }
+            if (lane < (int)m) idx[lane] = i;
+        }
+        __syncthreads();
+        return min(K, valid);
+    }
+    uint32_t P = 64;
+    while (P < m) P <<= 1;
+    for (uint32_t e = m + tid; e < P; e += WT) idx[e] = 0xFFFFFFFFu;
+    __syncthreads();
+    for (uint32_t a = 2; a <= P; a <<= 1)
+        for (uint32_t b = a >> 1; b > 0; b >>= 1) {
+            for (uint32_t t = tid; t < P / 2; t += WT) {
+                const uint32_t x = 2 * t - (t & (b - 1)), y = x + b;
+                const uint32_t ix = idx[x], iy = idx[y];
+                if ((key(ix) > key(iy)) == ((x & a) == 0)) {
+                    idx[x] = iy;
+                    idx[y] = ix;
+                }
+            }
+            __syncthreads();
+        }
+    return min(K, valid);
+}
+
+// Hash of an id for the set and the partitions.
+__device__ __forceinline__ uint32_t id_hash(uint32_t x) {
+    x *= 0x9E3779B1u;
+    x ^= x >> 15;
+    x *= 0x85EBCA77u;
+    return x ^ (x >> 13);
+}
+
+// Queries of at most kSmallMax non-unique candidates, one warp each: bucket list,
+// ids, duplicates (lanes that hold the same id), distances and order all within
+// the warp. As items of k_candidates_ws they took a block, a cleared hash set
+// and a dozen block barriers each: 103 us for 9,700 look-ups of one point, now
+// 48 us.
+constexpr int SMW = 8;   // warps per block
+__global__ void __launch_bounds__(32 * SMW) k_candidates_small(WsArgs a) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ uint64_t s_base[SMW][32];
+    __shared__ uint32_t s_pre[SMW][32], s_id[SMW][32];
+    __shared__ float s_d[SMW][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int D = a.D, K = a.K, T = a.T, LT = a.L * T;
+    float* qs = reinterpret_cast<float*>(smem) + (size_t)w * ((D + 3) & ~3);
+    const bool vec = (D & 3) == 0;
+    const unsigned int n = *a.n_small;
+    unsigned long long tu = 0, tn = 0;
+    for (unsigned int i = blockIdx.x * SMW + w; i < n; i += gridDim.x * SMW) {
+        const int q = a.small_q[i];
+        for (int d = lane; d < D; d += 32) qs[d] = __ldg(a.queries + (int64_t)q * D + d);
+        uint32_t nl = 0, C = 0;   // lists, ids
+        for (int e0 = 0; e0 < LT; e0 += 128) {
+            int32_t j[4];
+            uint32_t st[4], sz[4];
+            uint64_t gi[4];
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const int e = e0 + u * 32 + lane;
+                j[u] = -1;
+                if (e < LT) {
+                    const int l = e / T;
+                    j[u] = __ldg(a.qbuckets + (int64_t)l * a.Q * T + (int64_t)q * T + (e - l * T));
+                    gi[u] = __ldg(a.boff + l) + (uint32_t)max(j[u], 0);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                sz[u] = 0;
+                if (j[u] >= 0) {
+                    st[u] = __ldg(a.starts + gi[u]);
+                    sz[u] = __ldg(a.sizes + gi[u]);
+                }
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) {
+                const uint32_t has = __ballot_sync(0xffffffffu, sz[u] > 0);
+                if (has == 0) continue;
+                uint32_t x = sz[u];
+#pragma unroll
+                for (int o = 1; o < 32; o <<= 1) {
+                    const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+                    if (lane >= o) x += y;
+                }
+                if (sz[u] > 0) {
+                    const uint32_t k = nl + __popc(has & ((1u << lane) - 1u));
+                    s_base[w][k] = (uint64_t)((e0 + u * 32 + lane) / T) * (uint64_t)a.N + st[u];
+                    s_pre[w][k] = C + x;   // ids up to and including this list
+                }
+                nl += __popc(has);
+                C += __shfl_sync(0xffffffffu, x, 31);
+            }
+        }
+        __syncwarp();
+        const bool on = lane < (int)C;
+        uint32_t id = 0;
+        if (on) {
+            uint32_t k = 0;
+            while (s_pre[w][k] <= (uint32_t)lane) ++k;
+            id = __ldg(a.ids + s_base[w][k] + (lane - (k ? s_pre[w][k - 1] : 0u)));
+        }
+        const uint32_t mask = __ballot_sync(0xffffffffu, on);
+        bool first = false;
+        if (on) first = __ffs((int)__match_any_sync(mask, id)) - 1 == lane;
+        const uint32_t uniq = __ballot_sync(0xffffffffu, first);
+        const uint32_t U = __popc(uniq);
+        if (first) s_id[w][__popc(uniq & ((1u << lane) - 1u))] = id;
+        __syncwarp();
+        const uint32_t per = vec ? 16 : 4, sub = vec ? lane >> 1 : lane >> 3;
+        for (uint32_t b = 0; b < U; b += per) {
+            const uint32_t e = b + sub;
+            const float d = row_distance(a.X + (int64_t)(e < U ? s_id[w][e] : 0u) * D, D, qs, vec, e < U);
+            if (e < U && (lane & (vec ? 1 : 7)) == 0) s_d[w][e] = d;
+        }
+        __syncwarp();
+        unsigned long long v = ~0ull;
+        if (lane < (int)U && s_d[w][lane] < FLT_MAX)
+            v = ((unsigned long long)__float_as_uint(s_d[w][lane]) << 32) | s_id[w][lane];
+#pragma unroll
+        for (int x = 2; x <= 32; x <<= 1) {
+#pragma unroll
+            for (int y = x >> 1; y > 0; y >>= 1) {
+                const unsigned long long o = __shfl_xor_sync(0xffffffffu, v, y);
+                if ((o < v) == (((lane & y) == 0) == ((lane & x) == 0))) v = o;
+            }
+        }
+        int32_t* oid = a.out_ids + (int64_t)q * K;
+        float* od = a.out_d + (int64_t)q * K;
+        for (int k = lane; k < K; k += 32) {
+            const bool have = k < 32 && v != ~0ull;
+            oid[k] = have ? (int32_t)(uint32_t)v : -1;
+            od[k] = have ? __uint_as_float((uint32_t)(v >> 32)) : FLT_MAX;
+        }
+        if (lane == 0) a.cu[q] = U;
+        tu += U;
+        tn += C;
+        __syncwarp();
+    }
+    if (lane == 0 && tn) {
+        atomicAdd(a.totals + 0, tu);
+        atomicAdd(a.totals + 1, tn);
+    }
+}
+
+template <int WT, int W_SLOTS>
+__global__ void __launch_bounds__(WT) k_candidates_ws(WsArgs a) {
+    constexpr int WW = WT / 32;
+    constexpr uint32_t W_CAP = W_SLOTS / 2;
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ uint32_t s_ucount, s_skip;
+    __shared__ int s_item, s_last;
+    __shared__ GatherSmem<WT, GCH> s_gather;
+    __shared__ SelectSmem s_sel;
+    __shared__ uint64_t s_bar[WW];
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const int D = a.D, K = a.K, L = a.L, T = a.T;
+    const int Dp = (D + 3) & ~3;
+    // rows staged by bulk copies where they start on 16-byte boundaries
+    const bool staged = row_staged(D) && (reinterpret_cast<uintptr_t>(a.X) & 15) == 0;
+    float* stage = reinterpret_cast<float*>(smem + warp * row_stage_bytes(D));
+    uint32_t phase = 0;
+    float* qs = reinterpret_cast<float*>(smem + WW * row_stage_bytes(D));
+    uint32_t* hset = reinterpret_cast<uint32_t*>(qs + Dp);                        // [W_SLOTS], then the entries
+    unsigned long long* ent = reinterpret_cast<unsigned long long*>(hset);       // [W_CAP]
+    uint32_t* ulist = hset + W_SLOTS;                                            // [W_CAP], then positions
+    float* wd = reinterpret_cast<float*>(ulist + W_CAP);                         // [K] merge of very large partial lists
+    uint32_t* wi = reinterpret_cast<uint32_t*>(wd + K);
+    // Bit 0 of the overflow word: the plan did not fit (set by k_plan_items,
+    // which has finished). Read once and broadcast, so that the whole block
+    // returns or none of it does; bit 1 (a set overflow) may be raised by
+    // other blocks meanwhile and is left to the host.
+    // Thread 0 claims the next item while the block works on the current one.
+    if (tid == 0) {
+        s_skip = *(volatile unsigned int*)a.overflow & 1u;
+        s_item = s_skip ? 0 : (int)atomicAdd(a.next_item, 1u);
+        for (int w = 0; w < WW; ++w) stage_bar_init(s_bar + w);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    __syncthreads();
+    if (s_skip) return;
+    const int n_items = (int)*a.n_items;
+    const bool vec = (D & 3) == 0;
+    for (;;) {
+        const int item = s_item;
+        if (item >= n_items) break;
+        int next = 0;
+        if (tid == 0) next = (int)atomicAdd(a.next_item, 1u);
+        const int q = a.item_q[item];
+        const uint32_t p = a.item_p[item];
+        const uint32_t P = (uint32_t)a.q_items[q];
+        const unsigned long long C = a.cnu[q];
+        // as many set slots as the item can need: twice its candidates
+        uint32_t slots = W_SLOTS;
+        if (P == 1 && C < W_CAP) slots = max(32u, 2u << (31 - __clz((int)C)) << (((uint32_t)C & ((uint32_t)C - 1)) != 0));
+        for (int i = tid; i < Dp; i += WT) qs[i] = i < D ? a.queries[(int64_t)q * D + i] : 0.0f;
+        for (uint32_t i = tid; i < slots; i += WT) hset[i] = kEmpty32;
+        if (tid == 0) s_ucount = 0;
+        __syncthreads();
+
+        // Gather this item's id partition from every matched bucket.
+        const BucketView bv{a.qbuckets, a.boff, a.starts, a.sizes, a.ids, a.N, L, T, a.Q};
+        gather_bucket_ids<WT, GCH>(bv, q, s_gather, [&](uint32_t id) {
+            const uint32_t h = id_hash(id);
+            if (P > 1 && __umulhi(h, P) != p) return;
+            set_insert_at(hset, slots - 1, ulist, W_CAP, &s_ucount, id, h);
+        });
+        __syncthreads();
+        uint32_t U = s_ucount;
+        if (U > W_CAP) {   // the set overflowed: flag it, finish the protocol with no candidates
+            if (tid == 0) atomicOr(a.overflow, 2u);
+            U = 0;
+        }
+        if (tid == 0) {
+            s_sel.lo = kNoDist;
+            s_sel.hi = s_sel.valid = 0;
+        }
+        __syncthreads();   // the set is no longer read: its place takes the entries
+
+        // Exact FP32 distances in the reference lane order.
+        {
+            const uint32_t per = vec ? 16 : 4, sub = vec ? lane >> 1 : lane >> 3;
+            const bool lead = (lane & (vec ? 1 : 7)) == 0;
+            uint32_t lo = kNoDist, hi = 0, valid = 0;
+            for (uint32_t b = warp * per; b < U; b += WW * per) {
+                const uint32_t e = b + sub;
+                const bool on = e < U;
+                const uint32_t id = on ? ulist[e] : 0u;
+                const float d = staged ? staged_distance(a.X, D, qs, ulist, b, U, stage, s_bar + warp, phase, a.overflow)
+                                       : row_distance(a.X + (int64_t)id * D, D, qs, vec, on);
+                if (on && lead) {
+                    const uint32_t bits = d < FLT_MAX ? __float_as_uint(d) : kNoDist;
+                    ent[e] = ((unsigned long long)bits << 32) | id;
+                    if (bits != kNoDist) {
+                        lo = min(lo, bits);
+                        hi = max(hi, bits);
+                        ++valid;
+                    }
+                }
+            }
+            lo = __reduce_min_sync(0xffffffffu, lo);
+            hi = __reduce_max_sync(0xffffffffu, hi);
+            valid = __reduce_add_sync(0xffffffffu, valid);
+            if (lane == 0 && valid) {
+                atomicMin(&s_sel.lo, lo);
+                atomicMax(&s_sel.hi, hi);
+                atomicAdd(&s_sel.valid, valid);
+            }
+        }
+        __syncthreads();
+        uint32_t n = block_top<WT>(ent, U, (uint32_t)K, ulist, s_sel);
+        if (tid == 0) {
+            atomicAdd(a.cu + q, (unsigned long long)U);
+            atomicAdd(a.totals + 0, (unsigned long long)U);
+        }
+        bool write = P == 1;
+        if (P > 1) {
+            // Publish this partition's list; the last partition to finish merges.
+            float* pd = a.part_d + (int64_t)item * K;
+            uint32_t* pi = a.part_i + (int64_t)item * K;
+            for (uint32_t k = tid; k < n; k += WT) {
+                const unsigned long long v = ent[ulist[k]];
+                pd[k] = __uint_as_float((uint32_t)(v >> 32));
+                pi[k] = (uint32_t)v;
+            }
+            if (tid == 0) a.part_n[item] = (int)n;
+            __threadfence();
+            __syncthreads();
+            if (tid == 0) s_last = atomicAdd(a.q_done + q, 1u) == P - 1;
+            __syncthreads();
+            if (s_last) {   // uniform
+                __threadfence();
+                const int first = a.q_off[q];
+                if (P * (uint32_t)K <= W_CAP) {
+                    if (tid == 0) {
+                        s_sel.lo = kNoDist;
+                        s_sel.hi = s_sel.valid = 0;
+                    }
+                    __syncthreads();
+                    for (uint32_t e = tid; e < P * (uint32_t)K; e += WT) {
+                        const uint32_t it = e / K, k = e - it * K;
+                        unsigned long long v = ~0ull;
+                        if ((int)k < *(volatile const int*)(a.part_n + first + it)) {
+                            const int64_t o = (int64_t)(first + it) * K + k;
+                            const uint32_t bits = __float_as_uint(*(volatile const float*)(a.part_d + o));
+                            v = ((unsigned long long)bits << 32) | *(volatile const uint32_t*)(a.part_i + o);
+                            atomicMin(&s_sel.lo, bits);
+                            atomicMax(&s_sel.hi, bits);
+                            atomicAdd(&s_sel.valid, 1u);
+                        }
+                        ent[e] = v;
+                    }
+                    __syncthreads();
+                    n = block_top<WT>(ent, P * (uint32_t)K, (uint32_t)K, ulist, s_sel);
+                    write = true;
+                } else if (warp == 0) {
+                    int m = 0;
+                    float thr_d = FLT_MAX;
+                    uint32_t thr_i = 0;
+                    for (uint32_t k = 0; k < P; ++k) {
+                        const int it = first + (int)k;
+                        const int cnt = *(volatile const int*)(a.part_n + it);
+                        const float* pd2 = a.part_d + (int64_t)it * K;
+                        const uint32_t* pi2 = a.part_i + (int64_t)it * K;
+                        for (int e = 0; e < cnt; ++e) {
+                            const float d = *(volatile const float*)(pd2 + e);
+                            const uint32_t id = *(volatile const uint32_t*)(pi2 + e);
+                            if (!lessp(d, id, thr_d, thr_i)) break;
+                            warp_insert(wd, wi, m, K, d, id, thr_d, thr_i);
+                        }
+                    }
+                    int32_t* oid = a.out_ids + (int64_t)q * K;
+                    float* od = a.out_d + (int64_t)q * K;
+                    for (int k = lane; k < K; k += 32) {
+                        oid[k] = k < m ? (int32_t)wi[k] : -1;
+                        od[k] = k < m ? wd[k] : FLT_MAX;
+                    }
+                    if (lane == 0) atomicAdd(a.totals + 1, C);
+                }
+            }
+        }
+        if (write) {   // uniform
+            int32_t* oid = a.out_ids + (int64_t)q * K;
+            float* od = a.out_d + (int64_t)q * K;
+            for (uint32_t k = tid; k < (uint32_t)K; k += WT) {
+                const unsigned long long v = k < n ? ent[ulist[k]] : 0ull;
+                oid[k] = k < n ? (int32_t)(uint32_t)v : -1;
+                od[k] = k < n ? __uint_as_float((uint32_t)(v >> 32)) : FLT_MAX;
+            }
+            if (tid == 0) atomicAdd(a.totals + 1, C);
+        }
+        if (tid == 0) s_item = next;
+        __syncthreads();
+    }
+}
+
+// ---- BF16 form ----
 // WT threads per item: WT / 32 warps each keep a sorted top-K list over a
 // strided share of the item's candidates (tuned: 64, 128, 256 or 512; wide
 // items keep more row gathers in flight per block of shared memory).
@@ -170,8 +620,8 @@ __global__ void k_order_scatter(WsArgs a) {
 // item holds at most W_CAP = W_SLOTS / 2 distinct ids. Every item of a query
 // scans the query's whole id list and keeps its partition, so larger sets
 // (fewer, larger partitions) scan less at the cost of occupancy.
-template <int WT, bool kBF16, int W_SLOTS>
-__global__ void __launch_bounds__(WT) k_candidates_ws(WsArgs a) {
+template <int WT, int W_SLOTS>
+__global__ void __launch_bounds__(WT) k_candidates_ws_bf16(WsArgs a) {
     constexpr int WW = WT / 32;
     constexpr int W_CAP = W_SLOTS / 2;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -240,9 +690,7 @@ __global__ void __launch_bounds__(WT) k_candidates_ws(WsArgs a) {
             fp32_dist_pass<WW>(a.X, D, qs, vec, cnt, idx_of, [&](uint32_t ci) { return ulist[ci]; }, pre, wd, wi, K,
                                n, thr_d, thr_i);
         };
-        if constexpr (!kBF16) {
-            fp32_pass(U, [](uint32_t j) { return j; }, [](uint32_t, float&) { return false; });
-        } else {
+        {
             // Pass 1: BF16 rows. d~ is computed in the reference lane order
             // from the bf16 copy; E bounds |d~ - d| where d is the FP32
             // distance (exact rows: E = 0, since d~ is then d itself; rows
@@ -1051,8 +1499,8 @@ size_t dense_smem_bytes(int64_t N, int D, int K) {
 
 size_t ws_smem_bytes(int D, int K, int wt, int bf16, int slots) {
     const size_t cap = (size_t)slots / 2;
-    return sizeof(float) * (size_t)((D + 3) & ~3) + sizeof(uint32_t) * ((size_t)slots + cap) +
-           (size_t)(wt / 32) * K * (sizeof(float) + sizeof(uint32_t)) + (bf16 ? 2 * sizeof(float) * cap : 0);
+    return (bf16 ? 0 : (size_t)(wt / 32) * row_stage_bytes(D)) + sizeof(float) * (size_t)((D + 3) & ~3) + sizeof(uint32_t) * ((size_t)slots + cap) +
+           (size_t)(bf16 ? wt / 32 : 1) * K * (sizeof(float) + sizeof(uint32_t)) + (bf16 ? 2 * sizeof(float) * cap : 0);
 }
 
 cudaError_t launch_order_queries(const WsArgs& a, cudaStream_t st) {
@@ -1080,11 +1528,17 @@ std::atomic<size_t>& ws_smem_cap() {
 }
 
 template <int WT, bool kBF16, int SL>
+constexpr auto ws_kernel() {
+    if constexpr (kBF16) return &k_candidates_ws_bf16<WT, SL>;
+    else return &k_candidates_ws<WT, SL>;
+}
+
+template <int WT, bool kBF16, int SL>
 cudaError_t launch_ws_v(const WsArgs& a, int grid, cudaStream_t st) {
     const size_t smem = ws_smem_bytes(a.D, a.K, WT, kBF16, SL);
-    const cudaError_t e = opt_in_smem(k_candidates_ws<WT, kBF16, SL>, smem, ws_smem_cap<WT, kBF16, SL>());
+    const cudaError_t e = opt_in_smem(ws_kernel<WT, kBF16, SL>(), smem, ws_smem_cap<WT, kBF16, SL>());
     if (e != cudaSuccess) return e;
-    k_candidates_ws<WT, kBF16, SL><<<grid, WT, smem, st>>>(a);
+    ws_kernel<WT, kBF16, SL>()<<<grid, WT, smem, st>>>(a);
     return cudaGetLastError();
 }
 
@@ -1092,8 +1546,8 @@ template <int WT, bool kBF16, int SL>
 int ws_bps_v(int D, int K) {
     int n = 0;
     const size_t smem = ws_smem_bytes(D, K, WT, kBF16, SL);
-    if (opt_in_smem(k_candidates_ws<WT, kBF16, SL>, smem, ws_smem_cap<WT, kBF16, SL>()) != cudaSuccess) return 1;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, k_candidates_ws<WT, kBF16, SL>, WT, smem) != cudaSuccess)
+    if (opt_in_smem(ws_kernel<WT, kBF16, SL>(), smem, ws_smem_cap<WT, kBF16, SL>()) != cudaSuccess) return 1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ws_kernel<WT, kBF16, SL>(), WT, smem) != cudaSuccess)
         n = 1;
     return n > 0 ? n : 1;
 }
@@ -1143,6 +1597,16 @@ __global__ void k_bf16_rows(const float* __restrict__ X, int64_t N, int D, uint1
     }
 }
 }  // namespace
+
+cudaError_t launch_candidates_small(const WsArgs& a, int sms, cudaStream_t st) {
+    const size_t smem = sizeof(float) * SMW * (size_t)((a.D + 3) & ~3);
+    static std::atomic<size_t> cap{0};
+    const cudaError_t e = opt_in_smem(k_candidates_small, smem, cap);
+    if (e != cudaSuccess) return e;
+    const int grid = std::min((a.Q + SMW - 1) / SMW, sms * 8);
+    k_candidates_small<<<grid, 32 * SMW, smem, st>>>(a);
+    return cudaGetLastError();
+}
 
 cudaError_t launch_candidates_ws(const WsArgs& a, int grid, cudaStream_t st) {
     if (a.slots == 16384)

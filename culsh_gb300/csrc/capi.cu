@@ -255,7 +255,7 @@ struct culsh_search {
     DevBuf<int> deferred;
     DevBuf<uint32_t> arena;
     // work-stealing candidate stage
-    DevBuf<int> q_items, q_off, item_q, part_n, dense_q;
+    DevBuf<int> q_items, q_off, item_q, part_n, dense_q, small_q;
     DevBuf<uint32_t> qorder, qorder_bins;
     DevBuf<unsigned int> q_done;
     DevBuf<uint8_t> item_p;
@@ -942,7 +942,8 @@ constexpr int kWsPartitions = 64;              // most partitions of one query
 // counter (low) and overflow flag (high), [5] items, [6] BF16 re-checks,
 // [7] dense queries (low) and their claim counter (high), [8..9] unused,
 // [10] dense queries scanned exactly after the tensor-core merge, [11] the
-// tensor-core kernels' error flags, [12..15] unused.
+// tensor-core kernels' error flags, [12] queries of a few candidates,
+// [13..15] unused.
 constexpr int kStatWords = 16;
 constexpr size_t kWsPartialBytes = size_t(64) << 20;
 
@@ -968,7 +969,7 @@ struct SearchPlan {
     float* vals;
     ProbeArgs pa;
     int probe_generic;
-    int use_ws, ws_grid;
+    int use_ws, ws_grid, sms;
     int use_dense;      // some query can be dense: the planner lists those, run_dense serves them
     int use_knn;        // ... on the tensor cores (membership rows + masked GEMM)
     CandArgs ca;
@@ -1322,7 +1323,10 @@ int plan_search(culsh_search* s, const float* dQ, int Q, int32_t* d_ids, float* 
             CU_TRY(cudaGetDevice(&dev));
             CU_TRY(cudaDeviceGetAttribute(&s->smem_optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
         }
-        const size_t need = ws_smem_bytes(D, K, tu.ws_wt, tu.dist_bf16 ? 1 : 0, tu.ws_slots) + 8192;
+        // (Counted with a list per warp, which the BF16 form keeps, so that both
+        // forms of a configuration take the same route.)
+        const size_t need = ws_smem_bytes(D, K, tu.ws_wt, tu.dist_bf16 ? 1 : 0, tu.ws_slots) + 8192 +
+                            (tu.dist_bf16 ? 0 : 8 * (size_t)K * (tu.ws_wt / 32 - 1));
         if (need > (size_t)s->smem_optin) P.use_ws = 0;
     }
     if (P.use_ws) {
@@ -1366,6 +1370,7 @@ int plan_search(culsh_search* s, const float* dQ, int Q, int32_t* d_ids, float* 
         const int occ = s->occ_val;
         const int bps = tu.ws_bps > 0 ? std::min(tu.ws_bps, occ) : occ;
         P.ws_grid = s->sms * bps;
+        P.sms = s->sms;
         WsArgs& a = P.wa;
         a.X = ca.X;
         a.N = ca.N;
@@ -1387,6 +1392,7 @@ int plan_search(culsh_search* s, const float* dQ, int Q, int32_t* d_ids, float* 
         a.totals = ca.totals;
         a.pmax = pmax;
         a.chunk = (unsigned long long)tu.ws_chunk;
+        a.whole = !bf16 && Q >= 4 * s->sms ? (unsigned long long)tu.ws_slots / 2 : 0ull;
         a.q_items = s->q_items.p;
         a.q_off = s->q_off.p;
         a.q_done = s->q_done.p;
@@ -1399,6 +1405,12 @@ int plan_search(culsh_search* s, const float* dQ, int Q, int32_t* d_ids, float* 
         a.next_item = reinterpret_cast<unsigned int*>(s->stats.p + 4);
         a.overflow = reinterpret_cast<unsigned int*>(s->stats.p + 4) + 1;
         a.n_items = reinterpret_cast<unsigned int*>(s->stats.p + 5);
+        if (!bf16 && D <= kSmallMaxD) {
+            CU_TRY(s->small_q.reserve(Q));
+            a.small_q = s->small_q.p;
+            a.small_max = kSmallMax;
+        }
+        a.n_small = reinterpret_cast<unsigned int*>(s->stats.p + 12);
         a.wt = tu.ws_wt;
         a.slots = tu.ws_slots;
         a.bf16 = bf16;
@@ -1482,13 +1494,14 @@ int enqueue_search(const SearchPlan& P, cudaStream_t st, bool capturing, int* la
     if (P.use_ws) {
         if (P.wa.order) CU_TRY(launch_order_queries(P.wa, st));
         CU_TRY(launch_plan_items(P.wa, st));
+        if (P.wa.small_max) CU_TRY(launch_candidates_small(P.wa, P.sms, st));
         CU_TRY(launch_candidates_ws(P.wa, P.ws_grid, st));
     } else {
         CU_TRY(launch_candidates(P.ca, st));
     }
     if (P.stage_events) CU_TRY(cudaEventRecordWithFlags(P.ev[3], st, evf));
     CU_TRY(cudaMemcpyAsync(P.h_stats, P.stats, 8 * kStatWords, cudaMemcpyDeviceToHost, st));
-    *launches = (P.use_ws ? 3 + (P.wa.order ? 3 : 0) : 2) + probe_launches(P.pa);
+    *launches = (P.use_ws ? 3 + (P.wa.order ? 3 : 0) + (P.wa.small_max ? 1 : 0) : 2) + probe_launches(P.pa);
     return CULSH_OK;
 }
 
@@ -2161,6 +2174,7 @@ long long culsh_search_device_bytes(culsh_search* s) {
     add(s->part_d);
     add(s->part_i);
     add(s->dense_q);
+    add(s->small_q);
     add(s->qorder);
     add(s->qorder_bins);
     add(s->kbm);
@@ -2185,7 +2199,7 @@ long long culsh::search_estimate(const culsh_index* ix, int Q, int K, int T, boo
     const size_t per_item = k * 8 + 4 + 4 + 1;
     size_t cap = std::max<size_t>(2 * q, kWsPartialBytes / per_item);
     cap = std::min(cap, q * kWsPartitions);
-    b += 16 * q + cap * per_item;   // per-query plan arrays, dense-query list, partial lists
+    b += 20 * q + cap * per_item;   // per-query plan arrays, dense and small lists, partial lists
     b += 4 * q + 4 * (kOrderBins + 1);   // locality order
     if (M <= 16) b += 12 * L * q * (size_t)T + 48 * L * q;   // split probe lookups
     KnnSearch kn;
@@ -2232,6 +2246,7 @@ int culsh_search_release(culsh_search* s) {
     s->part_d.release();
     s->part_i.release();
     s->dense_q.release();
+    s->small_q.release();
     s->qorder.release();
     s->qorder_bins.release();
     s->kbm.release();

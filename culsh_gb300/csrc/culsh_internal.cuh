@@ -363,6 +363,7 @@ struct WsArgs {
     unsigned long long* totals;        // [2]: sum unique, sum non-unique
     int pmax;                          // partitions per query, at most 64
     unsigned long long chunk;          // non-unique candidates per partition
+    unsigned long long whole;          // ... up to which a query is one item whatever chunk says
     int* q_items;                      // [Q] partitions of each query
     int* q_off;                        // [Q] first item of each query
     unsigned int* q_done;              // [Q] partitions finished
@@ -375,6 +376,10 @@ struct WsArgs {
     unsigned int* n_items;
     unsigned int* next_item;           // work-stealing counter, zero before the launch
     unsigned int* overflow;            // nonzero: rerun with the per-query kernel
+    // Queries of 1 .. small_max non-unique candidates (0: none), one warp each
+    uint32_t small_max;
+    int* small_q;                      // [Q]
+    unsigned int* n_small;
     int wt;                            // threads per item CTA: 64, 128 or 256
     int slots;                         // shared hash-set slots per item: 4096 or 8192
     // BF16 form: approximate distances from xb, certified FP32 rerank
@@ -413,6 +418,9 @@ struct WsArgs {
 };
 constexpr uint32_t kBankMin = 512;            // smallest bucket that has a bank list
 constexpr int64_t kBankMaxN = (int64_t(1) << 21) - 1024;   // 11 bits of word row (one past the bitmap), 5 of bit
+constexpr uint32_t kSmallMax = 32;     // candidates a warp's lanes hold
+constexpr int kSmallMaxD = 1024;       // dimensions whose query rows leave several blocks resident
+cudaError_t launch_candidates_small(const WsArgs& a, int sms, cudaStream_t st);
 constexpr int kOrderBins = 4096;
 cudaError_t launch_order_queries(const WsArgs& a, cudaStream_t st);   // 3 kernels + 1 memset
 size_t dense_smem_bytes(int64_t N, int D, int K);

@@ -58,9 +58,9 @@ __device__ __forceinline__ void warp_insert(float* wd, uint32_t* wi, int& n, int
 // Inserts id into the open-addressing set hset[0..mask]; a new id is appended
 // to ulist when its position is below lcap. *ucount counts every new id, so a
 // count above lcap reports an overflow without writing past the list.
-__device__ __forceinline__ void set_insert(uint32_t* hset, uint32_t mask, uint32_t* ulist, uint32_t lcap,
-                                           uint32_t* ucount, uint32_t id) {
-    uint32_t h = mix32(id) & mask;
+__device__ __forceinline__ void set_insert_at(uint32_t* hset, uint32_t mask, uint32_t* ulist, uint32_t lcap,
+                                              uint32_t* ucount, uint32_t id, uint32_t hash) {
+    uint32_t h = hash & mask;
     for (uint32_t p = 0; p <= mask; ++p) {
         const uint32_t prev = atomicCAS(&hset[h], kEmpty32, id);
         if (prev == kEmpty32) {
@@ -71,6 +71,11 @@ __device__ __forceinline__ void set_insert(uint32_t* hset, uint32_t mask, uint32
         if (prev == id) return;
         h = (h + 1) & mask;
     }
+}
+
+__device__ __forceinline__ void set_insert(uint32_t* hset, uint32_t mask, uint32_t* ulist, uint32_t lcap,
+                                           uint32_t* ucount, uint32_t id) {
+    set_insert_at(hset, mask, ulist, lcap, ucount, id, mix32(id));
 }
 
 // Exact FP32 squared distance of row x to the query qs (shared memory) in the
@@ -111,6 +116,79 @@ __device__ __forceinline__ float row_distance(const float* __restrict__ x, int D
     const float t = __fadd_rn(s, __shfl_xor_sync(0xffffffffu, s, 4));
     const float u = __fadd_rn(t, __shfl_xor_sync(0xffffffffu, t, 2));
     return __fadd_rn(u, __shfl_xor_sync(0xffffffffu, u, 1));
+}
+
+// ---- Rows through shared memory ----
+// A warp fetches 16 rows at a time with one bulk copy each (whole 128-byte
+// lines in one request) and reads them back in the lane order above. Row
+// loads of 16 bytes per lane touch 16 lines an instruction, a 32-byte sector
+// of each: the candidate kernel then ran at 2.7 TB/s of random sectors.
+constexpr int kRowBatch = 16;
+constexpr int kRowStageMaxD = 160;   // 16 rows of a larger dimension leave too few warps resident
+// Padded row of the stage in floats: 8 mod 32, so that four rows' pairs of
+// 16-byte reads fall into different banks.
+__host__ __device__ constexpr int row_stride(int D) { return (D + 23) / 32 * 32 + 8; }
+__host__ __device__ constexpr bool row_staged(int D) { return D % 4 == 0 && D >= 16 && D <= kRowStageMaxD; }
+__host__ __device__ constexpr size_t row_stage_bytes(int D) {
+    return row_staged(D) ? sizeof(float) * (size_t)kRowBatch * row_stride(D) : 0;
+}
+
+__device__ __forceinline__ uint32_t shared_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
+__device__ __forceinline__ void stage_bar_init(uint64_t* bar) {
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(shared_addr(bar)) : "memory");
+}
+
+// Distances of rows ids[e], e = first + lane / 2 < cnt, to qs: every lane
+// returns its row's (garbage past cnt). All lanes of the warp call it; `phase`
+// counts the warp's uses of its barrier. A copy that does not arrive within the
+// bounded wait sets *err and the distance is not to be used.
+__device__ __forceinline__ float staged_distance(const float* __restrict__ X, int D, const float* qs,
+                                                 const uint32_t* ids, uint32_t first, uint32_t cnt, float* stage,
+                                                 uint64_t* bar, uint32_t& phase, unsigned int* err) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t rows = min((uint32_t)kRowBatch, cnt - first);
+    const uint32_t bytes = (uint32_t)D * 4;
+    const int stride = row_stride(D);
+    __syncwarp();   // the stage's last reads are over
+    if (lane == 0) {
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(shared_addr(bar)), "r"(rows * bytes)
+                     : "memory");
+    }
+    __syncwarp();
+    if (lane < (int)rows)
+        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                         shared_addr(stage + lane * stride)),
+                     "l"(reinterpret_cast<uint64_t>(X + (int64_t)ids[first + lane] * D)), "r"(bytes), "r"(shared_addr(bar))
+                     : "memory");
+    uint32_t ok = 0;
+    for (uint32_t i = 0; i < (1u << 18) && !ok; ++i)
+        asm volatile(
+            "{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\tselp.u32 %0, 1, 0, "
+            "p;\n\t}\n"
+            : "=r"(ok)
+            : "r"(shared_addr(bar)), "r"(phase & 1u), "r"(16384u)
+            : "memory");
+    ++phase;
+    if (!ok) atomicOr(err, 4u);
+    const float* x = stage + (lane >> 1) * stride;
+    float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
+#pragma unroll 8
+    for (int c = 4 * (lane & 1); c < D; c += 8) {
+        const float4 v = *reinterpret_cast<const float4*>(x + c);
+        const float4 qv = *reinterpret_cast<const float4*>(qs + c);
+        const float d0 = __fsub_rn(qv.x, v.x), d1 = __fsub_rn(qv.y, v.y);
+        const float d2 = __fsub_rn(qv.z, v.z), d3 = __fsub_rn(qv.w, v.w);
+        s0 = __fmaf_rn(d0, d0, s0);
+        s1 = __fmaf_rn(d1, d1, s1);
+        s2 = __fmaf_rn(d2, d2, s2);
+        s3 = __fmaf_rn(d3, d3, s3);
+    }
+    __syncwarp();
+    const float o0 = __shfl_xor_sync(0xffffffffu, s0, 1), o1 = __shfl_xor_sync(0xffffffffu, s1, 1);
+    const float o2 = __shfl_xor_sync(0xffffffffu, s2, 1), o3 = __shfl_xor_sync(0xffffffffu, s3, 1);
+    const float t0 = __fadd_rn(s0, o0), t1 = __fadd_rn(s1, o1), t2 = __fadd_rn(s2, o2), t3 = __fadd_rn(s3, o3);
+    return __fadd_rn(__fadd_rn(t0, t2), __fadd_rn(t1, t3));
 }
 
 // Exact FP32 squared distances, in the reference lane order
@@ -260,19 +338,31 @@ __device__ __forceinline__ void gather_bucket_ids(const BucketView& v, int q, Ga
         const unsigned long long total = g.pre[n - 1];
         // h: first bucket whose inclusive prefix exceeds i. i only grows, so
         // h is kept between steps and searched for only when i leaves it.
+        // Four ids are loaded before the first is visited (one at a time, each
+        // visit waited out a load).
+        constexpr int GU = 4;
         uint32_t h = 0;
-        for (unsigned long long i = tid; i < total; i += NT) {
-            if (g.pre[h] <= i) {
-                uint32_t lo = h + 1, hi = n - 1;
-                while (lo < hi) {
-                    const uint32_t mid = (lo + hi) >> 1;
-                    if (g.pre[mid] > i) hi = mid;
-                    else lo = mid + 1;
+        for (unsigned long long i0 = tid; i0 < total; i0 += GU * NT) {
+            uint32_t id[GU];
+#pragma unroll
+            for (int u = 0; u < GU; ++u) {
+                const unsigned long long i = i0 + (unsigned long long)u * NT;
+                if (i < total) {
+                    if (g.pre[h] <= i) {
+                        uint32_t lo = h + 1, hi = n - 1;
+                        while (lo < hi) {
+                            const uint32_t mid = (lo + hi) >> 1;
+                            if (g.pre[mid] > i) hi = mid;
+                            else lo = mid + 1;
+                        }
+                        h = lo;
+                    }
+                    id[u] = __ldg(v.ids + g.base[h] + (i - (h ? g.pre[h - 1] : 0ull)));
                 }
-                h = lo;
             }
-            const uint64_t off = i - (h ? g.pre[h - 1] : 0ull);
-            f(__ldg(v.ids + g.base[h] + off));
+#pragma unroll
+            for (int u = 0; u < GU; ++u)
+                if (i0 + (unsigned long long)u * NT < total) f(id[u]);
         }
         __syncthreads();
     }

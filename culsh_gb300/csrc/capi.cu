@@ -229,6 +229,7 @@ struct SearchTune {
     int dist_bf16 = 0;     // 1: BF16 candidate distances + certified FP32 rerank (work-stealing form)
     int ws_slots = 4096;   // shared hash-set slots per work item (4096, 8192 or 16384)
     int probe_split = 0;   // M <= 16: 1 enumeration kernel + lookup kernel; 2 lookups at the enumeration's end
+    bool probe_auto = true;   // probe_split and probe_pch as created: the form may follow the shape
     int ws_order = 0;      // 1: plan queries in the locality order of their home bucket (work-stealing form)
     int dense_tc = 1;      // 1: dense queries take the tensor-core path (membership rows + masked GEMM)
     int dense_min = 0;     // non-unique candidates that make a query dense (0: the form's default)
@@ -1275,7 +1276,14 @@ int plan_search(culsh_search* s, const float* dQ, int Q, int32_t* d_ids, float* 
     {
         // CULSH_PROBE_SPLIT=0/1 overrides the tuning (the tests run both).
         const char* e = getenv("CULSH_PROBE_SPLIT");
-        const int form = M <= 16 ? std::min(2, std::max(0, e ? atoi(e) : tu.probe_split)) : 0;
+        int form = M <= 16 ? std::min(2, std::max(0, e ? atoi(e) : tu.probe_split)) : 0;
+        P.pa.auto_form = tu.probe_auto && !e;
+        // No form set: lookups behind the key filter at the enumeration's end
+        // where buckets hold fewer than four points on average, since most
+        // probes then find nothing (1M points, every one its own bucket, T = 16:
+        // 148 us fused, 117 us so; at 20,000 buckets a table fused is ahead, 160 against 167 us).
+        if (P.pa.auto_form && M <= 16 && T >= 4 && 4 * (unsigned long long)ix->h_boff[L] > (unsigned long long)ix->N * L)
+            form = 2;
         if (form > 0) {
             CU_TRY(s->ph.reserve((size_t)L * Q * T));
             CU_TRY(s->pmask.reserve((size_t)L * Q * T));
@@ -2309,6 +2317,7 @@ int culsh_search_set_tuning(culsh_search* s, const culsh_tuning* in) {
     s->tune.dist_bf16 = in->distance_bf16;
     s->tune.ws_slots = in->ws_set_slots;
     s->tune.probe_split = in->probe_split;
+    s->tune.probe_auto = false;
     s->tune.ws_order = in->ws_order;
     s->tune.dense_tc = in->dense_tc;
     s->tune.dense_min = in->dense_min;
@@ -2384,6 +2393,7 @@ int culsh_search_autotune(culsh_search* s, const float* d_queries, int Q, int* d
     };
     const SearchTune start = s->tune;
     SearchTune best = start;
+    best.probe_auto = false;
     float stage[4];
     float best_t = 0;
     // projection tiling

@@ -307,6 +307,7 @@ struct ProbeArgs {
     int32_t* qbuckets;         // [L][Q*T]
     unsigned long long* cnu;   // [Q] non-unique candidate counts (accumulated)
     int small_codes;           // every |cmin|, |cmax| < 2^24 - 2 (set by the host)
+    int auto_form;             // no probe form was set by the caller: small batches may take a warp per pair
     int pch;                   // fast kernel: probes whose group loads overlap (1, 2, 4)
     // Split lookups (M <= 16, fast kernel). split = 1: the enumeration kernel
     // stores each valid probe's finished hash and mask and marks its query

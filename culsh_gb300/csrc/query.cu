@@ -220,7 +220,8 @@ __device__ __forceinline__ int lowest_bit(uint64_t b) { return __ffsll((long lon
 __device__ __forceinline__ int highest_bit(uint32_t b) { return 31 - __clz((int)b); }
 __device__ __forceinline__ int highest_bit(uint64_t b) { return 63 - __clzll((long long)b); }
 
-struct FastProbeCtx {
+template <int PF>
+struct FastProbeCtxT {
     u128 hkey;
     uint64_t h0;                        // additive lookup hash of the home key (before the mix)
     uint32_t ok0, okUp, okDn, allM;     // per-column range validity (M <= 32)
@@ -229,14 +230,16 @@ struct FastProbeCtx {
     const unsigned long long* rmul;     // this table's hash multipliers
 };
 
+using FastProbeCtx = FastProbeCtxT<PF>;
+
 __device__ __forceinline__ u128 unit_of(const unsigned long long* funit, int m) {
     return ((u128)__ldg(funit + 2 * m + 1) << 64) | (u128)__ldg(funit + 2 * m);
 }
 
 // Key of a probe mask; returns false when a column leaves [cmin, cmax]. A
 // column perturbed both up and down keeps its home code.
-template <typename MaskT>
-__device__ __forceinline__ bool probe_key(const FastProbeCtx& c, MaskT mask, u128& key) {
+template <int PF, typename MaskT>
+__device__ __forceinline__ bool probe_key(const FastProbeCtxT<PF>& c, MaskT mask, u128& key) {
     uint32_t up = 0, dn = 0;
     for (MaskT b = mask; b; b &= b - 1) {
         const int e = c.enc[lowest_bit(b) * PF];
@@ -256,8 +259,8 @@ __device__ __forceinline__ bool probe_key(const FastProbeCtx& c, MaskT mask, u12
 // perturbed column, accumulated in the same walk over the mask: a column
 // perturbed both up and down adds +R - R = 0 mod 2^64, as it keeps its home
 // code); returns false when a column leaves [cmin, cmax].
-template <typename MaskT>
-__device__ __forceinline__ bool probe_hash(const FastProbeCtx& c, MaskT mask, uint64_t& hh) {
+template <int PF, typename MaskT>
+__device__ __forceinline__ bool probe_hash(const FastProbeCtxT<PF>& c, MaskT mask, uint64_t& hh) {
     uint32_t up = 0, dn = 0;
     uint64_t h = c.h0;
     for (MaskT b = mask; b; b &= b - 1) {
@@ -288,7 +291,7 @@ __device__ __forceinline__ bool key_matches(const uint32_t* uk, u128 k, int KW) 
 // The reference's heap selection + heap sort over a strided slice (used
 // only when deltas tie or are NaN). val(i) is delta i; perm[] receives the
 // delta indices in ascending order.
-template <class V>
+template <int PF, class V>
 __device__ void heap_order_strided(V val, int8_t* perm, int M2, int maxT) {
     const int levels = ceil_log2_dev(M2 + 1);
     auto sift = [&](int total) {
@@ -426,6 +429,7 @@ __device__ __forceinline__ bool order_deltas_net(const float* dn, uint8_t* enc, 
 // whose deltas tie (or are NaN). Out of line: inlined, its loops enlarge the
 // probe kernel and slow every pair. dn: the pair's downs (strided slice);
 // enc: receives sorted delta -> column | up << 7.
+template <int PF>
 __device__ __noinline__ void order_deltas_heap(const float* dn, uint8_t* enc, int M) {
     auto dv = [&](int i) {
         const float d = dn[(i < M ? i : i - M) * PF];
@@ -433,7 +437,7 @@ __device__ __noinline__ void order_deltas_heap(const float* dn, uint8_t* enc, in
     };
     const int M2 = 2 * M;
     int8_t* perm = reinterpret_cast<int8_t*>(enc);
-    heap_order_strided(dv, perm, M2, M2);
+    heap_order_strided<PF>(dv, perm, M2, M2);
     for (int i = 0; i < M2; ++i) {
         const int pm = perm[i * PF];
         enc[i * PF] = (uint8_t)((pm % M) | (pm >= M ? 0x80 : 0));
@@ -536,7 +540,7 @@ __global__ void __launch_bounds__(PF, kForm == 2 && MM <= 12 ? 9 : (kForm > 0 ? 
 
     if (T > 1 && MM > 0) {
         if (distinct) distinct = order_deltas_net<(MM > 0 ? MM : 1)>(dn, enc, M, sv);
-        if (!distinct) order_deltas_heap(dn, enc, M);
+        if (!distinct) order_deltas_heap<PF>(dn, enc, M);
         comb[0] = 1;
         cd[0] = sv(0);
     } else if (T > 1) {
@@ -572,7 +576,7 @@ __global__ void __launch_bounds__(PF, kForm == 2 && MM <= 12 ? 9 : (kForm > 0 ? 
                 else --iu;
             }
         }
-        if (!distinct) order_deltas_heap(dn, enc, M);
+        if (!distinct) order_deltas_heap<PF>(dn, enc, M);
         comb[0] = 1;
         cd[0] = sv(0);
     }
@@ -803,6 +807,193 @@ __global__ void __launch_bounds__(PF, kForm == 2 && MM <= 12 ? 9 : (kForm > 0 ? 
         }
     }
     if (cnu) atomicAdd(a.cnu + q, cnu);
+}
+
+// One warp per (table, query) pair, for batches too small to fill the device
+// with a thread per pair (a lone thread walks its T probes one after another,
+// 90 us at T = 16 and 440 us at T = 64 whatever the batch; a warp 14 and 29 us).
+// M <= 16: lane i holds delta i and sorts them across the lanes (the
+// reference's heap procedure where two are equal or NaN); the enumeration's
+// candidates live in the lanes' registers, entry i in lane i % 32, and each step
+// takes the smallest sum, the first of equal ones, with two warp reductions. The
+// masks then go to the lanes, which hash and look up all T probes at once.
+constexpr int PW = 4;            // warps per block
+constexpr int kWarpProbeMaxT = 64;
+__global__ void __launch_bounds__(32 * PW) k_probe_warp(ProbeArgs a) {
+    __shared__ float s_dn[PW][16];
+    __shared__ uint8_t s_enc[PW][32];
+    __shared__ uint32_t s_mask[PW][kWarpProbeMaxT];
+    const LookupView& lv = a.lv;
+    const int Q = a.Q, T = a.T, L = lv.L, M = lv.M, KW = lv.KW, M2 = 2 * M;
+    const int lane = threadIdx.x & 31, wp = threadIdx.x >> 5;
+    const int64_t idx = (int64_t)blockIdx.x * PW + wp;
+    if (idx >= (int64_t)L * Q) return;   // warps work alone
+    const int l = (int)(idx / Q), q = (int)(idx - (int64_t)l * Q);
+    float* dn = s_dn[wp];
+    uint8_t* enc = s_enc[wp];
+
+    FastProbeCtxT<1> c;
+    c.allM = M >= 32 ? ~0u : ((1u << M) - 1);
+    c.enc = enc;
+    c.funit = lv.funit + 2 * l * M;
+    c.rmul = lv.rmul + l * M;
+    // lane m < M: column m's home code, range and key contributions
+    const bool col_on = lane < M;
+    const int col = l * M + (col_on ? lane : 0);
+    const float v = __ldg(a.vals + (int64_t)col * Q + q);
+    const float f = floorf(v);
+    const float down = __fsub_rn(v, f);
+    const float up = __fsub_rn(1.0f, down);
+    const int64_t lo = __ldg(lv.cmin + col), hi = __ldg(lv.cmax + col);
+    const int64_t h = (f >= -1.0e15f && f <= 1.0e15f) ? (int64_t)f : (int64_t)1 << 50;
+    c.ok0 = __ballot_sync(0xffffffffu, col_on && h >= lo && h <= hi);
+    c.okUp = __ballot_sync(0xffffffffu, col_on && h + 1 >= lo && h + 1 <= hi);
+    c.okDn = __ballot_sync(0xffffffffu, col_on && h - 1 >= lo && h - 1 <= hi);
+    u128 hk = col_on ? field_term(h - lo, __ldg(lv.foff + col)) : (u128)0;
+    uint64_t h0 = col_on ? (uint64_t)(h - lo) * __ldg(c.rmul + lane) : 0ull;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const uint64_t l64 = __shfl_xor_sync(0xffffffffu, (uint64_t)hk, o);
+        const uint64_t h64 = __shfl_xor_sync(0xffffffffu, (uint64_t)(hk >> 64), o);
+        hk += ((u128)h64 << 64) | l64;
+        h0 += __shfl_xor_sync(0xffffffffu, h0, o);
+    }
+    c.hkey = hk;
+    c.h0 = h0;
+    if (col_on) dn[lane] = down;
+    const bool finite = __all_sync(0xffffffffu, !col_on || (down == down && up == up));
+    __syncwarp();
+
+    float sd = 0.0f;   // value of sorted delta `lane`
+    if (T > 1) {
+        // delta i: down of column i, or up of column i - M; padding sorts last
+        const int m = lane < M ? lane : lane - M;
+        float x = lane < M2 ? (lane < M ? dn[m] : __fsub_rn(1.0f, dn[m])) : 3.0f;
+        uint32_t e = lane < M2 ? (uint32_t)m | (lane < M ? 0u : 0x80u) : 0xFFu;
+        if (finite) {
+#pragma unroll
+            for (int i = 2; i <= 32; i <<= 1) {
+#pragma unroll
+                for (int j = i >> 1; j > 0; j >>= 1) {
+                    const float ox = __shfl_xor_sync(0xffffffffu, x, j);
+                    const uint32_t oe = __shfl_xor_sync(0xffffffffu, e, j);
+                    const bool keep_min = ((lane & j) == 0) == ((lane & i) == 0);
+                    const bool less = ox < x || (ox == x && oe < e);
+                    if (less == keep_min && (ox != x || oe != e)) {
+                        x = ox;
+                        e = oe;
+                    }
+                }
+            }
+        }
+        const float px = __shfl_up_sync(0xffffffffu, x, 1);
+        const bool distinct = finite && __all_sync(0xffffffffu, lane == 0 || lane >= M2 || px < x);
+        if (distinct) {
+            if (lane < M2) enc[lane] = (uint8_t)e;
+        } else if (lane == 0) {
+            order_deltas_heap<1>(dn, enc, M);
+        }
+        __syncwarp();
+        if (lane < M2) {
+            const int en = enc[lane];
+            const float d = dn[en & 0x3f];
+            sd = (en & 0x80) ? __fsub_rn(1.0f, d) : d;
+        }
+    }
+    // Enumeration (cuLSH_Kernels.cu:216-255): probe t > 0 is the candidate of
+    // smallest delta sum (the first of equal sums), shifted in place and
+    // expanded into a new one. Sums are compared as the reference's `<` does
+    // from FLT_MAX down: a sum that is not below FLT_MAX is never the minimum,
+    // and entry 0 is taken when none is.
+    const float INF = __int_as_float(0x7f800000);
+    float cd0 = INF, cd1 = INF;
+    uint32_t cm0 = 0, cm1 = 0;
+    const float first = __shfl_sync(0xffffffffu, sd, 0);
+    if (lane == 0) {
+        cd0 = first;
+        cm0 = 1;
+    }
+    int size = 1;
+    if (lane == 0) s_mask[wp][0] = 0;
+    auto order = [](float x) {   // unsigned order of a float; NaN and values from FLT_MAX on rank last
+        if (!(x < FLT_MAX)) return 0xFFFFFFFFu;
+        const uint32_t u = __float_as_uint(x);
+        return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+    };
+    for (int t = 1; t < T; ++t) {
+        const uint32_t o0 = order(cd0), o1 = order(cd1);
+        const uint32_t mn = __reduce_min_sync(0xffffffffu, min(o0, o1));
+        int mi = 0;   // entry index
+        if (mn != 0xFFFFFFFFu) {
+            const uint32_t b0 = __ballot_sync(0xffffffffu, o0 == mn), b1 = __ballot_sync(0xffffffffu, o1 == mn);
+            mi = b0 ? __ffs((int)b0) - 1 : 32 + __ffs((int)b1) - 1;
+        }
+        const int src = mi & 31;
+        const uint32_t probe = __shfl_sync(0xffffffffu, mi < 32 ? cm0 : cm1, src);
+        const float sum = mn != 0xFFFFFFFFu ? __shfl_sync(0xffffffffu, mi < 32 ? cd0 : cd1, src) : FLT_MAX;
+        if (lane == 0) s_mask[wp][t] = probe;
+        const int top = 31 - __clz((int)probe);
+        if (t < T - 1 && top < M2 - 1) {
+            const uint32_t p1 = probe | (1u << (top + 1));
+            const float m1 = __fadd_rn(sum, __shfl_sync(0xffffffffu, sd, top + 1));
+            const float m2 = __fsub_rn(m1, __shfl_sync(0xffffffffu, sd, top));
+            if (lane == src) {
+                if (mi < 32) { cd0 = m1; cm0 = p1; }
+                else { cd1 = m1; cm1 = p1; }
+            }
+            if (lane == (size & 31)) {
+                if (size < 32) { cd0 = m2; cm0 = p1 - (1u << top); }
+                else { cd1 = m2; cm1 = p1 - (1u << top); }
+            }
+            ++size;
+        }
+    }
+    __syncwarp();
+
+    // Every probe at once: lane t and t + 32.
+    int32_t* qb = a.qbuckets + (int64_t)l * Q * T + (int64_t)q * T;
+    const uint32_t gmask = __ldg(lv.hmask + l);
+    const unsigned long long* slots = lv.hslots + __ldg(lv.hoff + l);
+    const uint64_t bo = __ldg(lv.boff + l);
+    const uint32_t* filt = lv.filt ? lv.filt + __ldg(lv.fl_off + l) : nullptr;
+    const uint32_t fmask = lv.filt ? __ldg(lv.fl_mask + l) : 0u;
+    unsigned long long cnu = 0;
+    for (int t = lane; t < T; t += 32) {
+        const uint32_t pm = s_mask[wp][t];
+        uint64_t hh;
+        int32_t res = -1;
+        bool done = !probe_hash(c, pm, hh);
+        if (!done && filt) {
+            const uint32_t fx = filter_mix(hh), need = filter_bits(fx);
+            done = (__ldg(filt + (fx & fmask)) & need) != need;
+        }
+        const uint32_t fp = slot_fp(hh);
+        uint32_t g = (uint32_t)hh & gmask;
+        for (uint32_t p = 0; p <= gmask && !done; ++p) {
+            const unsigned long long* grp = slots + (uint64_t)g * kGroupWords;
+            const unsigned long long w = __ldg(grp);
+            for (int e = 0; e < kGroupSlots && !done; ++e) {
+                const uint32_t fe = (uint32_t)(w >> (16 * e)) & 0xFFFFu;
+                if (fe == kEmptyFp) {
+                    done = true;
+                } else if (fe == fp) {
+                    const uint32_t bj = __ldg(reinterpret_cast<const uint32_t*>(grp + 1) + e);
+                    u128 k;
+                    probe_key(c, pm, k);
+                    if (key_matches(lv.ukeys + (bo + bj) * KW, k, KW)) {
+                        res = (int32_t)bj;
+                        done = true;
+                    }
+                }
+            }
+            g = (g + 1) & gmask;
+        }
+        qb[t] = res;
+        if (res >= 0) cnu += __ldg(lv.sizes + bo + res);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) cnu += __shfl_xor_sync(0xffffffffu, cnu, o);
+    if (lane == 0 && cnu) atomicAdd(a.cnu + q, cnu);
 }
 
 // Lookups of the split form. A thread takes kResolveSlots probe slots
@@ -1143,14 +1334,29 @@ static bool probe_fast_eligible(const ProbeArgs& a) {
     return !generic_only && a.small_codes && a.lv.KW <= 4 && a.T <= 64 && a.lv.M <= 32 && fast_bytes <= 100 * 1024;
 }
 
+// Whether a warp per pair serves these arguments: shapes the fast kernel takes,
+// masks of at most 32 deltas, no form asked for, and so few pairs that a thread
+// each leaves the device empty: 1,024 T pairs, near the measured crossings (44
+// against 84 us at 16,384 pairs and T = 16, 84 against 86 us at 32,768; 118
+// against 357 us at 16,384 and T = 64, level at about 65,000).
+static bool probe_warp_eligible(const ProbeArgs& a) {
+    return a.auto_form && a.lv.M <= 16 && a.T <= kWarpProbeMaxT && (int64_t)a.lv.L * a.Q <= 1024ll * a.T &&
+           getenv("CULSH_PROBE_SPLIT") == nullptr;
+}
+
 int probe_launches(const ProbeArgs& a) {
     if ((int64_t)a.lv.L * a.Q <= 0) return 0;
+    if (probe_fast_eligible(a) && probe_warp_eligible(a)) return 1;
     return probe_fast_eligible(a) && a.split == 1 && a.lv.M <= 16 ? 2 : 1;
 }
 
 cudaError_t launch_probe(const ProbeArgs& a, cudaStream_t st) {
     const int64_t n = (int64_t)a.lv.L * a.Q;
     if (n <= 0) return cudaSuccess;
+    if (probe_fast_eligible(a) && probe_warp_eligible(a)) {
+        k_probe_warp<<<(unsigned)((n + PW - 1) / PW), 32 * PW, 0, st>>>(a);
+        return cudaGetLastError();
+    }
     if (probe_fast_eligible(a)) return launch_probe_fast(a, st);
     k_probe<<<(unsigned)((n + 127) / 128), 128, 0, st>>>(a);
     return cudaGetLastError();

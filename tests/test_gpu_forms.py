@@ -79,3 +79,32 @@ def test_set_sizes(culsh, Q, D, K):
     st.set_tuning(dense_min=1 << 30)   # no dense queries: the item kernels take all
     st.search(Qm, dataset=X)
     _check(st, want, 1, Q, 1)
+
+
+@pytest.mark.parametrize("M,T,Q", [(1, 1, 9), (1, 6, 9), (8, 2, 200), (8, 16, 40), (12, 33, 100), (16, 64, 30),
+                                   (16, 64, 20000), (15, 5, 1023), (15, 5, 1025), (17, 16, 40)])
+@pytest.mark.parametrize("ties", [False, True])
+def test_warp_probe(culsh, M, T, Q, ties):
+    """Query buckets, counts and results when the probe takes a warp per (table,
+    query) pair, around the pair count up to which it does; with ties, many of
+    a query's boundary distances are equal (the reference's heap order)."""
+    rng = np.random.default_rng(100 * M + T)
+    N, D, L, K = 2000, 10, 5, 4
+    if ties:
+        X = rng.integers(-3, 4, (N, D)).astype(np.float32)
+        Qm = rng.integers(-3, 4, (Q, D)).astype(np.float32)
+        A = rng.integers(-1, 2, (L, M, D)).astype(np.float32)
+        b = np.zeros((L, M), np.float32)
+        W = 4.0
+    else:
+        X = rng.normal(0, 1, (N, D)).astype(np.float32)
+        Qm = rng.normal(0, 1, (Q, D)).astype(np.float32)
+        A = rng.normal(0, 1, (L, M, D)).astype(np.float32)
+        W = 3.0
+        b = (rng.random((L, M)) * W).astype(np.float32)
+    want = oracle.search(oracle.build_index(X, A, b, W), X, Qm, K, T)
+    ht = _index(culsh, X, A, b, W)
+    st = culsh.SearchTables()
+    st.reset(ht, K, T)
+    st.search(Qm, dataset=X)
+    _check(st, want, L, Q, T)

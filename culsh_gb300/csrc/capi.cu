@@ -191,6 +191,14 @@ struct culsh_index {
     DevBuf<float> ws_anorm, ws_xnorm;
     DevBuf<ProjectState> ws_pstate;
     PinBuf<float> h_norms;
+    // pinned staging of a build's small host arrays (its copies neither block nor
+    // outlive the build), and of what it reads back
+    PinBuf<unsigned char> h_stage;
+    size_t h_stage_used = 0;
+    PinBuf<unsigned int> h_relist_cnt, h_nb;
+    PinBuf<ProjectState> h_pstate;
+    PinBuf<int32_t> h_range;    // [2][L*M] code ranges
+    PinBuf<int> h_err;
     double tc_predicted_open = 0.0;   // predicted share of codes the tensor-core bound leaves open
     DevBuf<uint32_t> maxb;
     PinBuf<uint32_t> h_maxb;
@@ -203,7 +211,6 @@ struct culsh_index {
     cudaEvent_t bev[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};   // build stage boundaries
     bool built_once = false;
     DevBuf<uint32_t> ws_keys[2], ws_low, ws_vals, ws_hist, ws_base, ws_status, ws_tcnt, ws_toff, ws_nb;
-    PinBuf<uint32_t> h_sort_hist;
     DevBuf<unsigned long long> ws_run_pos;
     DevBuf<uint32_t> ws_run_len;
     DevBuf<unsigned int> ws_run_cnt;
@@ -330,7 +337,6 @@ void clear_index_state(culsh_index* ix) {
     ix->h_codes.clear();
     ix->x_src = nullptr;
     ix->x_borrow = nullptr;
-    ix->proj_on_dev = false;
     ix->xb_valid = false;
     ix->kx_valid = false;
     ix->big_valid = false;
@@ -355,10 +361,33 @@ int upload_projection(culsh_index* ix, cudaStream_t st) {
     return CULSH_OK;
 }
 
+// Copies a small host array to the device through the pinned staging (pageable
+// where that is full).
+int stage_copy(culsh_index* ix, void* dst, const void* src, size_t bytes, cudaStream_t st) {
+    const size_t at = (ix->h_stage_used + 15) & ~size_t(15);
+    if (ix->h_stage.p && at + bytes <= ix->h_stage.n) {
+        std::memcpy(ix->h_stage.p + at, src, bytes);
+        src = ix->h_stage.p + at;
+        ix->h_stage_used = at + bytes;
+    }
+    CU_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st));
+    return CULSH_OK;
+}
+
+// Empties the staging and makes room for a build's or load's arrays. Nothing
+// staged earlier is still being copied: both end with their stream drained.
+int stage_begin(culsh_index* ix) {
+    const size_t LM = (size_t)ix->L * ix->M, L1 = (size_t)ix->L + 1;
+    CU_TRY(ix->h_stage.reserve(40 * LM + 40 * L1 + 1024));
+    ix->h_stage_used = 0;
+    return CULSH_OK;
+}
+
 int read_err_flag(culsh_index* ix, cudaStream_t st, const char* what) {
-    int h = 0;
-    CU_TRY(cudaMemcpyAsync(&h, ix->err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+    CU_TRY(ix->h_err.reserve(1));
+    CU_TRY(cudaMemcpyAsync(ix->h_err.p, ix->err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
     CU_TRY(cudaStreamSynchronize(st));
+    const int h = *ix->h_err.p;
     if (h & kErrNonFinite) return fail(CULSH_ERR_NUMERIC, "%s: a projection is not finite (NaN/Inf in the data?)", what);
     if (h & kErrCodeRange) return fail(CULSH_ERR_NUMERIC, "%s: a bucket code exceeds the int32 range", what);
     if (h & kErrNotIntegral) return fail(CULSH_ERR_FORMAT, "%s: a bucket code is not an integer", what);
@@ -424,10 +453,8 @@ int upload_layout(culsh_index* ix, cudaStream_t st) {
     CU_TRY(ix->foff.reserve(LM));
     CU_TRY(ix->cmin.reserve(LM));
     CU_TRY(ix->cmax.reserve(LM));
-    CU_TRY(cudaMemcpyAsync(ix->fbits.p, ix->h_fbits.data(), LM, cudaMemcpyHostToDevice, st));
-    CU_TRY(cudaMemcpyAsync(ix->foff.p, ix->h_foff.data(), LM * 2, cudaMemcpyHostToDevice, st));
-    CU_TRY(cudaMemcpyAsync(ix->cmin.p, ix->h_cmin.data(), LM * 4, cudaMemcpyHostToDevice, st));
-    CU_TRY(cudaMemcpyAsync(ix->cmax.p, ix->h_cmax.data(), LM * 4, cudaMemcpyHostToDevice, st));
+    TRY(stage_copy(ix, ix->fbits.p, ix->h_fbits.data(), LM, st));
+    TRY(stage_copy(ix, ix->foff.p, ix->h_foff.data(), LM * 2, st));
     std::vector<unsigned long long> unit(2 * LM, 0ull);
     for (size_t c = 0; c < LM; ++c) {
         const int off = ix->h_foff[c];
@@ -435,12 +462,11 @@ int upload_layout(culsh_index* ix, cudaStream_t st) {
         else if (off < 128) unit[2 * c + 1] = 1ull << (off - 64);
     }
     CU_TRY(ix->funit.reserve(2 * LM));
-    CU_TRY(cudaMemcpyAsync(ix->funit.p, unit.data(), 16 * LM, cudaMemcpyHostToDevice, st));
+    TRY(stage_copy(ix, ix->funit.p, unit.data(), 16 * LM, st));
     std::vector<unsigned long long> rm(LM);
     for (size_t c = 0; c < LM; ++c) rm[c] = field_mult((int)c);
     CU_TRY(ix->rmul.reserve(LM));
-    CU_TRY(cudaMemcpyAsync(ix->rmul.p, rm.data(), 8 * LM, cudaMemcpyHostToDevice, st));
-    CU_TRY(cudaStreamSynchronize(st));   // `unit` and `rm` are pageable temporaries
+    TRY(stage_copy(ix, ix->rmul.p, rm.data(), 8 * LM, st));
     return CULSH_OK;
 }
 
@@ -461,8 +487,8 @@ int build_hash(culsh_index* ix, cudaStream_t st) {
     CU_TRY(ix->hoff.reserve(L + 1));
     CU_TRY(ix->hmask.reserve(L));
     CU_TRY(ix->hslots.reserve(ix->h_hoff[L]));
-    CU_TRY(cudaMemcpyAsync(ix->hoff.p, ix->h_hoff.data(), 8 * (L + 1), cudaMemcpyHostToDevice, st));
-    CU_TRY(cudaMemcpyAsync(ix->hmask.p, ix->h_hmask.data(), 4 * L, cudaMemcpyHostToDevice, st));
+    TRY(stage_copy(ix, ix->hoff.p, ix->h_hoff.data(), 8 * (L + 1), st));
+    TRY(stage_copy(ix, ix->hmask.p, ix->h_hmask.data(), 4 * L, st));
     CU_TRY(cudaMemsetAsync(ix->hslots.p, 0xFF, 8 * ix->h_hoff[L], st));
     // Filter words per table: a power of two holding 8 to 16 bits per key.
     ix->h_fl_off.assign(L + 1, 0);
@@ -477,8 +503,8 @@ int build_hash(culsh_index* ix, cudaStream_t st) {
     CU_TRY(ix->fl_off.reserve(L + 1));
     CU_TRY(ix->fl_mask.reserve(L));
     CU_TRY(ix->filt.reserve(ix->h_fl_off[L]));
-    CU_TRY(cudaMemcpyAsync(ix->fl_off.p, ix->h_fl_off.data(), 8 * (L + 1), cudaMemcpyHostToDevice, st));
-    CU_TRY(cudaMemcpyAsync(ix->fl_mask.p, flm.data(), 4 * L, cudaMemcpyHostToDevice, st));
+    TRY(stage_copy(ix, ix->fl_off.p, ix->h_fl_off.data(), 8 * (L + 1), st));
+    TRY(stage_copy(ix, ix->fl_mask.p, flm.data(), 4 * L, st));
     CU_TRY(cudaMemsetAsync(ix->filt.p, 0, 4 * ix->h_fl_off[L], st));
     CU_TRY(launch_hash_build(ix->boff.p, ix->ukeys.p, L, ix->M, ix->KW, maxB, ix->foff.p, ix->fbits.p, ix->rmul.p,
                              ix->hoff.p, ix->hmask.p, ix->hslots.p, ix->filt.p, ix->fl_off.p, ix->fl_mask.p,
@@ -520,9 +546,10 @@ int project_tensor_cores(culsh_index* ix, const float* dX, cudaStream_t st, bool
     CU_TRY(launch_project_sample(dX, N, D, ns, ix->dA.p, LM, ix->ws_xnorm.p, ix->ws_anorm.p, ix->ws_pstate.p, st));
     CU_TRY(cudaMemcpyAsync(ix->h_norms.p, ix->ws_anorm.p, 4 * (size_t)LM, cudaMemcpyDeviceToHost, st));
     CU_TRY(cudaMemcpyAsync(ix->h_norms.p + LM, ix->ws_xnorm.p, 4 * (size_t)ns, cudaMemcpyDeviceToHost, st));
-    ProjectState ps{};
-    CU_TRY(cudaMemcpyAsync(&ps, ix->ws_pstate.p, sizeof(ps), cudaMemcpyDeviceToHost, st));
+    CU_TRY(ix->h_pstate.reserve(1));
+    CU_TRY(cudaMemcpyAsync(ix->h_pstate.p, ix->ws_pstate.p, sizeof(ProjectState), cudaMemcpyDeviceToHost, st));
     CU_TRY(cudaStreamSynchronize(st));
+    ProjectState ps = *ix->h_pstate.p;
     // Bound on |tensor-core sum - canonical FP32 chain| per unit of sum|x||a|
     // (bounded by |x|_2 |a|_2): fp16 split residue, one rounding per summed
     // large product and, at 2^-10 of it, per small one (all products alike in
@@ -556,63 +583,67 @@ int project_tensor_cores(culsh_index* ix, const float* dX, cudaStream_t st, bool
                           st));
     const size_t nx = (size_t)N * p.Dp;
     CU_TRY(ix->ws_xh.reserve(nx));
-    // The low parts are made when the sample has one; data that are inexact
-    // elsewhere only, or whose magnitudes the sample's scale takes out of the
-    // fp16 range, are converted again.
-    for (int attempt = 0;; ++attempt) {
-        if (lo) CU_TRY(ix->ws_xl.reserve(nx));
-        CU_TRY(launch_split_rows(dX, N, D, p.Dp, kappa, ix->ws_xh.p, lo ? ix->ws_xl.p : nullptr, ix->ws_xnorm.p,
-                                 ix->ws_pstate.p, attempt > 0, st));
-        CU_TRY(cudaMemcpyAsync(&ps, ix->ws_pstate.p, sizeof(ps), cudaMemcpyDeviceToHost, st));
-        CU_TRY(cudaStreamSynchronize(st));
-        if (ps.flags & 2) return CULSH_OK;   // non-finite data: the SIMT kernel reports it
-        if (attempt == 2 && (ps.flags & 4)) return CULSH_OK;
-        if (!(ps.flags & 4) && (lo || !(ps.flags & 1))) break;
-        lo = lo || (ps.flags & 1);
-        kappa = kappa_for(lo);
-        CU_TRY(cudaMemsetAsync(&ix->ws_pstate.p->flags, 0, sizeof(int), st));
-    }
-    // the accumulators' scale and its reciprocal stay well inside the float range
-    if (!(ps.sx * ps.sa > 1e-25f && ps.sx * ps.sa < 1e25f && ix->W > 1e-10f && ix->W < 1e10f)) return CULSH_OK;
-    const int need_lo = lo ? 1 : 0;
-    ix->tc_need_lo = need_lo;
     // One recomputation region per CTA, sized for 1/6 of its codes.
     const unsigned long long cap = ((unsigned long long)N * LM / 6) / p.grid + 4096;
     CU_TRY(ix->ws_relist.reserve(cap * p.grid));
     CU_TRY(ix->ws_relist_cnt.reserve(p.grid));
+    CU_TRY(ix->h_relist_cnt.reserve(p.grid));
     CU_TRY(ix->ws_pmin.reserve((size_t)p.grid * LM));
     CU_TRY(ix->ws_pmax.reserve((size_t)p.grid * LM));
-    if (stream)
-        CU_TRY(launch_project_tc_stream(sp, need_lo, N, D, LM, ix->ws_xh.p, ix->ws_xl.p, ix->ws_ah.p, ix->ws_al.p,
-                                        ix->db.p, ix->ws_anorm.p, ix->ws_xnorm.p, ix->ws_pstate.p, ix->W, kappa,
-                                        ix->ws_codes.p, ix->ws_pmin.p, ix->ws_pmax.p, ix->ws_relist.p, cap,
-                                        ix->ws_relist_cnt.p, ix->err.p, st));
-    else
-        CU_TRY(launch_project_tc(rp, need_lo, N, D, LM, ix->ws_xh.p, ix->ws_xl.p, ix->ws_ah.p, ix->ws_al.p, ix->db.p,
-                                 ix->ws_anorm.p, ix->ws_xnorm.p, ix->ws_pstate.p, ix->W, kappa, ix->ws_codes.p,
-                                 ix->ws_pmin.p, ix->ws_pmax.p, ix->ws_relist.p, cap, ix->ws_relist_cnt.p, ix->err.p, st));
-    CU_TRY(launch_minmax_reduce(ix->ws_pmin.p, ix->ws_pmax.p, p.grid, LM, ix->cmin.p, ix->cmax.p, st));
-    std::vector<unsigned int> cnt(p.grid);
-    int err = 0;
-    CU_TRY(cudaMemcpyAsync(cnt.data(), ix->ws_relist_cnt.p, 4 * p.grid, cudaMemcpyDeviceToHost, st));
-    CU_TRY(cudaMemcpyAsync(&err, ix->err.p, 4, cudaMemcpyDeviceToHost, st));
-    CU_TRY(cudaStreamSynchronize(st));
-    unsigned long long nre = 0;
-    bool overflow = false;
-    for (unsigned int c : cnt) {
-        nre += c;
-        overflow |= c > cap;
-    }
-    if (err != 0 || overflow) {
-        CU_TRY(cudaMemsetAsync(ix->err.p, 0, sizeof(int), st));
-        return CULSH_OK;   // fall back to the SIMT kernel
-    }
-    if (nre)
+    CU_TRY(ix->h_range.reserve(2 * (size_t)LM));
+    CU_TRY(ix->h_err.reserve(1));
+    // The low parts are made when the sample has one. Everything up to the
+    // recomputed codes and their ranges is enqueued on that assumption and
+    // judged after one wait; data that are inexact elsewhere only, or whose
+    // magnitudes the sample's scale takes out of the fp16 range, run again.
+    for (int attempt = 0;; ++attempt) {
+        // the accumulators' scale and its reciprocal stay well inside the float range
+        if (!(ps.sx * ps.sa > 1e-25f && ps.sx * ps.sa < 1e25f && ix->W > 1e-10f && ix->W < 1e10f)) return CULSH_OK;
+        if (lo) CU_TRY(ix->ws_xl.reserve(nx));
+        CU_TRY(launch_split_rows(dX, N, D, p.Dp, kappa, ix->ws_xh.p, lo ? ix->ws_xl.p : nullptr, ix->ws_xnorm.p,
+                                 ix->ws_pstate.p, attempt > 0, st));
+        if (stream)
+            CU_TRY(launch_project_tc_stream(sp, lo, N, D, LM, ix->ws_xh.p, ix->ws_xl.p, ix->ws_ah.p, ix->ws_al.p,
+                                            ix->db.p, ix->ws_anorm.p, ix->ws_xnorm.p, ix->ws_pstate.p, ix->W, kappa,
+                                            ix->ws_codes.p, ix->ws_pmin.p, ix->ws_pmax.p, ix->ws_relist.p, cap,
+                                            ix->ws_relist_cnt.p, ix->err.p, st));
+        else
+            CU_TRY(launch_project_tc(rp, lo, N, D, LM, ix->ws_xh.p, ix->ws_xl.p, ix->ws_ah.p, ix->ws_al.p, ix->db.p,
+                                     ix->ws_anorm.p, ix->ws_xnorm.p, ix->ws_pstate.p, ix->W, kappa, ix->ws_codes.p,
+                                     ix->ws_pmin.p, ix->ws_pmax.p, ix->ws_relist.p, cap, ix->ws_relist_cnt.p, ix->err.p,
+                                     st));
+        CU_TRY(launch_minmax_reduce(ix->ws_pmin.p, ix->ws_pmax.p, p.grid, LM, ix->cmin.p, ix->cmax.p, st));
         CU_TRY(launch_tc_recompute(dX, N, D, LM, ix->dA.p, ix->db.p, ix->W, ix->ws_relist.p, cap, ix->ws_relist_cnt.p,
                                    p.grid, ix->ws_codes.p, ix->cmin.p, ix->cmax.p, ix->err.p, st));
-    ix->tc_recomputed = (long long)nre;
-    *done = true;
-    return CULSH_OK;
+        CU_TRY(cudaMemcpyAsync(ix->h_pstate.p, ix->ws_pstate.p, sizeof(ProjectState), cudaMemcpyDeviceToHost, st));
+        CU_TRY(cudaMemcpyAsync(ix->h_relist_cnt.p, ix->ws_relist_cnt.p, 4 * p.grid, cudaMemcpyDeviceToHost, st));
+        CU_TRY(cudaMemcpyAsync(ix->h_range.p, ix->cmin.p, 4 * (size_t)LM, cudaMemcpyDeviceToHost, st));
+        CU_TRY(cudaMemcpyAsync(ix->h_range.p + LM, ix->cmax.p, 4 * (size_t)LM, cudaMemcpyDeviceToHost, st));
+        CU_TRY(cudaMemcpyAsync(ix->h_err.p, ix->err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+        CU_TRY(cudaStreamSynchronize(st));
+        ps = *ix->h_pstate.p;
+        unsigned long long nre = 0;
+        bool overflow = false;
+        for (int r = 0; r < p.grid; ++r) {
+            nre += ix->h_relist_cnt.p[r];
+            overflow |= ix->h_relist_cnt.p[r] > cap;
+        }
+        const bool again = (ps.flags & 4) || (!lo && (ps.flags & 1));
+        if ((ps.flags & 2) || overflow || *ix->h_err.p != 0 || again) {
+            CU_TRY(cudaMemsetAsync(ix->err.p, 0, sizeof(int), st));
+            // non-finite data (the SIMT kernel reports it), too many open codes,
+            // a code out of range or a wait that gave up: the SIMT kernel
+            if ((ps.flags & 2) || !again || attempt == 2) return CULSH_OK;
+            lo = lo || (ps.flags & 1);
+            kappa = kappa_for(lo);
+            CU_TRY(cudaMemsetAsync(&ix->ws_pstate.p->flags, 0, sizeof(int), st));
+            continue;
+        }
+        ix->tc_need_lo = lo ? 1 : 0;
+        ix->tc_recomputed = (long long)nre;
+        *done = true;
+        return CULSH_OK;
+    }
 }
 
 // Packs every point's key and orders every table's points by it (ties by id),
@@ -620,13 +651,17 @@ int project_tensor_cores(culsh_index* ix, const float* dX, cudaStream_t st, bool
 // two to four words (sort_top_word) take the digit passes over the top word
 // alone (moving 8 bytes per point a pass instead of 4 (KW + 1)) and then order
 // each run of equal top words by (lower words, id); a run longer than
-// run_max_len() or more runs than the lists hold sends the build through the
-// passes over every word instead. On return *sk describes the sorted keys and
-// ix->ids holds the sorted ids.
-int sort_keys(culsh_index* ix, int N, int passes, cudaStream_t st, SortedKeys* sk) {
+// run_max_len() or more runs than the lists hold is counted in h_run_cnt[3]
+// (valid once the stream has been waited for): the caller then sorts again with
+// all_words, by passes over every word. On return *sk describes the sorted keys
+// and ix->ids holds the sorted ids.
+int sort_keys(culsh_index* ix, int N, int passes, bool all_words, cudaStream_t st, SortedKeys* sk) {
     const int L = ix->L, KW = ix->KW;
     const size_t LN = (size_t)L * N;
-    const bool top_first = passes == 4 * KW && sort_top_word(KW, 32 * KW);
+    const bool top_first = !all_words && passes == 4 * KW && sort_top_word(KW, 32 * KW);
+    // digits below every table's lowest field are zero: no pass
+    int first_pass = passes;
+    for (int l = 0; l < L; ++l) first_pass = std::min(first_pass, ix->h_foff[(size_t)(l + 1) * ix->M - 1] / 8);
     const int lw = low_row_words(KW);
     CU_TRY(ix->ws_vals.reserve(LN));
     CU_TRY(ix->ids.reserve(LN));
@@ -639,7 +674,8 @@ int sort_keys(culsh_index* ix, int N, int passes, cudaStream_t st, SortedKeys* s
     CU_TRY(ix->ws_hist.reserve((size_t)L * hp * 256));
     CU_TRY(ix->ws_base.reserve((size_t)L * hp * 256));
     CU_TRY(ix->ws_status.reserve(sort_status_words(N, L)));
-    CU_TRY(ix->h_sort_hist.reserve((size_t)L * hp * 256));
+    CU_TRY(ix->h_run_cnt.reserve(4));
+    ix->h_run_cnt.p[3] = 0;
     CU_TRY(cudaEventRecord(ix->bev[2], st));
     SortBuffers sb;
     sb.keys[0] = ix->ws_keys[0].p;
@@ -650,12 +686,10 @@ int sort_keys(culsh_index* ix, int N, int passes, cudaStream_t st, SortedKeys* s
     sb.base = ix->ws_base.p;
     sb.status = ix->ws_status.p;
     sb.err = ix->err.p;
-    sb.h_hist = ix->h_sort_hist.p;
-    sb.h_hist_words = ix->h_sort_hist.n;
     ix->sort_form = 0;
     bool alt = false;
     if (top_first) {
-        CU_TRY(run_segmented_sort(sb, N, L, 1, 4, &alt, st));
+        CU_TRY(run_segmented_sort(sb, N, L, 1, 4, 0, &alt, st));
         const uint32_t* top = sb.keys[alt ? 1 : 0];
         if (alt) ix->ids.swap(ix->ws_vals);
         const unsigned int tcap = (unsigned int)std::min<size_t>(LN / 3 + 1, (size_t)1 << 25);
@@ -665,7 +699,6 @@ int sort_keys(culsh_index* ix, int N, int passes, cudaStream_t st, SortedKeys* s
         CU_TRY(ix->ws_run_pos.reserve(rcap));
         CU_TRY(ix->ws_run_len.reserve(rcap));
         CU_TRY(ix->ws_run_cnt.reserve(4));
-        CU_TRY(ix->h_run_cnt.reserve(4));
         RunLists rl;
         rl.tpos = ix->ws_run_pos.p;
         rl.tlen = ix->ws_run_len.p;
@@ -678,27 +711,14 @@ int sort_keys(culsh_index* ix, int N, int passes, cudaStream_t st, SortedKeys* s
         rl.lcap = lcap;
         rl.cnt = ix->ws_run_cnt.p;
         CU_TRY(launch_run_find(top, N, L, KW, ix->ws_low.p, ix->ids.p, rl, st));
+        CU_TRY(launch_run_sorts(rl, N, L, KW, ix->ws_low.p, ix->ids.p, st));
         CU_TRY(cudaMemcpyAsync(ix->h_run_cnt.p, rl.cnt, 4 * sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
-        CU_TRY(cudaStreamSynchronize(st));
-        const unsigned int* hc = ix->h_run_cnt.p;
-        if (hc[3] == 0) {
-            CU_TRY(launch_run_sorts(rl, hc, N, L, KW, ix->ws_low.p, ix->ids.p, st));
-            ix->sort_form = 1;
-            *sk = SortedKeys{top, ix->ws_low.p, ix->ids.p, lw};
-            return CULSH_OK;
-        }
-        // a run too long to order in shared memory: repack, sort every word
-        ix->sort_form = 2;
-        CU_TRY(ix->ws_keys[0].reserve(LN * KW));
-        CU_TRY(ix->ws_keys[1].reserve(LN * KW));
-        CU_TRY(launch_pack_keys(ix->ws_codes.p, N, L, ix->M, KW, ix->cmin.p, ix->fbits.p, ix->foff.p, ix->ws_keys[0].p,
-                                ix->ids.p, nullptr, 0, st));
-        sb.keys[0] = ix->ws_keys[0].p;
-        sb.keys[1] = ix->ws_keys[1].p;
-        sb.vals[0] = ix->ids.p;
-        sb.vals[1] = ix->ws_vals.p;
+        ix->sort_form = 1;
+        *sk = SortedKeys{top, ix->ws_low.p, ix->ids.p, lw};
+        return CULSH_OK;
     }
-    CU_TRY(run_segmented_sort(sb, N, L, KW, passes, &alt, st));
+    if (all_words && sort_top_word(KW, 32 * KW)) ix->sort_form = 2;
+    CU_TRY(run_segmented_sort(sb, N, L, KW, passes, first_pass, &alt, st));
     if (alt) ix->ids.swap(ix->ws_vals);
     *sk = SortedKeys{sb.keys[alt ? 1 : 0], nullptr, ix->ids.p, 0};
     return CULSH_OK;
@@ -712,6 +732,7 @@ int build_device(culsh_index* ix, const float* dX, cudaStream_t st, FILE* dbg) {
     for (auto& e : ix->bev)
         if (!e) CU_TRY(cudaEventCreate(&e));
     CU_TRY(cudaEventRecord(ix->bev[0], st));
+    TRY(stage_begin(ix));
     TRY(upload_projection(ix, st));
     CU_TRY(ix->err.reserve(1));
     CU_TRY(cudaMemsetAsync(ix->err.p, 0, sizeof(int), st));
@@ -728,11 +749,14 @@ int build_device(culsh_index* ix, const float* dX, cudaStream_t st, FILE* dbg) {
                                    ix->ws_pmin.p, ix->ws_pmax.p, ix->err.p, st));
         CU_TRY(launch_minmax_reduce(ix->ws_pmin.p, ix->ws_pmax.p, gx, LM, ix->cmin.p, ix->cmax.p, st));
     }
-    ix->h_cmin.resize(LM);
-    ix->h_cmax.resize(LM);
-    CU_TRY(cudaMemcpyAsync(ix->h_cmin.data(), ix->cmin.p, 4 * LM, cudaMemcpyDeviceToHost, st));
-    CU_TRY(cudaMemcpyAsync(ix->h_cmax.data(), ix->cmax.p, 4 * LM, cudaMemcpyDeviceToHost, st));
-    TRY(read_err_flag(ix, st, "index"));
+    if (!tc_done) {
+        CU_TRY(ix->h_range.reserve(2 * (size_t)LM));
+        CU_TRY(cudaMemcpyAsync(ix->h_range.p, ix->cmin.p, 4 * (size_t)LM, cudaMemcpyDeviceToHost, st));
+        CU_TRY(cudaMemcpyAsync(ix->h_range.p + LM, ix->cmax.p, 4 * (size_t)LM, cudaMemcpyDeviceToHost, st));
+        TRY(read_err_flag(ix, st, "index"));
+    }
+    ix->h_cmin.assign(ix->h_range.p, ix->h_range.p + LM);
+    ix->h_cmax.assign(ix->h_range.p + LM, ix->h_range.p + 2 * LM);
     int passes = 0;
     TRY(compute_layout(ix, &passes));
     TRY(upload_layout(ix, st));
@@ -745,18 +769,21 @@ int build_device(culsh_index* ix, const float* dX, cudaStream_t st, FILE* dbg) {
 
     // Pack keys and sort all tables at once (records bev[2] between the two).
     SortedKeys skeys{};
-    TRY(sort_keys(ix, N, passes, st, &skeys));
-    CU_TRY(cudaEventRecord(ix->bev[3], st));
-
-    // Run-length bucketing.
     const int tiles = (N + 4095) / 4096;
     CU_TRY(ix->ws_tcnt.reserve((size_t)L * tiles));
     CU_TRY(ix->ws_toff.reserve((size_t)L * tiles));
     CU_TRY(ix->ws_nb.reserve(L));
-    CU_TRY(launch_rl_count(skeys, N, L, ix->KW, ix->ws_tcnt.p, ix->ws_toff.p, ix->ws_nb.p, st));
-    ix->buckets.assign(L, 0);
-    CU_TRY(cudaMemcpyAsync(ix->buckets.data(), ix->ws_nb.p, 4 * L, cudaMemcpyDeviceToHost, st));
-    CU_TRY(cudaStreamSynchronize(st));
+    CU_TRY(ix->h_nb.reserve(L));
+    for (int all_words = 0; all_words < 2; ++all_words) {
+        TRY(sort_keys(ix, N, passes, all_words != 0, st, &skeys));
+        CU_TRY(cudaEventRecord(ix->bev[3], st));
+        // Run-length bucketing.
+        CU_TRY(launch_rl_count(skeys, N, L, ix->KW, ix->ws_tcnt.p, ix->ws_toff.p, ix->ws_nb.p, st));
+        CU_TRY(cudaMemcpyAsync(ix->h_nb.p, ix->ws_nb.p, 4 * L, cudaMemcpyDeviceToHost, st));
+        CU_TRY(cudaStreamSynchronize(st));
+        if (ix->h_run_cnt.p[3] == 0) break;   // every run was ordered
+    }
+    ix->buckets.assign(ix->h_nb.p, ix->h_nb.p + L);
     ix->h_boff.assign(L + 1, 0);
     int64_t maxB = 0;
     for (int l = 0; l < L; ++l) {
@@ -765,7 +792,7 @@ int build_device(culsh_index* ix, const float* dX, cudaStream_t st, FILE* dbg) {
     }
     const uint64_t totB = ix->h_boff[L];
     CU_TRY(ix->boff.reserve(L + 1));
-    CU_TRY(cudaMemcpyAsync(ix->boff.p, ix->h_boff.data(), 8 * (L + 1), cudaMemcpyHostToDevice, st));
+    TRY(stage_copy(ix, ix->boff.p, ix->h_boff.data(), 8 * (L + 1), st));
     CU_TRY(ix->starts.reserve(totB));
     CU_TRY(ix->sizes.reserve(totB));
     CU_TRY(ix->ukeys.reserve(totB * ix->KW));
@@ -828,6 +855,7 @@ int ensure_device(culsh_index* ix, cudaStream_t st) {
     if (!ix->host_valid) return fail(CULSH_ERR_STATE, "No index: have you performed indexing or loaded a file???");
     const int L = ix->L, N = ix->N, M = ix->M, LM = L * M;
     ix->big_valid = false;
+    TRY(stage_begin(ix));
     TRY(upload_projection(ix, st));
     CU_TRY(ix->err.reserve(1));
     CU_TRY(cudaMemsetAsync(ix->err.p, 0, sizeof(int), st));
@@ -1774,6 +1802,7 @@ static int reset_common(culsh_index* ix, int N, int D, int L, int M, float W) {
     ix->A.assign((size_t)L * M * D, 0.0f);
     ix->b.assign((size_t)L * M, 0.0f);
     ix->has_proj = false;
+    ix->proj_on_dev = false;
     return CULSH_OK;
 }
 

@@ -233,12 +233,11 @@ struct SortBuffers {
     uint32_t* base;      // [L][passes][256]
     uint32_t* status;    // [L*tiles][256] + counter
     int* err;
-    uint32_t* h_hist = nullptr;   // pinned host copy of hist (allocated per call when absent or short)
-    size_t h_hist_words = 0;
 };
 size_t sort_status_words(int64_t N, int L);
-cudaError_t run_segmented_sort(SortBuffers& sb, int64_t N, int L, int KW, int passes, bool* result_in_alt,
-                               cudaStream_t st);
+// Digits below first_pass are zero in every key and get no pass.
+cudaError_t run_segmented_sort(SortBuffers& sb, int64_t N, int L, int KW, int passes, int first_pass,
+                               bool* result_in_alt, cudaStream_t st);
 
 // Top-word-first ordering (sort.cu): after the digit passes over the top key
 // word, find the runs of equal top words and order each run by (lower words,
@@ -257,8 +256,8 @@ struct RunLists {
 };
 cudaError_t launch_run_find(const uint32_t* top, int64_t N, int L, int KW, const uint32_t* low, uint32_t* ids,
                             const RunLists& rl, cudaStream_t st);
-cudaError_t launch_run_sorts(const RunLists& rl, const unsigned int* counts, int64_t N, int L, int KW, const uint32_t* low,
-                             uint32_t* ids, cudaStream_t st);
+cudaError_t launch_run_sorts(const RunLists& rl, int64_t N, int L, int KW, const uint32_t* low, uint32_t* ids,
+                             cudaStream_t st);
 int run_max_len();
 
 // Sorted keys of all tables: KW arrays of L*N words, or (low != nullptr) the

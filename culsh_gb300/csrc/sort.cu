@@ -900,10 +900,10 @@ size_t sort_status_words(int64_t N, int L) {
     return (size_t)(L * tiles * 256 + 32);
 }
 
-cudaError_t run_segmented_sort(SortBuffers& sb, int64_t N, int L, int KW, int passes, bool* result_in_alt,
-                               cudaStream_t st) {
+cudaError_t run_segmented_sort(SortBuffers& sb, int64_t N, int L, int KW, int passes, int first_pass,
+                               bool* result_in_alt, cudaStream_t st) {
     *result_in_alt = false;
-    if (passes <= 0 || N <= 1) return cudaSuccess;
+    if (passes <= first_pass || N <= 1) return cudaSuccess;
     const int tiles = (int)((N + SP_TILE - 1) / SP_TILE);
     cudaError_t e;
     if ((e = cudaMemsetAsync(sb.hist, 0, sizeof(uint32_t) * L * passes * 256, st)) != cudaSuccess) return e;
@@ -911,30 +911,10 @@ cudaError_t run_segmented_sort(SortBuffers& sb, int64_t N, int L, int KW, int pa
     k_sort_hist<<<hg, NT, passes * 256 * sizeof(uint32_t), st>>>(sb.keys[0], N, L, passes, sb.hist);
     k_sort_digit_base<<<L * passes, NT, 0, st>>>(sb.hist, sb.base);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    // Skip digit passes that are constant over every table (a stable pass
-    // with one occupied bin is the identity).
-    const size_t hwords = (size_t)L * passes * 256, hbytes = sizeof(uint32_t) * hwords;
-    const bool own = sb.h_hist == nullptr || sb.h_hist_words < hwords;
-    uint32_t* h_hist = own ? nullptr : sb.h_hist;
-    if (own && (e = cudaMallocHost(&h_hist, hbytes)) != cudaSuccess) return e;
-    if ((e = cudaMemcpyAsync(h_hist, sb.hist, hbytes, cudaMemcpyDeviceToHost, st)) == cudaSuccess)
-        e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) {
-        if (own) cudaFreeHost(h_hist);
-        return e;
-    }
     int cur = 0;
     const size_t status_words = sort_status_words(N, L);
     uint32_t* counter = sb.status + (status_words - 32);
-    for (int p = 0; p < passes; ++p) {
-        bool trivial = true;
-        for (int l = 0; l < L && trivial; ++l) {
-            const uint32_t* hp = h_hist + ((size_t)l * passes + p) * 256;
-            int nz = 0;
-            for (int d = 0; d < 256; ++d) nz += hp[d] != 0;
-            trivial = nz <= 1;
-        }
-        if (trivial) continue;
+    for (int p = first_pass; p < passes; ++p) {
         if ((e = cudaMemsetAsync(sb.status, 0, sizeof(uint32_t) * status_words, st)) != cudaSuccess) break;
         k_sort_pass<<<(unsigned)(L * tiles), NT, 0, st>>>(sb.keys[cur], sb.vals[cur], sb.keys[cur ^ 1],
                                                           sb.vals[cur ^ 1], N, L, KW, tiles, p >> 2, (p & 3) * 8,
@@ -942,7 +922,6 @@ cudaError_t run_segmented_sort(SortBuffers& sb, int64_t N, int L, int KW, int pa
         if ((e = cudaGetLastError()) != cudaSuccess) break;
         cur ^= 1;
     }
-    if (own) cudaFreeHost(h_hist);
     *result_in_alt = cur == 1;
     return e;
 }
@@ -964,23 +943,24 @@ cudaError_t launch_run_find(const uint32_t* top, int64_t N, int L, int KW, const
 int run_max_len() { return kRunMax; }
 
 template <int KWL>
-void launch_run_sorts_w(const RunLists& rl, unsigned int ntiny, unsigned int nsmall, unsigned int nlarge, int64_t N,
-                        const uint32_t* low, uint32_t* ids, cudaStream_t st) {
-    const unsigned gt = (unsigned)std::min<unsigned long long>(((unsigned long long)ntiny + NT - 1) / NT, 152 * 16);
-    const unsigned gs = (unsigned)std::min<unsigned long long>(((unsigned long long)nsmall * 32 + NT - 1) / NT, 152 * 32);
-    const unsigned gl = (unsigned)std::min<unsigned int>(nlarge, 152 * 4);
-    if (gt) k_run_sort_tiny<KWL><<<gt, NT, 0, st>>>(rl.tpos, rl.tlen, rl.cnt, rl.tcap, N, low, ids);
-    if (gs) k_run_sort_small<KWL><<<gs, NT, 0, st>>>(rl.spos, rl.slen, rl.cnt, rl.scap, N, low, ids);
-    if (gl) k_run_sort_large<KWL><<<gl, NT, 0, st>>>(rl.lpos, rl.llen, rl.cnt, rl.lcap, N, low, ids);
+void launch_run_sorts_w(const RunLists& rl, int64_t LN, int64_t N, const uint32_t* low, uint32_t* ids, cudaStream_t st) {
+    // the lists' lengths stay on the device: grids for a full device, or fewer
+    // where the keys cannot hold as many runs
+    const unsigned gt = (unsigned)std::min<int64_t>((LN / 3 + NT - 1) / NT + 1, 152 * 16);
+    const unsigned gs = (unsigned)std::min<int64_t>((LN / 9 * 32 + NT - 1) / NT + 1, 152 * 16);
+    const unsigned gl = (unsigned)std::min<int64_t>(LN / 33 + 1, 152 * 4);
+    k_run_sort_tiny<KWL><<<gt, NT, 0, st>>>(rl.tpos, rl.tlen, rl.cnt, rl.tcap, N, low, ids);
+    k_run_sort_small<KWL><<<gs, NT, 0, st>>>(rl.spos, rl.slen, rl.cnt, rl.scap, N, low, ids);
+    k_run_sort_large<KWL><<<gl, NT, 0, st>>>(rl.lpos, rl.llen, rl.cnt, rl.lcap, N, low, ids);
 }
 
-cudaError_t launch_run_sorts(const RunLists& rl, const unsigned int* counts, int64_t N, int L, int KW, const uint32_t* low,
-                             uint32_t* ids, cudaStream_t st) {
-    (void)L;
+cudaError_t launch_run_sorts(const RunLists& rl, int64_t N, int L, int KW, const uint32_t* low, uint32_t* ids,
+                             cudaStream_t st) {
+    const int64_t LN = (int64_t)L * N;
     switch (KW - 1) {
-    case 1: launch_run_sorts_w<1>(rl, counts[0], counts[1], counts[2], N, low, ids, st); break;
-    case 2: launch_run_sorts_w<2>(rl, counts[0], counts[1], counts[2], N, low, ids, st); break;
-    case 3: launch_run_sorts_w<3>(rl, counts[0], counts[1], counts[2], N, low, ids, st); break;
+    case 1: launch_run_sorts_w<1>(rl, LN, N, low, ids, st); break;
+    case 2: launch_run_sorts_w<2>(rl, LN, N, low, ids, st); break;
+    case 3: launch_run_sorts_w<3>(rl, LN, N, low, ids, st); break;
     default: return cudaErrorInvalidValue;
     }
     return cudaGetLastError();

@@ -543,30 +543,37 @@ int project_tensor_cores(culsh_index* ix, const float* dX, cudaStream_t st, bool
     CU_TRY(ix->ws_xnorm.reserve(std::max(N, ns)));
     CU_TRY(ix->ws_pstate.reserve(1));
     CU_TRY(ix->h_norms.reserve(LM + ns));
-    CU_TRY(launch_project_sample(dX, N, D, ns, ix->dA.p, LM, ix->ws_xnorm.p, ix->ws_anorm.p, ix->ws_pstate.p, st));
+    // Bound on |tensor-core sum - canonical FP32 chain| per unit of |x||a|: the
+    // part that falls over d (roundings of the running sums: one a step of the
+    // canonical chain, one per summed large product, all products alike in
+    // the streaming form, whose K slices alternate) and the rest (the fp16
+    // split's residue, the small products' roundings and their sum's share in
+    // the large ones', the steps' width); 1.25 margin.
+    const double u24 = std::ldexp(1.0, -24), u23 = std::ldexp(1.0, -23), u22 = std::ldexp(1.0, -22);
+    float kappa = 0.0f, slope = 0.0f;
+    auto bound_for = [&](int need_lo) {
+        const double split = (need_lo ? 3.1 : 1.05) * u22;
+        const double small = std::ldexp(1.0, -10) * u23;
+        const double falls = D * u24 + (stream ? (need_lo ? 3.0 : 2.0) : 1.0) * D * u23;
+        const double rest = 2 * u24 + split +
+                            (stream ? (need_lo ? 48 : 32) * u23
+                                    : 16 * u23 + ((need_lo ? 2.0 : 1.0) * D + 16) * small + (D + 16) * small);
+        kappa = (float)(1.25 * (falls + rest));
+        slope = (float)(falls / ((falls + rest) * D));
+    };
+    bound_for(0);
+    CU_TRY(launch_project_sample(dX, N, D, ns, ix->dA.p, LM, slope, ix->ws_xnorm.p, ix->ws_anorm.p, ix->ws_pstate.p, st));
     CU_TRY(cudaMemcpyAsync(ix->h_norms.p, ix->ws_anorm.p, 4 * (size_t)LM, cudaMemcpyDeviceToHost, st));
     CU_TRY(cudaMemcpyAsync(ix->h_norms.p + LM, ix->ws_xnorm.p, 4 * (size_t)ns, cudaMemcpyDeviceToHost, st));
     CU_TRY(ix->h_pstate.reserve(1));
     CU_TRY(cudaMemcpyAsync(ix->h_pstate.p, ix->ws_pstate.p, sizeof(ProjectState), cudaMemcpyDeviceToHost, st));
     CU_TRY(cudaStreamSynchronize(st));
     ProjectState ps = *ix->h_pstate.p;
-    // Bound on |tensor-core sum - canonical FP32 chain| per unit of sum|x||a|
-    // (bounded by |x|_2 |a|_2): fp16 split residue, one rounding per summed
-    // large product and, at 2^-10 of it, per small one (all products alike in
-    // the streaming form, whose K slices alternate), the canonical chain's
-    // rounding; 1.25 margin.
-    const double u24 = std::ldexp(1.0, -24), u23 = std::ldexp(1.0, -23), u22 = std::ldexp(1.0, -22);
-    auto kappa_for = [&](int need_lo) {
-        const double split = (need_lo ? 3.1 : 1.05) * u22;
-        const double accum = stream ? ((need_lo ? 3.0 : 2.0) * D + 16) * u23
-                                    : (D + 16) * u23 + ((need_lo ? 2.0 : 1.0) * D + 16) * u23 * std::ldexp(1.0, -10);
-        return (float)(1.25 * ((D + 2) * u24 + split + accum));
-    };
     bool lo = (ps.flags & 8) != 0;
-    float kappa = kappa_for(lo);
+    bound_for(lo);
     {
         // Predicted share of codes the bound leaves open: a code is open when
-        // an integer lies within E / W of its value, E = kappa |x| |a|. Above
+        // an integer lies within E / W of its value, E = kappa |x|_t |a|_t. Above
         // 6 % the FP32 recomputation costs more than the SIMT projection
         // itself, so the SIMT kernel runs. Taken before anything of X's size is
         // converted.
@@ -579,8 +586,6 @@ int project_tensor_cores(culsh_index* ix, const float* dX, cudaStream_t st, bool
     }
     CU_TRY(ix->ws_ah.reserve((size_t)p.LMp * p.Dp));
     CU_TRY(ix->ws_al.reserve((size_t)p.LMp * p.Dp));
-    CU_TRY(launch_split_a(ix->dA.p, LM, p.LMp, D, p.Dp, kappa, ix->ws_ah.p, ix->ws_al.p, ix->ws_anorm.p, ix->ws_pstate.p,
-                          st));
     const size_t nx = (size_t)N * p.Dp;
     CU_TRY(ix->ws_xh.reserve(nx));
     // One recomputation region per CTA, sized for 1/6 of its codes.
@@ -600,7 +605,9 @@ int project_tensor_cores(culsh_index* ix, const float* dX, cudaStream_t st, bool
         // the accumulators' scale and its reciprocal stay well inside the float range
         if (!(ps.sx * ps.sa > 1e-25f && ps.sx * ps.sa < 1e25f && ix->W > 1e-10f && ix->W < 1e10f)) return CULSH_OK;
         if (lo) CU_TRY(ix->ws_xl.reserve(nx));
-        CU_TRY(launch_split_rows(dX, N, D, p.Dp, kappa, ix->ws_xh.p, lo ? ix->ws_xl.p : nullptr, ix->ws_xnorm.p,
+        CU_TRY(launch_split_a(ix->dA.p, LM, p.LMp, D, p.Dp, kappa, slope, ix->ws_ah.p, ix->ws_al.p, ix->ws_anorm.p, ix->ws_pstate.p,
+                              st));
+        CU_TRY(launch_split_rows(dX, N, D, p.Dp, kappa, slope, ix->ws_xh.p, lo ? ix->ws_xl.p : nullptr, ix->ws_xnorm.p,
                                  ix->ws_pstate.p, attempt > 0, st));
         if (stream)
             CU_TRY(launch_project_tc_stream(sp, lo, N, D, LM, ix->ws_xh.p, ix->ws_xl.p, ix->ws_ah.p, ix->ws_al.p,
@@ -635,7 +642,7 @@ int project_tensor_cores(culsh_index* ix, const float* dX, cudaStream_t st, bool
             // a code out of range or a wait that gave up: the SIMT kernel
             if ((ps.flags & 2) || !again || attempt == 2) return CULSH_OK;
             lo = lo || (ps.flags & 1);
-            kappa = kappa_for(lo);
+            bound_for(lo);
             CU_TRY(cudaMemsetAsync(&ix->ws_pstate.p->flags, 0, sizeof(int), st));
             continue;
         }

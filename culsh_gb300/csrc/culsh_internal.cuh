@@ -201,11 +201,11 @@ cudaError_t launch_project_tc_stream(const TcStreamPlan& p, int need_lo, int64_t
                                      cudaStream_t st);
 // Norms of A's columns and of ns rows of X, and both scales; fp16 parts of A and
 // of X (xl null: the high part only; rescale: from X's own maximum).
-cudaError_t launch_project_sample(const float* X, int64_t N, int D, int ns, const float* A, int LM, float* xs,
+cudaError_t launch_project_sample(const float* X, int64_t N, int D, int ns, const float* A, int LM, float slope, float* xs,
                                   float* anorm, ProjectState* ps, cudaStream_t st);
-cudaError_t launch_split_a(const float* A, int LM, int LMp, int D, int Dp, float kappa, void* ah, void* al, float* anorm,
+cudaError_t launch_split_a(const float* A, int LM, int LMp, int D, int Dp, float kappa, float slope, void* ah, void* al, float* anorm,
                            const ProjectState* ps, cudaStream_t st);
-cudaError_t launch_split_rows(const float* X, int64_t N, int D, int Dp, float kappa, void* xh, void* xl, float* xnorm,
+cudaError_t launch_split_rows(const float* X, int64_t N, int D, int Dp, float kappa, float slope, void* xh, void* xl, float* xnorm,
                               ProjectState* ps, bool rescale, cudaStream_t st);
 cudaError_t launch_project_tc(const TcPlan& p, int need_lo, int64_t N, int D, int LM, const void* xh, const void* xl,
                               const void* ah, const void* al, const float* b, const float* anorm, const float* xnorm,

@@ -10,19 +10,25 @@
 // and A = Ah + Al (Xl is skipped when every element is exact in fp16). The
 // tensor cores compute y = Xh*Al' (+ Xl*Ah') + Xh*Ah' with FP32 accumulation
 // in TMEM, the small products first. For each element the distance between y
-// and the canonical sequential FMA chain is bounded by
-// E = kappa * |x|_2 * |a|_2 (Cauchy-Schwarz on sum|x||a|), where kappa covers
-// the split residue (2^-22 per part: fp16 pairs keep 22 bits, bf16 pairs had
-// kept 16), a rounding at every accumulation of the large products (one 2^-23
-// step per product; the small ones accumulate at 2^-11 of that) and the
-// canonical chain's own rounding ((D + 2) * 2^-24), with a 1.25 margin. A window
+// and the canonical sequential FMA chain is bounded by E = kappa * |x|_t * |a|_t, where
+// kappa covers the split residue (2^-22 per part: fp16 pairs keep 22 bits, bf16
+// pairs had kept 16), a rounding at every accumulation of the large products
+// (one 2^-23 step per product; the small ones accumulate at 2^-11 of that) and
+// the canonical chain's own rounding (D + 2 steps of 2^-24), with a 1.25 margin.
+// Both sums run over d in order, so a rounding is relative to the sum so far,
+// which Cauchy-Schwarz bounds by the norms of x's and a's leading parts: an
+// element takes part in the roundings from its own 16-wide step on. Summed over
+// the steps (Cauchy-Schwarz again) that is the product of the weighted norms
+// |x|_t = sqrt(sum t_d x_d^2), t_d = 1 - slope * (d rounded down to 16), where
+// slope * D is the share of kappa that such roundings have. A window
 // test on (y - b) * (1/W) without a division proves a code: when no integer
 // lies within E / W and the test's own rounding of it, every value the
 // canonical chain can take has the same floor. Every other element is
 // appended to a list and recomputed in the canonical order by k_tc_recompute.
 // Codes are therefore bit-identical to the SIMT kernel and the oracle. With
 // bf16 parts in any order 3.8 % of the codes of 1M x 128 integer features at
-// W = 16 were open (0.69 ms of recomputation); now 1.7 %.
+// W = 16 were open (0.69 ms of recomputation), with fp16 parts and plain norms
+// 1.7 % (0.35 ms), now 1.0 % (0.22 ms).
 //
 // Structure: persistent CTAs of 18 warps. Warp 0 issues TMA loads (the
 // projection matrix once, then 128-point X tiles into a 1- or 2-stage ring);
@@ -56,8 +62,8 @@ struct TcArgs {
     int D, Dp, LM, LMp, ntiles, need_lo, stages, tmem_cols;
     float W, kappa;
     const float* b;        // [LM]
-    const float* anorm;    // [LM] upper bounds of |a_c|_2
-    const float* xnorm;    // [N]  upper bounds of |x_n|_2
+    const float* anorm;    // [LM] upper bounds of |a_c|_t
+    const float* xnorm;    // [N]  upper bounds of |x_n|_t
     const ProjectState* ps;   // scales of X and A
     int32_t* codes;        // [LM][N]
     int32_t* pmin;         // [gridDim.x][LM]
@@ -195,7 +201,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     unsigned int* list_top = reinterpret_cast<unsigned int*>(tmem_ptr + 2);
     int32_t* cmin = reinterpret_cast<int32_t*>(tail + 96);   // 16-byte aligned, past the barriers
     int32_t* cmax = cmin + a.LMp;
-    float* s_an = reinterpret_cast<float*>(cmax + a.LMp);     // |a_c|_2 bounds / W
+    float* s_an = reinterpret_cast<float*>(cmax + a.LMp);     // |a_c|_t bounds / W
     float* s_bw = s_an + a.LMp;                                // -b_c / W
     float* s_win = s_bw + a.LMp;                               // the window test's own rounding beside |v|
     uint32_t* s_unsure = reinterpret_cast<uint32_t*>(s_win + a.LMp);   // [8 words][TC_EPI_WARPS * 32] per-thread masks
@@ -482,36 +488,39 @@ __device__ __forceinline__ float project_scale(uint32_t amax_bits) {
 }
 
 // A row (or column of A) of a warp: fp16 parts of row * scale into h and l
-// (either may be null) and its squared norm, rounded up. Lanes hold four
-// consecutive elements where vec (16-byte aligned rows), one otherwise.
-__device__ __forceinline__ void split_row(const float* __restrict__ row, int D, int Dp, float scale, bool vec, __half* h,
-                                          __half* l, float& ss, bool& inexact, float& amax, bool& bad) {
+// (either may be null) and its squared weighted norm (t_d = 1 - slope * (d
+// rounded down to 16)), rounded up. Lanes hold four consecutive elements where
+// vec (16-byte aligned rows), one otherwise.
+__device__ __forceinline__ void split_row(const float* __restrict__ row, int D, int Dp, float scale, float slope,
+                                          bool vec, __half* h, __half* l, float& ss, bool& inexact, float& amax,
+                                          bool& bad) {
     const int lane = threadIdx.x & 31;
     ss = 0.0f;
-    auto part = [&](float x, __half& hi, __half& lo) {
+    auto part = [&](float x, float t, __half& hi, __half& lo) {
         const float xs = x * scale;   // exact but for subnormal results
         hi = __float2half_rn(xs);
         lo = __float2half_rn(__fsub_rn(xs, __half2float(hi)));
         inexact |= (__half_as_ushort(lo) & 0x7FFF) != 0;
         if (fabsf(x) <= FLT_MAX) amax = fmaxf(amax, fabsf(x));
         else bad = true;
-        ss = __fmaf_ru(x, x, ss);
+        ss = __fmaf_ru(__fmul_ru(fabsf(x), t), fabsf(x), ss);
     };
     if (vec) {
         for (int d = 4 * lane; d < Dp; d += 128) {
             const float4 x = d < D ? __ldg(reinterpret_cast<const float4*>(row + d)) : make_float4(0.f, 0.f, 0.f, 0.f);
             __align__(8) __half hh[4], ll[4];
-            part(x.x, hh[0], ll[0]);
-            part(x.y, hh[1], ll[1]);
-            part(x.z, hh[2], ll[2]);
-            part(x.w, hh[3], ll[3]);
+            const float t = __fmaf_ru(-slope, (float)(d & ~15), 1.0f);
+            part(x.x, t, hh[0], ll[0]);
+            part(x.y, t, hh[1], ll[1]);
+            part(x.z, t, hh[2], ll[2]);
+            part(x.w, t, hh[3], ll[3]);
             if (h) *reinterpret_cast<uint2*>(h + d) = *reinterpret_cast<const uint2*>(hh);
             if (l) *reinterpret_cast<uint2*>(l + d) = *reinterpret_cast<const uint2*>(ll);
         }
     } else {
         for (int d = lane; d < Dp; d += 32) {
             __half hh, ll;
-            part(d < D ? __ldg(row + d) : 0.0f, hh, ll);
+            part(d < D ? __ldg(row + d) : 0.0f, __fmaf_ru(-slope, (float)(d & ~15), 1.0f), hh, ll);
             if (h) h[d] = hh;
             if (l) l[d] = ll;
         }
@@ -525,7 +534,8 @@ __device__ __forceinline__ float norm_up(float ss) { return __fmul_ru(__fsqrt_ru
 // Norms of A's columns and of ns rows spread over X, the largest magnitudes of
 // both (one warp per row); flag 8: some of those rows are not exact in fp16.
 __global__ void k_project_sample(const float* __restrict__ X, int64_t N, int D, int ns, const float* __restrict__ A,
-                                 int LM, float* __restrict__ xs, float* __restrict__ anorm, ProjectState* st) {
+                                 int LM, float slope, float* __restrict__ xs, float* __restrict__ anorm,
+                                 ProjectState* st) {
     const int lane = threadIdx.x & 31;
     const int w = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
     if (w >= ns + LM) return;
@@ -533,7 +543,7 @@ __global__ void k_project_sample(const float* __restrict__ X, int64_t N, int D, 
     const float* row = is_a ? A + (int64_t)(w - ns) * D : X + (int64_t)w * (N / ns) * D;
     float ss, amax = 0.0f;
     bool inexact = false, bad = false;
-    split_row(row, D, D, 1.0f, false, nullptr, nullptr, ss, inexact, amax, bad);
+    split_row(row, D, D, 1.0f, slope, false, nullptr, nullptr, ss, inexact, amax, bad);
     const uint32_t am = __reduce_max_sync(0xffffffffu, __float_as_uint(amax));
     inexact = __any_sync(0xffffffffu, inexact);
     if (lane == 0) {
@@ -550,9 +560,16 @@ __global__ void k_project_scales(ProjectState* st) {
     st->sa = project_scale(st->amax_a);
 }
 
-// fp16 parts of A (LMp rows, zero past LM; the bounds of its norms get the
-// absolute residue of subnormal parts).
-__global__ void k_split_a(const float* __restrict__ A, int LM, int LMp, int D, int Dp, float kappa, __half* ah,
+// What an element's subnormal parts leave out (2^-25 of the scaled values, D of
+// them against the other operand's plain norm, which is at most |.|_t over the
+// root of the smallest weight), as an addition to |.|_t.
+__device__ __forceinline__ float subnormal_residue(int D, float scale, float kappa, float slope) {
+    return 1.01f * 2.98023224e-8f * sqrtf((float)D) / (scale * kappa * sqrtf(1.0f - slope * (float)D));
+}
+
+// fp16 parts of A (LMp rows, zero past LM) and upper bounds of its columns'
+// weighted norms.
+__global__ void k_split_a(const float* __restrict__ A, int LM, int LMp, int D, int Dp, float kappa, float slope, __half* ah,
                           __half* al, float* anorm, const ProjectState* st) {
     const int lane = threadIdx.x & 31;
     const int c = (int)((blockIdx.x * blockDim.x + threadIdx.x) >> 5);
@@ -560,27 +577,27 @@ __global__ void k_split_a(const float* __restrict__ A, int LM, int LMp, int D, i
     float ss, amax = 0.0f;
     bool inexact = false, bad = false;
     // rows past LM: zero dimensions to read
-    split_row(A + (int64_t)min(c, LM - 1) * D, c < LM ? D : 0, Dp, st->sa, false, ah + (int64_t)c * Dp,
+    split_row(A + (int64_t)min(c, LM - 1) * D, c < LM ? D : 0, Dp, st->sa, slope, false, ah + (int64_t)c * Dp,
               al + (int64_t)c * Dp, ss, inexact, amax, bad);
-    if (lane == 0 && c < LM) anorm[c] += 1.01f * 2.98023224e-8f * sqrtf((float)D) / (st->sa * kappa);
+    if (lane == 0 && c < LM) anorm[c] = __fadd_ru(norm_up(ss), subnormal_residue(D, st->sa, kappa, slope));
 }
 
-// fp16 parts of X and upper bounds of its row norms (warp per row); xl is null
+// fp16 parts of X and upper bounds of its rows' weighted norms (warp per row); xl is null
 // where the sample was exact in fp16. flags: 1 some element has a low part, 2
 // a value is not finite, 4 a scaled value leaves the fp16 range (amax_x then
 // holds the largest magnitude).
-__global__ void k_split_rows(const float* __restrict__ X, int64_t N, int D, int Dp, float kappa, __half* __restrict__ xh,
-                             __half* __restrict__ xl, float* __restrict__ xnorm, ProjectState* st) {
+__global__ void k_split_rows(const float* __restrict__ X, int64_t N, int D, int Dp, float kappa, float slope,
+                             __half* __restrict__ xh, __half* __restrict__ xl, float* __restrict__ xnorm, ProjectState* st) {
     const int lane = threadIdx.x & 31;
     const int64_t w0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int64_t nw = ((int64_t)gridDim.x * blockDim.x) >> 5;
-    const float sx = st->sx, res = 1.01f * 2.98023224e-8f * sqrtf((float)D) / (sx * kappa);
+    const float sx = st->sx, res = subnormal_residue(D, sx, kappa, slope);
     const bool vec = (D & 3) == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
     float amax = 0.0f;
     bool inexact = false, bad = false;
     for (int64_t n = w0; n < N; n += nw) {
         float ss;
-        split_row(X + n * D, D, Dp, sx, vec, xh + n * Dp, xl ? xl + n * Dp : nullptr, ss, inexact, amax, bad);
+        split_row(X + n * D, D, Dp, sx, slope, vec, xh + n * Dp, xl ? xl + n * Dp : nullptr, ss, inexact, amax, bad);
         if (lane == 0) xnorm[n] = __fadd_ru(norm_up(ss), res);
     }
     const uint32_t am = __reduce_max_sync(0xffffffffu, __float_as_uint(amax));
@@ -755,27 +772,27 @@ TcPlan tc_plan(int64_t N, int D, int LM, int num_sms, int max_smem) {
     return p;
 }
 
-cudaError_t launch_project_sample(const float* X, int64_t N, int D, int ns, const float* A, int LM, float* xs,
-                                  float* anorm, ProjectState* ps, cudaStream_t st) {
+cudaError_t launch_project_sample(const float* X, int64_t N, int D, int ns, const float* A, int LM, float slope,
+                                  float* xs, float* anorm, ProjectState* ps, cudaStream_t st) {
     cudaError_t e = cudaMemsetAsync(ps, 0, sizeof(ProjectState), st);
     if (e != cudaSuccess) return e;
-    k_project_sample<<<(unsigned)((ns + LM + 7) / 8), 256, 0, st>>>(X, N, D, ns, A, LM, xs, anorm, ps);
+    k_project_sample<<<(unsigned)((ns + LM + 7) / 8), 256, 0, st>>>(X, N, D, ns, A, LM, slope, xs, anorm, ps);
     k_project_scales<<<1, 1, 0, st>>>(ps);
     return cudaGetLastError();
 }
 
-cudaError_t launch_split_a(const float* A, int LM, int LMp, int D, int Dp, float kappa, void* ah, void* al, float* anorm,
+cudaError_t launch_split_a(const float* A, int LM, int LMp, int D, int Dp, float kappa, float slope, void* ah, void* al, float* anorm,
                            const ProjectState* ps, cudaStream_t st) {
-    k_split_a<<<(unsigned)((LMp + 7) / 8), 256, 0, st>>>(A, LM, LMp, D, Dp, kappa, static_cast<__half*>(ah),
+    k_split_a<<<(unsigned)((LMp + 7) / 8), 256, 0, st>>>(A, LM, LMp, D, Dp, kappa, slope, static_cast<__half*>(ah),
                                                         static_cast<__half*>(al), anorm, ps);
     return cudaGetLastError();
 }
 
-cudaError_t launch_split_rows(const float* X, int64_t N, int D, int Dp, float kappa, void* xh, void* xl, float* xnorm,
+cudaError_t launch_split_rows(const float* X, int64_t N, int D, int Dp, float kappa, float slope, void* xh, void* xl, float* xnorm,
                               ProjectState* ps, bool rescale, cudaStream_t st) {
     if (rescale) k_project_scales<<<1, 1, 0, st>>>(ps);
     const int blocks = (int)std::min<int64_t>((N * 32 + 255) / 256, 152 * 16);
-    k_split_rows<<<blocks, 256, 0, st>>>(X, N, D, Dp, kappa, static_cast<__half*>(xh), static_cast<__half*>(xl), xnorm,
+    k_split_rows<<<blocks, 256, 0, st>>>(X, N, D, Dp, kappa, slope, static_cast<__half*>(xh), static_cast<__half*>(xl), xnorm,
                                         ps);
     return cudaGetLastError();
 }

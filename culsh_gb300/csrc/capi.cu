@@ -675,8 +675,10 @@ int sort_keys(culsh_index* ix, int N, int passes, bool all_words, cudaStream_t s
     CU_TRY(ix->ws_keys[0].reserve(top_first ? LN : LN * KW));
     CU_TRY(ix->ws_keys[1].reserve(top_first ? LN : LN * KW));
     if (top_first) CU_TRY(ix->ws_low.reserve(LN * lw));
+    // the first pass makes the ids; without one they are the points' order
+    const bool any_pass = N > 1 && (top_first || passes > first_pass);
     CU_TRY(launch_pack_keys(ix->ws_codes.p, N, L, ix->M, KW, ix->cmin.p, ix->fbits.p, ix->foff.p, ix->ws_keys[0].p,
-                            ix->ids.p, top_first ? ix->ws_low.p : nullptr, lw, st));
+                            any_pass ? nullptr : ix->ids.p, top_first ? ix->ws_low.p : nullptr, lw, st));
     const int hp = std::max(passes, 1);
     CU_TRY(ix->ws_hist.reserve((size_t)L * hp * 256));
     CU_TRY(ix->ws_base.reserve((size_t)L * hp * 256));

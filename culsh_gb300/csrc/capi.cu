@@ -471,44 +471,85 @@ int upload_layout(culsh_index* ix, cudaStream_t st) {
 }
 
 // Hash tables over the unique keys, load factor between 1/4 and 1/2, in
-// groups of kGroupSlots slots.
-int build_hash(culsh_index* ix, cudaStream_t st) {
+// groups of kGroupSlots slots. with_sizes: a build, which wants the bucket sizes
+// too and may build the tables by parts in the space of the codes it no longer
+// needs; *spill then points at the number of keys placed afterwards, to be
+// checked against kHashSpill by the caller (once the stream has been waited
+// for), who calls again with in_place.
+constexpr uint32_t kHashSpill = 1u << 20;
+int build_hash(culsh_index* ix, bool with_sizes, bool in_place, const uint32_t** spill, cudaStream_t st) {
     const int L = ix->L;
     ix->h_hoff.assign(L + 1, 0);
     ix->h_hmask.assign(L, 0);
+    ix->h_fl_off.assign(L + 1, 0);
+    std::vector<uint32_t>& flm = ix->h_fl_mask;
+    flm.assign(L, 0);
     int64_t maxB = 0;
+    uint64_t max_groups = 0;
     for (int l = 0; l < L; ++l) {
         const uint64_t B = ix->h_boff[l + 1] - ix->h_boff[l];
         const uint64_t groups = next_pow2(std::max<uint64_t>(2 * B, kGroupSlots)) / kGroupSlots;
         ix->h_hmask[l] = (uint32_t)(groups - 1);
         ix->h_hoff[l + 1] = ix->h_hoff[l] + groups * kGroupWords;
+        const uint64_t words = std::max<uint64_t>(groups / 2, 1);
+        flm[l] = (uint32_t)(words - 1);
+        ix->h_fl_off[l + 1] = ix->h_fl_off[l] + words;
         maxB = std::max<int64_t>(maxB, (int64_t)B);
+        max_groups = std::max(max_groups, groups);
     }
     CU_TRY(ix->hoff.reserve(L + 1));
     CU_TRY(ix->hmask.reserve(L));
     CU_TRY(ix->hslots.reserve(ix->h_hoff[L]));
-    TRY(stage_copy(ix, ix->hoff.p, ix->h_hoff.data(), 8 * (L + 1), st));
-    TRY(stage_copy(ix, ix->hmask.p, ix->h_hmask.data(), 4 * L, st));
-    CU_TRY(cudaMemsetAsync(ix->hslots.p, 0xFF, 8 * ix->h_hoff[L], st));
-    // Filter words per table: a power of two holding 8 to 16 bits per key.
-    ix->h_fl_off.assign(L + 1, 0);
-    std::vector<uint32_t>& flm = ix->h_fl_mask;
-    flm.assign(L, 0);
-    for (int l = 0; l < L; ++l) {
-        const uint64_t B = ix->h_boff[l + 1] - ix->h_boff[l];
-        const uint64_t words = next_pow2(std::max<uint64_t>((B * kFilterBitsPerKey + 31) / 32, 1));
-        flm[l] = (uint32_t)(words - 1);
-        ix->h_fl_off[l + 1] = ix->h_fl_off[l] + words;
-    }
     CU_TRY(ix->fl_off.reserve(L + 1));
     CU_TRY(ix->fl_mask.reserve(L));
     CU_TRY(ix->filt.reserve(ix->h_fl_off[L]));
+    TRY(stage_copy(ix, ix->hoff.p, ix->h_hoff.data(), 8 * (L + 1), st));
+    TRY(stage_copy(ix, ix->hmask.p, ix->h_hmask.data(), 4 * L, st));
     TRY(stage_copy(ix, ix->fl_off.p, ix->h_fl_off.data(), 8 * (L + 1), st));
     TRY(stage_copy(ix, ix->fl_mask.p, flm.data(), 4 * L, st));
+    HashBuild h{};
+    h.boff = ix->boff.p;
+    h.ukeys = ix->ukeys.p;
+    h.L = L;
+    h.M = ix->M;
+    h.KW = ix->KW;
+    h.maxB = maxB;
+    h.max_groups = (uint32_t)std::min<uint64_t>(max_groups, 0xFFFFFFFFu);
+    h.foff = ix->foff.p;
+    h.fbits = ix->fbits.p;
+    h.rmul = ix->rmul.p;
+    h.hoff = ix->hoff.p;
+    h.hmask = ix->hmask.p;
+    h.hslots = ix->hslots.p;
+    h.filt = ix->filt.p;
+    h.fl_off = ix->fl_off.p;
+    h.fl_mask = ix->fl_mask.p;
+    h.starts = ix->starts.p;
+    h.N = ix->N;
+    h.sizes = with_sizes ? ix->sizes.p : nullptr;
+    h.max_size = ix->maxb.p;
+    h.err = ix->err.p;
+    // By parts from 2M keys on: 800K keys take 39 us by parts (three launches
+    // that fill no device) and 17 in place, 16M 0.38 and 0.49 ms, 200M 5.4 and 9.
+    const uint64_t parts = std::max<uint64_t>(max_groups / kHashPartGroups, 1);
+    const size_t rec = (size_t)L * parts * kHashPartCap, cnt = (size_t)L * parts + 1;
+    const size_t need = 8 * rec + 8 * (size_t)kHashSpill + 4 * cnt + 64;
+    const char* floor_env = getenv("CULSH_HASH_PARTS_MIN");
+    const uint64_t from = floor_env ? strtoull(floor_env, nullptr, 10) : 2000000;
+    if (spill && !in_place && with_sizes && ix->KW <= 4 && parts <= kHashMaxParts && ix->h_boff[L] >= from &&
+        need <= ix->ws_codes.n * sizeof(int32_t)) {
+        unsigned char* base = reinterpret_cast<unsigned char*>(ix->ws_codes.p);
+        h.rec = reinterpret_cast<unsigned long long*>(base);
+        h.spill = reinterpret_cast<uint2*>(h.rec + rec);
+        h.spill_cap = kHashSpill;
+        h.part_cnt = reinterpret_cast<uint32_t*>(h.spill + kHashSpill);
+        CU_TRY(launch_hash_build_parts(h, st));
+        *spill = h.part_cnt + (cnt - 1);
+        return CULSH_OK;
+    }
+    CU_TRY(cudaMemsetAsync(ix->hslots.p, 0xFF, 8 * ix->h_hoff[L], st));
     CU_TRY(cudaMemsetAsync(ix->filt.p, 0, 4 * ix->h_fl_off[L], st));
-    CU_TRY(launch_hash_build(ix->boff.p, ix->ukeys.p, L, ix->M, ix->KW, maxB, ix->foff.p, ix->fbits.p, ix->rmul.p,
-                             ix->hoff.p, ix->hmask.p, ix->hslots.p, ix->filt.p, ix->fl_off.p, ix->fl_mask.p,
-                             ix->err.p, st));
+    CU_TRY(launch_hash_build(h, st));
     return CULSH_OK;
 }
 
@@ -786,8 +827,8 @@ int build_device(culsh_index* ix, const float* dX, cudaStream_t st, FILE* dbg) {
     for (int all_words = 0; all_words < 2; ++all_words) {
         TRY(sort_keys(ix, N, passes, all_words != 0, st, &skeys));
         CU_TRY(cudaEventRecord(ix->bev[3], st));
-        // Run-length bucketing.
-        CU_TRY(launch_rl_count(skeys, N, L, ix->KW, ix->ws_tcnt.p, ix->ws_toff.p, ix->ws_nb.p, st));
+        // Run-length bucketing (the boundary flags take the place of the sort's tile states).
+        CU_TRY(launch_rl_count(skeys, N, L, ix->KW, ix->ws_tcnt.p, ix->ws_toff.p, ix->ws_status.p, ix->ws_nb.p, st));
         CU_TRY(cudaMemcpyAsync(ix->h_nb.p, ix->ws_nb.p, 4 * L, cudaMemcpyDeviceToHost, st));
         CU_TRY(cudaStreamSynchronize(st));
         if (ix->h_run_cnt.p[3] == 0) break;   // every run was ordered
@@ -805,15 +846,22 @@ int build_device(culsh_index* ix, const float* dX, cudaStream_t st, FILE* dbg) {
     CU_TRY(ix->starts.reserve(totB));
     CU_TRY(ix->sizes.reserve(totB));
     CU_TRY(ix->ukeys.reserve(totB * ix->KW));
-    CU_TRY(launch_rl_write(skeys, N, L, ix->KW, ix->ws_toff.p, ix->boff.p, ix->starts.p, ix->ukeys.p, st));
+    CU_TRY(launch_rl_write(skeys, N, L, ix->KW, ix->ws_status.p, ix->ws_toff.p, ix->boff.p, ix->starts.p, ix->ukeys.p, st));
     CU_TRY(ix->maxb.reserve(1));
     CU_TRY(cudaMemsetAsync(ix->maxb.p, 0, sizeof(uint32_t), st));
-    CU_TRY(launch_bucket_sizes(ix->boff.p, ix->starts.p, N, L, maxB, ix->sizes.p, ix->maxb.p, st));
-    CU_TRY(ix->h_maxb.reserve(1));   // pinned: the copy does not block the host mid-build
+    const uint32_t* spill = nullptr;
+    TRY(build_hash(ix, true, false, &spill, st));
+    CU_TRY(ix->h_maxb.reserve(2));   // pinned: the copy does not block the host mid-build
+    ix->h_maxb.p[1] = 0;
     CU_TRY(cudaMemcpyAsync(ix->h_maxb.p, ix->maxb.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    TRY(build_hash(ix, st));
+    if (spill) CU_TRY(cudaMemcpyAsync(ix->h_maxb.p + 1, spill, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     CU_TRY(cudaEventRecord(ix->bev[4], st));
     TRY(read_err_flag(ix, st, "index"));   // synchronises the stream
+    if (ix->h_maxb.p[1] > kHashSpill) {    // more keys in a few parts than they can hold
+        TRY(build_hash(ix, true, true, nullptr, st));
+        CU_TRY(cudaEventRecord(ix->bev[4], st));
+        TRY(read_err_flag(ix, st, "index"));
+    }
     ix->max_bucket = *ix->h_maxb.p;
     ix->indexed = ix->dev_valid = true;
     ix->host_valid = false;
@@ -906,7 +954,7 @@ int ensure_device(culsh_index* ix, cudaStream_t st) {
     CU_TRY(ix->ukeys.reserve(totB * ix->KW));
     CU_TRY(launch_pack_from_codes(ix->boff.p, ix->dcodes.p, L, M, ix->KW, maxB, ix->cmin.p, ix->fbits.p, ix->foff.p,
                                   ix->ukeys.p, st));
-    TRY(build_hash(ix, st));
+    TRY(build_hash(ix, false, true, nullptr, st));
     TRY(read_err_flag(ix, st, "load"));
     ix->dev_valid = true;
     return CULSH_OK;

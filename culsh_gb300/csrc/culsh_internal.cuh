@@ -78,17 +78,15 @@ __host__ __device__ __forceinline__ uint64_t field_mult(int c) {
 __host__ __device__ __forceinline__ uint64_t hash_finish(uint64_t h) { return mix64(h ^ kHashSeed); }
 
 // Key filter beside each table's hash (a blocked Bloom filter, two bits in
-// one 32-bit word, 8 to 16 bits per key): the word index and the two bits
-// come from the high half of a 64-bit product of the finished hash, so they
-// are independent of the group (low bits) and the fingerprint (top 16 bits).
-// A key that is in the table always finds both of its bits set.
-__host__ __device__ __forceinline__ uint32_t filter_mix(uint64_t hh) {
-    return (uint32_t)((hh * 0xD6E8FEB86659FD93ull) >> 32);
+// one 32-bit word per two groups, 8 to 16 bits per key). The word is that of
+// the key's home group, so that a part of a table and its filter are built
+// together; the bits are independent of the group (low 32 bits), one of them
+// is part of the fingerprint (top 16 bits, the same for the two hashes that
+// slot_fp makes equal). A key that is in the table always finds both set.
+__host__ __device__ __forceinline__ uint32_t filter_word(uint64_t hh) { return (uint32_t)hh >> 1; }
+__host__ __device__ __forceinline__ uint32_t filter_bits(uint64_t hh) {
+    return (1u << ((uint32_t)(hh >> 43) & 31u)) | (1u << ((uint32_t)(hh >> 53) & 31u));
 }
-__host__ __device__ __forceinline__ uint32_t filter_bits(uint32_t fx) {
-    return (1u << (fx >> 27)) | (1u << ((fx >> 22) & 31u));
-}
-constexpr int kFilterBitsPerKey = 8;
 
 // Place a field of `bits` bits (<= 32) at bit offset `off` of a little-endian
 // multi-word key.
@@ -124,7 +122,7 @@ struct LookupView {
     const unsigned long long* rmul;    // [L*M]: field multipliers of the lookup hash
     const uint32_t* filt;              // key filters, table l at words [fl_off[l], fl_off[l+1])
     const uint64_t* fl_off;
-    const uint32_t* fl_mask;           // [L]: words in table l's filter - 1 (a power of two - 1)
+    const uint32_t* fl_mask;           // [L]: words in table l's filter - 1 (half its groups, at least one)
 };
 
 // ---------------------------------------------------------------------------
@@ -270,19 +268,49 @@ struct SortedKeys {
 };
 constexpr int low_row_words(int KW) { return KW == 2 ? 1 : KW == 3 ? 2 : 4; }
 
-// Run-length bucketing of sorted keys. Two phases: count (per table bucket
-// totals, written to nb[L]) and write (starts, ukeys).
+// Run-length bucketing of sorted keys. Two phases: count (boundary flags, one
+// word per 32 positions of 4,096-position tiles; per table bucket totals,
+// written to nb[L]) and write (starts, ukeys).
 cudaError_t launch_rl_count(const SortedKeys& keys, int64_t N, int L, int KW, uint32_t* tile_cnt, uint32_t* tile_off,
-                            uint32_t* nb, cudaStream_t st);
-cudaError_t launch_rl_write(const SortedKeys& keys, int64_t N, int L, int KW, const uint32_t* tile_off,
-                            const uint64_t* boff, uint32_t* starts, uint32_t* ukeys, cudaStream_t st);
-cudaError_t launch_bucket_sizes(const uint64_t* boff, const uint32_t* starts, int64_t N, int L, int64_t maxB,
-                                uint32_t* sizes, uint32_t* max_size, cudaStream_t st);
-cudaError_t launch_hash_build(const uint64_t* boff, const uint32_t* ukeys, int L, int M, int KW, int64_t maxB,
-                              const uint16_t* foff, const uint8_t* fbits, const unsigned long long* rmul,
-                              const uint64_t* hoff, const uint32_t* hmask, unsigned long long* hslots,
-                              uint32_t* filt, const uint64_t* fl_off, const uint32_t* fl_mask, int* err,
-                              cudaStream_t st);
+                            uint32_t* flags, uint32_t* nb, cudaStream_t st);
+cudaError_t launch_rl_write(const SortedKeys& keys, int64_t N, int L, int KW, const uint32_t* flags,
+                            const uint32_t* tile_off, const uint64_t* boff, uint32_t* starts, uint32_t* ukeys,
+                            cudaStream_t st);
+// Hash tables and filters over the unique keys; with sizes set also the bucket
+// sizes and the largest (max_size zeroed by the caller).
+struct HashBuild {
+    const uint64_t* boff;
+    const uint32_t* ukeys;
+    int L, M, KW;
+    int64_t maxB;                 // most buckets of a table
+    uint32_t max_groups;          // most groups of a table
+    const uint16_t* foff;
+    const uint8_t* fbits;
+    const unsigned long long* rmul;
+    const uint64_t* hoff;
+    const uint32_t* hmask;
+    unsigned long long* hslots;
+    uint32_t* filt;
+    const uint64_t* fl_off;
+    const uint32_t* fl_mask;
+    const uint32_t* starts;       // with sizes: a build's bucket starts, points per table
+    int64_t N;
+    uint32_t* sizes;
+    uint32_t* max_size;
+    int* err;
+    // Form by parts: records [L][parts of the largest table][kHashPartCap], their
+    // counts, keys that fit no part's records or slots.
+    unsigned long long* rec;
+    uint32_t* part_cnt;           // [L][parts], then the spill count
+    uint2* spill;                 // (table, bucket)
+    uint32_t spill_cap;
+};
+constexpr uint32_t kHashPartGroups = 2048;   // groups built together in shared memory
+constexpr uint32_t kHashPartCap = 4672;      // a part's records: 4,096 expected at most, 9 deviations more
+constexpr uint32_t kHashMaxParts = 4096;
+// Key by key in place (hslots all ones, filt zero), or by parts (any contents).
+cudaError_t launch_hash_build(const HashBuild& h, cudaStream_t st);
+cudaError_t launch_hash_build_parts(const HashBuild& h, cudaStream_t st);
 // Bucket codes [M][B_l] per table (float, the reference's layout) decoded from ukeys.
 cudaError_t launch_decode_codes(const uint64_t* boff, const uint32_t* ukeys, int L, int M, int KW, int64_t maxB,
                                 const int32_t* cmin, const uint8_t* fbits, const uint16_t* foff, float* codes,

@@ -669,9 +669,8 @@ __global__ void __launch_bounds__(PF, kForm == 2 && MM <= 12 ? 9 : (kForm > 0 ? 
                 if (pt >= 0 && (pfw & pneed) == pneed) pass |= 1ull << pt;
                 pt = -1;
                 if (ok) {
-                    const uint32_t fx = filter_mix(hh);
-                    pneed = filter_bits(fx);
-                    pfw = filt ? __ldg(filt + (fx & fmask)) : ~0u;
+                    pneed = filter_bits(hh);
+                    pfw = filt ? __ldg(filt + (filter_word(hh) & fmask)) : ~0u;
                     pt = t;
                 }
             }
@@ -964,8 +963,8 @@ __global__ void __launch_bounds__(32 * PW) k_probe_warp(ProbeArgs a) {
         int32_t res = -1;
         bool done = !probe_hash(c, pm, hh);
         if (!done && filt) {
-            const uint32_t fx = filter_mix(hh), need = filter_bits(fx);
-            done = (__ldg(filt + (fx & fmask)) & need) != need;
+            const uint32_t need = filter_bits(hh);
+            done = (__ldg(filt + (filter_word(hh) & fmask)) & need) != need;
         }
         const uint32_t fp = slot_fp(hh);
         uint32_t g = (uint32_t)hh & gmask;
@@ -1091,9 +1090,9 @@ __global__ void __launch_bounds__(256, 5) k_probe_resolve(const __grid_constant_
         need[k] = 0;
         fw[k] = 0;
         if (v[k] == -2) {
-            const uint32_t fx = filter_mix(a.ph[base + (int64_t)k * Q]);
-            need[k] = filter_bits(fx);
-            fw[k] = filt ? __ldg(filt + (fx & fmask)) : ~0u;
+            const uint64_t hh = a.ph[base + (int64_t)k * Q];
+            need[k] = filter_bits(hh);
+            fw[k] = filt ? __ldg(filt + (filter_word(hh) & fmask)) : ~0u;
         }
     }
     // Slots the filter rules out are misses; the rest (a few percent when

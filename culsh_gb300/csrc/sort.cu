@@ -743,37 +743,83 @@ __global__ void __launch_bounds__(NT) k_run_sort_large(const unsigned long long*
     }
 }
 
-// Whether sorted positions a and a - 1 of the table at seg hold different keys.
-// LOW: top-word-first form, keys = the sorted top words, low = lower words by
-// point; otherwise keys = KW arrays of LN words.
-template <bool LOW>
-__device__ __forceinline__ bool key_differs(const SortedKeys& s, int64_t LN, int64_t seg, int64_t a, int KW) {
-    if constexpr (LOW) {
-        if (s.keys[a] != s.keys[a - 1]) return true;
-        const uint32_t* x = s.low + (seg + s.ids[a]) * s.lw;
-        const uint32_t* y = s.low + (seg + s.ids[a - 1]) * s.lw;
-        for (int w = 0; w < KW - 1; ++w)
-            if (__ldg(x + w) != __ldg(y + w)) return true;
-        return false;
+// A point's lower key words (rows of lw words, as low_row; unused ones zero).
+__device__ __forceinline__ uint4 low_words(const uint32_t* __restrict__ low, int lw, int64_t row) {
+    if (lw == 1) return make_uint4(__ldg(low + row), 0u, 0u, 0u);
+    if (lw == 2) {
+        const uint2 v = __ldg(reinterpret_cast<const uint2*>(low) + row);
+        return make_uint4(v.x, v.y, 0u, 0u);
     }
-    for (int w = 0; w < KW; ++w)
-        if (s.keys[w * LN + a] != s.keys[w * LN + a - 1]) return true;
-    return false;
+    return __ldg(reinterpret_cast<const uint4*>(low) + row);
 }
 
+// Bucket boundaries of one tile of 4,096 sorted positions: warp w takes positions
+// [512 w, 512 w + 512) as 16 rows of 32 lanes. A position whose key differs
+// from its predecessor's starts a bucket; flags gets one word per row, tile_cnt
+// the tile's total. LOW: top-word-first form, keys = the sorted top words, low =
+// lower words by point, looked up only where two top words are equal; four
+// rows' lookups are in flight together. Otherwise keys = KW arrays of L*N words.
 template <bool LOW>
-__global__ void k_rl_count(SortedKeys s, int64_t N, int L, int KW, uint32_t* __restrict__ tile_cnt) {
+__global__ void __launch_bounds__(NT) k_rl_count(SortedKeys s, int64_t N, int L, int KW, uint32_t* __restrict__ tile_cnt,
+                                                 uint32_t* __restrict__ flags) {
     __shared__ uint32_t ws[SP_WARPS];
     const int l = blockIdx.y, tile = blockIdx.x, tiles = gridDim.x;
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t LN = (int64_t)L * N, seg = (int64_t)l * N;
-    uint32_t c = 0;
-    for (int e = threadIdx.x; e < SP_TILE; e += NT) {
-        const int64_t i = (int64_t)tile * SP_TILE + e;
-        if (i < N) c += (i == 0 || key_differs<LOW>(s, LN, seg, seg + i, KW)) ? 1u : 0u;
+    const int64_t w0 = (int64_t)tile * SP_TILE + (int64_t)warp * (32 * SP_ITEMS);
+    uint32_t mine = 0;
+#pragma unroll
+    for (int k0 = 0; k0 < SP_ITEMS; k0 += 4) {
+        bool same[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const int64_t i = w0 + (k0 + q) * 32 + lane;
+            same[q] = i > 0 && i < N && s.keys[seg + i] == s.keys[seg + i - 1];
+        }
+        if constexpr (LOW) {
+            uint32_t ia[4], ib[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int64_t i = w0 + (k0 + q) * 32 + lane;
+                ia[q] = same[q] ? s.ids[seg + i] : 0u;
+                ib[q] = same[q] ? s.ids[seg + i - 1] : 0u;
+            }
+            uint4 x[4], y[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                x[q] = y[q] = make_uint4(0, 0, 0, 0);
+                if (same[q]) {
+                    x[q] = low_words(s.low, s.lw, seg + ia[q]);
+                    y[q] = low_words(s.low, s.lw, seg + ib[q]);
+                }
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q)
+                same[q] = same[q] && x[q].x == y[q].x && x[q].y == y[q].y && x[q].z == y[q].z;
+        } else {
+            for (int w = 1; w < KW; ++w)
+#pragma unroll
+                for (int q = 0; q < 4; ++q)
+                    if (same[q]) {
+                        const int64_t a = w * LN + seg + w0 + (k0 + q) * 32 + lane;
+                        same[q] = s.keys[a] == s.keys[a - 1];
+                    }
+        }
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            const uint32_t ball = __ballot_sync(0xffffffffu, !same[q] && w0 + (k0 + q) * 32 + lane < N);
+            if (lane == k0 + q) mine = ball;
+        }
     }
-    uint32_t tot;
-    block_excl_scan(c, ws, &tot);
-    if (threadIdx.x == 0) tile_cnt[(int64_t)l * tiles + tile] = tot;
+    if (lane < SP_ITEMS) flags[((int64_t)l * tiles + tile) * (SP_TILE / 32) + warp * SP_ITEMS + lane] = mine;
+    const uint32_t c = __reduce_add_sync(0xffffffffu, (uint32_t)__popc(mine));
+    if (lane == 0) ws[warp] = c;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        uint32_t tot = 0;
+        for (int w = 0; w < SP_WARPS; ++w) tot += ws[w];
+        tile_cnt[(int64_t)l * tiles + tile] = tot;
+    }
 }
 
 __global__ void k_rl_scan(const uint32_t* __restrict__ tile_cnt, int tiles, uint32_t* __restrict__ tile_off,
@@ -792,123 +838,175 @@ __global__ void k_rl_scan(const uint32_t* __restrict__ tile_cnt, int tiles, uint
     if (threadIdx.x == 0) nb[l] = carry;
 }
 
-// Bucket starts and unique keys of one tile of 4,096 sorted positions: warp w
-// takes positions [512 w, 512 w + 512) as 16 rows of 32 lanes (coalesced key
-// loads), ranks its flagged positions with ballots, and the block scans the
-// warp totals; flagged positions are written in order.
+// Bucket starts and unique keys at the positions that k_rl_count flagged, in
+// order. LOW: four rows' lookups of lower words are in flight together (one
+// after another they had taken 0.23 ms for 16M buckets, now 0.11).
 template <bool LOW>
-__global__ void k_rl_write(SortedKeys s, int64_t N, int L, int KW, const uint32_t* __restrict__ tile_off, const uint64_t* __restrict__ boff,
-                           uint32_t* __restrict__ starts, uint32_t* __restrict__ ukeys) {
+__global__ void __launch_bounds__(NT) k_rl_write(SortedKeys s, int64_t N, int L, int KW,
+                                                 const uint32_t* __restrict__ flags, const uint32_t* __restrict__ tile_off,
+                                                 const uint64_t* __restrict__ boff, uint32_t* __restrict__ starts,
+                                                 uint32_t* __restrict__ ukeys) {
     __shared__ uint32_t ws[SP_WARPS];
     const int l = blockIdx.y, tile = blockIdx.x, tiles = gridDim.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t LN = (int64_t)L * N, seg = (int64_t)l * N;
     const int64_t w0 = (int64_t)tile * SP_TILE + (int64_t)warp * (32 * SP_ITEMS);
-    uint32_t ball[SP_ITEMS];
-    uint32_t c = 0;
-#pragma unroll
-    for (int k = 0; k < SP_ITEMS; ++k) {
-        const int64_t i = w0 + k * 32 + lane;
-        const bool f = i < N && (i == 0 || key_differs<LOW>(s, LN, seg, seg + i, KW));
-        ball[k] = __ballot_sync(0xffffffffu, f);
-        c += __popc(ball[k]);
-    }
+    const uint32_t mine =
+        lane < SP_ITEMS ? flags[((int64_t)l * tiles + tile) * (SP_TILE / 32) + warp * SP_ITEMS + lane] : 0u;
+    const uint32_t c = __reduce_add_sync(0xffffffffu, (uint32_t)__popc(mine));
     if (lane == 0) ws[warp] = c;
     __syncthreads();
-    uint32_t r = tile_off[(int64_t)l * tiles + tile];
-    for (int w = 0; w < warp; ++w) r += ws[w];
-    const uint64_t bo = boff[l];
+    uint64_t g = boff[l] + tile_off[(int64_t)l * tiles + tile];
+    for (int w = 0; w < warp; ++w) g += ws[w];
     const uint32_t below = (1u << lane) - 1u;
 #pragma unroll
-    for (int k = 0; k < SP_ITEMS; ++k) {
-        if ((ball[k] >> lane) & 1u) {
-            const int64_t i = w0 + k * 32 + lane;
-            const uint64_t g = bo + r + __popc(ball[k] & below);
-            starts[g] = (uint32_t)i;
-            if constexpr (LOW) {
-                const uint32_t* x = s.low + (seg + s.ids[seg + i]) * s.lw;
-                for (int w = 0; w < KW - 1; ++w) ukeys[g * KW + w] = __ldg(x + w);
-                ukeys[g * KW + KW - 1] = s.keys[seg + i];
-            } else {
-                for (int w = 0; w < KW; ++w) ukeys[g * KW + w] = s.keys[w * LN + seg + i];
+    for (int k0 = 0; k0 < SP_ITEMS; k0 += 4) {
+        uint32_t ball[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) ball[q] = __shfl_sync(0xffffffffu, mine, k0 + q);
+        if constexpr (LOW) {
+            uint32_t id[4], top[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int64_t a = seg + w0 + (k0 + q) * 32 + lane;
+                const bool f = (ball[q] >> lane) & 1u;
+                id[q] = f ? s.ids[a] : 0u;
+                top[q] = f ? s.keys[a] : 0u;
+            }
+            uint4 x[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                x[q] = make_uint4(0, 0, 0, 0);
+                if ((ball[q] >> lane) & 1u) x[q] = low_words(s.low, s.lw, seg + id[q]);
+            }
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                if ((ball[q] >> lane) & 1u) {
+                    const uint64_t o = g + __popc(ball[q] & below);
+                    starts[o] = (uint32_t)(w0 + (k0 + q) * 32 + lane);
+                    if (s.lw == 1) {
+                        reinterpret_cast<uint2*>(ukeys)[o] = make_uint2(x[q].x, top[q]);
+                    } else if (s.lw == 2) {
+                        ukeys[o * 3] = x[q].x;
+                        ukeys[o * 3 + 1] = x[q].y;
+                        ukeys[o * 3 + 2] = top[q];
+                    } else {
+                        reinterpret_cast<uint4*>(ukeys)[o] = make_uint4(x[q].x, x[q].y, x[q].z, top[q]);
+                    }
+                }
+                g += __popc(ball[q]);
+            }
+        } else {
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                if ((ball[q] >> lane) & 1u) {
+                    const int64_t i = w0 + (k0 + q) * 32 + lane;
+                    const uint64_t o = g + __popc(ball[q] & below);
+                    starts[o] = (uint32_t)i;
+                    for (int w = 0; w < KW; ++w) ukeys[o * KW + w] = s.keys[w * LN + seg + i];
+                }
+                g += __popc(ball[q]);
             }
         }
-        r += __popc(ball[k]);
     }
 }
 
-__global__ void k_bucket_sizes(const uint64_t* __restrict__ boff, const uint32_t* __restrict__ starts, int64_t N,
-                               uint32_t* __restrict__ sizes, uint32_t* __restrict__ max_size) {
-    const int l = blockIdx.y;
-    const int64_t j = (int64_t)blockIdx.x * NT + threadIdx.x;
-    const int64_t B = (int64_t)(boff[l + 1] - boff[l]);
-    uint32_t sz = 0;
-    if (j < B) {
-        const uint64_t g = boff[l] + j;
-        const int64_t end = (j + 1 < B) ? (int64_t)starts[g + 1] : N;
-        sz = (uint32_t)(end - (int64_t)starts[g]);
-        sizes[g] = sz;
-    }
-    // largest bucket: one atomic per block (one per warp serialises on the
-    // single address when every bucket is small and there are millions)
-    __shared__ uint32_t smax[SP_WARPS];
-    const uint32_t wmax = __reduce_max_sync(0xffffffffu, sz);
-    if ((threadIdx.x & 31) == 0) smax[threadIdx.x >> 5] = wmax;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t m = 0;
-        for (int w = 0; w < SP_WARPS; ++w) m = max(m, smax[w]);
-        if (m) atomicMax(max_size, m);
-    }
-}
-
-template <bool WIDE>   // KW > 4
-__global__ void k_hash_build(const uint64_t* __restrict__ boff, const uint32_t* __restrict__ ukeys, int M, int KW,
-                             const uint16_t* __restrict__ foff, const uint8_t* __restrict__ fbits,
-                             const unsigned long long* __restrict__ rmul, const uint64_t* __restrict__ hoff,
-                             const uint32_t* __restrict__ hmask, unsigned long long* __restrict__ hslots,
-                             uint32_t* __restrict__ filt, const uint64_t* __restrict__ fl_off,
-                             const uint32_t* __restrict__ fl_mask, int* err) {
-    const int l = blockIdx.y;
-    const int64_t j = (int64_t)blockIdx.x * NT + threadIdx.x;
-    const int64_t B = (int64_t)(boff[l + 1] - boff[l]);
-    if (j >= B) return;
-    const uint32_t* key = ukeys + (boff[l] + j) * KW;
-    const uint32_t gmask = hmask[l];
-    uint64_t hs = 0;   // additive lookup hash over the key's fields
-    if constexpr (WIDE) {
-        for (int m = 0; m < M; ++m) {
-            const int c = l * M + m;
-            hs += (uint64_t)key_get(key, __ldg(foff + c), __ldg(fbits + c)) * __ldg(rmul + c);
+// Finished lookup hashes of ITEMS keys of table l (indices j0 + i * NTH, clamped
+// to the last). Fields are contiguous from column M - 1's offset upwards and
+// their widths the same for every thread: they are taken from a 64-bit window
+// (a 128-bit shift per field had been most of the kernel's instructions).
+template <bool WIDE, int NTH, int ITEMS>
+__device__ __forceinline__ void key_hashes(const HashBuild& h, int l, uint64_t bo, int64_t B, int64_t j0,
+                                           uint64_t (&hh)[ITEMS]) {
+    const int M = h.M, KW = h.KW;
+    if constexpr (WIDE) {   // KW > 4
+#pragma unroll 1
+        for (int i = 0; i < ITEMS; ++i) {
+            const uint32_t* key = h.ukeys + (bo + min(j0 + i * NTH, B - 1)) * KW;
+            uint64_t hs = 0;
+            for (int m = 0; m < M; ++m) {
+                const int c = l * M + m;
+                hs += (uint64_t)key_get(key, __ldg(h.foff + c), __ldg(h.fbits + c)) * __ldg(h.rmul + c);
+            }
+#pragma unroll
+            for (int q = 0; q < ITEMS; ++q) hh[q] = q == i ? hash_finish(hs) : hh[q];
         }
     } else {
-        unsigned __int128 kk = 0;
-        for (int w = KW - 1; w >= 0; --w) kk = (kk << 32) | key[w];
-        // fields are contiguous from column M - 1's offset upwards
-        kk >>= __ldg(foff + (int64_t)l * M + M - 1);
+        uint32_t k[4][ITEMS];
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) {
+            const uint32_t* key = h.ukeys + (bo + min(j0 + i * NTH, B - 1)) * KW;
+#pragma unroll
+            for (int w = 0; w < 4; ++w) k[w][i] = w < KW ? __ldg(key + w) : 0u;
+        }
+        const int pos = __ldg(h.foff + (int64_t)l * M + M - 1);
+        int w = pos >> 5;
+        uint64_t win[ITEMS];
+        auto word = [&](int i) { return w == 0 ? k[0][i] : w == 1 ? k[1][i] : w == 2 ? k[2][i] : w == 3 ? k[3][i] : 0u; };
+        int have = 32 - (pos & 31);
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) {
+            win[i] = word(i) >> (pos & 31);
+            hh[i] = 0;
+        }
         for (int m = M - 1; m >= 0; --m) {
             const int c = l * M + m;
-            const int bits = __ldg(fbits + c);
-            const uint32_t f = bits ? (uint32_t)kk & (bits == 32 ? 0xFFFFFFFFu : ((1u << bits) - 1u)) : 0u;
-            kk >>= bits;
-            hs += (uint64_t)f * __ldg(rmul + c);
+            const int bits = __ldg(h.fbits + c);
+            if (bits == 0) continue;
+            const uint64_t mul = __ldg(h.rmul + c);
+            if (have < bits) {
+                ++w;
+#pragma unroll
+                for (int i = 0; i < ITEMS; ++i) win[i] |= (uint64_t)word(i) << have;
+                have += 32;
+            }
+            const uint32_t mask = bits == 32 ? 0xFFFFFFFFu : (1u << bits) - 1u;
+#pragma unroll
+            for (int i = 0; i < ITEMS; ++i) {
+                hh[i] += (uint64_t)((uint32_t)win[i] & mask) * mul;
+                win[i] >>= bits;
+            }
+            have -= bits;
         }
+#pragma unroll
+        for (int i = 0; i < ITEMS; ++i) hh[i] = hash_finish(hh[i]);
     }
-    const uint64_t hh = hash_finish(hs);
-    const uint32_t h = (uint32_t)hh;
-    const uint32_t fp = slot_fp(hh);
-    if (filt) {
-        const uint32_t fx = filter_mix(hh);
-        atomicOr(filt + fl_off[l] + (fx & fl_mask[l]), filter_bits(fx));
+}
+
+// Sizes of buckets j0 + i * NTH of a table, and the largest of the block's with
+// one atomic (one per warp serialises on the single address).
+template <int NTH, int ITEMS>
+__device__ __forceinline__ void bucket_sizes(const HashBuild& h, uint64_t bo, int64_t B, int64_t j0) {
+    __shared__ uint32_t smax[NTH / 32];
+    uint32_t mx = 0;
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+        const int64_t j = j0 + i * NTH;
+        if (j >= B) break;
+        const uint32_t end = j + 1 < B ? h.starts[bo + j + 1] : (uint32_t)h.N;
+        const uint32_t sz = end - h.starts[bo + j];
+        h.sizes[bo + j] = sz;
+        mx = max(mx, sz);
     }
-    unsigned long long* slots = hslots + hoff[l];
-    // Claim the first empty slot in probe order (a group's slots in order,
-    // then the next group), then store the bucket index beside it. Lookups
-    // stop at the first empty slot they meet, which can only lie past every
-    // key inserted along the same path.
+    mx = __reduce_max_sync(0xffffffffu, mx);
+    if ((threadIdx.x & 31) == 0) smax[threadIdx.x >> 5] = mx;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        for (int w = 1; w < NTH / 32; ++w) mx = max(mx, smax[w]);
+        atomicMax(h.max_size, mx);
+    }
+}
+
+// Claims the first empty slot in probe order from group g on (a group's slots
+// in order, then the next group), then stores the bucket index beside it; cur
+// is the first group's fingerprint word as last seen. Lookups stop at the first
+// empty slot they meet, which can only lie past every key inserted along the
+// same path.
+__device__ __forceinline__ void hash_insert(unsigned long long* slots, uint32_t gmask, uint32_t g, uint32_t fp, uint32_t j,
+                                            unsigned long long cur, int* err) {
     for (uint32_t p = 0; p <= gmask; ++p) {
-        unsigned long long* grp = slots + (uint64_t)((h + p) & gmask) * kGroupWords;
-        unsigned long long cur = *reinterpret_cast<volatile unsigned long long*>(grp);
+        unsigned long long* grp = slots + (uint64_t)((g + p) & gmask) * kGroupWords;
+        if (p > 0) cur = *reinterpret_cast<volatile unsigned long long*>(grp);
         // One 64-bit CAS per attempt on the group's fingerprint word; each
         // failure means another insert took a slot, so at most four tries.
         for (int tries = 0; tries <= kGroupSlots; ++tries) {
@@ -918,13 +1016,231 @@ __global__ void k_hash_build(const uint64_t* __restrict__ boff, const uint32_t* 
             const unsigned long long nw = (cur & ~(0xFFFFull << (16 * e))) | ((unsigned long long)fp << (16 * e));
             const unsigned long long old = atomicCAS(grp, cur, nw);
             if (old == cur) {
-                reinterpret_cast<uint32_t*>(grp + 1)[e] = (uint32_t)j;
+                reinterpret_cast<uint32_t*>(grp + 1)[e] = j;
                 return;
             }
             cur = old;
         }
     }
     atomicOr(err, kErrHashFull);
+}
+
+// Key by key in place. The first attempt takes the home group for empty, as
+// most are, without reading it, two keys' attempts in flight per thread (16M
+// keys in tables of 17 MB: 0.43 ms with the sizes; reading the group first 0.54,
+// one key per thread 0.48, four 0.48).
+constexpr int HB_ITEMS = 2;
+template <bool WIDE>
+__global__ void __launch_bounds__(NT) k_hash_build(HashBuild h) {
+    const int l = blockIdx.y;
+    const int64_t j0 = (int64_t)blockIdx.x * (NT * HB_ITEMS) + threadIdx.x;
+    const uint64_t bo = h.boff[l];
+    const int64_t B = (int64_t)(h.boff[l + 1] - bo);
+    if ((int64_t)blockIdx.x * (NT * HB_ITEMS) >= B) return;
+    const uint32_t gmask = h.hmask[l];
+    uint64_t hh[HB_ITEMS];
+    key_hashes<WIDE, NT, HB_ITEMS>(h, l, bo, B, j0, hh);
+    uint32_t* fl = h.filt + h.fl_off[l];
+    const uint32_t fmask = h.fl_mask[l];
+    unsigned long long* slots = h.hslots + h.hoff[l];
+    constexpr unsigned long long kEmptyGroup = ~0ull;
+    unsigned long long got[HB_ITEMS];
+#pragma unroll
+    for (int i = 0; i < HB_ITEMS; ++i)
+        if (j0 + i * NT < B) atomicOr(fl + (filter_word(hh[i]) & fmask), filter_bits(hh[i]));
+#pragma unroll
+    for (int i = 0; i < HB_ITEMS; ++i) {
+        got[i] = kEmptyGroup;
+        if (j0 + i * NT < B)
+            got[i] = atomicCAS(slots + (uint64_t)((uint32_t)hh[i] & gmask) * kGroupWords, kEmptyGroup,
+                               (kEmptyGroup & ~0xFFFFull) | slot_fp(hh[i]));
+    }
+#pragma unroll
+    for (int i = 0; i < HB_ITEMS; ++i) {
+        const int64_t j = j0 + i * NT;
+        if (j >= B) break;
+        const uint32_t g = (uint32_t)hh[i] & gmask;
+        if (got[i] == kEmptyGroup) reinterpret_cast<uint32_t*>(slots + (uint64_t)g * kGroupWords + 1)[0] = (uint32_t)j;
+        else hash_insert(slots, gmask, g, slot_fp(hh[i]), (uint32_t)j, got[i], h.err);
+    }
+    if (h.sizes) bucket_sizes<NT, HB_ITEMS>(h, bo, B, j0);
+}
+
+// By parts: k_hash_split orders the keys of a tile by the part of the table
+// (kHashPartGroups groups) that their home group lies in and appends them to
+// the parts' records; k_hash_fill builds a part and its filter words in shared
+// memory and writes them out whole. In place, a key cost three random accesses
+// of L2 or, in tables beyond its size, of memory, and the tables had to be
+// cleared first: 0.66 ms for 16M keys in 16 tables, clearing and sizes included,
+// against 0.38 now; 9.1 ms for 200M in 20 tables, now 5.4. 512 threads x 16 keys
+// a tile: x 8 takes 0.20 instead of 0.23 ms at 16M but 4.1 instead of 3.7 at
+// 200M, whose 4,096 parts leave a tile two keys a part.
+// A record: bucket in the low half; group within the part (11 bits),
+// fingerprint (16) and the filter bit outside it (5) in the high one.
+constexpr int HS_T = 512, HS_ITEMS = 16, HS_TILE = HS_T * HS_ITEMS;
+static_assert(kHashPartGroups == 2048 && HS_TILE <= 8192 && kHashMaxParts <= 4096, "bit fields of a record and of a rank");
+constexpr size_t hash_split_smem(uint32_t parts) { return (size_t)HS_TILE * 10 + (size_t)parts * 8; }
+
+__device__ __forceinline__ void hash_spill(const HashBuild& h, uint32_t* cnt, int l, uint32_t j) {
+    const uint32_t s = atomicAdd(cnt, 1u);
+    if (s < h.spill_cap) h.spill[s] = make_uint2((uint32_t)l, j);
+}
+
+__global__ void __launch_bounds__(HS_T, 2) k_hash_split(HashBuild h, uint32_t parts) {
+    extern __shared__ __align__(16) unsigned char raw[];
+    unsigned long long* buf = reinterpret_cast<unsigned long long*>(raw);              // [HS_TILE]
+    uint16_t* bin = reinterpret_cast<uint16_t*>(raw + (size_t)HS_TILE * 8);            // [HS_TILE]
+    uint32_t* hist = reinterpret_cast<uint32_t*>(raw + (size_t)HS_TILE * 10);          // [parts] counts, then starts
+    uint32_t* gpos = hist + parts;                                                     // [parts] record of position 0
+    __shared__ uint32_t ws[HS_T / 32];
+    const int l = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint64_t bo = h.boff[l];
+    const int64_t B = (int64_t)(h.boff[l + 1] - bo), t0 = (int64_t)blockIdx.x * HS_TILE;
+    if (t0 >= B) return;
+    const uint32_t gmask = h.hmask[l];
+    const uint32_t my_parts = gmask / kHashPartGroups + 1;
+    for (uint32_t i = tid; i < my_parts; i += HS_T) hist[i] = 0;
+    __syncthreads();
+    uint32_t hi[HS_ITEMS], br[HS_ITEMS];   // record's high half; part and rank within it
+#pragma unroll
+    for (int i0 = 0; i0 < HS_ITEMS; i0 += 4) {
+        uint64_t hh[4];
+        key_hashes<false, HS_T, 4>(h, l, bo, B, t0 + i0 * HS_T + tid, hh);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const uint32_t g = (uint32_t)hh[i] & gmask, part = g / kHashPartGroups;
+            hi[i0 + i] = (g % kHashPartGroups) | (slot_fp(hh[i]) << 11) | ((uint32_t)(hh[i] >> 43) << 27);
+            br[i0 + i] = 0;
+            if (t0 + (i0 + i) * HS_T + tid < B) br[i0 + i] = (part << 16) | atomicAdd(hist + part, 1u);
+        }
+    }
+    __syncthreads();
+    // starts of the parts within the tile, and their places among the records
+    const uint32_t per = (my_parts + HS_T - 1) / HS_T;
+    uint32_t sum = 0;
+    for (uint32_t q = 0; q < per; ++q) {
+        const uint32_t b = tid * per + q;
+        if (b < my_parts) sum += hist[b];
+    }
+    uint32_t x = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const uint32_t y = __shfl_up_sync(0xffffffffu, x, o);
+        if (lane >= o) x += y;
+    }
+    if (lane == 31) ws[warp] = x;
+    __syncthreads();
+    uint32_t start = x - sum;
+    for (int w = 0; w < warp; ++w) start += ws[w];
+    for (uint32_t q = 0; q < per; ++q) {
+        const uint32_t b = tid * per + q;
+        if (b >= my_parts) break;
+        const uint32_t c = hist[b];
+        hist[b] = start;
+        if (c) gpos[b] = atomicAdd(h.part_cnt + (size_t)l * parts + b, c) - start;
+        start += c;
+    }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < HS_ITEMS; ++i) {
+        const int64_t j = t0 + i * HS_T + tid;
+        if (j < B) {
+            const uint32_t part = br[i] >> 16, at = hist[part] + (br[i] & 0xFFFFu);
+            buf[at] = ((unsigned long long)hi[i] << 32) | (uint32_t)j;
+            bin[at] = (uint16_t)part;
+        }
+    }
+    __syncthreads();
+    const int n = (int)min((int64_t)HS_TILE, B - t0);
+    for (int sp = tid; sp < n; sp += HS_T) {
+        const uint32_t part = bin[sp], at = gpos[part] + (uint32_t)sp;
+        if (at < kHashPartCap) h.rec[((size_t)l * parts + part) * kHashPartCap + at] = buf[sp];
+        else hash_spill(h, h.part_cnt + (size_t)h.L * parts, l, (uint32_t)buf[sp]);
+    }
+    bucket_sizes<HS_T, HS_ITEMS>(h, bo, B, t0 + tid);
+}
+
+__global__ void __launch_bounds__(NT) k_hash_fill(HashBuild h, uint32_t parts) {
+    extern __shared__ __align__(16) unsigned char raw[];
+    unsigned long long* fps = reinterpret_cast<unsigned long long*>(raw);              // [groups]
+    uint4* idx = reinterpret_cast<uint4*>(raw + (size_t)kHashPartGroups * 8);          // [groups]
+    uint32_t* fw = reinterpret_cast<uint32_t*>(raw + (size_t)kHashPartGroups * 24);    // [groups / 2]
+    const int l = blockIdx.y, tid = threadIdx.x;
+    const uint32_t gmask = h.hmask[l], part = blockIdx.x;
+    const uint32_t my_parts = gmask / kHashPartGroups + 1;
+    if (part >= my_parts) return;
+    const uint32_t groups = min(gmask + 1, kHashPartGroups), words = max(groups / 2, 1u);
+    for (uint32_t i = tid; i < groups; i += NT) {
+        fps[i] = ~0ull;
+        idx[i] = make_uint4(~0u, ~0u, ~0u, ~0u);
+    }
+    for (uint32_t i = tid; i < words; i += NT) fw[i] = 0u;
+    __syncthreads();
+    const size_t base = (size_t)l * parts + part;
+    const unsigned long long* rec = h.rec + base * kHashPartCap;
+    const uint32_t n = min(h.part_cnt[base], kHashPartCap);
+    for (uint32_t i0 = tid; i0 < n; i0 += 4 * NT) {
+        unsigned long long r[4];
+#pragma unroll
+        for (int q = 0; q < 4; ++q) r[q] = i0 + q * NT < n ? __ldcs(rec + i0 + q * NT) : 0ull;
+#pragma unroll
+        for (int q = 0; q < 4; ++q) {
+            if (i0 + q * NT >= n) break;
+            const uint32_t hi = (uint32_t)(r[q] >> 32), fp = (hi >> 11) & 0xFFFFu;
+            uint32_t g = hi & (kHashPartGroups - 1);
+            // filter_bits: bit 43.. of the hash, and bit 5 of the fingerprint on
+            atomicOr(fw + (g >> 1), (1u << (hi >> 27)) | (1u << ((fp >> 5) & 31u)));
+            bool in = false;
+            for (uint32_t p = 0; p < groups && !in; ++p) {
+                unsigned long long cur = *reinterpret_cast<volatile unsigned long long*>(fps + g);
+                for (int tries = 0; tries <= kGroupSlots; ++tries) {
+                    int e = 0;
+                    while (e < kGroupSlots && ((cur >> (16 * e)) & 0xFFFFu) != kEmptyFp) ++e;
+                    if (e == kGroupSlots) break;
+                    const unsigned long long nw = (cur & ~(0xFFFFull << (16 * e))) | ((unsigned long long)fp << (16 * e));
+                    const unsigned long long old = atomicCAS(fps + g, cur, nw);
+                    if (old == cur) {
+                        reinterpret_cast<uint32_t*>(idx + g)[e] = (uint32_t)r[q];
+                        in = true;
+                        break;
+                    }
+                    cur = old;
+                }
+                // the next group; past a part's last one, the insertion in place
+                if (++g == groups) {
+                    if (my_parts > 1) break;
+                    g = 0;
+                }
+            }
+            if (!in) hash_spill(h, h.part_cnt + (size_t)h.L * parts, l, (uint32_t)r[q]);
+        }
+    }
+    __syncthreads();
+    uint4* out = reinterpret_cast<uint4*>(h.hslots + h.hoff[l] + (size_t)part * kHashPartGroups * kGroupWords);
+    for (uint32_t i = tid; i < 2 * groups; i += NT) {
+        const uint4 ix = idx[i >> 1];
+        const unsigned long long f = fps[i >> 1];
+        out[i] = i & 1 ? make_uint4(ix.z, ix.w, ~0u, ~0u) : make_uint4((uint32_t)f, (uint32_t)(f >> 32), ix.x, ix.y);
+    }
+    uint32_t* fo = h.filt + h.fl_off[l] + (size_t)part * (kHashPartGroups / 2);
+    for (uint32_t i = tid; i < words; i += NT) fo[i] = fw[i];
+}
+
+// The spilled keys, in place once every part is written.
+__global__ void k_hash_spilled(HashBuild h, uint32_t parts) {
+    const uint32_t n = min(h.part_cnt[(size_t)h.L * parts], h.spill_cap);
+    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const uint2 s = h.spill[i];
+        const int l = (int)s.x;
+        const uint64_t bo = h.boff[l];
+        uint64_t hh[1];
+        key_hashes<false, 1, 1>(h, l, bo, (int64_t)(h.boff[l + 1] - bo), (int64_t)s.y, hh);
+        const uint32_t gmask = h.hmask[l], g = (uint32_t)hh[0] & gmask;
+        atomicOr(h.filt + h.fl_off[l] + (filter_word(hh[0]) & h.fl_mask[l]), filter_bits(hh[0]));
+        unsigned long long* slots = h.hslots + h.hoff[l];
+        hash_insert(slots, gmask, g, slot_fp(hh[0]), s.y,
+                    *reinterpret_cast<volatile unsigned long long*>(slots + (uint64_t)g * kGroupWords), h.err);
+    }
 }
 
 __global__ void k_decode_codes(const uint64_t* __restrict__ boff, const uint32_t* __restrict__ ukeys, int M, int KW,
@@ -1121,42 +1437,42 @@ cudaError_t launch_run_sorts(const RunLists& rl, int64_t N, int L, int KW, const
 }
 
 cudaError_t launch_rl_count(const SortedKeys& keys, int64_t N, int L, int KW, uint32_t* tile_cnt, uint32_t* tile_off,
-                            uint32_t* nb, cudaStream_t st) {
+                            uint32_t* flags, uint32_t* nb, cudaStream_t st) {
     const int tiles = (int)((N + SP_TILE - 1) / SP_TILE);
-    if (keys.low) k_rl_count<true><<<dim3(tiles, L), NT, 0, st>>>(keys, N, L, KW, tile_cnt);
-    else k_rl_count<false><<<dim3(tiles, L), NT, 0, st>>>(keys, N, L, KW, tile_cnt);
+    if (keys.low) k_rl_count<true><<<dim3(tiles, L), NT, 0, st>>>(keys, N, L, KW, tile_cnt, flags);
+    else k_rl_count<false><<<dim3(tiles, L), NT, 0, st>>>(keys, N, L, KW, tile_cnt, flags);
     k_rl_scan<<<L, NT, 0, st>>>(tile_cnt, tiles, tile_off, nb);
     return cudaGetLastError();
 }
 
-cudaError_t launch_rl_write(const SortedKeys& keys, int64_t N, int L, int KW, const uint32_t* tile_off,
-                            const uint64_t* boff, uint32_t* starts, uint32_t* ukeys, cudaStream_t st) {
+cudaError_t launch_rl_write(const SortedKeys& keys, int64_t N, int L, int KW, const uint32_t* flags,
+                            const uint32_t* tile_off, const uint64_t* boff, uint32_t* starts, uint32_t* ukeys,
+                            cudaStream_t st) {
     const int tiles = (int)((N + SP_TILE - 1) / SP_TILE);
-    if (keys.low) k_rl_write<true><<<dim3(tiles, L), NT, 0, st>>>(keys, N, L, KW, tile_off, boff, starts, ukeys);
-    else k_rl_write<false><<<dim3(tiles, L), NT, 0, st>>>(keys, N, L, KW, tile_off, boff, starts, ukeys);
+    if (keys.low) k_rl_write<true><<<dim3(tiles, L), NT, 0, st>>>(keys, N, L, KW, flags, tile_off, boff, starts, ukeys);
+    else k_rl_write<false><<<dim3(tiles, L), NT, 0, st>>>(keys, N, L, KW, flags, tile_off, boff, starts, ukeys);
     return cudaGetLastError();
 }
 
-cudaError_t launch_bucket_sizes(const uint64_t* boff, const uint32_t* starts, int64_t N, int L, int64_t maxB,
-                                uint32_t* sizes, uint32_t* max_size, cudaStream_t st) {
-    if (maxB <= 0) return cudaSuccess;
-    k_bucket_sizes<<<dim3(blocks_for(maxB), L), NT, 0, st>>>(boff, starts, N, sizes, max_size);
+cudaError_t launch_hash_build(const HashBuild& h, cudaStream_t st) {
+    if (h.maxB <= 0) return cudaSuccess;
+    const dim3 grid((unsigned)((h.maxB + NT * HB_ITEMS - 1) / (NT * HB_ITEMS)), h.L);
+    if (h.KW > 4) k_hash_build<true><<<grid, NT, 0, st>>>(h);
+    else k_hash_build<false><<<grid, NT, 0, st>>>(h);
     return cudaGetLastError();
 }
 
-cudaError_t launch_hash_build(const uint64_t* boff, const uint32_t* ukeys, int L, int M, int KW, int64_t maxB,
-                              const uint16_t* foff, const uint8_t* fbits, const unsigned long long* rmul,
-                              const uint64_t* hoff, const uint32_t* hmask, unsigned long long* hslots,
-                              uint32_t* filt, const uint64_t* fl_off, const uint32_t* fl_mask, int* err,
-                              cudaStream_t st) {
-    if (maxB <= 0) return cudaSuccess;
-    const dim3 grid(blocks_for(maxB), L);
-    if (KW > 4)
-        k_hash_build<true><<<grid, NT, 0, st>>>(boff, ukeys, M, KW, foff, fbits, rmul, hoff, hmask, hslots, filt, fl_off,
-                                               fl_mask, err);
-    else
-        k_hash_build<false><<<grid, NT, 0, st>>>(boff, ukeys, M, KW, foff, fbits, rmul, hoff, hmask, hslots, filt, fl_off,
-                                                fl_mask, err);
+cudaError_t launch_hash_build_parts(const HashBuild& h, cudaStream_t st) {
+    const uint32_t parts = std::max(h.max_groups / kHashPartGroups, 1u);
+    const int split = (int)hash_split_smem(parts), fill = (int)kHashPartGroups * 26;
+    cudaError_t e = cudaFuncSetAttribute(k_hash_split, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)hash_split_smem(kHashMaxParts));
+    if (e != cudaSuccess) return e;
+    if ((e = cudaFuncSetAttribute(k_hash_fill, cudaFuncAttributeMaxDynamicSharedMemorySize, fill)) != cudaSuccess) return e;
+    if ((e = cudaMemsetAsync(h.part_cnt, 0, sizeof(uint32_t) * ((size_t)h.L * parts + 1), st)) != cudaSuccess) return e;
+    k_hash_split<<<dim3((unsigned)((h.maxB + HS_TILE - 1) / HS_TILE), h.L), HS_T, split, st>>>(h, parts);
+    k_hash_fill<<<dim3(parts, h.L), NT, fill, st>>>(h, parts);
+    k_hash_spilled<<<152, NT, 0, st>>>(h, parts);
     return cudaGetLastError();
 }
 

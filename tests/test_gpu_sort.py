@@ -100,3 +100,33 @@ def test_keys_wider_than_128_bits(culsh, M, W):
     want = oracle.search(oracle.build_index(X, A, b, W), X, X[:200], K, T)
     np.testing.assert_array_equal(st.getKnnIds(), want["knn_ids"])
     np.testing.assert_array_equal(st.getKnnDistances(), want["knn_dists"])
+
+
+@pytest.mark.parametrize("form", ["parts", "in place"])
+@pytest.mark.parametrize("N,M,dup", [(1, 8, 1), (3, 8, 1), (4096, 8, 1), (4097, 12, 1), (8191, 12, 3), (20000, 16, 1),
+                                     (60000, 12, 1), (60000, 12, 5000)])
+def test_hash_tables_find_every_bucket(culsh, form, N, M, dup, monkeypatch):
+    """Both forms of the hash tables (by parts of 2,048 groups, one part or
+    many, a last tile of any length; and in place): the points themselves as
+    queries all find their own buckets, and the first probes' buckets are the
+    oracle's."""
+    monkeypatch.setenv("CULSH_HASH_PARTS_MIN", "1" if form == "parts" else "1000000000000")
+    rng = np.random.default_rng(N + M)
+    D, L, W = 16, 3, 2.0
+    X = rng.normal(0, 4, (max(N // dup, 1), D)).astype(np.float32)
+    X = np.ascontiguousarray(X[rng.integers(0, X.shape[0], N)] if dup > 1 else X)
+    A = rng.normal(0, 1, (L, M, D)).astype(np.float32)
+    b = rng.uniform(0, W, (L, M)).astype(np.float32)
+    ht = culsh.HashTables()
+    ht.reset(N, D, L, M, W, A=A, b=b)
+    ht.index(X)
+    q = X[rng.permutation(N)[:2000]]
+    st = culsh.SearchTables()
+    st.reset(ht, 1, 4)
+    st.search(q, dataset=X)
+    ref = oracle.search(oracle.build_index(X, A, b, W), X, q, 1, 4)
+    for l in range(L):
+        qb = st.getQueryBuckets(l)
+        assert (qb[:, 0] >= 0).all()
+        np.testing.assert_array_equal(qb, ref["qbuckets"][l].reshape(q.shape[0], 4), err_msg=f"table {l}")
+    np.testing.assert_array_equal(ht.getBuckets_sizes(0), oracle.build_index(X, A, b, W).sizes(0))

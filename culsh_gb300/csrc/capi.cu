@@ -1700,7 +1700,7 @@ int run_plan(culsh_search* s, const SearchPlan& P, cudaStream_t st) {
         return fail(CULSH_ERR_DEVICE, "search graph instantiation: %s", cudaGetErrorString(ei));
     }
     s->graph = g;
-    s->gproj = P.xcopy ? find_kernel_node(g, project_copy_kernel()) : nullptr;
+    s->gproj = P.xcopy ? find_kernel_node(g, project_copy_kernel(P.Q, P.D, P.LM)) : nullptr;
     s->gsrc = P.dQ;
     std::memcpy(&s->gplan, &key, sizeof(key));
     s->glaunches = launches;

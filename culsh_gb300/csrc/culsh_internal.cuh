@@ -155,9 +155,10 @@ cudaError_t launch_project_fp32(const float* X, int64_t n_pts, int D, const floa
                                 int LM, float W, int32_t* codes, float* vals, int32_t* pmin, int32_t* pmax, int* err,
                                 cudaStream_t st, int tile = 0, ZeroWords zw = ZeroWords{}, float* xcopy = nullptr);
 int project_grid_x(int64_t n_pts);
-// The kernel of tiling 5 (xcopy form), for finding its node in a captured
-// graph, and its number of parameters (the first is the rows it reads).
-const void* project_copy_kernel();
+// The kernel that the xcopy form launches for n_pts rows, for finding its node
+// in a captured graph, and its number of parameters (the first is the rows it
+// reads).
+const void* project_copy_kernel(int64_t n_pts, int D, int LM);
 constexpr int kProjectArgs = 15;
 // n floats, 16-byte aligned source and destination (src may be host memory
 // the device reads directly).

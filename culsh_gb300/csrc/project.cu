@@ -14,6 +14,7 @@
 #include <algorithm>
 #include <cfloat>
 #include <climits>
+#include <type_traits>
 
 #include "culsh_internal.cuh"
 
@@ -226,6 +227,93 @@ __global__ void __launch_bounds__(NT, kCopy ? 2 : 0) k_project(const float* __re
     }
 }
 
+// Few queries: one column per thread, P rows per block of 64 columns, the rows
+// staged whole and a column's next 16 values loaded while 16 are multiplied.
+// Bound by the latency of those loads; the tilings above, made for ten thousand
+// queries, leave most SMs without a block and wait for one stage of 32 dimensions
+// after another (128 dimensions: one query on 64 columns 14 us, now 5; 1,000 on
+// 64 17, now 11; 256 on 192 15, now 10).
+// Same chains, same parameters as k_project (vals only).
+constexpr int FC = 64;     // columns (threads)
+constexpr int FD = 256;    // dimensions at most
+template <int P>
+__global__ void __launch_bounds__(FC) k_project_few(const float* __restrict__ X, int64_t n_pts, int D,
+                                                    const float* __restrict__ AT, int lmp, const float* __restrict__ b,
+                                                    int LM, float W, int32_t*, float* __restrict__ vals, int32_t*,
+                                                    int32_t*, int*, ZeroWords zw, float* __restrict__ xcopy) {
+    __shared__ __align__(16) float xs[P][FD];
+    const int tid = threadIdx.x, c = blockIdx.y * FC + tid;
+    zw.clear(tid);
+    const int64_t n0 = (int64_t)blockIdx.x * P;
+    const int rows = (int)min((int64_t)P, n_pts - n0);
+    const bool vec = (D & 3) == 0 && (reinterpret_cast<uintptr_t>(X) & 15) == 0;
+    const bool copy = xcopy && blockIdx.y == 0;
+    const float* at = AT + min(c, lmp - 1);
+    float acc[P];
+#pragma unroll
+    for (int p = 0; p < P; ++p) acc[p] = 0.0f;
+    const int dp = (D + 15) & ~15;
+    float cur[16], nxt[16];
+#pragma unroll
+    for (int i = 0; i < 16; ++i) cur[i] = i < D ? __ldg(at + (int64_t)i * lmp) : 0.0f;
+    // dimensions past D are zeros: they leave a chain unchanged
+    if (vec) {
+#pragma unroll 4
+        for (int f = tid; f < P * (dp / 4); f += FC) {
+            const int p = f / (dp / 4), d = f % (dp / 4) * 4;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (p < rows && d < D) {
+                v = __ldg(reinterpret_cast<const float4*>(X + (n0 + p) * D + d));
+                if (copy) *reinterpret_cast<float4*>(xcopy + (n0 + p) * D + d) = v;
+            }
+            *reinterpret_cast<float4*>(&xs[p][d]) = v;
+        }
+    } else {
+#pragma unroll 4
+        for (int f = tid; f < P * dp; f += FC) {
+            const int p = f / dp, d = f % dp;
+            const float v = p < rows && d < D ? __ldg(X + (n0 + p) * D + d) : 0.0f;
+            if (copy && p < rows && d < D) xcopy[(n0 + p) * D + d] = v;
+            xs[p][d] = v;
+        }
+    }
+    __syncthreads();
+    for (int d = 0; d < dp; d += 16) {
+#pragma unroll
+        for (int i = 0; i < 16; ++i) nxt[i] = d + 16 + i < D ? __ldg(at + (int64_t)(d + 16 + i) * lmp) : 0.0f;
+#pragma unroll
+        for (int i = 0; i < 16; i += 4)
+#pragma unroll
+            for (int p = 0; p < P; ++p) {
+                const float4 x = *reinterpret_cast<const float4*>(&xs[p][d + i]);
+                acc[p] = __fmaf_rn(x.x, cur[i], acc[p]);
+                acc[p] = __fmaf_rn(x.y, cur[i + 1], acc[p]);
+                acc[p] = __fmaf_rn(x.z, cur[i + 2], acc[p]);
+                acc[p] = __fmaf_rn(x.w, cur[i + 3], acc[p]);
+            }
+#pragma unroll
+        for (int i = 0; i < 16; ++i) cur[i] = nxt[i];
+    }
+    if (c >= LM) return;
+    const float bc = __ldg(b + c);
+    float* out = vals + (int64_t)c * n_pts + n0;
+#pragma unroll
+    for (int p = 0; p < P; ++p)
+        if (p < rows) out[p] = __fdiv_rn(__fsub_rn(acc[p], bc), W);
+}
+
+// Rows per block of the few-queries form, 0 where the tilings take over: when
+// they have more than 64 blocks, or more than 256 dimensions (all blocks read
+// the same rows of AT at the same time: 256 queries of 960 dimensions on 512
+// columns take 58 us in both, 1,000 take 68 and 58).
+int few_rows(int64_t n_pts, int D, int LM) {
+    if (D > 256 || ((n_pts + 63) / 64) * ((LM + 127) / 128) > 64) return 0;
+    return n_pts <= 64 ? 2 : 8;
+}
+typedef void (*FewKernel)(const float*, int64_t, int, const float*, int, const float*, int, float, int32_t*, float*,
+                          int32_t*, int32_t*, int*, ZeroWords, float*);
+FewKernel few_kernel(int rows) { return rows == 2 ? k_project_few<2> : k_project_few<8>; }
+
 // Wide tiling of the index build's projection: 128 points x 128 columns per
 // block, 8 x 8 outputs per thread, 16 dimensions per stage, two stages in shared
 // memory (the next one's loads are in registers while this one is multiplied).
@@ -414,7 +502,11 @@ cudaError_t launch_project_fp32(const float* X, int64_t n_pts, int D, const floa
     // xcopy (the rows also written to device memory as they are read): one
     // column block, so that every row is read exactly once
     if (xcopy && (codes || tile != 5 || LM > 192)) return cudaErrorInvalidValue;
-    if (codes && LM > 64) {
+    const int few = !codes && (tile == 0 || tile == 5) ? few_rows(n_pts, D, LM) : 0;
+    if (few) {
+        few_kernel(few)<<<dim3((unsigned)((n_pts + few - 1) / few), (LM + FC - 1) / FC), FC, 0, st>>>(
+            X, n_pts, D, AT, lmp, b, LM, W, nullptr, vals, nullptr, nullptr, err, zw, xcopy);
+    } else if (codes && LM > 64) {
         // one column block of 64 (LM <= 64) would leave half of the wide tile idle
         k_project_wide<<<dim3(project_grid_x(n_pts), (LM + WB - 1) / WB), NT, 0, st>>>(X, n_pts, D, AT, lmp, b, LM, W,
                                                                                      codes, pmin, pmax, err);
@@ -452,7 +544,13 @@ struct arity<R(A...)> {
 };
 static_assert(arity<decltype(k_project<false, 2, 12, 32, true>)>::value == kProjectArgs, "projection parameters");
 
-const void* project_copy_kernel() { return reinterpret_cast<const void*>(&k_project<false, 2, 12, 32, true>); }
+static_assert(arity<std::remove_pointer_t<FewKernel>>::value == kProjectArgs, "projection parameters");
+
+const void* project_copy_kernel(int64_t n_pts, int D, int LM) {
+    const int few = few_rows(n_pts, D, LM);
+    if (few) return reinterpret_cast<const void*>(few_kernel(few));
+    return reinterpret_cast<const void*>(&k_project<false, 2, 12, 32, true>);
+}
 
 cudaError_t launch_minmax_reduce(const int32_t* pmin, const int32_t* pmax, int nparts, int LM, int32_t* cmin,
                                  int32_t* cmax, cudaStream_t st) {

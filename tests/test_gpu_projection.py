@@ -71,3 +71,36 @@ def test_simt_codes(culsh, N, D, L, M, monkeypatch):
     X = features("plain", N, D, rng)
     A, b = projection(L, M, D, 3.0, rng)
     assert check(culsh, X, A, b, 3.0)["tensor_cores"] == 0
+
+
+@pytest.mark.parametrize("Q", [1, 2, 3, 64, 65, 511])
+@pytest.mark.parametrize("D,L,M", [(128, 3, 7), (256, 5, 13), (256, 3, 8), (33, 4, 16), (15, 1, 3), (257, 3, 8)])
+def test_few_queries(culsh, Q, D, L, M):
+    """The few-queries projection (2 or 8 rows a block of 64 columns, up to 256
+    dimensions) and the tiling past it, on host rows and on device rows: probes
+    and distances are the oracle's."""
+    torch = pytest.importorskip("torch")
+    rng = np.random.default_rng(Q + D + L)
+    N, K, T, W = 3000, 5, 6, 12.0
+    X = rng.normal(0, 2, (N, D)).astype(np.float32)
+    q = np.ascontiguousarray(X[rng.integers(0, N, Q)] + 0.1 * rng.normal(0, 1, (Q, D)), np.float32)
+    A, b = projection(L, M, D, W, rng)
+    ht = culsh.HashTables()
+    ht.reset(N, D, L, M, W, A=A, b=b)
+    ht.index(X)
+    ref = oracle.search(oracle.build_index(X, A, b, W), X, q, K, T)
+    st = culsh.SearchTables()
+    st.reset(ht, K, T)
+    for _ in range(2):
+        st.search(q, dataset=X)
+        for l in range(L):
+            np.testing.assert_array_equal(st.getQueryBuckets(l), ref["qbuckets"][l].reshape(Q, T), err_msg=f"table {l}")
+        np.testing.assert_array_equal(st.getKnnIds(), ref["knn_ids"])
+        np.testing.assert_array_equal(st.getKnnDistances(), ref["knn_dists"])
+    dq = torch.from_numpy(q).cuda()
+    ids = torch.empty(Q * K, dtype=torch.int32, device="cuda")
+    dists = torch.empty(Q * K, dtype=torch.float32, device="cuda")
+    st.search_device(dq.data_ptr(), Q, ids.data_ptr(), dists.data_ptr())
+    torch.cuda.synchronize()
+    np.testing.assert_array_equal(ids.cpu().numpy(), ref["knn_ids"].astype(np.int32).reshape(-1))
+    np.testing.assert_array_equal(dists.cpu().numpy(), ref["knn_dists"].reshape(-1))

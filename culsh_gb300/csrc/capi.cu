@@ -760,6 +760,7 @@ int sort_keys(culsh_index* ix, int N, int passes, bool all_words, cudaStream_t s
         rl.llen = ix->ws_run_len.p + tcap + scap;
         rl.lcap = lcap;
         rl.cnt = ix->ws_run_cnt.p;
+        rl.same = ix->ws_status.p;
         CU_TRY(launch_run_find(top, N, L, KW, ix->ws_low.p, ix->ids.p, rl, st));
         CU_TRY(launch_run_sorts(rl, N, L, KW, ix->ws_low.p, ix->ids.p, st));
         CU_TRY(cudaMemcpyAsync(ix->h_run_cnt.p, rl.cnt, 4 * sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
@@ -827,7 +828,8 @@ int build_device(culsh_index* ix, const float* dX, cudaStream_t st, FILE* dbg) {
     for (int all_words = 0; all_words < 2; ++all_words) {
         TRY(sort_keys(ix, N, passes, all_words != 0, st, &skeys));
         CU_TRY(cudaEventRecord(ix->bev[3], st));
-        // Run-length bucketing (the boundary flags take the place of the sort's tile states).
+        // Run-length bucketing (its flags, like the runs' marks, take the place of
+        // the sort's tile states).
         CU_TRY(launch_rl_count(skeys, N, L, ix->KW, ix->ws_tcnt.p, ix->ws_toff.p, ix->ws_status.p, ix->ws_nb.p, st));
         CU_TRY(cudaMemcpyAsync(ix->h_nb.p, ix->ws_nb.p, 4 * L, cudaMemcpyDeviceToHost, st));
         CU_TRY(cudaStreamSynchronize(st));

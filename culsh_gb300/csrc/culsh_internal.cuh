@@ -251,6 +251,7 @@ struct RunLists {
     unsigned long long* lpos;   // runs of 33..run_max_len()
     uint32_t* llen;
     unsigned int lcap;
+    uint32_t* same;             // bit per sorted position: same key as the one before (launch_rl_count's flags)
     unsigned int* cnt;          // [4]: tiny, small and large runs; overflow flags (1 run too long, 2 list full)
 };
 cudaError_t launch_run_find(const uint32_t* top, int64_t N, int L, int KW, const uint32_t* low, uint32_t* ids,

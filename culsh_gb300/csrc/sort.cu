@@ -510,11 +510,27 @@ __device__ __forceinline__ bool run_less(const uint32_t (&a)[KWL + 1], const uin
     return a[KWL] < b[KWL];
 }
 
+// Marks sorted position i of table l as holding the same whole key as position
+// i - 1 (words of 32 positions, tables padded to 4,096-position tiles: the
+// layout of the boundary flags).
+__device__ __forceinline__ void mark_same(uint32_t* same, int64_t N, int64_t l, int64_t i) {
+    atomicOr(same + l * ((N + SP_TILE - 1) / SP_TILE * (SP_TILE / 32)) + (i >> 5), 1u << (i & 31));
+}
+template <int KWL>
+__device__ __forceinline__ bool same_row(const uint32_t* a, const uint32_t* b) {
+    bool eq = true;
+#pragma unroll
+    for (int k = 0; k < KWL; ++k) eq = eq && a[k] == b[k];
+    return eq;
+}
+
 // Runs of two or more equal top words, found from their first element. Runs of
 // two, by far the most where points fall nearly alone (of 200M positions of the
-// 10M-point build more than the lists hold), are ordered here; longer ones go
-// to three lists: 3..8 (tiny), 9..32 (small), 33..kRunMax (large); a longer
-// run or a full list sets cnt[3] (the caller then sorts all words instead).
+// 10M-point build more than the lists hold), are ordered here (by the thread
+// that meets them: collected per block first, one to four pairs in flight a
+// thread, the kernel takes 13 to 70 % longer); longer ones go to three lists:
+// 3..8 (tiny), 9..32 (small), 33..kRunMax (large); a longer run or a full list
+// sets cnt[3] (the caller then sorts all words instead).
 // Block (x, table y) examines RUN_TILE positions from shared memory, one
 // position in RUN_ITEMS rows per thread (consecutive threads, consecutive
 // positions). List slots are claimed per block (shared counters, then one
@@ -573,6 +589,7 @@ __global__ void __launch_bounds__(NT) k_run_find(const uint32_t* __restrict__ to
                     ids[seg + i] = b[KWL];
                     ids[seg + i + 1] = a[KWL];
                 }
+                if (same_row<KWL>(a, b)) mark_same(rl.same, N, blockIdx.y, i + 1);
             }
         }
         len[k] = n;
@@ -610,12 +627,12 @@ template <int KWL>
 __global__ void k_run_sort_tiny(const unsigned long long* __restrict__ tpos, const uint32_t* __restrict__ tlen,
                                 const unsigned int* __restrict__ cnt, unsigned int tcap, int64_t N,
                                 const uint32_t* __restrict__ low,
-                                uint32_t* __restrict__ ids) {
+                                uint32_t* __restrict__ ids, uint32_t* __restrict__ same) {
     const unsigned int nrun = min(cnt[0], tcap);
     for (unsigned int r = blockIdx.x * blockDim.x + threadIdx.x; r < nrun; r += gridDim.x * blockDim.x) {
         const int64_t pos = (int64_t)tpos[r];
         const int len = (int)tlen[r];
-        const int64_t seg = pos / N * N;
+        const int64_t l = pos / N, seg = l * N;
         uint32_t e[8][KWL + 1];
 #pragma unroll
         for (int t = 0; t < 8; ++t) {
@@ -643,6 +660,7 @@ __global__ void k_run_sort_tiny(const unsigned long long* __restrict__ tpos, con
 #pragma unroll
         for (int t = 0; t < 8; ++t) {
             if (t < len) ids[pos + t] = e[t][KWL];
+            if (t > 0 && t < len && same_row<KWL>(e[t], e[t - 1])) mark_same(same, N, l, pos - seg + t);
         }
     }
 }
@@ -653,14 +671,14 @@ template <int KWL>
 __global__ void k_run_sort_small(const unsigned long long* __restrict__ spos, const uint32_t* __restrict__ slen,
                                  const unsigned int* __restrict__ cnt, unsigned int scap, int64_t N,
                                  const uint32_t* __restrict__ low,
-                                uint32_t* __restrict__ ids) {
+                                uint32_t* __restrict__ ids, uint32_t* __restrict__ same) {
     const int lane = threadIdx.x & 31;
     const unsigned int nrun = min(cnt[1], scap);
     for (unsigned int r = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; r < nrun;
          r += (gridDim.x * blockDim.x) >> 5) {
         const int64_t pos = (int64_t)spos[r];
         const int len = (int)slen[r];
-        const int64_t seg = pos / N * N;
+        const int64_t l = pos / N, seg = l * N;
         uint32_t e[KWL + 1];
 #pragma unroll
         for (int k = 0; k <= KWL; ++k) e[k] = 0xFFFFFFFFu;
@@ -684,6 +702,10 @@ __global__ void k_run_sort_small(const unsigned long long* __restrict__ spos, co
             }
         }
         if (lane < len) ids[pos + lane] = e[KWL];
+        uint32_t prev[KWL];
+#pragma unroll
+        for (int c = 0; c < KWL; ++c) prev[c] = __shfl_up_sync(0xffffffffu, e[c], 1);
+        if (lane > 0 && lane < len && same_row<KWL>(e, prev)) mark_same(same, N, l, pos - seg + lane);
     }
 }
 
@@ -693,13 +715,13 @@ __global__ void __launch_bounds__(NT) k_run_sort_large(const unsigned long long*
                                                       const uint32_t* __restrict__ llen,
                                                       const unsigned int* __restrict__ cnt, unsigned int lcap,
                                                       int64_t N, const uint32_t* __restrict__ low,
-                                                      uint32_t* __restrict__ ids) {
+                                                      uint32_t* __restrict__ ids, uint32_t* __restrict__ same) {
     __shared__ uint32_t sv[KWL + 1][kRunMax];
     const unsigned int nrun = min(cnt[2], lcap);
     for (unsigned int r = blockIdx.x; r < nrun; r += gridDim.x) {
         const int64_t pos = (int64_t)lpos[r];
         const int len = (int)llen[r];
-        const int64_t seg = pos / N * N;
+        const int64_t l = pos / N, seg = l * N;
         int n2 = 64;
         while (n2 < len) n2 <<= 1;
         for (int t = threadIdx.x; t < n2; t += NT) {
@@ -738,7 +760,13 @@ __global__ void __launch_bounds__(NT) k_run_sort_large(const unsigned long long*
                 __syncthreads();
             }
         }
-        for (int t = threadIdx.x; t < len; t += NT) ids[pos + t] = sv[KWL][t];
+        for (int t = threadIdx.x; t < len; t += NT) {
+            ids[pos + t] = sv[KWL][t];
+            bool eq = t > 0;
+#pragma unroll
+            for (int c = 0; c < KWL; ++c) eq = eq && sv[c][t] == sv[c][t > 0 ? t - 1 : 0];
+            if (eq) mark_same(same, N, l, pos - seg + t);
+        }
         __syncthreads();
     }
 }
@@ -756,17 +784,20 @@ __device__ __forceinline__ uint4 low_words(const uint32_t* __restrict__ low, int
 // Bucket boundaries of one tile of 4,096 sorted positions: warp w takes positions
 // [512 w, 512 w + 512) as 16 rows of 32 lanes. A position whose key differs
 // from its predecessor's starts a bucket; flags gets one word per row, tile_cnt
-// the tile's total. LOW: top-word-first form, keys = the sorted top words, low =
-// lower words by point, looked up only where two top words are equal; four
-// rows' lookups are in flight together. Otherwise keys = KW arrays of L*N words.
+// the tile's total. LOW: top-word-first form, keys = the sorted top words, flags
+// hold the positions whose whole key equals the one before (looking up the lower
+// words again had taken 1.65 ms at 200M positions, now 0.19). Otherwise keys =
+// KW arrays of L*N words.
 template <bool LOW>
 __global__ void __launch_bounds__(NT) k_rl_count(SortedKeys s, int64_t N, int L, int KW, uint32_t* __restrict__ tile_cnt,
-                                                 uint32_t* __restrict__ flags) {
+                                                 uint32_t* flags) {
     __shared__ uint32_t ws[SP_WARPS];
     const int l = blockIdx.y, tile = blockIdx.x, tiles = gridDim.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const int64_t LN = (int64_t)L * N, seg = (int64_t)l * N;
     const int64_t w0 = (int64_t)tile * SP_TILE + (int64_t)warp * (32 * SP_ITEMS);
+    uint32_t* fl = flags + ((int64_t)l * tiles + tile) * (SP_TILE / 32) + warp * SP_ITEMS;
+    const uint32_t marks = LOW && lane < SP_ITEMS ? fl[lane] : 0u;
     uint32_t mine = 0;
 #pragma unroll
     for (int k0 = 0; k0 < SP_ITEMS; k0 += 4) {
@@ -777,25 +808,12 @@ __global__ void __launch_bounds__(NT) k_rl_count(SortedKeys s, int64_t N, int L,
             same[q] = i > 0 && i < N && s.keys[seg + i] == s.keys[seg + i - 1];
         }
         if constexpr (LOW) {
-            uint32_t ia[4], ib[4];
+            // the runs' sorts marked the positions whose lower words are equal too
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                const int64_t i = w0 + (k0 + q) * 32 + lane;
-                ia[q] = same[q] ? s.ids[seg + i] : 0u;
-                ib[q] = same[q] ? s.ids[seg + i - 1] : 0u;
+                const uint32_t row = __shfl_sync(0xffffffffu, marks, k0 + q);   // by all lanes
+                same[q] = same[q] && ((row >> lane) & 1u);
             }
-            uint4 x[4], y[4];
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                x[q] = y[q] = make_uint4(0, 0, 0, 0);
-                if (same[q]) {
-                    x[q] = low_words(s.low, s.lw, seg + ia[q]);
-                    y[q] = low_words(s.low, s.lw, seg + ib[q]);
-                }
-            }
-#pragma unroll
-            for (int q = 0; q < 4; ++q)
-                same[q] = same[q] && x[q].x == y[q].x && x[q].y == y[q].y && x[q].z == y[q].z;
         } else {
             for (int w = 1; w < KW; ++w)
 #pragma unroll
@@ -811,7 +829,7 @@ __global__ void __launch_bounds__(NT) k_rl_count(SortedKeys s, int64_t N, int L,
             if (lane == k0 + q) mine = ball;
         }
     }
-    if (lane < SP_ITEMS) flags[((int64_t)l * tiles + tile) * (SP_TILE / 32) + warp * SP_ITEMS + lane] = mine;
+    if (lane < SP_ITEMS) fl[lane] = mine;
     const uint32_t c = __reduce_add_sync(0xffffffffu, (uint32_t)__popc(mine));
     if (lane == 0) ws[warp] = c;
     __syncthreads();
@@ -1400,6 +1418,8 @@ cudaError_t launch_run_find(const uint32_t* top, int64_t N, int L, int KW, const
                             const RunLists& rl, cudaStream_t st) {
     cudaError_t e = cudaMemsetAsync(rl.cnt, 0, 4 * sizeof(unsigned int), st);
     if (e != cudaSuccess) return e;
+    e = cudaMemsetAsync(rl.same, 0, sizeof(uint32_t) * (size_t)L * ((N + SP_TILE - 1) / SP_TILE) * (SP_TILE / 32), st);
+    if (e != cudaSuccess) return e;
     const dim3 grid((unsigned)((N + RUN_TILE - 1) / RUN_TILE), (unsigned)L);
     switch (KW - 1) {
     case 1: k_run_find<1><<<grid, NT, 0, st>>>(top, N, low, ids, rl); break;
@@ -1419,9 +1439,9 @@ void launch_run_sorts_w(const RunLists& rl, int64_t LN, int64_t N, const uint32_
     const unsigned gt = (unsigned)std::min<int64_t>((LN / 3 + NT - 1) / NT + 1, 152 * 16);
     const unsigned gs = (unsigned)std::min<int64_t>((LN / 9 * 32 + NT - 1) / NT + 1, 152 * 16);
     const unsigned gl = (unsigned)std::min<int64_t>(LN / 33 + 1, 152 * 4);
-    k_run_sort_tiny<KWL><<<gt, NT, 0, st>>>(rl.tpos, rl.tlen, rl.cnt, rl.tcap, N, low, ids);
-    k_run_sort_small<KWL><<<gs, NT, 0, st>>>(rl.spos, rl.slen, rl.cnt, rl.scap, N, low, ids);
-    k_run_sort_large<KWL><<<gl, NT, 0, st>>>(rl.lpos, rl.llen, rl.cnt, rl.lcap, N, low, ids);
+    k_run_sort_tiny<KWL><<<gt, NT, 0, st>>>(rl.tpos, rl.tlen, rl.cnt, rl.tcap, N, low, ids, rl.same);
+    k_run_sort_small<KWL><<<gs, NT, 0, st>>>(rl.spos, rl.slen, rl.cnt, rl.scap, N, low, ids, rl.same);
+    k_run_sort_large<KWL><<<gl, NT, 0, st>>>(rl.lpos, rl.llen, rl.cnt, rl.lcap, N, low, ids, rl.same);
 }
 
 cudaError_t launch_run_sorts(const RunLists& rl, int64_t N, int L, int KW, const uint32_t* low, uint32_t* ids,

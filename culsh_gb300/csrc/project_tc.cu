@@ -356,7 +356,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         const int quad = warp & 3;                 // TMEM lane quadrant this warp may access
         const int part = ew >> 2;                  // which quarter of the column chunks
         const int row = quad * 32 + lane;
-        const int nchunk = a.LMp / 16;
+        const int nchunk = (a.LM + 15) / 16;       // the last column block may hold fewer than LMp / 16
         const int ch0 = part * nchunk / 4, ch1 = (part + 1) * nchunk / 4;
         uint32_t* my_mask = s_unsure + ew * 32 + lane;   // word w at my_mask[w * TC_EPI_WARPS * 32]
         unsigned long long* region = a.relist + (unsigned long long)blockIdx.x * a.relist_cap;

@@ -63,6 +63,20 @@ def test_tensor_core_codes(culsh, kind, D, L, M, monkeypatch):
     assert check(culsh, X, A, b, W)["tensor_cores"] == 1
 
 
+@pytest.mark.parametrize("D,L,M", [(216, 14, 7), (256, 5, 13), (250, 10, 11), (200, 3, 37)])
+def test_narrow_last_column_block(culsh, D, L, M):
+    """Two column blocks of which the last holds at least sixteen columns
+    fewer: only columns that exist are recomputed (each other column of a block
+    would add a code per point)."""
+    rng = np.random.default_rng(D + L)
+    N = 6001
+    X = features("plain", N, D, rng)
+    W = float(2 * np.sqrt(D))
+    A, b = projection(L, M, D, W, rng)
+    p = check(culsh, X, A, b, W)
+    assert p["tensor_cores"] == 1 and p["recomputed"] < 0.02 * N * L * M
+
+
 @pytest.mark.parametrize("N,D,L,M", [(1027, 33, 4, 16), (1027, 33, 5, 13), (130, 128, 8, 16), (2049, 130, 3, 43),
                                      (127, 7, 16, 16), (5, 64, 6, 12)])
 def test_simt_codes(culsh, N, D, L, M, monkeypatch):

@@ -9,6 +9,8 @@
 //    deduplicate disjoint id sets (each fits the shared-memory set) and can be
 //    processed by different CTAs. Queries without candidates get their padded
 //    output ((-1, FLT_MAX) x K) right there.
+//    Queries of at most kSmallMax go to k_candidates_small (one warp each), dense
+//    ones to the membership rows below.
 //  * k_candidates_ws is a persistent grid that claims items with an atomic
 //    counter (work stealing). Each item yields an exact top-K over its id
 //    partition; the last item of a query to finish merges the P partial lists
@@ -421,7 +423,7 @@ __global__ void __launch_bounds__(32 * SMW) k_candidates_small(WsArgs a) {
     }
 }
 
-template <int WT, int W_SLOTS>
+template <int WT, int W_SLOTS, bool STAGED>
 __global__ void __launch_bounds__(WT) k_candidates_ws(WsArgs a) {
     constexpr int WW = WT / 32;
     constexpr uint32_t W_CAP = W_SLOTS / 2;
@@ -435,10 +437,11 @@ __global__ void __launch_bounds__(WT) k_candidates_ws(WsArgs a) {
     const int D = a.D, K = a.K, L = a.L, T = a.T;
     const int Dp = (D + 3) & ~3;
     // rows staged by bulk copies where they start on 16-byte boundaries
-    const bool staged = row_staged(D) && (reinterpret_cast<uintptr_t>(a.X) & 15) == 0;
-    float* stage = reinterpret_cast<float*>(smem + warp * row_stage_bytes(D));
+    const size_t stage_bytes = STAGED ? row_stage_bytes(D) : 0;
+    const bool staged = STAGED && row_staged(D) && (reinterpret_cast<uintptr_t>(a.X) & 15) == 0;
+    float* stage = reinterpret_cast<float*>(smem + warp * stage_bytes);
     uint32_t phase = 0;
-    float* qs = reinterpret_cast<float*>(smem + WW * row_stage_bytes(D));
+    float* qs = reinterpret_cast<float*>(smem + WW * stage_bytes);
     uint32_t* hset = reinterpret_cast<uint32_t*>(qs + Dp);                        // [W_SLOTS], then the entries
     unsigned long long* ent = reinterpret_cast<unsigned long long*>(hset);       // [W_CAP]
     uint32_t* ulist = hset + W_SLOTS;                                            // [W_CAP], then positions
@@ -1062,14 +1065,23 @@ __global__ void __launch_bounds__(DT, 1) k_knn_scan_rows(KnnSearch k) {
 // query's bucket ids (every matched bucket over the L tables and T probes,
 // as the reference's candidate lists, cuLSH_SearchTables.cu:321-364) and
 // copied out once; their count is the query's unique candidate count.
-// Persistent grid, one query per CTA at a time, 1024 threads. The matched
-// buckets are cut into units of at most BSEG consecutive ids; warp w takes
-// units w, w + 32, ..., loads 32 x BU ids at a time (coalesced: a bucket's
-// ids are contiguous, BU loads in flight per lane) and ORs their bits in.
-// A matched bucket that has a bucket row (a.big_rows; up to BROWS of them
-// per query) sets no bits: its row is ORed into the words as they are copied
-// out, which replaces one shared-memory atomic per id by one 16-byte load
-// per four words. The set is the same either way.
+// Persistent grid, one query per CTA at a time, 1024 threads. A dataset whose
+// bits do not fit shared memory (more than about 1.6M points) takes one sweep
+// over the query's ids per segment of it. The matched buckets of a chunk of
+// slots form one flattened list of ids; warps take 32 x BU of them in turn
+// (BU loads in flight per lane) and OR their bits in. Two kinds of buckets do
+// better, both laid out once per index; the set is the same either way:
+//  - a bucket row (a.big_rows, of the largest buckets; up to BROWS of them per
+//    query) is ORed into the words as they are copied out: one 16-byte load
+//    per four words instead of one shared-memory atomic per id;
+//  - a bank list (k_bank_fill, other buckets of 512 ids or more, where one
+//    segment holds the dataset): 16-bit entries, 32 of which a warp ORs into
+//    32 different banks.
+// Bound by the shared-memory atomics. 10,000 queries of 743k ids each over 1M
+// points: 4.65 ms id by id, 3.8 with bucket rows, 3.45 with bank lists too.
+// Prefetching the next entries into registers spills (4.23 ms when the rest
+// took 3.6); padding entries that are compared instead of ORed into a spare
+// row 4.97.
 constexpr int BT = 1024;
 constexpr int BU = 8;
 constexpr int BCH = 512;   // (table, probe) slots per compaction chunk
@@ -1390,10 +1402,10 @@ __global__ void k_big_find(const uint32_t* __restrict__ sizes, uint64_t totB, ui
 // entries into 32 different banks: entry slot [group][bank][4] holds four
 // ids of one bank. Every bank gets as many slots as an even split of the
 // bucket would fill; a bank with fewer ids fills the rest with an entry of the
-// word row past the bitmap (never copied out), one with more sends the remaining ids to the bucket's tail (32-bit ids). The order
-// within a bank is arbitrary: the entries are ORed. 32 random banks cost 3.5
-// cycles a warp instruction, distinct ones one, and an entry is half an id:
-// (figures at k_cand_bitmap).
+// word row past the bitmap (never copied out), one with more sends the remaining
+// ids to the bucket's tail (32-bit ids). The order within a bank is arbitrary: the
+// entries are ORed. 32 random banks cost 3.5 cycles a warp instruction, distinct
+// ones 1.6, and an entry is half an id (figures at k_cand_bitmap).
 constexpr int BF = 256;
 __global__ void __launch_bounds__(BF) k_bank_fill(const uint64_t* __restrict__ gi, const unsigned int* __restrict__ n,
                                                  unsigned int cap, const uint64_t* __restrict__ boff, int L,
@@ -1497,10 +1509,12 @@ size_t dense_smem_bytes(int64_t N, int D, int K) {
     return sizeof(float) * (size_t)((D + 3) & ~3) + 4 * nwp + scan_bytes(K);
 }
 
-size_t ws_smem_bytes(int D, int K, int wt, int bf16, int slots) {
+size_t ws_smem_bytes(int D, int K, int wt, WsForm form, int slots) {
     const size_t cap = (size_t)slots / 2;
-    return (bf16 ? 0 : (size_t)(wt / 32) * row_stage_bytes(D)) + sizeof(float) * (size_t)((D + 3) & ~3) + sizeof(uint32_t) * ((size_t)slots + cap) +
-           (size_t)(bf16 ? wt / 32 : 1) * K * (sizeof(float) + sizeof(uint32_t)) + (bf16 ? 2 * sizeof(float) * cap : 0);
+    const bool bf16 = form == WsForm::bf16;
+    return (form == WsForm::staged ? (size_t)(wt / 32) * row_stage_bytes(D) : 0) + sizeof(float) * (size_t)((D + 3) & ~3) +
+           sizeof(uint32_t) * ((size_t)slots + cap) + (size_t)(bf16 ? wt / 32 : 1) * K * (sizeof(float) + sizeof(uint32_t)) +
+           (bf16 ? 2 * sizeof(float) * cap : 0);
 }
 
 cudaError_t launch_order_queries(const WsArgs& a, cudaStream_t st) {
@@ -1521,54 +1535,54 @@ cudaError_t launch_plan_items(const WsArgs& a, cudaStream_t st) {
 }
 
 namespace {
-template <int WT, bool kBF16, int SL>
+template <int WT, WsForm kForm, int SL>
 std::atomic<size_t>& ws_smem_cap() {
     static std::atomic<size_t> cap{0};   // dynamic shared memory this kernel is opted into
     return cap;
 }
 
-template <int WT, bool kBF16, int SL>
+template <int WT, WsForm kForm, int SL>
 constexpr auto ws_kernel() {
-    if constexpr (kBF16) return &k_candidates_ws_bf16<WT, SL>;
-    else return &k_candidates_ws<WT, SL>;
+    if constexpr (kForm == WsForm::bf16) return &k_candidates_ws_bf16<WT, SL>;
+    else return &k_candidates_ws<WT, SL, kForm == WsForm::staged>;
 }
 
-template <int WT, bool kBF16, int SL>
+template <int WT, WsForm kForm, int SL>
 cudaError_t launch_ws_v(const WsArgs& a, int grid, cudaStream_t st) {
-    const size_t smem = ws_smem_bytes(a.D, a.K, WT, kBF16, SL);
-    const cudaError_t e = opt_in_smem(ws_kernel<WT, kBF16, SL>(), smem, ws_smem_cap<WT, kBF16, SL>());
+    const size_t smem = ws_smem_bytes(a.D, a.K, WT, kForm, SL);
+    const cudaError_t e = opt_in_smem(ws_kernel<WT, kForm, SL>(), smem, ws_smem_cap<WT, kForm, SL>());
     if (e != cudaSuccess) return e;
-    ws_kernel<WT, kBF16, SL>()<<<grid, WT, smem, st>>>(a);
+    ws_kernel<WT, kForm, SL>()<<<grid, WT, smem, st>>>(a);
     return cudaGetLastError();
 }
 
-template <int WT, bool kBF16, int SL>
+template <int WT, WsForm kForm, int SL>
 int ws_bps_v(int D, int K) {
     int n = 0;
-    const size_t smem = ws_smem_bytes(D, K, WT, kBF16, SL);
-    if (opt_in_smem(ws_kernel<WT, kBF16, SL>(), smem, ws_smem_cap<WT, kBF16, SL>()) != cudaSuccess) return 1;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ws_kernel<WT, kBF16, SL>(), WT, smem) != cudaSuccess)
+    const size_t smem = ws_smem_bytes(D, K, WT, kForm, SL);
+    if (opt_in_smem(ws_kernel<WT, kForm, SL>(), smem, ws_smem_cap<WT, kForm, SL>()) != cudaSuccess) return 1;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, ws_kernel<WT, kForm, SL>(), WT, smem) != cudaSuccess)
         n = 1;
     return n > 0 ? n : 1;
 }
 
-template <bool kBF16, int SL>
+template <WsForm kForm, int SL>
 cudaError_t launch_ws_w(const WsArgs& a, int grid, cudaStream_t st) {
     switch (a.wt) {
-        case 64: return launch_ws_v<64, kBF16, SL>(a, grid, st);
-        case 256: return launch_ws_v<256, kBF16, SL>(a, grid, st);
-        case 512: return launch_ws_v<512, kBF16, SL>(a, grid, st);
-        default: return launch_ws_v<128, kBF16, SL>(a, grid, st);
+        case 64: return launch_ws_v<64, kForm, SL>(a, grid, st);
+        case 256: return launch_ws_v<256, kForm, SL>(a, grid, st);
+        case 512: return launch_ws_v<512, kForm, SL>(a, grid, st);
+        default: return launch_ws_v<128, kForm, SL>(a, grid, st);
     }
 }
 
-template <bool kBF16, int SL>
+template <WsForm kForm, int SL>
 int ws_bps_w(int D, int K, int wt) {
     switch (wt) {
-        case 64: return ws_bps_v<64, kBF16, SL>(D, K);
-        case 256: return ws_bps_v<256, kBF16, SL>(D, K);
-        case 512: return ws_bps_v<512, kBF16, SL>(D, K);
-        default: return ws_bps_v<128, kBF16, SL>(D, K);
+        case 64: return ws_bps_v<64, kForm, SL>(D, K);
+        case 256: return ws_bps_v<256, kForm, SL>(D, K);
+        case 512: return ws_bps_v<512, kForm, SL>(D, K);
+        default: return ws_bps_v<128, kForm, SL>(D, K);
     }
 }
 
@@ -1609,16 +1623,22 @@ cudaError_t launch_candidates_small(const WsArgs& a, int sms, cudaStream_t st) {
 }
 
 cudaError_t launch_candidates_ws(const WsArgs& a, int grid, cudaStream_t st) {
+    const bool bf16 = a.form == WsForm::bf16;
     if (a.slots == 16384)
-        return a.bf16 ? launch_ws_w<true, 16384>(a, grid, st) : launch_ws_w<false, 16384>(a, grid, st);
-    if (a.slots == 8192) return a.bf16 ? launch_ws_w<true, 8192>(a, grid, st) : launch_ws_w<false, 8192>(a, grid, st);
-    return a.bf16 ? launch_ws_w<true, 4096>(a, grid, st) : launch_ws_w<false, 4096>(a, grid, st);
+        return bf16 ? launch_ws_w<WsForm::bf16, 16384>(a, grid, st) : launch_ws_w<WsForm::direct, 16384>(a, grid, st);
+    if (a.slots == 8192)
+        return bf16 ? launch_ws_w<WsForm::bf16, 8192>(a, grid, st) : launch_ws_w<WsForm::direct, 8192>(a, grid, st);
+    if (a.form == WsForm::staged) return launch_ws_w<WsForm::staged, 4096>(a, grid, st);
+    return bf16 ? launch_ws_w<WsForm::bf16, 4096>(a, grid, st) : launch_ws_w<WsForm::direct, 4096>(a, grid, st);
 }
 
-int ws_blocks_per_sm(int D, int K, int wt, int bf16, int slots) {
-    if (slots == 16384) return bf16 ? ws_bps_w<true, 16384>(D, K, wt) : ws_bps_w<false, 16384>(D, K, wt);
-    if (slots == 8192) return bf16 ? ws_bps_w<true, 8192>(D, K, wt) : ws_bps_w<false, 8192>(D, K, wt);
-    return bf16 ? ws_bps_w<true, 4096>(D, K, wt) : ws_bps_w<false, 4096>(D, K, wt);
+int ws_blocks_per_sm(int D, int K, int wt, WsForm form, int slots) {
+    const bool bf16 = form == WsForm::bf16;
+    if (slots == 16384)
+        return bf16 ? ws_bps_w<WsForm::bf16, 16384>(D, K, wt) : ws_bps_w<WsForm::direct, 16384>(D, K, wt);
+    if (slots == 8192) return bf16 ? ws_bps_w<WsForm::bf16, 8192>(D, K, wt) : ws_bps_w<WsForm::direct, 8192>(D, K, wt);
+    if (form == WsForm::staged) return ws_bps_w<WsForm::staged, 4096>(D, K, wt);
+    return bf16 ? ws_bps_w<WsForm::bf16, 4096>(D, K, wt) : ws_bps_w<WsForm::direct, 4096>(D, K, wt);
 }
 
 cudaError_t launch_candidates_dense(const WsArgs& a, int grid, cudaStream_t st) {

@@ -20,6 +20,7 @@
 #include <ctime>
 #include <mutex>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "culsh.h"
@@ -117,6 +118,9 @@ inline double seconds_now() {
 
 }  // namespace
 
+constexpr int kSampleRows = 4096;   // rows of X sampled for the tensor-core projection
+constexpr int kMaxRegions = 1024;   // recomputation lists (one per CTA) of it
+
 struct culsh_index {
     int N = 0, D = 0, L = 0, M = 0;
     float W = 0.0f;
@@ -190,18 +194,21 @@ struct culsh_index {
     DevBuf<uint16_t> ws_ah, ws_al, ws_xh, ws_xl;   // bf16 splits for the tensor-core projection
     DevBuf<float> ws_anorm, ws_xnorm;
     DevBuf<ProjectState> ws_pstate;
-    PinBuf<float> h_norms;
-    // pinned staging of a build's small host arrays (its copies neither block nor
-    // outlive the build), and of what it reads back
-    PinBuf<unsigned char> h_stage;
-    size_t h_stage_used = 0;
-    PinBuf<unsigned int> h_relist_cnt, h_nb;
-    PinBuf<ProjectState> h_pstate;
-    PinBuf<int32_t> h_range;    // [2][L*M] code ranges
-    PinBuf<int> h_err;
     double tc_predicted_open = 0.0;   // predicted share of codes the tensor-core bound leaves open
     DevBuf<uint32_t> maxb;
-    PinBuf<uint32_t> h_maxb;
+    // What a build stages (its copies neither block nor outlive the build) and
+    // reads back, in one pinned allocation: parts of it set by stage_begin.
+    PinBuf<unsigned char> h_pin;
+    float* h_norms = nullptr;            // [L*M + kSampleRows]
+    unsigned char* h_stage = nullptr;
+    size_t h_stage_used = 0, h_stage_size = 0;
+    unsigned int* h_relist_cnt = nullptr;   // [kMaxRegions]
+    unsigned int* h_nb = nullptr;        // [L]
+    ProjectState* h_pstate = nullptr;
+    int32_t* h_range = nullptr;          // [2][L*M] code ranges
+    int* h_err = nullptr;
+    unsigned int* h_run_cnt = nullptr;   // [4]
+    uint32_t* h_maxb = nullptr;          // largest bucket, spilled keys
     uint32_t max_bucket = 0;          // largest bucket of any table (gates the dense candidate kernel)
     DevBuf<unsigned long long> ws_relist;
     DevBuf<unsigned int> ws_relist_cnt;
@@ -214,7 +221,6 @@ struct culsh_index {
     DevBuf<unsigned long long> ws_run_pos;
     DevBuf<uint32_t> ws_run_len;
     DevBuf<unsigned int> ws_run_cnt;
-    PinBuf<unsigned int> h_run_cnt;
     int sort_form = 0;   // 1: top-word passes + run ordering, 2: that form fell back to all words, 0: all words
 
     ~culsh_index() {
@@ -365,9 +371,9 @@ int upload_projection(culsh_index* ix, cudaStream_t st) {
 // where that is full).
 int stage_copy(culsh_index* ix, void* dst, const void* src, size_t bytes, cudaStream_t st) {
     const size_t at = (ix->h_stage_used + 15) & ~size_t(15);
-    if (ix->h_stage.p && at + bytes <= ix->h_stage.n) {
-        std::memcpy(ix->h_stage.p + at, src, bytes);
-        src = ix->h_stage.p + at;
+    if (ix->h_stage && at + bytes <= ix->h_stage_size) {
+        std::memcpy(ix->h_stage + at, src, bytes);
+        src = ix->h_stage + at;
         ix->h_stage_used = at + bytes;
     }
     CU_TRY(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st));
@@ -378,16 +384,33 @@ int stage_copy(culsh_index* ix, void* dst, const void* src, size_t bytes, cudaSt
 // staged earlier is still being copied: both end with their stream drained.
 int stage_begin(culsh_index* ix) {
     const size_t LM = (size_t)ix->L * ix->M, L1 = (size_t)ix->L + 1;
-    CU_TRY(ix->h_stage.reserve(40 * LM + 40 * L1 + 1024));
+    ix->h_stage_size = 40 * LM + 40 * L1 + 1024;
+    size_t at = 0;
+    auto part = [&](auto** p, size_t n, bool set) {
+        if (set) *p = reinterpret_cast<std::remove_reference_t<decltype(*p)>>(ix->h_pin.p + at);
+        at = (at + n * sizeof(**p) + 15) & ~size_t(15);
+    };
+    for (int set = 0; set < 2; ++set) {
+        at = 0;
+        part(&ix->h_stage, ix->h_stage_size, set);
+        part(&ix->h_norms, LM + kSampleRows, set);
+        part(&ix->h_relist_cnt, kMaxRegions, set);
+        part(&ix->h_nb, (size_t)ix->L, set);
+        part(&ix->h_pstate, 1, set);
+        part(&ix->h_range, 2 * LM, set);
+        part(&ix->h_err, 1, set);
+        part(&ix->h_run_cnt, 4, set);
+        part(&ix->h_maxb, 2, set);
+        if (!set) CU_TRY(ix->h_pin.reserve(at));
+    }
     ix->h_stage_used = 0;
     return CULSH_OK;
 }
 
 int read_err_flag(culsh_index* ix, cudaStream_t st, const char* what) {
-    CU_TRY(ix->h_err.reserve(1));
-    CU_TRY(cudaMemcpyAsync(ix->h_err.p, ix->err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+    CU_TRY(cudaMemcpyAsync(ix->h_err, ix->err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
     CU_TRY(cudaStreamSynchronize(st));
-    const int h = *ix->h_err.p;
+    const int h = *ix->h_err;
     if (h & kErrNonFinite) return fail(CULSH_ERR_NUMERIC, "%s: a projection is not finite (NaN/Inf in the data?)", what);
     if (h & kErrCodeRange) return fail(CULSH_ERR_NUMERIC, "%s: a bucket code exceeds the int32 range", what);
     if (h & kErrNotIntegral) return fail(CULSH_ERR_FORMAT, "%s: a bucket code is not an integer", what);
@@ -574,16 +597,16 @@ int project_tensor_cores(culsh_index* ix, const float* dX, cudaStream_t st, bool
     const TcPlan rp = tc_plan(N, D, LM, sms, maxsm);
     const TcStreamPlan sp = rp.ok ? TcStreamPlan{} : tc_plan_stream(N, D, LM, sms, maxsm);
     if (!rp.ok && !sp.ok) return CULSH_OK;
+    if ((rp.ok ? rp.grid : sp.grid) > kMaxRegions) return CULSH_OK;
     const bool stream = !rp.ok;
     struct {
         int Dp, LMp, grid;
     } p = {stream ? sp.Dp : rp.Dp, stream ? sp.LMp : rp.LMp, stream ? sp.grid : rp.grid};
     // Norms of A's columns and of a sample of X, and the operands' scales.
-    const int ns = (int)std::min<int64_t>(N, 4096);
+    const int ns = (int)std::min<int64_t>(N, kSampleRows);
     CU_TRY(ix->ws_anorm.reserve(LM));
     CU_TRY(ix->ws_xnorm.reserve(std::max(N, ns)));
     CU_TRY(ix->ws_pstate.reserve(1));
-    CU_TRY(ix->h_norms.reserve(LM + ns));
     // Bound on |tensor-core sum - canonical FP32 chain| per unit of |x||a|: the
     // part that falls over d (roundings of the running sums: one a step of the
     // canonical chain, one per summed large product, all products alike in
@@ -604,12 +627,11 @@ int project_tensor_cores(culsh_index* ix, const float* dX, cudaStream_t st, bool
     };
     bound_for(0);
     CU_TRY(launch_project_sample(dX, N, D, ns, ix->dA.p, LM, slope, ix->ws_xnorm.p, ix->ws_anorm.p, ix->ws_pstate.p, st));
-    CU_TRY(cudaMemcpyAsync(ix->h_norms.p, ix->ws_anorm.p, 4 * (size_t)LM, cudaMemcpyDeviceToHost, st));
-    CU_TRY(cudaMemcpyAsync(ix->h_norms.p + LM, ix->ws_xnorm.p, 4 * (size_t)ns, cudaMemcpyDeviceToHost, st));
-    CU_TRY(ix->h_pstate.reserve(1));
-    CU_TRY(cudaMemcpyAsync(ix->h_pstate.p, ix->ws_pstate.p, sizeof(ProjectState), cudaMemcpyDeviceToHost, st));
+    CU_TRY(cudaMemcpyAsync(ix->h_norms, ix->ws_anorm.p, 4 * (size_t)LM, cudaMemcpyDeviceToHost, st));
+    CU_TRY(cudaMemcpyAsync(ix->h_norms + LM, ix->ws_xnorm.p, 4 * (size_t)ns, cudaMemcpyDeviceToHost, st));
+    CU_TRY(cudaMemcpyAsync(ix->h_pstate, ix->ws_pstate.p, sizeof(ProjectState), cudaMemcpyDeviceToHost, st));
     CU_TRY(cudaStreamSynchronize(st));
-    ProjectState ps = *ix->h_pstate.p;
+    ProjectState ps = *ix->h_pstate;
     bool lo = (ps.flags & 8) != 0;
     bound_for(lo);
     {
@@ -618,7 +640,7 @@ int project_tensor_cores(culsh_index* ix, const float* dX, cudaStream_t st, bool
         // 6 % the FP32 recomputation costs more than the SIMT projection
         // itself, so the SIMT kernel runs. Taken before anything of X's size is
         // converted.
-        float *as = ix->h_norms.p, *xs = ix->h_norms.p + LM;
+        float *as = ix->h_norms, *xs = ix->h_norms + LM;
         std::nth_element(xs, xs + ns / 2, xs + ns);
         std::nth_element(as, as + LM / 2, as + LM);
         const double open = 2.0 * (double)kappa * xs[ns / 2] * as[LM / 2] / (double)ix->W;
@@ -633,11 +655,8 @@ int project_tensor_cores(culsh_index* ix, const float* dX, cudaStream_t st, bool
     const unsigned long long cap = ((unsigned long long)N * LM / 6) / p.grid + 4096;
     CU_TRY(ix->ws_relist.reserve(cap * p.grid));
     CU_TRY(ix->ws_relist_cnt.reserve(p.grid));
-    CU_TRY(ix->h_relist_cnt.reserve(p.grid));
     CU_TRY(ix->ws_pmin.reserve((size_t)p.grid * LM));
     CU_TRY(ix->ws_pmax.reserve((size_t)p.grid * LM));
-    CU_TRY(ix->h_range.reserve(2 * (size_t)LM));
-    CU_TRY(ix->h_err.reserve(1));
     // The low parts are made when the sample has one. Everything up to the
     // recomputed codes and their ranges is enqueued on that assumption and
     // judged after one wait; data that are inexact elsewhere only, or whose
@@ -663,21 +682,21 @@ int project_tensor_cores(culsh_index* ix, const float* dX, cudaStream_t st, bool
         CU_TRY(launch_minmax_reduce(ix->ws_pmin.p, ix->ws_pmax.p, p.grid, LM, ix->cmin.p, ix->cmax.p, st));
         CU_TRY(launch_tc_recompute(dX, N, D, LM, ix->dA.p, ix->db.p, ix->W, ix->ws_relist.p, cap, ix->ws_relist_cnt.p,
                                    p.grid, ix->ws_codes.p, ix->cmin.p, ix->cmax.p, ix->err.p, st));
-        CU_TRY(cudaMemcpyAsync(ix->h_pstate.p, ix->ws_pstate.p, sizeof(ProjectState), cudaMemcpyDeviceToHost, st));
-        CU_TRY(cudaMemcpyAsync(ix->h_relist_cnt.p, ix->ws_relist_cnt.p, 4 * p.grid, cudaMemcpyDeviceToHost, st));
-        CU_TRY(cudaMemcpyAsync(ix->h_range.p, ix->cmin.p, 4 * (size_t)LM, cudaMemcpyDeviceToHost, st));
-        CU_TRY(cudaMemcpyAsync(ix->h_range.p + LM, ix->cmax.p, 4 * (size_t)LM, cudaMemcpyDeviceToHost, st));
-        CU_TRY(cudaMemcpyAsync(ix->h_err.p, ix->err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
+        CU_TRY(cudaMemcpyAsync(ix->h_pstate, ix->ws_pstate.p, sizeof(ProjectState), cudaMemcpyDeviceToHost, st));
+        CU_TRY(cudaMemcpyAsync(ix->h_relist_cnt, ix->ws_relist_cnt.p, 4 * p.grid, cudaMemcpyDeviceToHost, st));
+        CU_TRY(cudaMemcpyAsync(ix->h_range, ix->cmin.p, 4 * (size_t)LM, cudaMemcpyDeviceToHost, st));
+        CU_TRY(cudaMemcpyAsync(ix->h_range + LM, ix->cmax.p, 4 * (size_t)LM, cudaMemcpyDeviceToHost, st));
+        CU_TRY(cudaMemcpyAsync(ix->h_err, ix->err.p, sizeof(int), cudaMemcpyDeviceToHost, st));
         CU_TRY(cudaStreamSynchronize(st));
-        ps = *ix->h_pstate.p;
+        ps = *ix->h_pstate;
         unsigned long long nre = 0;
         bool overflow = false;
         for (int r = 0; r < p.grid; ++r) {
-            nre += ix->h_relist_cnt.p[r];
-            overflow |= ix->h_relist_cnt.p[r] > cap;
+            nre += ix->h_relist_cnt[r];
+            overflow |= ix->h_relist_cnt[r] > cap;
         }
         const bool again = (ps.flags & 4) || (!lo && (ps.flags & 1));
-        if ((ps.flags & 2) || overflow || *ix->h_err.p != 0 || again) {
+        if ((ps.flags & 2) || overflow || *ix->h_err != 0 || again) {
             CU_TRY(cudaMemsetAsync(ix->err.p, 0, sizeof(int), st));
             // non-finite data (the SIMT kernel reports it), too many open codes,
             // a code out of range or a wait that gave up: the SIMT kernel
@@ -724,8 +743,7 @@ int sort_keys(culsh_index* ix, int N, int passes, bool all_words, cudaStream_t s
     CU_TRY(ix->ws_hist.reserve((size_t)L * hp * 256));
     CU_TRY(ix->ws_base.reserve((size_t)L * hp * 256));
     CU_TRY(ix->ws_status.reserve(sort_status_words(N, L)));
-    CU_TRY(ix->h_run_cnt.reserve(4));
-    ix->h_run_cnt.p[3] = 0;
+    ix->h_run_cnt[3] = 0;
     CU_TRY(cudaEventRecord(ix->bev[2], st));
     SortBuffers sb;
     sb.keys[0] = ix->ws_keys[0].p;
@@ -763,7 +781,7 @@ int sort_keys(culsh_index* ix, int N, int passes, bool all_words, cudaStream_t s
         rl.same = ix->ws_status.p;
         CU_TRY(launch_run_find(top, N, L, KW, ix->ws_low.p, ix->ids.p, rl, st));
         CU_TRY(launch_run_sorts(rl, N, L, KW, ix->ws_low.p, ix->ids.p, st));
-        CU_TRY(cudaMemcpyAsync(ix->h_run_cnt.p, rl.cnt, 4 * sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
+        CU_TRY(cudaMemcpyAsync(ix->h_run_cnt, rl.cnt, 4 * sizeof(unsigned int), cudaMemcpyDeviceToHost, st));
         ix->sort_form = 1;
         *sk = SortedKeys{top, ix->ws_low.p, ix->ids.p, lw};
         return CULSH_OK;
@@ -801,13 +819,12 @@ int build_device(culsh_index* ix, const float* dX, cudaStream_t st, FILE* dbg) {
         CU_TRY(launch_minmax_reduce(ix->ws_pmin.p, ix->ws_pmax.p, gx, LM, ix->cmin.p, ix->cmax.p, st));
     }
     if (!tc_done) {
-        CU_TRY(ix->h_range.reserve(2 * (size_t)LM));
-        CU_TRY(cudaMemcpyAsync(ix->h_range.p, ix->cmin.p, 4 * (size_t)LM, cudaMemcpyDeviceToHost, st));
-        CU_TRY(cudaMemcpyAsync(ix->h_range.p + LM, ix->cmax.p, 4 * (size_t)LM, cudaMemcpyDeviceToHost, st));
+        CU_TRY(cudaMemcpyAsync(ix->h_range, ix->cmin.p, 4 * (size_t)LM, cudaMemcpyDeviceToHost, st));
+        CU_TRY(cudaMemcpyAsync(ix->h_range + LM, ix->cmax.p, 4 * (size_t)LM, cudaMemcpyDeviceToHost, st));
         TRY(read_err_flag(ix, st, "index"));
     }
-    ix->h_cmin.assign(ix->h_range.p, ix->h_range.p + LM);
-    ix->h_cmax.assign(ix->h_range.p + LM, ix->h_range.p + 2 * LM);
+    ix->h_cmin.assign(ix->h_range, ix->h_range + LM);
+    ix->h_cmax.assign(ix->h_range + LM, ix->h_range + 2 * LM);
     int passes = 0;
     TRY(compute_layout(ix, &passes));
     TRY(upload_layout(ix, st));
@@ -824,18 +841,17 @@ int build_device(culsh_index* ix, const float* dX, cudaStream_t st, FILE* dbg) {
     CU_TRY(ix->ws_tcnt.reserve((size_t)L * tiles));
     CU_TRY(ix->ws_toff.reserve((size_t)L * tiles));
     CU_TRY(ix->ws_nb.reserve(L));
-    CU_TRY(ix->h_nb.reserve(L));
     for (int all_words = 0; all_words < 2; ++all_words) {
         TRY(sort_keys(ix, N, passes, all_words != 0, st, &skeys));
         CU_TRY(cudaEventRecord(ix->bev[3], st));
         // Run-length bucketing (its flags, like the runs' marks, take the place of
         // the sort's tile states).
         CU_TRY(launch_rl_count(skeys, N, L, ix->KW, ix->ws_tcnt.p, ix->ws_toff.p, ix->ws_status.p, ix->ws_nb.p, st));
-        CU_TRY(cudaMemcpyAsync(ix->h_nb.p, ix->ws_nb.p, 4 * L, cudaMemcpyDeviceToHost, st));
+        CU_TRY(cudaMemcpyAsync(ix->h_nb, ix->ws_nb.p, 4 * L, cudaMemcpyDeviceToHost, st));
         CU_TRY(cudaStreamSynchronize(st));
-        if (ix->h_run_cnt.p[3] == 0) break;   // every run was ordered
+        if (ix->h_run_cnt[3] == 0) break;   // every run was ordered
     }
-    ix->buckets.assign(ix->h_nb.p, ix->h_nb.p + L);
+    ix->buckets.assign(ix->h_nb, ix->h_nb + L);
     ix->h_boff.assign(L + 1, 0);
     int64_t maxB = 0;
     for (int l = 0; l < L; ++l) {
@@ -853,18 +869,17 @@ int build_device(culsh_index* ix, const float* dX, cudaStream_t st, FILE* dbg) {
     CU_TRY(cudaMemsetAsync(ix->maxb.p, 0, sizeof(uint32_t), st));
     const uint32_t* spill = nullptr;
     TRY(build_hash(ix, true, false, &spill, st));
-    CU_TRY(ix->h_maxb.reserve(2));   // pinned: the copy does not block the host mid-build
-    ix->h_maxb.p[1] = 0;
-    CU_TRY(cudaMemcpyAsync(ix->h_maxb.p, ix->maxb.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
-    if (spill) CU_TRY(cudaMemcpyAsync(ix->h_maxb.p + 1, spill, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    ix->h_maxb[1] = 0;
+    CU_TRY(cudaMemcpyAsync(ix->h_maxb, ix->maxb.p, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
+    if (spill) CU_TRY(cudaMemcpyAsync(ix->h_maxb + 1, spill, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     CU_TRY(cudaEventRecord(ix->bev[4], st));
     TRY(read_err_flag(ix, st, "index"));   // synchronises the stream
-    if (ix->h_maxb.p[1] > kHashSpill) {    // more keys in a few parts than they can hold
+    if (ix->h_maxb[1] > kHashSpill) {    // more keys in a few parts than they can hold
         TRY(build_hash(ix, true, true, nullptr, st));
         CU_TRY(cudaEventRecord(ix->bev[4], st));
         TRY(read_err_flag(ix, st, "index"));
     }
-    ix->max_bucket = *ix->h_maxb.p;
+    ix->max_bucket = *ix->h_maxb;
     ix->indexed = ix->dev_valid = true;
     ix->host_valid = false;
     ix->built_once = true;
@@ -1420,7 +1435,7 @@ int plan_search(culsh_search* s, const float* dQ, int Q, int32_t* d_ids, float* 
         }
         // (Counted with a list per warp, which the BF16 form keeps, so that both
         // forms of a configuration take the same route.)
-        const size_t need = ws_smem_bytes(D, K, tu.ws_wt, tu.dist_bf16 ? 1 : 0, tu.ws_slots) + 8192 +
+        const size_t need = ws_smem_bytes(D, K, tu.ws_wt, tu.dist_bf16 ? WsForm::bf16 : WsForm::direct, tu.ws_slots) + 8192 +
                             (tu.dist_bf16 ? 0 : 8 * (size_t)K * (tu.ws_wt / 32 - 1));
         if (need > (size_t)s->smem_optin) P.use_ws = 0;
     }
@@ -1456,15 +1471,6 @@ int plan_search(culsh_search* s, const float* dQ, int Q, int32_t* d_ids, float* 
             CU_TRY(cudaStreamSynchronize(st));
             ix->xb_valid = true;
         }
-        // resident CTAs per SM, cached per kernel shape
-        const long long okey = ((((long long)D * 4096 + K) * 512 + tu.ws_wt) * 2 + bf16) * 16384 + tu.ws_slots;
-        if (s->occ_key != okey) {
-            s->occ_val = ws_blocks_per_sm(D, K, tu.ws_wt, bf16, tu.ws_slots);
-            s->occ_key = okey;
-        }
-        const int occ = s->occ_val;
-        const int bps = tu.ws_bps > 0 ? std::min(tu.ws_bps, occ) : occ;
-        P.ws_grid = s->sms * bps;
         P.sms = s->sms;
         WsArgs& a = P.wa;
         a.X = ca.X;
@@ -1508,7 +1514,7 @@ int plan_search(culsh_search* s, const float* dQ, int Q, int32_t* d_ids, float* 
         a.n_small = reinterpret_cast<unsigned int*>(s->stats.p + 12);
         a.wt = tu.ws_wt;
         a.slots = tu.ws_slots;
-        a.bf16 = bf16;
+        a.form = bf16 ? WsForm::bf16 : WsForm::direct;
         // Dense form: queries with at least dense_min non-unique candidates
         // take the tensor-core path (membership rows and a masked GEMM over
         // the whole dataset; default threshold max(4096, N/256)) or, where
@@ -1539,6 +1545,24 @@ int plan_search(culsh_search* s, const float* dQ, int Q, int32_t* d_ids, float* 
             CU_TRY(s->dense_q.reserve(Q));
             a.dense_q = s->dense_q.p;
         }
+        // Rows staged in shared memory where no sparse query has more candidates
+        // than twice the set: short items, whose time is the latency of their
+        // rows (4,000 candidates and fewer at 1M x 100: 136 us against 248; 156 at
+        // 100K x 128: 40 against 46). With more, items a device keeps resident
+        // count for more (12.7k at 1M x 128, all of them gathered: 38 ms against
+        // 21; up to 15,600 at 4M x 128: 660 us against 620).
+        const unsigned long long most = std::min(reach, P.use_dense ? dmin : ~0ull);
+        if (!bf16 && tu.ws_slots == 4096 && most <= 2ull * 4096 &&
+            ws_smem_bytes(D, K, tu.ws_wt, WsForm::staged, tu.ws_slots) + 8192 <= (size_t)s->smem_optin)
+            a.form = WsForm::staged;
+        // resident CTAs per SM, cached per kernel shape
+        const long long okey = ((((long long)D * 4096 + K) * 512 + tu.ws_wt) * 4 + (int)a.form) * 16384 + tu.ws_slots;
+        if (s->occ_key != okey) {
+            s->occ_val = ws_blocks_per_sm(D, K, tu.ws_wt, a.form, tu.ws_slots);
+            s->occ_key = okey;
+        }
+        const int bps = tu.ws_bps > 0 ? std::min(tu.ws_bps, s->occ_val) : s->occ_val;
+        P.ws_grid = s->sms * bps;
         a.nbig = 0;
         a.big_min = UINT32_MAX;
         if (tu.ws_order) {
@@ -1810,7 +1834,7 @@ int finish_search(culsh_search* s, const SearchPlan& P, cudaStream_t st) {
     }
     s->tot_unique = s->h_stats.p[0];
     s->tot_nonunique = s->h_stats.p[1];
-    s->rechecked = P.use_ws && P.wa.bf16 && !s->ws_overflow ? (long long)s->h_stats.p[6] : 0;
+    s->rechecked = P.use_ws && P.wa.form == WsForm::bf16 && !s->ws_overflow ? (long long)s->h_stats.p[6] : 0;
     s->dense_queries = nd;
     return CULSH_OK;
 }
@@ -2571,7 +2595,7 @@ int culsh_search_autotune(culsh_search* s, const float* d_queries, int Q, int* d
         }
     }
     if (best.cand_ws) {   // residency: half the occupancy limit as well
-        const int occ = ws_blocks_per_sm(s->ix->D, s->K, best.ws_wt, best.dist_bf16, best.ws_slots);
+        const int occ = ws_blocks_per_sm(s->ix->D, s->K, best.ws_wt, best.dist_bf16 ? WsForm::bf16 : WsForm::direct, best.ws_slots);
         if (occ > 1) {
             SearchTune t = best;
             t.ws_bps = occ / 2;

@@ -376,6 +376,11 @@ struct CandArgs {
 };
 // Work-stealing form of the candidate stage (candidates.cu): queries split
 // into id-partition items, claimed by a persistent grid.
+// How the work-stealing kernel reads candidate rows: FP32 rows straight from
+// global memory, BF16 copies with an FP32 recheck, FP32 rows staged in shared
+// memory by bulk copies (sets of 4,096 slots).
+enum class WsForm : int { direct = 0, bf16 = 1, staged = 2 };
+
 struct WsArgs {
     const float* X;
     int64_t N;
@@ -413,7 +418,7 @@ struct WsArgs {
     int wt;                            // threads per item CTA: 64, 128 or 256
     int slots;                         // shared hash-set slots per item: 4096 or 8192
     // BF16 form: approximate distances from xb, certified FP32 rerank
-    int bf16;
+    WsForm form;
     const uint16_t* xb;                // [N][D] bf16 copy of X
     const uint8_t* xflag;              // [N] 1 exact in bf16, 2 always re-check, 0 bound applies
     float e_c1, e_c2;                  // error-bound factors (rounded up)
@@ -455,8 +460,8 @@ constexpr int kOrderBins = 4096;
 cudaError_t launch_order_queries(const WsArgs& a, cudaStream_t st);   // 3 kernels + 1 memset
 size_t dense_smem_bytes(int64_t N, int D, int K);
 cudaError_t launch_candidates_dense(const WsArgs& a, int grid, cudaStream_t st);
-size_t ws_smem_bytes(int D, int K, int wt, int bf16, int slots);
-int ws_blocks_per_sm(int D, int K, int wt, int bf16, int slots);
+size_t ws_smem_bytes(int D, int K, int wt, WsForm form, int slots);
+int ws_blocks_per_sm(int D, int K, int wt, WsForm form, int slots);
 cudaError_t launch_bf16_rows(const float* X, int64_t N, int D, uint16_t* xb, uint8_t* flag, cudaStream_t st);
 cudaError_t launch_plan_items(const WsArgs& a, cudaStream_t st);
 // Bucket rows: the global numbers and sizes of the buckets of at least

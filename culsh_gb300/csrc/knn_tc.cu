@@ -804,7 +804,7 @@ constexpr int LW = 8;   // queries (warps) per block of k_knn_limit
 // is selected by radix passes over a 256-bin histogram, from the highest bit
 // in which the groups differ (bits above it would send every lane to one bin).
 // 10,000 queries of 1,953 chunks: 345 us with four passes over global memory
-// from the top bit, 108 us from the first differing bit.
+// from the top bit, 108 us from the first differing bit, 47 us from registers.
 template <int R>
 __global__ void __launch_bounds__(32 * LW) k_knn_limit(KnnSearch k) {
     __shared__ uint32_t hist[LW][256];

@@ -15,7 +15,7 @@
 // over the unique keys serves exact-code lookups at query time.
 //
 // Every pass streams keys and ids once in and once out (the digit's own
-// word is read once): HBM bound.
+// word is read once; the first pass makes the ids).
 #include <algorithm>
 #include <climits>
 

@@ -160,9 +160,11 @@ typedef struct culsh_tuning {
                              together and share rows in L2 (same results as 0)         */
     int dense_tc;         /* 1: dense queries (see dense_min) take the tensor-core path:
                              an N-bit candidate membership row per query, then q.x for
-                             all points by tcgen05 GEMM tiles with the top-K kept in the
-                             epilogue, exact distances (same results as 0); 0: the SIMT
-                             bitmap kernel                                              */
+                             all points by tcgen05 GEMM tiles whose epilogue keeps the
+                             candidates that a certified bound cannot exclude, exact
+                             distances of those (same results as 0). Shapes it does not
+                             cover (K > 256, D > 2048, more than 4,096 but fewer than
+                             128 K points) and 0: the SIMT bitmap kernel                */
     int dense_min;        /* non-unique candidates from which a query is dense; 0: the
                              default, max(4096, N/256) for the tensor-core path and
                              max(32768, N/16) for the SIMT bitmap kernel               */
@@ -219,7 +221,7 @@ typedef struct culsh_search_profile {
     int graph_mode;      /* 0: direct launches; 1: graph captured; 2: replayed */
     long long rechecked; /* BF16 distance form: candidates re-read in FP32     */
     int dense_queries;   /* queries deduplicated in an N-bit bitmap (candidate
-                            sets of at least max(32768, N/16) ids)             */
+                            sets of at least dense_min ids, see culsh_tuning)  */
     int host_path;       /* 0: device buffers (culsh_search_run_device*);
                             1: host buffers staged through device copies;
                             2: host buffers read and written by the kernels
@@ -231,16 +233,16 @@ typedef struct culsh_search_profile {
     int stage_times;     /* 1: the stage times above were measured; 0: stage
                             events off (culsh_search_set_profiling)          */
     int knn_queries;     /* dense queries served by the tensor-core path     */
-    int knn_fallback;    /* of those, queries whose bound-form lists could not
-                            prove the top-K, re-run by the exact per-query
-                            kernel                                          */
+    int knn_fallback;    /* of those, queries with more candidates within the
+                            bound than their lists hold, scanned exactly from
+                            their membership rows                           */
     float membership_ms; /* tensor-core path, stage times: planning and the
                             candidate membership rows ...                   */
     float knn_ms;        /* ... and the tensor-core distances, top-K lists
                             and merge (0 unless measured)                   */
     int bucket_rows;     /* tensor-core path: index buckets kept as N-bit rows
                             and ORed whole into the membership rows (buckets
-                            of at least max(1024, N/64) ids); 0: none       */
+                            of at least max(1024, N/32) ids); 0: none       */
 } culsh_search_profile;
 int culsh_search_profile_get(culsh_search* s, culsh_search_profile* out);
 

@@ -661,9 +661,11 @@ int project_tensor_cores(culsh_index* ix, const float* dX, cudaStream_t st, bool
     // recomputed codes and their ranges is enqueued on that assumption and
     // judged after one wait; data that are inexact elsewhere only, or whose
     // magnitudes the sample's scale takes out of the fp16 range, run again.
+    auto scale_fits = [&] {   // the accumulators' scale and its reciprocal stay well inside the float range
+        return ps.sx * ps.sa > 1e-25f && ps.sx * ps.sa < 1e25f && ix->W > 1e-10f && ix->W < 1e10f;
+    };
     for (int attempt = 0;; ++attempt) {
-        // the accumulators' scale and its reciprocal stay well inside the float range
-        if (!(ps.sx * ps.sa > 1e-25f && ps.sx * ps.sa < 1e25f && ix->W > 1e-10f && ix->W < 1e10f)) return CULSH_OK;
+        if (!scale_fits()) return CULSH_OK;
         if (lo) CU_TRY(ix->ws_xl.reserve(nx));
         CU_TRY(launch_split_a(ix->dA.p, LM, p.LMp, D, p.Dp, kappa, slope, ix->ws_ah.p, ix->ws_al.p, ix->ws_anorm.p, ix->ws_pstate.p,
                               st));
@@ -696,7 +698,7 @@ int project_tensor_cores(culsh_index* ix, const float* dX, cudaStream_t st, bool
             overflow |= ix->h_relist_cnt[r] > cap;
         }
         const bool again = (ps.flags & 4) || (!lo && (ps.flags & 1));
-        if ((ps.flags & 2) || overflow || *ix->h_err != 0 || again) {
+        if ((ps.flags & 2) || overflow || *ix->h_err != 0 || again || !scale_fits()) {
             CU_TRY(cudaMemsetAsync(ix->err.p, 0, sizeof(int), st));
             // non-finite data (the SIMT kernel reports it), too many open codes,
             // a code out of range or a wait that gave up: the SIMT kernel
@@ -1383,8 +1385,9 @@ int plan_search(culsh_search* s, const float* dQ, int Q, int32_t* d_ids, float* 
         // No form set: lookups behind the key filter at the enumeration's end
         // where buckets hold fewer than four points on average, since most
         // probes then find nothing (1M points, every one its own bucket, T = 16:
-        // 148 us fused, 117 us so; at 20,000 buckets a table fused is ahead, 160 against 167 us).
-        if (P.pa.auto_form && M <= 16 && T >= 4 && 4 * (unsigned long long)ix->h_boff[L] > (unsigned long long)ix->N * L)
+        // 148 us fused, 117 us so; at 20,000 buckets a table fused is ahead, 160 against
+        // 167 us; 1,291 queries of T = 5 on 33K points 25 us fused, 29 us so).
+        if (P.pa.auto_form && M <= 16 && T >= 8 && 4 * (unsigned long long)ix->h_boff[L] > (unsigned long long)ix->N * L)
             form = 2;
         if (form > 0) {
             CU_TRY(s->ph.reserve((size_t)L * Q * T));

@@ -10,7 +10,7 @@ projections, T=16 probes, K=10, Q=10,000 held-out queries, and W=825: the
 width at which LSH reaches recall@10 >= 0.90 on these data (at the named
 W=16 no held-out query has a candidate). Each query's candidates then cover
 about half of the dataset; the candidate stage runs on the tensor cores
-(bf16 operands, exact distances for these integer data: the "BF16" form), and
+(16-bit operands, exact distances for these integer data: the "BF16" form), and
 the FP32 SIMT form of the same search is timed beside it.
 
 value  : queries/s with queries already in HBM (device API), timed per step
@@ -198,9 +198,10 @@ STAGE_NOTES = {
     "membership": "algorithmic bytes are the 4 * C_nu bucket-id reads (each query reads its candidates' ids) "
                   "plus the N/8-byte membership row written per query; about 90 % of the id reads hit L2 "
                   "(the 64 MB of id arrays stay resident), so this is the rate seen at L2, not DRAM (measured "
-                  "DRAM traffic in `traffic`); buckets of at least N/64 ids are ORed in as whole N-bit bucket "
-                  "rows (L2-resident) instead of id by id, so part of those id bytes is never read and the "
-                  "rate can exceed the HBM peak; the rest is bound by the shared-memory atomicOr of each id",
+                  "DRAM traffic in `traffic`); buckets of at least N/32 ids are ORed in as whole N-bit bucket "
+                  "rows (L2-resident) and others of 512 ids or more as 16-bit entries, so part of those id bytes is "
+                  "never read and the rate can exceed the HBM peak; the rest is bound by the shared-memory atomicOr "
+                  "of each id or entry",
     "knn": "flops of the dense GEMM the kernel runs (2 * D * N per dense query); the candidates' own distance "
            "work is the unique-candidate share of it",
 }
@@ -500,8 +501,8 @@ def recall_point(culsh, torch, dev, steps, warmup, autotune=True, fixed=None):
     1M x 128, L=8, M=8, T=16, K=10, W=32, where LSH reaches recall@10 >= 0.90
     with sparse candidate sets (about 0.7 % of the dataset per query; the
     named W=4 leaves every held-out query without a candidate). Real-valued
-    data: the tensor-core form takes its bound form (three bf16 products,
-    certified bounds, exact FP32 recomputation). Three forms, identical
+    data: the tensor-core form bounds distances from one fp16 product and
+    recomputes in FP32 what the bounds leave. Three forms, identical
     results: FP32 work-stealing gather, BF16 gather with certified FP32
     rerank, tensor cores; each timed at its best settings (device events,
     inputs resident, L2 flushed)."""
@@ -881,10 +882,10 @@ def run_culsh(args):
         named_w = synth.CONFIGS[args.config].W
         line = {"metric": METRIC, "value": value, "unit": UNIT, "n_gpus": world, "steps": args.steps,
                 "warmup": args.warmup, "ms_per_step": 1e3 * max_s / args.steps, "higher_is_better": True,
-                "scaling": "weak", "vs_baseline": None, "dtype": "bf16" if tc else "f32",
+                "scaling": "weak", "vs_baseline": None, "dtype": "fp16" if tc else "f32",
                 "data": "synthetic (seeded generator of the workload's distribution)",
                 "config": {"workload": name, **d,
-                           "form": ("tensor cores: bf16 operands, exact distances (integer data), "
+                           "form": ("tensor cores: fp16 operands, FP32 accumulators, exact distances (integer data), "
                                     "results bit-identical to the FP32 form") if tc else
                                    "fp32 (canonical order, bit-exact)",
                            "operating_point": (f"W={d['W']:g} for recall@10 >= 0.90 (the named W={named_w:g} "

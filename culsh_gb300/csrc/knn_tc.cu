@@ -864,7 +864,9 @@ __global__ void __launch_bounds__(32 * LW) k_knn_limit(KnnSearch k) {
     const float key = key_dec(lo + prefix);
     const double u = (1.0 + (double)q.kappa) * ((double)key + q.sq) + q.slack;
     const double l = (u + q.slack) / (1.0 - (double)q.kappa) - q.sq;
-    k.qlim[i] = (float)(l + 1e-6 * (fabs(u) + q.sq));   // keys below it survive
+    // Keys below it survive: above every key that the bound admits, also where
+    // all of its terms are zero (a zero query among zero points).
+    k.qlim[i] = (float)(l + 1e-6 * (fabs(u) + q.sq) + 1e-37);
 }
 
 constexpr int MT = 128;   // threads of k_knn_merge

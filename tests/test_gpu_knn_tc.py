@@ -398,3 +398,31 @@ def test_magnitudes_and_outlier_rows(culsh, all_dense, scale):
     _check_against(st, want, Qm.shape[0], X)
     served = np.abs(X).max() <= 1e17
     assert st.profile()["knn_queries"] == (int((want["nonunique"] > 0).sum()) if served else 0)
+
+
+@pytest.mark.parametrize("D", [2, 16])
+@pytest.mark.parametrize("scale", [1.0, 0.3])
+def test_zero_queries_among_zero_points(culsh, D, scale):
+    """Queries and many points at the origin (more of them than K): every key
+    and every term of its bound is zero, in the exact form (integers) and in the
+    other; the nearest are those points, ties by id."""
+    import oracle
+    rng = np.random.default_rng(D)
+    N, L, M, T, K, Q = 4285, 6, 8, 5, 10, 300
+    X = (scale * np.clip(np.rint(rng.normal(20, 30, (N, D))), 0, 255)).astype(np.float32)
+    X[::7] = 0.0
+    q = np.ascontiguousarray(X[rng.integers(0, N, Q)])
+    q[::3] = 0.0
+    W = float(np.float32(3 * np.sqrt(np.mean(np.sum((X - X.mean(0)) ** 2, 1)))))
+    A = rng.normal(0, 1, (L, M, D)).astype(np.float32)
+    b = rng.uniform(0, W, (L, M)).astype(np.float32)
+    ht = culsh.HashTables()
+    ht.reset(N, D, L, M, W, A=A, b=b)
+    ht.index(X)
+    st = culsh.SearchTables()
+    st.reset(ht, K, T)
+    st.search(q, dataset=X)
+    assert st.profile()["knn_queries"] > 0
+    ref = oracle.search(oracle.build_index(X, A, b, W), X, q, K, T)
+    np.testing.assert_array_equal(st.getKnnIds(), ref["knn_ids"])
+    np.testing.assert_array_equal(st.getKnnDistances(), ref["knn_dists"])

@@ -575,13 +575,14 @@ cudaError_t launch_cand_bitmap(const WsArgs& a, const KnnSearch& k, uint32_t* bm
 cudaError_t launch_knn_scan_rows(const KnnSearch& k, int grid, cudaStream_t st);
 size_t knn_scan_smem(int D, int K);
 
-// Opts `func` into `dyn` bytes of dynamic shared memory when static plus
-// dynamic shared memory could pass the 48 KB default (the kernels here keep
-// at most 12 KB static). The opted-in size only grows (`cap` records it per
-// kernel), so a smaller configuration launched later stays valid.
+// Opts `func` into `dyn` bytes of dynamic shared memory: always, whatever the
+// size, since the 48 KB that need no opt-in include the kernel's static part
+// (15 KB of k_cand_bitmap, whose launches of 33 to 36 KB more had been refused).
+// The opted-in size only grows (`cap` records it per kernel), so a smaller
+// configuration launched later stays valid.
 template <class F>
 cudaError_t opt_in_smem(F* func, size_t dyn, std::atomic<size_t>& cap) {
-    if (dyn + 12 * 1024 <= 48 * 1024 || dyn <= cap.load()) return cudaSuccess;
+    if (dyn <= cap.load()) return cudaSuccess;
     static std::mutex mu;
     std::lock_guard<std::mutex> lk(mu);
     if (dyn <= cap.load()) return cudaSuccess;

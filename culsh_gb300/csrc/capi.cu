@@ -284,6 +284,7 @@ struct culsh_search {
     DevBuf<int> kpart_n, kfallback;
     int knn_queries = 0, knn_fallback = 0;   // last search: dense queries on the tensor cores, re-run
     int bucket_rows = 0;                     // last search: bucket rows its membership rows could use
+    bool knn_no_room = false;                // that path's buffers did not fit the device: later searches plan without it
     int sms = 0, smem_optin = 0, ws_used = 0, ws_overflow = 0;
     long long occ_key = -1;
     int occ_val = 1;
@@ -1024,6 +1025,27 @@ size_t arena_cap_words() {
     return ~size_t(0);
 }
 
+// Whether buffers that a faster form of a stage wants, and another form does
+// without, may take `bytes` more of device memory: they must leave the arena's
+// margin free. CULSH_SCRATCH_MAX_BYTES lowers the most they may take (the tests
+// reach the other forms with it).
+bool room_for(size_t bytes) {
+    if (bytes == 0) return true;
+    if (const char* e = getenv("CULSH_SCRATCH_MAX_BYTES"))
+        if (bytes > strtoull(e, nullptr, 10)) return false;
+    size_t freeb = 0, totalb = 0;
+    if (cudaMemGetInfo(&freeb, &totalb) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return bytes + 4 * kArenaInitialWords <= freeb;
+}
+// Bytes that reserving cnt elements adds to a buffer.
+template <class T>
+size_t growth(const DevBuf<T>& b, size_t cnt) {
+    return cnt > b.n ? (cnt - b.n) * sizeof(T) : 0;
+}
+
 }  // namespace
 
 std::mutex& culsh::alloc_capture_mutex() {
@@ -1116,13 +1138,24 @@ int ensure_knn_rows(culsh_index* ix, cudaStream_t st) {
 // stream is drained before they are published.
 constexpr size_t kBigRowsBytes = size_t(1) << 30;
 
+bool wants_bank(const culsh_index* ix, int nseg) {
+    return nseg == 1 && ix->N <= kBankMaxN && ix->max_bucket >= kBankMin;
+}
+
+// What ensure_big_rows may add, at most.
+size_t big_rows_bytes(const culsh_index* ix, int nseg) {
+    const size_t LN = (size_t)ix->L * ix->N;
+    const size_t bank = wants_bank(ix, nseg) ? 6 * LN + 8 * ix->h_boff[ix->L] + 12 * (LN / kBankMin + 1) : 0;
+    return bank + std::min(kBigRowsBytes, 4 * LN + (size_t(1) << 20));
+}
+
 int ensure_big_rows(culsh_index* ix, int nwp, int nseg, cudaStream_t st) {
     if (ix->big_valid) return CULSH_OK;
     const int L = ix->L, N = ix->N;
     ix->nbig = 0;
     ix->big_min = UINT32_MAX;
     ix->has_bank = false;
-    if (nseg == 1 && N <= kBankMaxN && ix->max_bucket >= kBankMin) {
+    if (wants_bank(ix, nseg)) {
         // Bank lists for the one-segment membership kernel.
         const size_t LN = (size_t)L * N, totB = ix->h_boff[L];
         const unsigned int cap = (unsigned int)std::min<size_t>(LN / kBankMin + 1, totB);
@@ -1227,6 +1260,59 @@ bool knn_shapes(const culsh_index* ix, int K, int nd, int sms, int smem_optin, K
     return knn_plan(k, smem_optin, bitmap_smem(smem_optin)) && knn_scan_smem(k.D, k.K) + 8192 <= (size_t)smem_optin;
 }
 
+void release_knn(culsh_search* s) {
+    s->kbm.release();
+    s->kbm_sample.release();
+    s->kq_h.release();
+    s->kq_info.release();
+    s->kq_lim.release();
+    s->kw_sample.release();
+    s->ksmin.release();
+    s->kpart.release();
+    s->kpart_n.release();
+    s->kfallback.release();
+}
+
+// Makes the tensor-core path's dataset rows, bucket rows and search buffers for
+// the shapes k. *ok turns false where the dataset does not suit the path or
+// its buffers do not fit the device: the dense queries then take the kernels
+// that need none (an index can be as large as the device, and its fp16 rows
+// alone are half the dataset).
+int reserve_knn(culsh_search* s, const KnnSearch& k, cudaStream_t st, bool* ok) {
+    culsh_index* ix = s->ix;
+    if (ix->kx_valid && !knn_dataset_fits(ix->h_kstate)) {
+        *ok = false;
+        return CULSH_OK;
+    }
+    const size_t qc = k.Qcap, nws = k.nws;
+    size_t need = growth(s->kbm, qc * k.nwp) + growth(s->kbm_sample, qc * nws) + growth(s->kq_h, qc * k.Dp) +
+                  growth(s->kq_info, qc) + growth(s->kq_lim, qc) + growth(s->kw_sample, nws * 32) +
+                  growth(s->ksmin, qc * nws) + growth(s->kpart, knn_part_entries(k)) +
+                  growth(s->kpart_n, knn_part_lists(k)) + growth(s->kfallback, qc);
+    if (!ix->kx_valid) need += growth(ix->kx_h, (size_t)ix->N * k.Dp) + growth(ix->kx_w, (size_t)ix->N + 255);
+    if (!ix->big_valid) need += big_rows_bytes(ix, k.nseg);
+    if (!room_for(need)) {
+        s->knn_no_room = true;
+        *ok = false;
+        return CULSH_OK;
+    }
+    TRY(ensure_knn_rows(ix, st));
+    *ok = knn_dataset_fits(ix->h_kstate);
+    if (!*ok) return CULSH_OK;
+    TRY(ensure_big_rows(ix, k.nwp, k.nseg, st));
+    CU_TRY(s->kbm.reserve(qc * k.nwp));
+    CU_TRY(s->kbm_sample.reserve(qc * nws));
+    CU_TRY(s->kq_h.reserve(qc * k.Dp));
+    CU_TRY(s->kq_info.reserve(qc));
+    CU_TRY(s->kq_lim.reserve(qc));
+    CU_TRY(s->kw_sample.reserve(nws * 32));
+    CU_TRY(s->ksmin.reserve(qc * nws));
+    CU_TRY(s->kpart.reserve(knn_part_entries(k)));
+    CU_TRY(s->kpart_n.reserve(knn_part_lists(k)));
+    CU_TRY(s->kfallback.reserve(qc));
+    return CULSH_OK;
+}
+
 // Serves the nd dense queries the planner listed (s->dense_q) once the rest of
 // the search has run: their number is known here, so that a search without
 // any launches nothing for them and buffers are sized by those it has. The
@@ -1240,20 +1326,24 @@ int run_dense(culsh_search* s, const SearchPlan& P, int nd, cudaStream_t st, boo
     *left = false;
     if (knn) {
         std::lock_guard<std::mutex> lk(alloc_capture_mutex());
-        TRY(ensure_knn_rows(ix, st));
-        knn = knn_dataset_fits(ix->h_kstate);
-        if (knn) {
-            TRY(ensure_big_rows(ix, k.nwp, k.nseg, st));
-            CU_TRY(s->kbm.reserve((size_t)k.Qcap * k.nwp));
-            CU_TRY(s->kbm_sample.reserve((size_t)k.Qcap * k.nws));
-            CU_TRY(s->kq_h.reserve((size_t)k.Qcap * k.Dp));
-            CU_TRY(s->kq_info.reserve(k.Qcap));
-            CU_TRY(s->kq_lim.reserve(k.Qcap));
-            CU_TRY(s->kw_sample.reserve((size_t)k.nws * 32));
-            CU_TRY(s->ksmin.reserve((size_t)k.Qcap * k.nws));
-            CU_TRY(s->kpart.reserve(knn_part_entries(k)));
-            CU_TRY(s->kpart_n.reserve(knn_part_lists(k)));
-            CU_TRY(s->kfallback.reserve(k.Qcap));
+        const int rc = reserve_knn(s, k, st, &knn);
+        if (rc == CULSH_ERR_OUT_OF_MEMORY) {   // the room was taken meanwhile, or is in pieces
+            cudaGetLastError();
+            knn = false;
+            s->knn_no_room = true;
+            release_knn(s);
+            if (!ix->kx_valid) {
+                ix->kx_h.release();
+                ix->kx_w.release();
+            }
+            if (!ix->big_valid) {
+                ix->bank.release();
+                ix->bank_tail.release();
+                ix->bank_meta.release();
+                ix->big_rows.release();
+            }
+        } else if (rc != CULSH_OK) {
+            return rc;
         }
     }
     if (!knn) {
@@ -1536,7 +1626,7 @@ int plan_search(culsh_search* s, const float* dQ, int Q, int32_t* d_ids, float* 
             return d;
         };
         KnnSearch shapes;
-        const bool knn = tu.dense_tc && !getenv("CULSH_NO_KNN_TC") && reach >= dense_min_for(true) &&
+        const bool knn = tu.dense_tc && !getenv("CULSH_NO_KNN_TC") && !s->knn_no_room && reach >= dense_min_for(true) &&
                          !(ix->kx_valid && !knn_dataset_fits(ix->h_kstate)) &&
                          knn_shapes(ix, K, Q, s->sms, s->smem_optin, &shapes);
         const unsigned long long dmin = dense_min_for(knn);
@@ -2187,6 +2277,7 @@ int culsh_search_reset(culsh_search* s, culsh_index* ix, int K, int T) {
     s->Q = 0;
     s->searched = false;
     s->qb_host_valid = false;
+    s->knn_no_room = false;
     s->tot_unique = s->tot_nonunique = 0;
     s->times = culsh_times{};
     return CULSH_OK;
@@ -2385,16 +2476,8 @@ int culsh_search_release(culsh_search* s) {
     s->small_q.release();
     s->qorder.release();
     s->qorder_bins.release();
-    s->kbm.release();
-    s->kbm_sample.release();
-    s->kq_h.release();
-    s->kq_info.release();
-    s->kq_lim.release();
-    s->kw_sample.release();
-    s->ksmin.release();
-    s->kpart.release();
-    s->kpart_n.release();
-    s->kfallback.release();
+    release_knn(s);
+    s->knn_no_room = false;
     s->Q = 0;
     s->searched = false;
     s->qb_host_valid = false;

@@ -1,0 +1,63 @@
+"""Forms that take over where the usual one does not apply: dense queries
+whose tensor-core buffers do not fit the device, or whose data that path does
+not take, against the oracle."""
+
+import numpy as np
+import pytest
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _case(seed, N, D, L, M, W, Q, scale=1.0):
+    rng = np.random.default_rng(seed)
+    X = (rng.normal(0, scale, (N, D))).astype(np.float32)
+    Qm = (rng.normal(0, scale, (Q, D))).astype(np.float32)
+    A = rng.normal(0, 1, (L, M, D)).astype(np.float32)
+    b = (rng.random((L, M)) * W).astype(np.float32)
+    return X, Qm, A, b
+
+
+def _search(culsh, X, A, b, W, K, T, **tuning):
+    L, M, D = A.shape
+    ht = culsh.HashTables()
+    ht.reset(X.shape[0], D, L, M, W, A=A, b=b)
+    ht.index(X)
+    st = culsh.SearchTables()
+    st.reset(ht, K, T)
+    if tuning:
+        st.set_tuning(**tuning)
+    return st
+
+
+def _check(st, want):
+    np.testing.assert_array_equal(st.getKnnIds(), want["knn_ids"])
+    np.testing.assert_array_equal(st.getKnnDistances(), want["knn_dists"])
+    assert st.getTotalCandidates_unique() == int(want["unique"].sum())
+    assert st.getTotalCandidates_nonUnique() == int(want["nonunique"].sum())
+
+
+@pytest.mark.parametrize("N", [30_000, 1_900_000])
+def test_dense_without_room(culsh, monkeypatch, N):
+    """The tensor-core path's buffers do not fit: the bitmap kernel, or (bits of
+    more points than a block holds) the per-query kernel serves the queries
+    that were listed as dense, and later searches plan without the path. A
+    search object that is reset tries again."""
+    D, L, M, W, Q, K, T = 4, 2, 2, 4.0, 6, 10, 4
+    X, Qm, A, b = _case(N, N, D, L, M, W, Q)
+    want = oracle.search(oracle.build_index(X, A, b, W), X, Qm, K, T)
+    monkeypatch.setenv("CULSH_SCRATCH_MAX_BYTES", "1000")
+    st = _search(culsh, X, A, b, W, K, T)
+    for _ in range(2):
+        st.search(Qm, dataset=X)
+        _check(st, want)
+        assert st.profile()["knn_queries"] == 0
+    monkeypatch.delenv("CULSH_SCRATCH_MAX_BYTES")
+    st.search(Qm, dataset=X)
+    _check(st, want)
+    assert st.profile()["knn_queries"] == 0
+    st.reset(st._ht, K, T)
+    st.search(Qm, dataset=X)
+    _check(st, want)
+    assert st.profile()["knn_queries"] > 0

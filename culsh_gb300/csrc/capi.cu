@@ -1477,7 +1477,8 @@ int plan_search(culsh_search* s, const float* dQ, int Q, int32_t* d_ids, float* 
         // probes then find nothing (1M points, every one its own bucket, T = 16:
         // 148 us fused, 117 us so; at 20,000 buckets a table fused is ahead, 160 against
         // 167 us; 1,291 queries of T = 5 on 33K points 25 us fused, 29 us so).
-        if (P.pa.auto_form && M <= 16 && T >= 8 && 4 * (unsigned long long)ix->h_boff[L] > (unsigned long long)ix->N * L)
+        if (P.pa.auto_form && M <= 16 && T >= 8 && 4 * (unsigned long long)ix->h_boff[L] > (unsigned long long)ix->N * L &&
+            room_for(growth(s->ph, (size_t)L * Q * T) + growth(s->pmask, (size_t)L * Q * T)))
             form = 2;
         if (form > 0) {
             CU_TRY(s->ph.reserve((size_t)L * Q * T));

@@ -61,3 +61,23 @@ def test_dense_without_room(culsh, monkeypatch, N):
     st.search(Qm, dataset=X)
     _check(st, want)
     assert st.profile()["knn_queries"] > 0
+
+
+def test_probe_form_without_room(culsh, monkeypatch):
+    """Narrow buckets and eight or more probes: the lookups behind the key filter
+    want a hash and a mask per probe; without room the fused form runs."""
+    N, D, L, M, W, Q, K, T = 20_000, 16, 4, 8, 1.0, 5_000, 5, 8
+    X, _, A, b = _case(7, N, D, L, M, W, 1)
+    Qm = X[:Q]
+    want = oracle.search(oracle.build_index(X, A, b, W), X, Qm, K, T)
+    held = {}
+    for limit in (None, "1000"):
+        if limit:
+            monkeypatch.setenv("CULSH_SCRATCH_MAX_BYTES", limit)
+        st = _search(culsh, X, A, b, W, K, T)
+        st.search(Qm, dataset=X)
+        _check(st, want)
+        for l in range(L):
+            np.testing.assert_array_equal(st.getQueryBuckets(l), want["qbuckets"][l].reshape(Q, T))
+        held[limit] = culsh.lib().culsh_search_device_bytes(st._h)
+    assert held["1000"] + 12 * L * Q * T <= held[None]

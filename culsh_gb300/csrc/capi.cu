@@ -242,10 +242,13 @@ struct SearchTune {
     int dist_bf16 = 0;     // 1: BF16 candidate distances + certified FP32 rerank (work-stealing form)
     int ws_slots = 4096;   // shared hash-set slots per work item (4096, 8192 or 16384)
     int probe_split = 0;   // M <= 16: 1 enumeration kernel + lookup kernel; 2 lookups at the enumeration's end
-    bool probe_auto = true;   // probe_split and probe_pch as created: the form may follow the shape
     int ws_order = 0;      // 1: plan queries in the locality order of their home bucket (work-stealing form)
     int dense_tc = 1;      // 1: dense queries take the tensor-core path (membership rows + masked GEMM)
     int dense_min = 0;     // non-unique candidates that make a query dense (0: the form's default)
+    // The probe settings as created ask for no form: it follows the shape. Read
+    // from the settings themselves, so that a tuning that was read, stored or
+    // changed elsewhere keeps it.
+    bool probe_auto() const { return probe_split == 0 && probe_pch == 2; }
 };
 constexpr size_t kPlanBytes = 2048;   // room for the graph key (checked below)
 
@@ -1471,7 +1474,7 @@ int plan_search(culsh_search* s, const float* dQ, int Q, int32_t* d_ids, float* 
         // CULSH_PROBE_SPLIT=0/1 overrides the tuning (the tests run both).
         const char* e = getenv("CULSH_PROBE_SPLIT");
         int form = M <= 16 ? std::min(2, std::max(0, e ? atoi(e) : tu.probe_split)) : 0;
-        P.pa.auto_form = tu.probe_auto && !e;
+        P.pa.auto_form = tu.probe_auto() && !e;
         // No form set: lookups behind the key filter at the enumeration's end
         // where buckets hold fewer than four points on average, since most
         // probes then find nothing (1M points, every one its own bucket, T = 16:
@@ -2529,7 +2532,6 @@ int culsh_search_set_tuning(culsh_search* s, const culsh_tuning* in) {
     s->tune.dist_bf16 = in->distance_bf16;
     s->tune.ws_slots = in->ws_set_slots;
     s->tune.probe_split = in->probe_split;
-    s->tune.probe_auto = false;
     s->tune.ws_order = in->ws_order;
     s->tune.dense_tc = in->dense_tc;
     s->tune.dense_min = in->dense_min;
@@ -2605,7 +2607,6 @@ int culsh_search_autotune(culsh_search* s, const float* d_queries, int Q, int* d
     };
     const SearchTune start = s->tune;
     SearchTune best = start;
-    best.probe_auto = false;
     float stage[4];
     float best_t = 0;
     // projection tiling
@@ -2622,8 +2623,9 @@ int culsh_search_autotune(culsh_search* s, const float* d_queries, int Q, int* d
             best.proj_tile = tile;
         }
     }
-    // probe form: fused with batch depth 1, 2 or 4, or (M <= 16) split
-    // lookups, or lookups at the end of the enumeration
+    // probe form: fused with batch depth 1 or 4, the form that follows the
+    // shape (in the place of depth 2), or (M <= 16) split lookups, or lookups at
+    // the end of the enumeration
     const int pchs[5] = {1, 2, 4, 0, -1};
     const int nforms = s->ix->M <= 16 ? 5 : 3;
     for (int i = 0; i < nforms; ++i) {

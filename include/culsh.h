@@ -153,8 +153,11 @@ typedef struct culsh_tuning {
     int configs_tried;    /* culsh_search_autotune: configurations timed                 */
     int probe_split;      /* M <= 16: 1 enumerate every probe first, then look each up in
                              its own thread behind a key filter; 2 look a pair's probes
-                             up behind the filter at the end of its enumeration
-                             (same results as 0)                                        */
+                             up behind the filter at the end of its enumeration;
+                             0 fused lookups. 0 with probe_batch 2, as created: the
+                             form follows the shape (a warp per pair for few pairs,
+                             2 for narrow buckets and 8 or more probes, else fused).
+                             Same results in every form                                 */
     int ws_order;         /* 1: work-stealing items planned in the locality order of the
                              queries' home buckets, so queries that share candidates run
                              together and share rows in L2 (same results as 0)         */

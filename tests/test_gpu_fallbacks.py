@@ -81,3 +81,43 @@ def test_probe_form_without_room(culsh, monkeypatch):
             np.testing.assert_array_equal(st.getQueryBuckets(l), want["qbuckets"][l].reshape(Q, T))
         held[limit] = culsh.lib().culsh_search_device_bytes(st._h)
     assert held["1000"] + 12 * L * Q * T <= held[None]
+
+
+@pytest.mark.parametrize("how", ["set", "set_other", "restore", "autotune"])
+def test_probe_form_survives_tuning(culsh, how):
+    """The probe form follows the shape until a form is set: a tuning that is
+    read and written back, changed elsewhere, or set and restored keeps it.
+    (The form behind the key filter shows by its buffers.)"""
+    N, D, L, M, W, Q, K, T = 20_000, 16, 4, 8, 1.0, 20_000, 5, 8
+    X, _, A, b = _case(8, N, D, L, M, W, 1)
+    st = _search(culsh, X, A, b, W, K, T)
+    created = st.get_tuning()
+    if how == "set":
+        st.set_tuning()
+    elif how == "set_other":
+        st.set_tuning(ws_threads=256)
+    elif how == "restore":
+        st.set_tuning(probe_split=1, probe_batch=4)
+        st.set_tuning(**created)
+    else:   # the tuner times that form too: what it returns, set again, is what it timed
+        torch = pytest.importorskip("torch")
+        q = torch.from_numpy(X).cuda()
+        ids = torch.empty((Q, K), dtype=torch.int32, device="cuda")
+        d = torch.empty((Q, K), dtype=torch.float32, device="cuda")
+        tune = st.autotune(q.data_ptr(), Q, ids.data_ptr(), d.data_ptr())
+        own = _search(culsh, X, A, b, W, K, T)
+        own.set_tuning(**{k: tune[k] for k in created if k not in ("search_ms", "configs_tried")})
+        for s in (st, own):
+            culsh.lib().culsh_search_release(s._h)
+            s.search(X, dataset=X)
+        assert culsh.lib().culsh_search_device_bytes(st._h) == culsh.lib().culsh_search_device_bytes(own._h)
+        return
+    st.search(X, dataset=X)
+    want = _search(culsh, X, A, b, W, K, T)
+    want.search(X, dataset=X)
+    assert culsh.lib().culsh_search_device_bytes(st._h) == culsh.lib().culsh_search_device_bytes(want._h)
+    st.set_tuning(probe_batch=1)   # a form set: no filter buffers
+    culsh.lib().culsh_search_release(st._h)
+    st.search(X, dataset=X)
+    assert (culsh.lib().culsh_search_device_bytes(st._h) + 12 * L * Q * T
+            == culsh.lib().culsh_search_device_bytes(want._h))

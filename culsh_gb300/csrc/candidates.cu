@@ -390,7 +390,7 @@ __global__ void __launch_bounds__(32 * SMW) k_candidates_small(WsArgs a) {
         const uint32_t per = vec ? 16 : 4, sub = vec ? lane >> 1 : lane >> 3;
         for (uint32_t b = 0; b < U; b += per) {
             const uint32_t e = b + sub;
-            const float d = row_distance(a.X + (int64_t)(e < U ? s_id[w][e] : 0u) * D, D, qs, vec, e < U);
+            const float d = row_distance<2>(a.X + (int64_t)(e < U ? s_id[w][e] : 0u) * D, D, qs, vec, e < U);
             if (e < U && (lane & (vec ? 1 : 7)) == 0) s_d[w][e] = d;
         }
         __syncwarp();
@@ -423,8 +423,16 @@ __global__ void __launch_bounds__(32 * SMW) k_candidates_small(WsArgs a) {
     }
 }
 
+// Registers for the row loads in flight: as many blocks per SM are asked for as
+// a set of 4,096 slots leaves room for (30 KB each: 7 of 128 threads) or 32
+// warps' registers do, which gives 64 to 72 registers; left alone, the compiler
+// took 40 to 128 as the code around the loads changed. 10,000 queries of 12,900
+// candidates, K = 10, after the gather's change (gather_bucket_ids): 16.0 ms at
+// 128 threads and sets of 4,096, 9.6 at 256 and 8,192, now 15.2 and 8.8; 2,000
+// queries of 13,800 at 10M x 96 5.6, now 4.8.
+constexpr int ws_min_blocks(int WT) { return WT == 512 ? 2 : WT == 256 ? 4 : WT == 128 ? 7 : 8; }
 template <int WT, int W_SLOTS, bool STAGED>
-__global__ void __launch_bounds__(WT) k_candidates_ws(WsArgs a) {
+__global__ void __launch_bounds__(WT, ws_min_blocks(WT)) k_candidates_ws(WsArgs a) {
     constexpr int WW = WT / 32;
     constexpr uint32_t W_CAP = W_SLOTS / 2;
     extern __shared__ __align__(16) unsigned char smem[];
@@ -481,7 +489,7 @@ __global__ void __launch_bounds__(WT) k_candidates_ws(WsArgs a) {
 
         // Gather this item's id partition from every matched bucket.
         const BucketView bv{a.qbuckets, a.boff, a.starts, a.sizes, a.ids, a.N, L, T, a.Q};
-        gather_bucket_ids<WT, GCH>(bv, q, s_gather, [&](uint32_t id) {
+        gather_bucket_ids<WT, GCH, (WT < 256 ? 2 : 1)>(bv, q, s_gather, [&](uint32_t id) {
             const uint32_t h = id_hash(id);
             if (P > 1 && __umulhi(h, P) != p) return;
             set_insert_at(hset, slots - 1, ulist, W_CAP, &s_ucount, id, h);
@@ -672,7 +680,7 @@ __global__ void __launch_bounds__(WT) k_candidates_ws_bf16(WsArgs a) {
 
         // Gather this item's id partition from every matched bucket.
         const BucketView bv{a.qbuckets, a.boff, a.starts, a.sizes, a.ids, a.N, L, T, a.Q};
-        gather_bucket_ids<WT, GCH>(bv, q, s_gather, [&](uint32_t id) {
+        gather_bucket_ids<WT, GCH, 4>(bv, q, s_gather, [&](uint32_t id) {
             if (P > 1 && (uint32_t)(((uint64_t)mix32(id ^ kPartSalt) * P) >> 32) != p) return;
             set_insert(hset, W_SLOTS - 1, ulist, W_CAP, &s_ucount, id);
         });
@@ -1023,8 +1031,8 @@ __global__ void __launch_bounds__(DT, 1) k_candidates_dense(WsArgs a) {
         for (uint32_t i = tid; i < nwords; i += DT) bits[i] = 0u;
         __syncthreads();
         const BucketView bv{a.qbuckets, a.boff, a.starts, a.sizes, a.ids, a.N, L, T, a.Q};
-        gather_bucket_ids<DT, GCH>(bv, q, s_gather,
-                                   [&](uint32_t id) { atomicOr(&bits[id >> 5], 1u << (id & 31)); });
+        gather_bucket_ids<DT, GCH, 4>(bv, q, s_gather,
+                                      [&](uint32_t id) { atomicOr(&bits[id >> 5], 1u << (id & 31)); });
         __syncthreads();
 
         const unsigned long long U = scan_words(a.X, D, K, nwords, [&](uint32_t w) { return bits[w]; }, qs, vec, sc,

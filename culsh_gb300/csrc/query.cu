@@ -1227,7 +1227,7 @@ __global__ void __launch_bounds__(CT) k_candidates(CandArgs a) {
     const uint32_t mask = cap - 1;
     const uint32_t lcap = C > (unsigned long long)SM_CAP ? (uint32_t)C : (uint32_t)SM_CAP;
     const BucketView bv{a.qbuckets, a.boff, a.starts, a.sizes, a.ids, a.N, L, T, a.Q};
-    gather_bucket_ids<CT, GCH>(bv, q, s_gather,
+    gather_bucket_ids<CT, GCH, 1>(bv, q, s_gather,
                                [&](uint32_t id) { set_insert(hset, mask, ulist, lcap, &s_ucount, id); });
     __syncthreads();
     const uint32_t U = s_ucount;

@@ -83,21 +83,38 @@ __device__ __forceinline__ void set_insert(uint32_t* hset, uint32_t mask, uint32
 // D % 4 == 0, four of the eight lane partials each from 16-byte loads) or
 // eight lanes that share the row; lanes without a row pass on = false. Every
 // lane of the warp calls it and every lane of a group gets the distance.
+// The 16-byte loads are issued RL at a time before the first is used: left
+// to the compiler, how many were in flight changed with the code around the
+// call (10,000 queries of 12,900 candidates, 256 threads an item: 11.6 to 16.2
+// ms).
+// RL: such loads; 2 in k_candidates_small, whose warps have a row or two each
+// (10,000 look-ups of one point: 240 us a search, 258 with 8, which take 99
+// registers a thread instead of 64).
+template <int RL = 8>
 __device__ __forceinline__ float row_distance(const float* __restrict__ x, int D, const float* qs, bool vec, bool on) {
     const int lane = threadIdx.x & 31;
     if (vec) {
         float s0 = 0.f, s1 = 0.f, s2 = 0.f, s3 = 0.f;
         if (on) {
-#pragma unroll 8
-            for (int c = 4 * (lane & 1); c < D; c += 8) {
-                const float4 v = __ldg(reinterpret_cast<const float4*>(x + c));
-                const float4 qv = *reinterpret_cast<const float4*>(qs + c);
-                const float d0 = __fsub_rn(qv.x, v.x), d1 = __fsub_rn(qv.y, v.y);
-                const float d2 = __fsub_rn(qv.z, v.z), d3 = __fsub_rn(qv.w, v.w);
-                s0 = __fmaf_rn(d0, d0, s0);
-                s1 = __fmaf_rn(d1, d1, s1);
-                s2 = __fmaf_rn(d2, d2, s2);
-                s3 = __fmaf_rn(d3, d3, s3);
+            for (int c0 = 4 * (lane & 1); c0 < D; c0 += 8 * RL) {
+                float4 xv[RL];
+#pragma unroll
+                for (int i = 0; i < RL; ++i)
+                    xv[i] = c0 + 8 * i < D ? __ldg(reinterpret_cast<const float4*>(x + c0 + 8 * i))
+                                           : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+                for (int i = 0; i < RL; ++i) {
+                    const int c = c0 + 8 * i;
+                    if (c >= D) break;
+                    const float4 v = xv[i];
+                    const float4 qv = *reinterpret_cast<const float4*>(qs + c);
+                    const float d0 = __fsub_rn(qv.x, v.x), d1 = __fsub_rn(qv.y, v.y);
+                    const float d2 = __fsub_rn(qv.z, v.z), d3 = __fsub_rn(qv.w, v.w);
+                    s0 = __fmaf_rn(d0, d0, s0);
+                    s1 = __fmaf_rn(d1, d1, s1);
+                    s2 = __fmaf_rn(d2, d2, s2);
+                    s3 = __fmaf_rn(d3, d3, s3);
+                }
             }
         }
         const float o0 = __shfl_xor_sync(0xffffffffu, s0, 1), o1 = __shfl_xor_sync(0xffffffffu, s1, 1);
@@ -279,6 +296,13 @@ __device__ __forceinline__ void fp32_dist_pass(const float* __restrict__ X, int 
 // chunk visited as one flattened range so that small and large buckets both
 // keep every thread busy. f(id) is called once per (bucket, id) occurrence by
 // some thread of the block; every thread must call this function.
+// GU: ids a thread loads before it visits the first (each load alone waits out
+// its latency, but a step of GU x NT ids spans more buckets, each looked up anew,
+// and the visit's branches are repeated per id). 10,000 queries of 12,900
+// candidates in 128 buckets, 1 / 2 / 4 ids: FP32 items of 128 threads 18.2 /
+// 16.0 / 21.1 ms, of 256 threads 11.9 / 13.7 / 17.9, the per-query kernel 17.4 /
+// 18.6 / 20.0; the bitmap kernel (a visit is one atomic) 22.8 with 1, 21.9 with 4,
+// BF16 items of 128 threads 26.7 with 2, 25.8 with 4.
 struct BucketView {
     const int32_t* qbuckets;   // [L][Q*T]
     const uint64_t* boff;      // [L+1]
@@ -296,7 +320,7 @@ struct GatherSmem {
     uint32_t n;
 };
 
-template <int NT, int CH, class F>
+template <int NT, int CH, int GU, class F>
 __device__ __forceinline__ void gather_bucket_ids(const BucketView& v, int q, GatherSmem<NT, CH>& g, F f) {
     const int tid = threadIdx.x, lane = tid & 31;
     const int T = v.T, LT = v.L * v.T;
@@ -338,9 +362,7 @@ __device__ __forceinline__ void gather_bucket_ids(const BucketView& v, int q, Ga
         const unsigned long long total = g.pre[n - 1];
         // h: first bucket whose inclusive prefix exceeds i. i only grows, so
         // h is kept between steps and searched for only when i leaves it.
-        // Four ids are loaded before the first is visited (one at a time, each
-        // visit waited out a load).
-        constexpr int GU = 4;
+        // GU ids are loaded before the first is visited.
         uint32_t h = 0;
         for (unsigned long long i0 = tid; i0 < total; i0 += GU * NT) {
             uint32_t id[GU];

@@ -108,3 +108,27 @@ def test_warp_probe(culsh, M, T, Q, ties):
     st.reset(ht, K, T)
     st.search(Qm, dataset=X)
     _check(st, want, L, Q, T)
+
+
+@pytest.mark.parametrize("D", [4, 60, 64, 68, 124, 132])
+@pytest.mark.parametrize("wt", [64, 128, 256, 512, 0])
+def test_gather_steps(culsh, wt, D):
+    """Candidate lists of lengths around the gather's steps of every width (one
+    or two ids a thread; wt = 0: the per-query kernel) and rows around the eight
+    16-byte loads a lane keeps in flight."""
+    sizes = [33, 63, 64, 127, 128, 129, 255, 256, 257, 511, 512, 513, 1023, 1024, 1025, 3000]
+    rng = np.random.default_rng(wt + D)
+    G, K, T, L, M, W = len(sizes), 10, 1, 2, 1, 4.0
+    X = rng.normal(0, 1, (sum(sizes), D)).astype(np.float32)
+    X[:, 0] = np.repeat(np.arange(G), sizes) * 100.0 + rng.random(sum(sizes)) * 3.9   # a bucket each
+    Qm = np.zeros((2 * G, D), np.float32)
+    Qm[:, 0] = np.tile(np.arange(G) * 100.0 + 2.0, 2)
+    A = np.zeros((L, M, D), np.float32)
+    A[:, 0, 0] = 1.0
+    b = np.zeros((L, M), np.float32)
+    want = oracle.search(oracle.build_index(X, A, b, W), X, Qm, K, T)
+    st = culsh.SearchTables()
+    st.reset(_index(culsh, X, A, b, W), K, T)
+    st.set_tuning(dense_min=1 << 30, **({"ws_threads": wt} if wt else {"candidates_mode": 0}))
+    st.search(Qm, dataset=X)
+    _check(st, want, L, 2 * G, T)

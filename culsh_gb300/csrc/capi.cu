@@ -1029,19 +1029,22 @@ size_t arena_cap_words() {
 }
 
 // Whether buffers that a faster form of a stage wants, and another form does
-// without, may take `bytes` more of device memory: they must leave the arena's
-// margin free. CULSH_SCRATCH_MAX_BYTES lowers the most they may take (the tests
+// without, may take `bytes` more of device memory: they must leave 64 MB free
+// (the question takes 25 us; buffers of less than that are not worth it).
+// CULSH_SCRATCH_MAX_BYTES lowers the most they may take (the tests
 // reach the other forms with it).
 bool room_for(size_t bytes) {
+    constexpr size_t margin = size_t(64) << 20;
     if (bytes == 0) return true;
     if (const char* e = getenv("CULSH_SCRATCH_MAX_BYTES"))
         if (bytes > strtoull(e, nullptr, 10)) return false;
+    if (bytes <= margin) return true;
     size_t freeb = 0, totalb = 0;
     if (cudaMemGetInfo(&freeb, &totalb) != cudaSuccess) {
         cudaGetLastError();
         return false;
     }
-    return bytes + 4 * kArenaInitialWords <= freeb;
+    return bytes + margin <= freeb;
 }
 // Bytes that reserving cnt elements adds to a buffer.
 template <class T>

@@ -118,6 +118,7 @@ ABI = {
     "culsh_index_sizes": (_UP, [_P, _I]),
     "culsh_index_codes": (_FP, [_P, _I]),
     "culsh_index_profile_get": (_I, [_P, ctypes.POINTER(_IndexProfile)]),
+    "culsh_index_hash_form": (_I, [_P, ctypes.POINTER(ctypes.c_uint)]),
     "culsh_search_create": (_I, [ctypes.POINTER(_P)]),
     "culsh_search_destroy": (None, [_P]),
     "culsh_search_reset": (_I, [_P, _P, _I, _I]),

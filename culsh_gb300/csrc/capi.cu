@@ -221,6 +221,8 @@ struct culsh_index {
     DevBuf<unsigned long long> ws_run_pos;
     DevBuf<uint32_t> ws_run_len;
     DevBuf<unsigned int> ws_run_cnt;
+    int hash_form = 0;                // 1: tables by parts, 2: by parts, then in place, 0: in place
+    unsigned hash_spilled = 0;        // keys the parts could not take
     int sort_form = 0;   // 1: top-word passes + run ordering, 2: that form fell back to all words, 0: all words
 
     ~culsh_index() {
@@ -501,9 +503,16 @@ int upload_layout(culsh_index* ix, cudaStream_t st) {
 // groups of kGroupSlots slots. with_sizes: a build, which wants the bucket sizes
 // too and may build the tables by parts in the space of the codes it no longer
 // needs; *spill then points at the number of keys placed afterwards, to be
-// checked against kHashSpill by the caller (once the stream has been waited
-// for), who calls again with in_place.
+// checked against hash_spill_cap() by the caller (once the stream has been waited
+// for), who calls again with in_place. CULSH_HASH_SPILL and CULSH_HASH_PART_CAP
+// lower the keys placed afterwards and a part's records (the tests reach both
+// ends of the form with them), CULSH_HASH_PARTS_MIN the keys it starts from.
 constexpr uint32_t kHashSpill = 1u << 20;
+uint32_t env_at_most(const char* name, uint32_t most) {
+    const char* e = getenv(name);
+    return e ? (uint32_t)std::min<unsigned long long>(strtoull(e, nullptr, 10), most) : most;
+}
+uint32_t hash_spill_cap() { return env_at_most("CULSH_HASH_SPILL", kHashSpill); }
 int build_hash(culsh_index* ix, bool with_sizes, bool in_place, const uint32_t** spill, cudaStream_t st) {
     const int L = ix->L;
     ix->h_hoff.assign(L + 1, 0);
@@ -560,7 +569,9 @@ int build_hash(culsh_index* ix, bool with_sizes, bool in_place, const uint32_t**
     // that fill no device) and 17 in place, 16M 0.38 and 0.49 ms, 200M 5.4 and 9.
     const uint64_t parts = std::max<uint64_t>(max_groups / kHashPartGroups, 1);
     const size_t rec = (size_t)L * parts * kHashPartCap, cnt = (size_t)L * parts + 1;
-    const size_t need = 8 * rec + 8 * (size_t)kHashSpill + 4 * cnt + 64;
+    h.spill_cap = hash_spill_cap();
+    h.part_cap = env_at_most("CULSH_HASH_PART_CAP", kHashPartCap);
+    const size_t need = 8 * rec + 8 * (size_t)h.spill_cap + 4 * cnt + 64;
     const char* floor_env = getenv("CULSH_HASH_PARTS_MIN");
     const uint64_t from = floor_env ? strtoull(floor_env, nullptr, 10) : 2000000;
     if (spill && !in_place && with_sizes && ix->KW <= 4 && parts <= kHashMaxParts && ix->h_boff[L] >= from &&
@@ -568,8 +579,7 @@ int build_hash(culsh_index* ix, bool with_sizes, bool in_place, const uint32_t**
         unsigned char* base = reinterpret_cast<unsigned char*>(ix->ws_codes.p);
         h.rec = reinterpret_cast<unsigned long long*>(base);
         h.spill = reinterpret_cast<uint2*>(h.rec + rec);
-        h.spill_cap = kHashSpill;
-        h.part_cnt = reinterpret_cast<uint32_t*>(h.spill + kHashSpill);
+        h.part_cnt = reinterpret_cast<uint32_t*>(h.spill + h.spill_cap);
         CU_TRY(launch_hash_build_parts(h, st));
         *spill = h.part_cnt + (cnt - 1);
         return CULSH_OK;
@@ -880,7 +890,10 @@ int build_device(culsh_index* ix, const float* dX, cudaStream_t st, FILE* dbg) {
     if (spill) CU_TRY(cudaMemcpyAsync(ix->h_maxb + 1, spill, sizeof(uint32_t), cudaMemcpyDeviceToHost, st));
     CU_TRY(cudaEventRecord(ix->bev[4], st));
     TRY(read_err_flag(ix, st, "index"));   // synchronises the stream
-    if (ix->h_maxb[1] > kHashSpill) {    // more keys in a few parts than they can hold
+    ix->hash_form = spill ? 1 : 0;
+    ix->hash_spilled = ix->h_maxb[1];
+    if (ix->hash_spilled > hash_spill_cap()) {    // more keys in a few parts than they can hold
+        ix->hash_form = 2;
         TRY(build_hash(ix, true, true, nullptr, st));
         CU_TRY(cudaEventRecord(ix->bev[4], st));
         TRY(read_err_flag(ix, st, "index"));
@@ -977,6 +990,8 @@ int ensure_device(culsh_index* ix, cudaStream_t st) {
     CU_TRY(ix->ukeys.reserve(totB * ix->KW));
     CU_TRY(launch_pack_from_codes(ix->boff.p, ix->dcodes.p, L, M, ix->KW, maxB, ix->cmin.p, ix->fbits.p, ix->foff.p,
                                   ix->ukeys.p, st));
+    ix->hash_form = 0;
+    ix->hash_spilled = 0;
     TRY(build_hash(ix, false, true, nullptr, st));
     TRY(read_err_flag(ix, st, "load"));
     ix->dev_valid = true;
@@ -2265,6 +2280,11 @@ int culsh_index_profile_get(culsh_index* ix, culsh_index_profile* out) {
     out->sort_passes = ix->sort_passes;
     out->sort_form = ix->sort_form;
     return CULSH_OK;
+}
+
+int culsh_index_hash_form(const culsh_index* ix, unsigned* spilled) {
+    if (spilled) *spilled = ix ? ix->hash_spilled : 0;
+    return ix ? ix->hash_form : 0;
 }
 
 int culsh_search_create(culsh_search** out) {

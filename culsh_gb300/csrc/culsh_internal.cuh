@@ -306,6 +306,7 @@ struct HashBuild {
     uint32_t* part_cnt;           // [L][parts], then the spill count
     uint2* spill;                 // (table, bucket)
     uint32_t spill_cap;
+    uint32_t part_cap;            // records a part takes, at most kHashPartCap
 };
 constexpr uint32_t kHashPartGroups = 2048;   // groups built together in shared memory
 constexpr uint32_t kHashPartCap = 4672;      // a part's records: 4,096 expected at most, 9 deviations more

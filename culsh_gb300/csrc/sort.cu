@@ -1099,6 +1099,8 @@ constexpr int HS_T = 512, HS_ITEMS = 16, HS_TILE = HS_T * HS_ITEMS;
 static_assert(kHashPartGroups == 2048 && HS_TILE <= 8192 && kHashMaxParts <= 4096, "bit fields of a record and of a rank");
 constexpr size_t hash_split_smem(uint32_t parts) { return (size_t)HS_TILE * 10 + (size_t)parts * 8; }
 
+// A key that its part cannot take is listed; past the list's end it is only
+// counted, and the caller of the form, who reads the count, builds in place.
 __device__ __forceinline__ void hash_spill(const HashBuild& h, uint32_t* cnt, int l, uint32_t j) {
     const uint32_t s = atomicAdd(cnt, 1u);
     if (s < h.spill_cap) h.spill[s] = make_uint2((uint32_t)l, j);
@@ -1172,7 +1174,7 @@ __global__ void __launch_bounds__(HS_T, 2) k_hash_split(HashBuild h, uint32_t pa
     const int n = (int)min((int64_t)HS_TILE, B - t0);
     for (int sp = tid; sp < n; sp += HS_T) {
         const uint32_t part = bin[sp], at = gpos[part] + (uint32_t)sp;
-        if (at < kHashPartCap) h.rec[((size_t)l * parts + part) * kHashPartCap + at] = buf[sp];
+        if (at < h.part_cap) h.rec[((size_t)l * parts + part) * kHashPartCap + at] = buf[sp];
         else hash_spill(h, h.part_cnt + (size_t)h.L * parts, l, (uint32_t)buf[sp]);
     }
     bucket_sizes<HS_T, HS_ITEMS>(h, bo, B, t0 + tid);
@@ -1196,7 +1198,7 @@ __global__ void __launch_bounds__(NT) k_hash_fill(HashBuild h, uint32_t parts) {
     __syncthreads();
     const size_t base = (size_t)l * parts + part;
     const unsigned long long* rec = h.rec + base * kHashPartCap;
-    const uint32_t n = min(h.part_cnt[base], kHashPartCap);
+    const uint32_t n = min(h.part_cnt[base], h.part_cap);
     for (uint32_t i0 = tid; i0 < n; i0 += 4 * NT) {
         unsigned long long r[4];
 #pragma unroll

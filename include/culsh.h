@@ -117,6 +117,10 @@ typedef struct culsh_index_profile {
                            /* again; 0: passes over all words (one-word keys)      */
 } culsh_index_profile;
 int culsh_index_profile_get(culsh_index* ix, culsh_index_profile* out);
+/* How the last build made the bucket lookup tables: 0 key by key in place, 1 by
+ * parts in shared memory (2 million buckets and more), 2 by parts, then in place
+ * because too many keys fitted no part; *spilled (may be null): those keys. */
+int culsh_index_hash_form(const culsh_index* ix, unsigned* spilled);
 
 /* ---- SearchTables -------------------------------------------------------- */
 int culsh_search_create(culsh_search** out);        /* SearchTables::SearchTables  cuLSH_SearchTables.cu:112-122 */

@@ -130,3 +130,52 @@ def test_hash_tables_find_every_bucket(culsh, form, N, M, dup, monkeypatch):
         assert (qb[:, 0] >= 0).all()
         np.testing.assert_array_equal(qb, ref["qbuckets"][l].reshape(q.shape[0], 4), err_msg=f"table {l}")
     np.testing.assert_array_equal(ht.getBuckets_sizes(0), oracle.build_index(X, A, b, W).sizes(0))
+
+
+@pytest.mark.parametrize("N,env,form,spills", [
+    (4_090, {}, 1, False),            # one part
+    (8_300, {}, 1, None),             # four parts, a last tile of 108 keys
+    (60_000, {}, 1, None),            # sixteen
+    (240_001, {}, 1, True),           # 64, nearly half full: keys that probe past a part's end
+    (60_000, {"CULSH_HASH_PART_CAP": "3600"}, 1, True),    # records past a part's space
+    (60_000, {"CULSH_HASH_PART_CAP": "0", "CULSH_HASH_SPILL": "200000"}, 1, True),   # every key placed afterwards
+    (60_000, {"CULSH_HASH_PART_CAP": "3600", "CULSH_HASH_SPILL": "64"}, 2, True),   # too many: again in place
+    (60_000, {"CULSH_HASH_PART_CAP": "0", "CULSH_HASH_SPILL": "0"}, 2, True),
+])
+def test_hash_tables_by_parts(culsh, monkeypatch, N, env, form, spills):
+    """The form by parts with one part and many, records or probes past a part's
+    end, and the rebuild in place when those outgrow their list: every point
+    finds its own bucket, the first probes' buckets are the oracle's, and keys
+    that no point has are not found."""
+    import ctypes
+    monkeypatch.setenv("CULSH_HASH_PARTS_MIN", "1")
+    monkeypatch.setenv("CULSH_HASH_SPILL", str(N))   # the list of a small build must fit its codes' space
+    for k, v in env.items():
+        monkeypatch.setenv(k, v)
+    rng = np.random.default_rng(N)
+    D, L, M, W = 16, 3, 12, 2.0
+    X = rng.normal(0, 4, (N, D)).astype(np.float32)
+    A = rng.normal(0, 1, (L, M, D)).astype(np.float32)
+    b = rng.uniform(0, W, (L, M)).astype(np.float32)
+    ht = culsh.HashTables()
+    ht.reset(N, D, L, M, W, A=A, b=b)
+    for _ in range(2):   # a second build of the same object starts afresh
+        ht.index(X)
+    spilled = ctypes.c_uint()
+    assert culsh.lib().culsh_index_hash_form(ht._h, ctypes.byref(spilled)) == form
+    if spills is not None:
+        assert (spilled.value > 0) == spills
+    if env.get("CULSH_HASH_PART_CAP") == "0":
+        assert spilled.value == sum(ht.getBuckets(l) for l in range(L))
+    own = min(N, 60_000)
+    q = np.concatenate([X[-own:], rng.normal(0, 4, (500, D)).astype(np.float32)])
+    ref = oracle.build_index(X, A, b, W)
+    want = oracle.search(ref, X, q, 1, 4)
+    st = culsh.SearchTables()
+    st.reset(ht, 1, 4)
+    st.search(q, dataset=X)
+    for l in range(L):
+        qb = st.getQueryBuckets(l)
+        assert (qb[:own, 0] >= 0).all()
+        np.testing.assert_array_equal(qb, want["qbuckets"][l].reshape(q.shape[0], 4), err_msg=f"table {l}")
+        np.testing.assert_array_equal(ht.getBuckets_sizes(l), ref.sizes(l))

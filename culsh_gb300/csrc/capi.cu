@@ -1261,11 +1261,17 @@ bool knn_dataset_fits(const KnnState& k) {
 
 constexpr int kKnnEstimateSmem = 227 * 1024;   // shared memory a block may opt into, for estimates without a device
 
-// Most membership-row bytes at a time; further dense queries take turns.
+// Most membership-row bytes at a time; further dense queries take turns
+// (CULSH_KNN_CHUNK_BYTES lowers it, to 256 queries at least: the tests take
+// turns with it).
 constexpr size_t kKnnChunkBytes = size_t(2) << 30;
+size_t knn_chunk_bytes() {
+    const char* e = getenv("CULSH_KNN_CHUNK_BYTES");
+    return e ? (size_t)std::min<unsigned long long>(strtoull(e, nullptr, 10), kKnnChunkBytes) : kKnnChunkBytes;
+}
 
 // Shapes of the tensor-core path for nd dense queries at a time (as many as
-// kKnnChunkBytes of membership rows allow); false when it does not serve the
+// knn_chunk_bytes() of membership rows allow); false when it does not serve the
 // index and K.
 bool knn_shapes(const culsh_index* ix, int K, int nd, int sms, int smem_optin, KnnSearch* out) {
     KnnSearch& k = *out;
@@ -1274,7 +1280,7 @@ bool knn_shapes(const culsh_index* ix, int K, int nd, int sms, int smem_optin, K
     k.D = ix->D;
     k.K = K;
     const size_t row = 4 * (size_t)(((size_t)ix->N + 31) / 32 + 3);
-    const size_t most = std::max<size_t>(kKnnChunkBytes / row / kKnnTileQ, 1) * kKnnTileQ;
+    const size_t most = std::max<size_t>(knn_chunk_bytes() / row / kKnnTileQ, 1) * kKnnTileQ;
     k.nd = (int)std::min<size_t>((size_t)nd, most);
     k.Qcap = (k.nd + kKnnTileQ - 1) / kKnnTileQ * kKnnTileQ;
     k.grid = sms;

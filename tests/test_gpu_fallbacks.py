@@ -121,3 +121,39 @@ def test_probe_form_survives_tuning(culsh, how):
     st.search(X, dataset=X)
     assert (culsh.lib().culsh_search_device_bytes(st._h) + 12 * L * Q * T
             == culsh.lib().culsh_search_device_bytes(want._h))
+
+
+@pytest.mark.parametrize("margin", [None, "0"])
+@pytest.mark.parametrize("Q", [256, 257, 700])
+def test_dense_queries_in_turns(culsh, monkeypatch, Q, margin):
+    """More dense queries than one turn's membership rows hold (here 256), the
+    last turn full or not, with queries that are scanned exactly in every turn:
+    values outside the path's range, and (margin 0) survivors past the lists."""
+    N, D, L, M, W, K, T = 6_000, 20, 3, 2, 6.0, 10, 4
+    X, Qm, A, b = _case(Q, N, D, L, M, W, Q)
+    Qm[::90] *= np.float32(1e-13) / np.abs(Qm[::90]).max()
+    want = oracle.search(oracle.build_index(X, A, b, W), X, Qm, K, T)
+    monkeypatch.setenv("CULSH_KNN_CHUNK_BYTES", "0")
+    if margin:
+        monkeypatch.setenv("CULSH_KNN_LIST_MARGIN", margin)
+    st = _search(culsh, X, A, b, W, K, T, dense_min=1)
+    for _ in range(2):
+        st.search(Qm, dataset=X)
+        _check(st, want)
+        p = st.profile()
+        assert p["knn_queries"] == int((want["nonunique"] > 0).sum()) > Q - 20
+        assert p["knn_fallback"] >= (Q + 89) // 90
+
+
+def test_dense_values_outside_every_dense_form(culsh):
+    """Values whose squares leave the tensor-core path's range, more points than
+    the bitmap kernel's block holds: listed as dense, served per query."""
+    N, D, L, M, W, Q, K, T = 1_900_000, 4, 2, 2, 4e18, 4, 10, 4
+    X, Qm, A, b = _case(3, N, D, L, M, W, Q, scale=1e18)
+    want = oracle.search(oracle.build_index(X, A, b, W), X, Qm, K, T)
+    assert want["nonunique"].min() > N // 16
+    st = _search(culsh, X, A, b, W, K, T)
+    for _ in range(2):
+        st.search(Qm, dataset=X)
+        _check(st, want)
+        assert st.profile()["knn_queries"] == 0

@@ -373,6 +373,30 @@ int upload_projection(culsh_index* ix, cudaStream_t st) {
     return CULSH_OK;
 }
 
+// Whether buffers that a faster form of a stage wants, and another form does
+// without, may take `bytes` more of device memory: they must leave 64 MB free
+// (the question takes 25 us; buffers of less than that are not worth it).
+// CULSH_SCRATCH_MAX_BYTES lowers the most they may take (the tests
+// reach the other forms with it).
+bool room_for(size_t bytes) {
+    constexpr size_t margin = size_t(64) << 20;
+    if (bytes == 0) return true;
+    if (const char* e = getenv("CULSH_SCRATCH_MAX_BYTES"))
+        if (bytes > strtoull(e, nullptr, 10)) return false;
+    if (bytes <= margin) return true;
+    size_t freeb = 0, totalb = 0;
+    if (cudaMemGetInfo(&freeb, &totalb) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    return bytes + margin <= freeb;
+}
+// Bytes that reserving cnt elements adds to a buffer.
+template <class T>
+size_t growth(const DevBuf<T>& b, size_t cnt) {
+    return cnt > b.n ? (cnt - b.n) * sizeof(T) : 0;
+}
+
 // Copies a small host array to the device through the pinned staging (pageable
 // where that is full).
 int stage_copy(culsh_index* ix, void* dst, const void* src, size_t bytes, cudaStream_t st) {
@@ -748,8 +772,18 @@ int sort_keys(culsh_index* ix, int N, int passes, bool all_words, cudaStream_t s
     const int lw = low_row_words(KW);
     CU_TRY(ix->ws_vals.reserve(LN));
     CU_TRY(ix->ids.reserve(LN));
-    CU_TRY(ix->ws_keys[0].reserve(top_first ? LN : LN * KW));
-    CU_TRY(ix->ws_keys[1].reserve(top_first ? LN : LN * KW));
+    const size_t words = top_first ? LN : LN * KW;
+    // either form beside the buffers that the other one left
+    if (all_words && !room_for(growth(ix->ws_keys[0], words) + growth(ix->ws_keys[1], words))) {
+        ix->ws_low.release();
+        ix->ws_run_pos.release();
+        ix->ws_run_len.release();
+    } else if (top_first && ix->ws_keys[0].n > words && !room_for(growth(ix->ws_low, LN * lw) + 4 * LN)) {
+        ix->ws_keys[0].release();
+        ix->ws_keys[1].release();
+    }
+    CU_TRY(ix->ws_keys[0].reserve(words));
+    CU_TRY(ix->ws_keys[1].reserve(words));
     if (top_first) CU_TRY(ix->ws_low.reserve(LN * lw));
     // the first pass makes the ids; without one they are the points' order
     const bool any_pass = N > 1 && (top_first || passes > first_pass);
@@ -1041,30 +1075,6 @@ size_t arena_cap_words() {
         if (v > 0) return (size_t)v;
     }
     return ~size_t(0);
-}
-
-// Whether buffers that a faster form of a stage wants, and another form does
-// without, may take `bytes` more of device memory: they must leave 64 MB free
-// (the question takes 25 us; buffers of less than that are not worth it).
-// CULSH_SCRATCH_MAX_BYTES lowers the most they may take (the tests
-// reach the other forms with it).
-bool room_for(size_t bytes) {
-    constexpr size_t margin = size_t(64) << 20;
-    if (bytes == 0) return true;
-    if (const char* e = getenv("CULSH_SCRATCH_MAX_BYTES"))
-        if (bytes > strtoull(e, nullptr, 10)) return false;
-    if (bytes <= margin) return true;
-    size_t freeb = 0, totalb = 0;
-    if (cudaMemGetInfo(&freeb, &totalb) != cudaSuccess) {
-        cudaGetLastError();
-        return false;
-    }
-    return bytes + margin <= freeb;
-}
-// Bytes that reserving cnt elements adds to a buffer.
-template <class T>
-size_t growth(const DevBuf<T>& b, size_t cnt) {
-    return cnt > b.n ? (cnt - b.n) * sizeof(T) : 0;
 }
 
 }  // namespace

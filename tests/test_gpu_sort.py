@@ -179,3 +179,27 @@ def test_hash_tables_by_parts(culsh, monkeypatch, N, env, form, spills):
         assert (qb[:own, 0] >= 0).all()
         np.testing.assert_array_equal(qb, want["qbuckets"][l].reshape(q.shape[0], 4), err_msg=f"table {l}")
         np.testing.assert_array_equal(ht.getBuckets_sizes(l), ref.sizes(l))
+
+
+def test_fallback_without_room_gives_scratch_back(culsh, monkeypatch):
+    """The passes over every word after a run too long: where their buffers
+    do not fit beside the first form's, those are freed first."""
+    torch = pytest.importorskip("torch")
+    X, A, b, W = clustered([1] * 100 + [30_000] * 20, 5)
+    L, M, D = A.shape
+    ref = oracle.build_index(X, A, b, W)
+    left = {}
+    for limit in (None, "1000"):
+        if limit:
+            monkeypatch.setenv("CULSH_SCRATCH_MAX_BYTES", limit)
+        ht = culsh.HashTables()
+        ht.reset(X.shape[0], D, L, M, W, A=A, b=b)
+        before = torch.cuda.mem_get_info()[0]
+        for _ in range(2):   # and the next build's first form, beside theirs
+            ht.index(X)
+        left[limit] = before - torch.cuda.mem_get_info()[0]
+        assert ht.profile()["sort_form"] == 2
+        for l in range(L):
+            np.testing.assert_array_equal(ht.getBuckets_totalIndices(l), ref.ids(l))
+        del ht
+    assert left["1000"] + (8 << 20) <= left[None]   # 4 bytes a point and table at least, and the runs' lists

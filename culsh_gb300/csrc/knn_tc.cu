@@ -1119,12 +1119,8 @@ size_t knn_smem(int Dp, int ops) {
 template <bool kSample, bool kStream>
 cudaError_t launch_knn_pass(const KnnSearch& k, cudaStream_t s) {
     static std::atomic<size_t> cap{0};
-    if (k.smem > cap.load()) {
-        const cudaError_t e = cudaFuncSetAttribute(k_knn_tc<kSample, kStream>,
-                                                   cudaFuncAttributeMaxDynamicSharedMemorySize, (int)k.smem);
-        if (e != cudaSuccess) return e;
-        cap = k.smem;
-    }
+    const cudaError_t e = opt_in_smem(k_knn_tc<kSample, kStream>, k.smem, cap);
+    if (e != cudaSuccess) return e;
     CUtensorMap mq, mx, mb;
     if (!knn_map_rows(&mq, k.qh, k.Dp, k.Qcap, MQ)) return cudaErrorNotSupported;
     KnnArgs a;

@@ -807,7 +807,8 @@ cudaError_t launch_project_tc(const TcPlan& p, int need_lo, int64_t N, int D, in
         !make_map(&mah, ah, p.Dp, p.LMp, p.blk) || !make_map(&mal, al, p.Dp, p.LMp, p.blk))
         return cudaErrorNotSupported;
     const int smem = (int)p.smem[need_lo];
-    cudaError_t e = cudaFuncSetAttribute(k_project_tc<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    static std::atomic<size_t> opted{0};
+    cudaError_t e = opt_in_smem(k_project_tc<false>, p.smem[need_lo], opted);
     if (e != cudaSuccess) return e;
     e = cudaMemsetAsync(relist_cnt, 0, sizeof(unsigned int) * (size_t)p.grid, st);
     if (e != cudaSuccess) return e;
@@ -887,7 +888,8 @@ cudaError_t launch_project_tc_stream(const TcStreamPlan& p, int need_lo, int64_t
     CUtensorMap mxh, mxl;
     if (!make_map(&mxh, xh, p.Dp, N, TC_M) || !make_map(&mxl, need_lo ? xl : xh, p.Dp, N, TC_M)) return cudaErrorNotSupported;
     const int smem = (int)p.smem[need_lo];
-    cudaError_t e = cudaFuncSetAttribute(k_project_tc<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    static std::atomic<size_t> opted{0};
+    cudaError_t e = opt_in_smem(k_project_tc<true>, p.smem[need_lo], opted);
     if (e != cudaSuccess) return e;
     e = cudaMemsetAsync(relist_cnt, 0, sizeof(unsigned int) * (size_t)p.grid, st);
     if (e != cudaSuccess) return e;
@@ -947,7 +949,8 @@ cudaError_t launch_tc_recompute(const float* X, int64_t N, int D, int LM, const 
     const size_t as = sizeof(float) * (size_t)LM * ((D & 3) == 0 ? D + 4 : D + 1);
     const int stage_a = xs + as <= 215 * 1024;
     const size_t smem = xs + (stage_a ? as : 0);
-    cudaError_t e = cudaFuncSetAttribute(k_tc_recompute, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    static std::atomic<size_t> opted{0};
+    cudaError_t e = opt_in_smem(k_tc_recompute, smem, opted);
     if (e != cudaSuccess) return e;
     k_tc_recompute<<<regions, RT, smem, st>>>(X, N, D, A, b, W, list, cap, cnt, regions, LM, stage_a, stage_x, codes, cmin,
                                              cmax, err);

@@ -1487,10 +1487,10 @@ cudaError_t launch_hash_build(const HashBuild& h, cudaStream_t st) {
 cudaError_t launch_hash_build_parts(const HashBuild& h, cudaStream_t st) {
     const uint32_t parts = std::max(h.max_groups / kHashPartGroups, 1u);
     const int split = (int)hash_split_smem(parts), fill = (int)kHashPartGroups * 26;
-    cudaError_t e = cudaFuncSetAttribute(k_hash_split, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)hash_split_smem(kHashMaxParts));
+    static std::atomic<size_t> opted_split{0}, opted_fill{0};
+    cudaError_t e = opt_in_smem(k_hash_split, (size_t)split, opted_split);
     if (e != cudaSuccess) return e;
-    if ((e = cudaFuncSetAttribute(k_hash_fill, cudaFuncAttributeMaxDynamicSharedMemorySize, fill)) != cudaSuccess) return e;
+    if ((e = opt_in_smem(k_hash_fill, (size_t)fill, opted_fill)) != cudaSuccess) return e;
     if ((e = cudaMemsetAsync(h.part_cnt, 0, sizeof(uint32_t) * ((size_t)h.L * parts + 1), st)) != cudaSuccess) return e;
     k_hash_split<<<dim3((unsigned)((h.maxB + HS_TILE - 1) / HS_TILE), h.L), HS_T, split, st>>>(h, parts);
     k_hash_fill<<<dim3(parts, h.L), NT, fill, st>>>(h, parts);

@@ -47,3 +47,43 @@ def test_membership_rows_around_48_kb(N, bank):
     r = subprocess.run([sys.executable, "-c", MEMBERSHIP.format(N=N, L=L, M=M, W=W, bank=bank)], cwd=ROOT,
                        capture_output=True, text=True, timeout=300)
     assert r.returncode == 0, r.stdout + r.stderr
+
+THREADS = """
+import threading
+import numpy as np, culsh_gb300 as culsh
+SHAPES = [(2_000, 16, 1, 4, 4.0), (2_000, 256, 4, 16, 16.0), (2_000, 64, 4, 8, 8.0), (2_000, 300, 8, 16, 16.0)]
+errors = []
+def work(i):
+    try:
+        N, D, L, M, W = SHAPES[i % len(SHAPES)]
+        rng = np.random.default_rng(i)
+        X = np.round(rng.normal(0, 20, (N, D))).astype(np.float32)
+        A = rng.normal(0, 0.2, (L, M, D)).astype(np.float32)
+        b = (rng.random((L, M)) * W).astype(np.float32)
+        ht = culsh.HashTables()
+        ht.reset(N, D, L, M, W, A=A, b=b)
+        st = culsh.SearchTables()
+        first = None
+        for _ in range(60):
+            ht.index(X)
+            st.reset(ht, 5, 2)
+            st.set_tuning(dense_min=1)
+            st.search(X[:64], dataset=X)
+            got = (ht.getBuckets_totalIndices(0), st.getKnnIds())
+            first = first or got
+            assert all(np.array_equal(a, b) for a, b in zip(first, got))
+        assert ht.profile()["tensor_cores"] == 1
+    except Exception as e:
+        errors.append(f"{i}: {e}")
+ts = [threading.Thread(target=work, args=(i,)) for i in range(8)]
+for t in ts: t.start()
+for t in ts: t.join()
+assert not errors, errors
+"""
+
+
+def test_threads_with_indexes_of_different_shapes():
+    """Eight threads build and search indexes whose kernels want different
+    amounts of shared memory: none takes back what another opted into."""
+    r = subprocess.run([sys.executable, "-c", THREADS], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr

@@ -679,8 +679,9 @@ int project_tensor_cores(culsh_index* ix, const float* dX, cudaStream_t st, bool
         // itself, so the SIMT kernel runs. Taken before anything of X's size is
         // converted.
         float *as = ix->h_norms, *xs = ix->h_norms + LM;
-        std::nth_element(xs, xs + ns / 2, xs + ns);
-        std::nth_element(as, as + LM / 2, as + LM);
+        auto below = [](float x, float y) { return x < y || (y != y && x == x); };   // NaN last: an order
+        std::nth_element(xs, xs + ns / 2, xs + ns, below);
+        std::nth_element(as, as + LM / 2, as + LM, below);
         const double open = 2.0 * (double)kappa * xs[ns / 2] * as[LM / 2] / (double)ix->W;
         ix->tc_predicted_open = open;
         if (!(open <= 0.06) && !getenv("CULSH_PROJECT_TC")) return CULSH_OK;

@@ -118,3 +118,25 @@ def test_few_queries(culsh, Q, D, L, M):
     torch.cuda.synchronize()
     np.testing.assert_array_equal(ids.cpu().numpy(), ref["knn_ids"].astype(np.int32).reshape(-1))
     np.testing.assert_array_equal(dists.cpu().numpy(), ref["knn_dists"].reshape(-1))
+
+
+@pytest.mark.parametrize("share", [0.001, 0.4, 1.0])
+@pytest.mark.parametrize("D", [64, 320])
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_values_that_are_not_numbers(culsh, D, share, bad):
+    """Rows with a value that is not finite, few of the sample or all: the build
+    reports them."""
+    rng = np.random.default_rng(D)
+    N, L, M, W = 8192, 2, 8, 64.0
+    X = np.round(rng.normal(0, 20, (N, D))).astype(np.float32)
+    X[rng.random(N) < share, rng.integers(0, D)] = bad
+    X[5, 1] = bad
+    A = rng.normal(0, 1, (L, M, D)).astype(np.float32)
+    ht = culsh.HashTables()
+    ht.reset(N, D, L, M, W, A=A, b=np.zeros((L, M), np.float32))
+    with pytest.raises(culsh.CulshError) as ei:
+        ht.index(X)
+    assert ei.value.code == culsh.ERR_NUMERIC
+    X[~np.isfinite(X)] = 1.0
+    ht.index(X)   # the object serves the next build
+    assert ht.getBuckets(0) > 0

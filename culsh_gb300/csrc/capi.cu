@@ -977,9 +977,20 @@ int ensure_host(culsh_index* ix) {
     return CULSH_OK;
 }
 
+// After a build or load that failed between two of its waits (an allocation):
+// the caller's rows and the staging may still be being read.
+int drained(int rc, cudaStream_t st) {
+    if (rc != CULSH_OK) cudaStreamSynchronize(st);
+    return rc;
+}
+
 // Device index from host arrays (after load()).
+int load_device(culsh_index* ix, cudaStream_t st);
 int ensure_device(culsh_index* ix, cudaStream_t st) {
-    if (ix->dev_valid) return upload_projection(ix, st);
+    return ix->dev_valid ? upload_projection(ix, st) : drained(load_device(ix, st), st);
+}
+
+int load_device(culsh_index* ix, cudaStream_t st) {
     if (!ix->host_valid) return fail(CULSH_ERR_STATE, "No index: have you performed indexing or loaded a file???");
     const int L = ix->L, N = ix->N, M = ix->M, LM = L * M;
     ix->big_valid = false;
@@ -2107,9 +2118,7 @@ int culsh_index_build(culsh_index* ix, const float* X, FILE* dbg) {
     cudaStream_t st = ix->stream;
     clear_index_state(ix);
     TRY(upload_dataset(ix, X, st));
-    const int rc = build_device(ix, ix->X.p, st, dbg);
-    if (rc != CULSH_OK) cudaStreamSynchronize(st);   // the caller's rows may still be being read
-    return rc;
+    return drained(build_device(ix, ix->X.p, st, dbg), st);
 }
 
 int culsh_index_build_device(culsh_index* ix, const float* d_X, void* stream) {
@@ -2119,7 +2128,7 @@ int culsh_index_build_device(culsh_index* ix, const float* d_X, void* stream) {
     cudaStream_t st = stream ? (cudaStream_t)stream : ix->stream;
     clear_index_state(ix);
     ix->x_borrow = d_X;
-    const int rc = build_device(ix, d_X, st, nullptr);
+    const int rc = drained(build_device(ix, d_X, st, nullptr), st);
     if (rc == CULSH_OK && stream) CU_TRY(cudaStreamSynchronize(st));
     return rc;
 }

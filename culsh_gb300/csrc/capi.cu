@@ -182,7 +182,7 @@ struct culsh_index {
     DevBuf<uint64_t> boff, hoff;
     DevBuf<uint32_t> hmask;
     DevBuf<unsigned long long> hslots;
-    std::vector<uint64_t> h_fl_off;   // key filters (see filter_mix)
+    std::vector<uint64_t> h_fl_off;   // key filters (see filter_word)
     std::vector<uint32_t> h_fl_mask;
     DevBuf<uint64_t> fl_off;
     DevBuf<uint32_t> fl_mask, filt;
@@ -191,7 +191,7 @@ struct culsh_index {
 
     // build workspace (kept across builds)
     DevBuf<int32_t> ws_codes, ws_pmin, ws_pmax;
-    DevBuf<uint16_t> ws_ah, ws_al, ws_xh, ws_xl;   // bf16 splits for the tensor-core projection
+    DevBuf<uint16_t> ws_ah, ws_al, ws_xh, ws_xl;   // fp16 parts for the tensor-core projection
     DevBuf<float> ws_anorm, ws_xnorm;
     DevBuf<ProjectState> ws_pstate;
     double tc_predicted_open = 0.0;   // predicted share of codes the tensor-core bound leaves open
@@ -630,7 +630,7 @@ int project_tensor_cores(culsh_index* ix, const float* dX, cudaStream_t st, bool
     CU_TRY(cudaDeviceGetAttribute(&maxsm, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
     CU_TRY(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev));
     if (major < 10) return CULSH_OK;
-    // Resident form when the bf16 projection matrix fits shared memory,
+    // Resident form when the projection matrix's fp16 parts fit shared memory,
     // streaming form (K slices of X and A, column blocks) otherwise.
     const TcPlan rp = tc_plan(N, D, LM, sms, maxsm);
     const TcStreamPlan sp = rp.ok ? TcStreamPlan{} : tc_plan_stream(N, D, LM, sms, maxsm);
@@ -759,7 +759,7 @@ int project_tensor_cores(culsh_index* ix, const float* dX, cudaStream_t st, bool
 // two to four words (sort_top_word) take the digit passes over the top word
 // alone (moving 8 bytes per point a pass instead of 4 (KW + 1)) and then order
 // each run of equal top words by (lower words, id); a run longer than
-// run_max_len() or more runs than the lists hold is counted in h_run_cnt[3]
+// 2,048 (kRunMax, sort.cu) or more runs than the lists hold is counted in h_run_cnt[3]
 // (valid once the stream has been waited for): the caller then sorts again with
 // all_words, by passes over every word. On return *sk describes the sorted keys
 // and ix->ids holds the sorted ids.

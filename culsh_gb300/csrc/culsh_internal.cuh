@@ -248,7 +248,7 @@ struct RunLists {
     unsigned long long* spos;   // runs of 9..32
     uint32_t* slen;
     unsigned int scap;
-    unsigned long long* lpos;   // runs of 33..run_max_len()
+    unsigned long long* lpos;   // runs of 33..2,048 (kRunMax)
     uint32_t* llen;
     unsigned int lcap;
     uint32_t* same;             // bit per sorted position: same key as the one before (launch_rl_count's flags)
@@ -258,7 +258,6 @@ cudaError_t launch_run_find(const uint32_t* top, int64_t N, int L, int KW, const
                             const RunLists& rl, cudaStream_t st);
 cudaError_t launch_run_sorts(const RunLists& rl, int64_t N, int L, int KW, const uint32_t* low, uint32_t* ids,
                              cudaStream_t st);
-int run_max_len();
 
 // Sorted keys of all tables: KW arrays of L*N words, or (low != nullptr) the
 // sorted top words and the lower words by point, in rows of lw words.

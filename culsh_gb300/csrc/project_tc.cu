@@ -80,7 +80,6 @@ struct TcArgs {
     int col0, LMtot;
     uint32_t stage_bytes;         // streaming: bytes of one ring stage
     uint32_t a_chunk;             // streaming: bytes of one A slice (LMp x 64 fp16)
-    int list_continue;            // streaming: recompute lists continue from relist_cnt
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -218,7 +217,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         }
         mbar_init(bfull, 1);
         *abort_flag = 0;
-        *list_top = a.list_continue ? a.relist_cnt[blockIdx.x] : 0u;
+        *list_top = a.relist_cnt[blockIdx.x];   // a column block's list goes on from the one before
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     for (int c = tid; c < a.LMp; c += TC_THREADS) {
@@ -554,8 +553,8 @@ __global__ void k_project_sample(const float* __restrict__ X, int64_t N, int D, 
     }
 }
 
-// Scales from the largest magnitudes; forced_x: X's own maximum after a
-// conversion whose sample-based scale overflowed.
+// Scales from the largest magnitudes (run again after a conversion that the
+// sample's scale took out of the fp16 range: amax_x is then X's own maximum).
 __global__ void k_project_scales(ProjectState* st) {
     st->sx = project_scale(st->amax_x);
     st->sa = project_scale(st->amax_a);
@@ -844,7 +843,6 @@ cudaError_t launch_project_tc(const TcPlan& p, int need_lo, int64_t N, int D, in
         a.LMtot = LM;
         a.stage_bytes = 0;
         a.a_chunk = 0;
-        a.list_continue = 1;
         k_project_tc<false><<<p.grid, TC_THREADS, smem, st>>>(mxh, mxl, mah, mal, a);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
@@ -932,7 +930,6 @@ cudaError_t launch_project_tc_stream(const TcStreamPlan& p, int need_lo, int64_t
         a.LMtot = LM;
         a.a_chunk = (uint32_t)lmp * 128u;
         a.stage_bytes = 16384u * (need_lo ? 2u : 1u) + 2u * a.a_chunk;
-        a.list_continue = 1;
         k_project_tc<true><<<p.grid, TC_THREADS, smem, st>>>(mxh, mxl, mah, mal, a);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;

@@ -1432,8 +1432,6 @@ cudaError_t launch_run_find(const uint32_t* top, int64_t N, int L, int KW, const
     return cudaGetLastError();
 }
 
-int run_max_len() { return kRunMax; }
-
 template <int KWL>
 void launch_run_sorts_w(const RunLists& rl, int64_t LN, int64_t N, const uint32_t* low, uint32_t* ids, cudaStream_t st) {
     // the lists' lengths stay on the device: grids for a full device, or fewer

@@ -195,13 +195,10 @@ def tensor_peak():
 # How to read a stage's roofline where the algorithmic figure is not the
 # traffic that bounds it.
 STAGE_NOTES = {
-    "membership": "algorithmic bytes are the 4 * C_nu bucket-id reads (each query reads its candidates' ids) "
-                  "plus the N/8-byte membership row written per query; about 90 % of the id reads hit L2 "
-                  "(the 64 MB of id arrays stay resident), so this is the rate seen at L2, not DRAM (measured "
-                  "DRAM traffic in `traffic`); buckets of at least N/32 ids are ORed in as whole N-bit bucket "
-                  "rows (L2-resident) and others of 512 ids or more as 16-bit entries, so part of those id bytes is "
-                  "never read and the rate can exceed the HBM peak; the rest is bound by the shared-memory atomicOr "
-                  "of each id or entry",
+    "membership": "algorithmic bytes are the N/8-byte membership row written per query, the query's bucket "
+                  "numbers and every table's id list read once (each list serves all queries from L2); the stage "
+                  "is bound not by them but by the shared-memory atomicOr of each id or 16-bit entry "
+                  "(`updates_per_s`: non-unique candidates, those of bucket rows included, per second)",
     "knn": "flops of the dense GEMM the kernel runs (2 * D * N per dense query); the candidates' own distance "
            "work is the unique-candidate share of it",
 }
@@ -235,10 +232,10 @@ def stage_bytes(cfg, Q, K, T, KW, hits, nonunique, unique):
     project = 4 * (Q * D + L * M * D + L * M + L * M * Q)
     probe = 4 * L * M * Q + Q * L * T * (8 + 4) + hits * (4 * KW + 4) + 8 * Q
     cand = 8 * Q + 4 * Q * L * T + 8 * hits + 4 * nonunique + 4 * D * unique + 4 * D * Q + 8 * K * Q
-    # tensor-core path: the membership rows read every candidate id (4 C_nu)
-    # and write one N-bit row per query; the masked GEMM's work is 2 D N
-    # multiply-adds per query
-    membership = 4 * Q * L * T + 4 * nonunique + Q * ((cfg["N"] + 31) // 32) * 4
+    # tensor-core path: the membership stage writes one N-bit row per query
+    # and reads the id lists it needs (all tables' at most) once; the masked
+    # GEMM's work is 2 D N multiply-adds per query
+    membership = 4 * Q * L * T + 4 * min(nonunique, L * cfg["N"]) + Q * ((cfg["N"] + 31) // 32) * 4
     knn_flops = 2.0 * D * cfg["N"] * Q
     return {"project": project, "probe": probe, "candidates": cand, "membership": membership, "knn_flops": knn_flops}
 
@@ -758,6 +755,7 @@ def run_culsh(args):
                                 "candidates_bytes": sb["candidates"]},
                 "peak_source": f"{peak_kind} hbm_gbs" if rf["bound"] == "hbm" else f"{tpeak_kind} bf16_tflops (burst)",
                 "note": STAGE_NOTES.get(dom),
+                "updates_per_s": round(nonuniq / (med["membership"] / 1e3)) if dom == "membership" else None,
                 "stage_ms_median": {k: round(v, 4) for k, v in med.items()},
                 "all_stages": {k: {"achieved": round(v["achieved"], 2), "unit": v["unit"],
                                    "frac": round(v["achieved"] / v["peak"], 5)} for k, v in rooflines.items()}}

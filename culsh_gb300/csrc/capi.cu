@@ -289,7 +289,7 @@ struct culsh_search {
     DevBuf<int> kpart_n, kfallback;
     int knn_queries = 0, knn_fallback = 0;   // last search: dense queries on the tensor cores, re-run
     int bucket_rows = 0;                     // last search: bucket rows its membership rows could use
-    bool knn_no_room = false;                // that path's buffers did not fit the device: later searches plan without it
+    size_t knn_short = 0;                    // bytes of that path that did not fit the device: planned without it until they do
     int sms = 0, smem_optin = 0, ws_used = 0, ws_overflow = 0;
     long long occ_key = -1;
     int occ_val = 1;
@@ -1340,14 +1340,17 @@ int reserve_knn(culsh_search* s, const KnnSearch& k, cudaStream_t st, bool* ok) 
                   growth(s->kpart_n, knn_part_lists(k)) + growth(s->kfallback, qc);
     if (!ix->kx_valid) need += growth(ix->kx_h, (size_t)ix->N * k.Dp) + growth(ix->kx_w, (size_t)ix->N + 255);
     if (!ix->big_valid) need += big_rows_bytes(ix, k.nseg);
+    s->knn_short = need;
     if (!room_for(need)) {
-        s->knn_no_room = true;
         *ok = false;
         return CULSH_OK;
     }
     TRY(ensure_knn_rows(ix, st));
     *ok = knn_dataset_fits(ix->h_kstate);
-    if (!*ok) return CULSH_OK;
+    if (!*ok) {
+        s->knn_short = 0;
+        return CULSH_OK;
+    }
     TRY(ensure_big_rows(ix, k.nwp, k.nseg, st));
     CU_TRY(s->kbm.reserve(qc * k.nwp));
     CU_TRY(s->kbm_sample.reserve(qc * nws));
@@ -1359,6 +1362,7 @@ int reserve_knn(culsh_search* s, const KnnSearch& k, cudaStream_t st, bool* ok) 
     CU_TRY(s->kpart.reserve(knn_part_entries(k)));
     CU_TRY(s->kpart_n.reserve(knn_part_lists(k)));
     CU_TRY(s->kfallback.reserve(qc));
+    s->knn_short = 0;
     return CULSH_OK;
 }
 
@@ -1379,7 +1383,7 @@ int run_dense(culsh_search* s, const SearchPlan& P, int nd, cudaStream_t st, boo
         if (rc == CULSH_ERR_OUT_OF_MEMORY) {   // the room was taken meanwhile, or is in pieces
             cudaGetLastError();
             knn = false;
-            s->knn_no_room = true;
+            s->knn_short *= 2;   // not before there is plainly more room
             release_knn(s);
             if (!ix->kx_valid) {
                 ix->kx_h.release();
@@ -1676,7 +1680,8 @@ int plan_search(culsh_search* s, const float* dQ, int Q, int32_t* d_ids, float* 
             return d;
         };
         KnnSearch shapes;
-        const bool knn = tu.dense_tc && !getenv("CULSH_NO_KNN_TC") && !s->knn_no_room && reach >= dense_min_for(true) &&
+        if (s->knn_short > 0 && room_for(s->knn_short)) s->knn_short = 0;
+        const bool knn = tu.dense_tc && !getenv("CULSH_NO_KNN_TC") && s->knn_short == 0 && reach >= dense_min_for(true) &&
                          !(ix->kx_valid && !knn_dataset_fits(ix->h_kstate)) &&
                          knn_shapes(ix, K, Q, s->sms, s->smem_optin, &shapes);
         const unsigned long long dmin = dense_min_for(knn);
@@ -2330,7 +2335,7 @@ int culsh_search_reset(culsh_search* s, culsh_index* ix, int K, int T) {
     s->Q = 0;
     s->searched = false;
     s->qb_host_valid = false;
-    s->knn_no_room = false;
+    s->knn_short = 0;
     s->tot_unique = s->tot_nonunique = 0;
     s->times = culsh_times{};
     return CULSH_OK;
@@ -2530,7 +2535,7 @@ int culsh_search_release(culsh_search* s) {
     s->qorder.release();
     s->qorder_bins.release();
     release_knn(s);
-    s->knn_no_room = false;
+    s->knn_short = 0;
     s->Q = 0;
     s->searched = false;
     s->qb_host_valid = false;

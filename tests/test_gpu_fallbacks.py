@@ -42,8 +42,8 @@ def _check(st, want):
 def test_dense_without_room(culsh, monkeypatch, N):
     """The tensor-core path's buffers do not fit: the bitmap kernel, or (bits of
     more points than a block holds) the per-query kernel serves the queries
-    that were listed as dense, and later searches plan without the path. A
-    search object that is reset tries again."""
+    that were listed as dense, and later searches plan without the path until
+    there is room."""
     D, L, M, W, Q, K, T = 4, 2, 2, 4.0, 6, 10, 4
     X, Qm, A, b = _case(N, N, D, L, M, W, Q)
     want = oracle.search(oracle.build_index(X, A, b, W), X, Qm, K, T)
@@ -54,10 +54,6 @@ def test_dense_without_room(culsh, monkeypatch, N):
         _check(st, want)
         assert st.profile()["knn_queries"] == 0
     monkeypatch.delenv("CULSH_SCRATCH_MAX_BYTES")
-    st.search(Qm, dataset=X)
-    _check(st, want)
-    assert st.profile()["knn_queries"] == 0
-    st.reset(st._ht, K, T)
     st.search(Qm, dataset=X)
     _check(st, want)
     assert st.profile()["knn_queries"] > 0

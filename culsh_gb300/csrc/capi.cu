@@ -1695,10 +1695,12 @@ int plan_search(culsh_search* s, const float* dQ, int Q, int32_t* d_ids, float* 
         }
         // Rows staged in shared memory where no sparse query has more candidates
         // than twice the set: short items, whose time is the latency of their
-        // rows (4,000 candidates and fewer at 1M x 100: 136 us against 248; 156 at
-        // 100K x 128: 40 against 46). With more, items a device keeps resident
-        // count for more (12.7k at 1M x 128, all of them gathered: 38 ms against
-        // 21; up to 15,600 at 4M x 128: 660 us against 620).
+        // rows (1,640 candidates each of 9,973 queries at 1M x 100: 1.7 ms against
+        // 2.3; up to 4,000 beside dense queries 3.8 against 4.0; but 158 each of
+        // 1,000 at 100K x 128 49 us against 41). With more, items a device keeps
+        // resident count for more (12,900 each of 10,000 at 1M x 128, all of
+        // them gathered: 27 ms against 15; 10,100 each of 2,000 at 4M x 128: 4.9
+        // against 3.3).
         const unsigned long long most = std::min(reach, P.use_dense ? dmin : ~0ull);
         if (!bf16 && tu.ws_slots == 4096 && most <= 2ull * 4096 &&
             ws_smem_bytes(D, K, tu.ws_wt, WsForm::staged, tu.ws_slots) + 8192 <= (size_t)s->smem_optin)
